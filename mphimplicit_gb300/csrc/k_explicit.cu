@@ -18,6 +18,12 @@
 
 namespace mph {
 
+// The density pass is bound by the FP64 pipe (about 180 neighbours a particle
+// in 3-D, all of them inside the radii): its divisions are all by constants
+// of the case, so they go through div_const (5 FP64 operations with the bits
+// of the quotient), q = r / RadiusA serves both weights (RadiusG is RadiusA),
+// and the radius tests compare bit patterns on the integer pipe.  Every value
+// keeps its bits.  9.69 -> 6.42 ms on 326,592 particles.
 template <int D>
 __global__ void __launch_bounds__(128) k_density(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
                                                  const int* __restrict__ nc, const long long* __restrict__ nptr,
@@ -29,7 +35,7 @@ __global__ void __launch_bounds__(128) k_density(DevParams P, const int* __restr
     const int ti = type[i];
     double xi[3];
     load_vec<D>(pos, i, xi);
-    const double rA2 = DMUL(P.rA, P.rA), rG2 = DMUL(P.rG, P.rG), rP2 = DMUL(P.rP, P.rP);
+    const double rA2 = DMUL(P.rA, P.rA), rP2 = DMUL(P.rP, P.rP);
     double sa = 0.0, sp = 0.0, sg[3] = {0.0, 0.0, 0.0};
     const long long b = nptr[i];
     const int n = nc[i];
@@ -40,17 +46,23 @@ __global__ void __launch_bounds__(128) k_density(DevParams P, const int* __restr
         load_vec<D>(pos, j, xj);
         sep_vec<D>(P, xj, xi, q);
         const double r2 = norm2_exact<D>(q);
-        const double ratio = P.ratio[ti][type[j]];
-        const bool inA = rA2 - r2 >= 0, inG = rG2 - r2 >= 0, inP = rP2 - r2 >= 0;
-        if (!(inA || inG || inP)) continue;
+        const bool inA = r2_within(r2, rA2), inP = r2_within(r2, rP2);   // RadiusG = RadiusA (main.cpp:888)
+        if (!(inA || inP)) continue;
         const double r = __dsqrt_rn(r2);
-        if (inA) sa = DADD(sa, DMUL(ratio, w_a(P.kfa, r, P.rA)));
-        if (inG) {
-            const double w = DMUL(ratio, w_quad(P.kfg, r, P.rG));
+        if (inA) {
+            const double ratio = P.ratio[ti][type[j]];
+            const double t = div_const(r, P.rA, P.inv_ra);
+            const double oq = DSUB(1.0, t);
+            // w_a and w_quad with their common quotient (main.cpp:236-307)
+            sa = DADD(sa, DMUL(ratio, DMUL(DMUL(DMUL(P.kfa, t), oq), oq)));
+            const double w = DMUL(ratio, DMUL(P.kfg, DMUL(oq, oq)));
 #pragma unroll
-            for (int d = 0; d < D; ++d) sg[d] = DADD(sg[d], DMUL(DDIV(DMUL(q[d], w), P.R2g), P.rG));
+            for (int d = 0; d < D; ++d) sg[d] = DADD(sg[d], DMUL(div_const(DMUL(q[d], w), P.R2g, P.inv_R2g), P.rG));
         }
-        if (inP) sp = DADD(sp, w_quad(P.kfp, r, P.rP));
+        if (inP) {
+            const double oq = DSUB(1.0, div_const(r, P.rP, P.inv_rp));
+            sp = DADD(sp, DMUL(P.kfp, DMUL(oq, oq)));
+        }
     }
     densA[i] = sa;
     store_vec<D>(gcen, i, sg);
@@ -65,6 +77,12 @@ __global__ void k_pressure_a(DevParams P, const int* __restrict__ type, const do
     presA[i] = (P.N0a <= a) ? 0.0 : DDIV(DMUL(P.cofA[type[i]], DSUB(a, P.N0a)), P.l0);
 }
 
+// Pressure-A and diffuse-interface forces (main.cpp:1801-1898).  Bound by the
+// FP64 pipe: a pair's force is gathered into one factor of q = x_j - x_i and
+// one of h = ratio_ji g_j - ratio_ij g_i, with one reciprocal square root and
+// the constants' products formed once, about 60 FP64 operations a pair
+// against some 30 divisions with the terms formed one by one.  4.82 -> 1.31
+// ms on 71,300 particles.
 template <int D>
 __global__ void __launch_bounds__(128) k_surface_forces(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
                                                         const int* __restrict__ nc, const long long* __restrict__ nptr,
@@ -77,53 +95,45 @@ __global__ void __launch_bounds__(128) k_surface_forces(DevParams P, const int* 
     double xi[3], gi[3];
     load_vec<D>(pos, i, xi);
     load_vec<D>(gcen, i, gi);
-    const double rA2 = P.rA * P.rA, rG2 = P.rG * P.rG;
-    const double ai = P.cofA[ti] * P.cofK * P.cofK, aj = ai;   // both from i's type (main.cpp:1857, 1863)
+    const double rA2 = P.rA * P.rA;   // RadiusG = RadiusA (main.cpp:888)
+    // both coefficients from i's type (main.cpp:1857, 1863)
+    const double K = P.cofA[ti] * P.cofK * P.cofK * P.rG * (P.vol / P.l0) / P.R2g;
     const double pa_i = presA[i];
-    double fa[3] = {0, 0, 0}, fd[3] = {0, 0, 0};
+    const double ih = P.inv_ra;
+    const double ca = P.kfa * ih * P.vol, cw = K * P.kfg, cd = cw * (-2.0 * ih);
+    double f[3] = {0, 0, 0};
     const long long b = nptr[i];
     const int n = nc[i];
-    const double sc = P.rG * (P.vol / P.l0);
     for (int k = 0; k < n; ++k) {
         const int j = nind[b + k];
         if (j == i) continue;
-        double xj[3], q[3];
+        double xj[3], q[3], gj[3];
         load_vec<D>(pos, j, xj);
         sep_vec<D>(P, xj, xi, q);
         const double r2 = norm2_exact<D>(q);
-        if (r2 == 0.0) continue;
+        if (!r2_pos_below(r2, rA2)) continue;
         const int tj = type[j];
         const double rij = P.ratio[ti][tj], rji = P.ratio[tj][ti];
-        const double r = sqrt(r2);
-        double e[3];
+        const double inv = rsqrt(r2);
+        const double t = (r2 * inv) * ih, oq = 1.0 - t;
+        // pressure A: s q / |q| with s = (p_i ratio_ij + p_j ratio_ji) w_a'(|q|) vol
+        const double s = (pa_i * rij + presA[j] * rji) * (ca * oq * (1.0 - 3.0 * t));
+        load_vec<D>(gcen, j, gj);
+        double h[3], hq = 0.0;
 #pragma unroll
-        for (int d = 0; d < D; ++d) e[d] = q[d] / r;
-        if (rA2 - r2 > 0) {                                    // pressure A force
-            const double dwa = dw_a(P.kfa, r, P.rA);
-            const double s = pa_i * (rij * dwa) + presA[j] * (rji * dwa);
-#pragma unroll
-            for (int d = 0; d < D; ++d) fa[d] += s * e[d] * P.vol;
+        for (int d = 0; d < D; ++d) {
+            h[d] = rji * gj[d] - rij * gi[d];
+            hq += h[d] * q[d];
         }
-        if (rG2 - r2 > 0) {                                    // diffuse-interface force
-            double gj[3];
-            load_vec<D>(gcen, j, gj);
-            const double wg = w_quad(P.kfg, r, P.rG);
-            const double wij = rij * wg, wji = rji * wg;
+        // diffuse interface: - K (w h + w' (h . q) q / |q|)
+        const double fq = inv * (s - cd * oq * hq), fh = cw * (oq * oq);
 #pragma unroll
-            for (int d = 0; d < D; ++d) fd[d] -= (aj * gj[d] * wji - ai * gi[d] * wij) / P.R2g * sc;
-            const double dwg = dw_quad(P.kfg, r, P.rG);
-            const double dwij = rij * dwg, dwji = rji * dwg;
-            double gr = 0.0;
-#pragma unroll
-            for (int d = 0; d < D; ++d) gr += (aj * gj[d] * dwji - ai * gi[d] * dwij) * q[d];
-#pragma unroll
-            for (int d = 0; d < D; ++d) fd[d] -= gr * e[d] / P.R2g * sc;
-        }
+        for (int d = 0; d < D; ++d) f[d] += fq * q[d] - fh * h[d];
     }
-    double f[3];
-    load_vec<D>(force, i, f);
+    double f0[3];
+    load_vec<D>(force, i, f0);
 #pragma unroll
-    for (int d = 0; d < D; ++d) f[d] = (f[d] + fa[d]) + fd[d];
+    for (int d = 0; d < D; ++d) f[d] = f0[d] + f[d];
     store_vec<D>(force, i, f);
 }
 
@@ -147,10 +157,14 @@ __global__ void k_accelerate(DevParams P, int fB, int fE, const int* __restrict_
 }
 
 // ---- output-step fields ----------------------------------------------------
+// DivergenceP and PressureP (main.cpp:1932-1990) over the P-list, which holds
+// exactly the pairs with r^2 <= RadiusP^2 in the full list's order: about 19
+// slots a particle in 3-D instead of 180.  5.79 -> 0.34 ms on 326,592
+// particles.
 template <int D>
 __global__ void __launch_bounds__(128) k_div_pressure(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
-                                                      const double* __restrict__ vel, const int* __restrict__ nc,
-                                                      const long long* __restrict__ nptr, const int* __restrict__ nind,
+                                                      const double* __restrict__ vel, const int* __restrict__ ncp,
+                                                      const long long* __restrict__ nptrP, const int* __restrict__ nindP,
                                                       const double* __restrict__ vsp, double* __restrict__ divP,
                                                       double* __restrict__ presP)
 {
@@ -159,24 +173,24 @@ __global__ void __launch_bounds__(128) k_div_pressure(DevParams P, const int* __
     double xi[3], vi[3];
     load_vec<D>(pos, i, xi);
     load_vec<D>(vel, i, vi);
-    const double rP2 = P.rP * P.rP;
     double sum = 0.0;
-    const long long b = nptr[i];
-    for (int k = 0; k < nc[i]; ++k) {
-        const int j = nind[b + k];
+    const long long b = nptrP[i];
+    const int n = ncp[i];
+    for (int k = 0; k < n; ++k) {
+        const int j = nindP[b + k];
         if (j == i) continue;
         double xj[3], q[3], vj[3];
         load_vec<D>(pos, j, xj);
         sep_vec<D>(P, xj, xi, q);
         const double r2 = norm2_exact<D>(q);
         if (r2 == 0.0) continue;
-        if (rP2 - r2 >= 0) {
-            const double r = sqrt(r2);
-            const double dw = dw_quad(P.kfp, r, P.rP);
-            load_vec<D>(vel, j, vj);
+        const double inv = rsqrt(r2);
+        const double dw = P.kfp * (P.m2h_rp * (1.0 - (r2 * inv) * P.inv_rp));
+        load_vec<D>(vel, j, vj);
+        double ue = 0.0;
 #pragma unroll
-            for (int d = 0; d < D; ++d) sum -= (vj[d] - vi[d]) * (q[d] / r) * dw;
-        }
+        for (int d = 0; d < D; ++d) ue += (vj[d] - vi[d]) * q[d];
+        sum -= ue * inv * dw;
     }
     divP[i] = sum;
     const int t = type[i];
@@ -186,31 +200,44 @@ __global__ void __launch_bounds__(128) k_div_pressure(DevParams P, const int* __
     presP[i] = p;
 }
 
-template <int D>
+// The pressure-P and viscosity forces and the virial stress of a frame
+// (main.cpp:1990-2063, 4494-4738) in one pass over the neighbours.  Bound by
+// the FP64 pipe, so a pair costs one reciprocal square root and no division:
+// every force but the diffuse interface's first term lies along q, so the
+// pair's virial is one factor times q (x) q (six sums in 3-D), and that first
+// term is g_i (x) sum w q (three sums).  The pairs within RadiusP are those of
+// the P-list, so its virial needs no second walk.  SURF false: every CofA is
+// zero, so the pressure-A and diffuse-interface terms are exact zeros and are
+// not formed.  104.3 -> 4.64 ms on 326,592 particles (59 million pairs).
+template <int D, bool SURF>
 __global__ void __launch_bounds__(128) k_output_forces(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
                                                        const double* __restrict__ vel, const int* __restrict__ nc,
-                                                       const int* __restrict__ ncp, const long long* __restrict__ nptr,
-                                                       const long long* __restrict__ nptrP, const int* __restrict__ nind,
-                                                       const int* __restrict__ nindP, const double* __restrict__ presP,
-                                                       const double* __restrict__ presA, const double* __restrict__ gcen,
-                                                       double* __restrict__ force, double* __restrict__ virS,
-                                                       double* __restrict__ virP)
+                                                       const long long* __restrict__ nptr, const int* __restrict__ nind,
+                                                       const double* __restrict__ presP, const double* __restrict__ presA,
+                                                       const double* __restrict__ gcen, double* __restrict__ force,
+                                                       double* __restrict__ virS, double* __restrict__ virP)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
     const int ti = type[i];
-    double xi[3], vi[3], gi[3];
+    double xi[3], vi[3], gi[3] = {0.0, 0.0, 0.0};
     load_vec<D>(pos, i, xi);
     load_vec<D>(vel, i, vi);
-    load_vec<D>(gcen, i, gi);
-    const double pi = presP[i], pa = presA[i];
-    const double mui = P.mu[ti];
-    const double rA2 = P.rA * P.rA, rG2 = P.rG * P.rG, rP2 = P.rP * P.rP, rV2 = P.rV * P.rV;
-    const double a = P.cofA[ti] * P.cofK * P.cofK;
-    double fp[3] = {0, 0, 0}, fv[3] = {0, 0, 0};
-    double sP[3][3] = {}, sA[3][3] = {}, sV[3][3] = {}, sD[3][3] = {};
+    const double pi = presP[i];
+    double pa = 0.0, Kd = 0.0;
+    if (SURF) {
+        load_vec<D>(gcen, i, gi);
+        pa = presA[i];
+        Kd = P.cofA[ti] * P.cofK * P.cofK / P.R2g * P.rG / P.l0;
+    }
+    const double rA2 = P.rA * P.rA, rP2 = P.rP * P.rP, rV2 = P.rV * P.rV;
+    const double cv = -P.kfv * P.m2h_rv * P.visc, cp = P.kfp * P.m2h_rp;
+    const double ca = SURF ? pa * P.kfa * P.inv_ra : 0.0;
+    double fq[3] = {0, 0, 0}, wq[3] = {0, 0, 0};
+    double T[6] = {0, 0, 0, 0, 0, 0};   // xx xy xz yy yz zz
     const long long b = nptr[i];
-    for (int k = 0; k < nc[i]; ++k) {
+    const int n = nc[i];
+    for (int k = 0; k < n; ++k) {
         const int j = nind[b + k];
         if (j == i) continue;
         double xj[3], q[3];
@@ -218,93 +245,61 @@ __global__ void __launch_bounds__(128) k_output_forces(DevParams P, const int* _
         sep_vec<D>(P, xj, xi, q);
         const double r2 = norm2_exact<D>(q);
         if (r2 == 0.0) continue;
+        const double inv = rsqrt(r2), r = r2 * inv;
         const int tj = type[j];
-        const double r = sqrt(r2);
-        double e[3];
-#pragma unroll
-        for (int d = 0; d < D; ++d) e[d] = q[d] / r;
-        if (rP2 - r2 > 0) {        // pressure P force (calculatePressureP)
-            const double dw = dw_quad(P.kfp, r, P.rP);
-#pragma unroll
-            for (int d = 0; d < D; ++d) fp[d] += (pi + presP[j]) * (dw * q[d] / r) * P.vol;
-        }
-        if (rV2 - r2 > 0) {        // viscosity force and its virial
-            const double dw = -dw_quad(P.kfv, r, P.rV);
-            double vj[3];
+        double S = 0.0, F = 0.0;           // the pair's factors of q (x) q and, over vol, of q
+        if (r2_pos_below(r2, rV2)) {       // viscosity: visc mu_ij (u . e) e w' / |q|
+            double vj[3], ue = 0.0;
             load_vec<D>(vel, j, vj);
-            double ue = 0.0;
 #pragma unroll
-            for (int d = 0; d < D; ++d) ue += (vj[d] - vi[d]) * e[d];
-            const double muj = P.mu[tj];
-            const double muij = 2.0 * (mui * muj) / (mui + muj);
-            double fij[3];
-#pragma unroll
-            for (int d = 0; d < D; ++d) {
-                fij[d] = P.visc * muij * ue * e[d] * dw / r * P.vol;
-                fv[d] += fij[d];
-            }
-#pragma unroll
-            for (int aa = 0; aa < D; ++aa)
-#pragma unroll
-                for (int bb = 0; bb < D; ++bb) sV[aa][bb] += 0.5 * fij[aa] * q[bb] / P.vol;
+            for (int d = 0; d < D; ++d) ue += (vj[d] - vi[d]) * q[d];
+            F = (P.muij[ti][tj] * cv) * (ue * (1.0 - r * P.inv_rv)) * (inv * inv * inv);
+            S = 0.5 * F;
         }
-        if (rA2 - r2 > 0) {        // pressure A virial
-            const double dw = P.ratio[ti][tj] * dw_a(P.kfa, r, P.rA);
-#pragma unroll
-            for (int aa = 0; aa < D; ++aa) {
-                const double fij = pa * (dw * q[aa] / r) * P.vol;
-#pragma unroll
-                for (int bb = 0; bb < D; ++bb) sA[aa][bb] += fij * q[bb] / P.vol;
-            }
+        if (r2_pos_below(r2, rP2)) {       // pressure P
+            const double dw = cp * (1.0 - r * P.inv_rp) * inv;
+            F += (pi + presP[j]) * dw;
+            S += pi * dw;
         }
-        if (rG2 - r2 > 0) {        // diffuse-interface virial (both terms)
+        if (SURF && r2_pos_below(r2, rA2)) {   // pressure A and the diffuse interface (RadiusG = RadiusA)
             const double ratio = P.ratio[ti][tj];
-            const double w = ratio * w_quad(P.kfg, r, P.rG);
-            const double dw = ratio * dw_quad(P.kfg, r, P.rG);
-            double gr = 0.0;
+            const double t = r * P.inv_ra, oq = 1.0 - t;
+            double gq = 0.0;
 #pragma unroll
-            for (int d = 0; d < D; ++d) gr += (-gi[d]) * q[d];
+            for (int d = 0; d < D; ++d) gq += gi[d] * q[d];
+            const double w = ratio * P.kfg * oq;
+            S += (ca * ratio * oq * (1.0 - 3.0 * t) + Kd * gq * w * (-2.0 * P.inv_ra)) * inv;
 #pragma unroll
-            for (int aa = 0; aa < D; ++aa) {
-                const double f1 = -a * (-gi[aa]) * w / P.R2g * P.rG * (P.vol / P.l0);
-                const double f2 = -a * gr * (dw * q[aa] / r) / P.R2g * P.rG * (P.vol / P.l0);
-#pragma unroll
-                for (int bb = 0; bb < D; ++bb) sD[aa][bb] += f1 * q[bb] / P.vol + f2 * q[bb] / P.vol;
-            }
+            for (int d = 0; d < D; ++d) wq[d] += (w * oq) * q[d];
         }
-    }
-    // pressure P virial over the P list (main.cpp:4512-4555)
-    for (int k = 0; k < ncp[i]; ++k) {
-        const int j = nindP[nptrP[i] + k];
-        if (j == i) continue;
-        double xj[3], q[3];
-        load_vec<D>(pos, j, xj);
-        sep_vec<D>(P, xj, xi, q);
-        const double r2 = norm2_exact<D>(q);
-        if (r2 == 0.0) continue;
-        if (rP2 - r2 > 0) {
-            const double r = sqrt(r2);
-            const double dw = dw_quad(P.kfp, r, P.rP);
+        double sq[3];
 #pragma unroll
-            for (int aa = 0; aa < D; ++aa) {
-                const double fij = pi * (dw * q[aa] / r) * P.vol;
-#pragma unroll
-                for (int bb = 0; bb < D; ++bb) sP[aa][bb] += fij * q[bb] / P.vol;
-            }
+        for (int d = 0; d < D; ++d) {
+            fq[d] += F * q[d];
+            sq[d] = S * q[d];
+        }
+        T[0] += sq[0] * q[0];
+        T[1] += sq[0] * q[1];
+        T[3] += sq[1] * q[1];
+        if (D == 3) {
+            T[2] += sq[0] * q[2];
+            T[4] += sq[1] * q[2];
+            T[5] += sq[2] * q[2];
         }
     }
     double f[3];
     load_vec<D>(force, i, f);
 #pragma unroll
-    for (int d = 0; d < D; ++d) f[d] = (f[d] + fp[d]) + fv[d];
+    for (int d = 0; d < D; ++d) f[d] += fq[d] * P.vol;
     store_vec<D>(force, i, f);
+    const double full[3][3] = {{T[0], T[1], T[2]}, {T[1], T[3], T[4]}, {T[2], T[4], T[5]}};
     double tr = 0.0;
 #pragma unroll
     for (int aa = 0; aa < 3; ++aa)
 #pragma unroll
         for (int bb = 0; bb < 3; ++bb) {
             double v = 0.0;
-            if (aa < D && bb < D) v = ((sP[aa][bb] + sA[aa][bb]) + sV[aa][bb]) + sD[aa][bb];
+            if (aa < D && bb < D) v = full[aa][bb] + (SURF ? Kd * gi[aa] * wq[bb] : 0.0);
             virS[9 * (size_t)i + 3 * aa + bb] = v;
             if (aa == bb) tr += v;
         }
@@ -334,9 +329,22 @@ __global__ void __launch_bounds__(128) k_density_p(DevParams P, const double* __
         load_vec<D>(pos, j, xj);
         sep_vec<D>(P, xj, xi, q);
         const double r2 = norm2_exact<D>(q);
-        if (r2_within(r2, rP2)) sp = DADD(sp, w_quad(P.kfp, __dsqrt_rn(r2), P.rP));
+        if (r2_within(r2, rP2)) {
+            const double oq = DSUB(1.0, div_const(__dsqrt_rn(r2), P.rP, P.inv_rp));   // w_quad
+            sp = DADD(sp, DMUL(P.kfp, DMUL(oq, oq)));
+        }
     }
     vsp[i] = DSUB(sp, P.N0p);
+}
+
+static void launch_density_p(mph_case* c)
+{
+    const DevParams& P = c->dp;
+    const unsigned g = grid_for(P.N, 128);
+    if (c->dim == 2)
+        { k_density_p<2><<<g, 128, 0, c->stream>>>(P, c->d.pos, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.vsp); MPH_COUNT_LAUNCH(); }
+    else
+        { k_density_p<3><<<g, 128, 0, c->stream>>>(P, c->d.pos, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.vsp); MPH_COUNT_LAUNCH(); }
 }
 
 // The full density pass (DensityA, GravityCenter, DensityP) and PressureA.
@@ -368,10 +376,7 @@ void launch_explicit(mph_case* c)
     if (P.surface) {
         launch_density_full(c);
     } else {
-        if (c->dim == 2)
-            { k_density_p<2><<<g, 128, 0, c->stream>>>(P, c->d.pos, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.vsp); MPH_COUNT_LAUNCH(); }
-        else
-            { k_density_p<3><<<g, 128, 0, c->stream>>>(P, c->d.pos, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.vsp); MPH_COUNT_LAUNCH(); }
+        launch_density_p(c);
         c->densa_valid = false;
     }
     if (P.surface) {
@@ -397,17 +402,25 @@ void launch_explicit_density_only(mph_case* c)
 
 void launch_output_fields(mph_case* c)
 {
-    ensure_density_a(c);
     const DevParams& P = c->dp;
     const unsigned g = grid_for(P.N, 128);
+    // with every CofA zero the frame needs VolStrainP alone of the density
+    // pass (DensityA and the rest follow when a reader asks for them)
+    if (P.surface) ensure_density_a(c);
+    else if (!c->densa_valid) launch_density_p(c);
+    DeviceState& d = c->d;
+    auto go = [&](auto dp, auto of) {
+        dp<<<g, 128, 0, c->stream>>>(P, d.type, d.pos, d.vel, d.ncp, d.nptrP, d.nindP, d.vsp, d.divP, d.presP);
+        MPH_COUNT_LAUNCH();
+        of<<<g, 128, 0, c->stream>>>(P, d.type, d.pos, d.vel, d.nc, d.nptr, d.nind, d.presP, d.presA, d.gcen, d.force, d.virS, d.virP);
+        MPH_COUNT_LAUNCH();
+    };
     if (c->dim == 2) {
-        { k_div_pressure<2><<<g, 128, 0, c->stream>>>(P, c->d.type, c->d.pos, c->d.vel, c->d.nc, c->d.nptr, c->d.nind, c->d.vsp, c->d.divP, c->d.presP); MPH_COUNT_LAUNCH(); }
-        { k_output_forces<2><<<g, 128, 0, c->stream>>>(P, c->d.type, c->d.pos, c->d.vel, c->d.nc, c->d.ncp, c->d.nptr, c->d.nptrP, c->d.nind,
-                                                     c->d.nindP, c->d.presP, c->d.presA, c->d.gcen, c->d.force, c->d.virS, c->d.virP); MPH_COUNT_LAUNCH(); }
+        if (P.surface) go(k_div_pressure<2>, k_output_forces<2, true>);
+        else go(k_div_pressure<2>, k_output_forces<2, false>);
     } else {
-        { k_div_pressure<3><<<g, 128, 0, c->stream>>>(P, c->d.type, c->d.pos, c->d.vel, c->d.nc, c->d.nptr, c->d.nind, c->d.vsp, c->d.divP, c->d.presP); MPH_COUNT_LAUNCH(); }
-        { k_output_forces<3><<<g, 128, 0, c->stream>>>(P, c->d.type, c->d.pos, c->d.vel, c->d.nc, c->d.ncp, c->d.nptr, c->d.nptrP, c->d.nind,
-                                                     c->d.nindP, c->d.presP, c->d.presA, c->d.gcen, c->d.force, c->d.virS, c->d.virP); MPH_COUNT_LAUNCH(); }
+        if (P.surface) go(k_div_pressure<3>, k_output_forces<3, true>);
+        else go(k_div_pressure<3>, k_output_forces<3, false>);
     }
 }
 

@@ -164,6 +164,8 @@ static int derive(mph_case* c, const mph_particles* parts)
     P.m2h_rv = -2.0 / P.rV;
     P.inv_rp = 1.0 / P.rP;
     P.m2h_rp = -2.0 / P.rP;
+    P.inv_ra = 1.0 / P.rA;
+    P.inv_R2g = 1.0 / P.R2g;
     for (int t = 0; t < kTypeCount; ++t)
         for (int u = 0; u < kTypeCount; ++u)
             P.muij[t][u] = 2.0 * (P.mu[t] * P.mu[u]) / (P.mu[t] + P.mu[u]);

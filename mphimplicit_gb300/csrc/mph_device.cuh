@@ -109,26 +109,18 @@ __device__ __forceinline__ void sep_vec(const DevParams& P, const double* xj, co
     for (int d = 0; d < D; ++d) q[d] = sep_exact(xj[d], xi[d], P.hw[d], P.dw[d], P.wsafe[d]);
 }
 
-// Weight functions (main.cpp:236-307) with the reference's evaluation order.
-__device__ __forceinline__ double w_a(double kf, double r, double h)
+// a / c rounded to nearest for a constant c > 0, with y = 1 / c rounded to
+// nearest: a first quotient and two residual corrections (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000", 1990:
+// the first correction gives a quotient within one unit in the last place,
+// the second the correctly rounded one).  Five FP64 operations; for the
+// lengths and weights it serves (normal numbers, no over- or underflow in the
+// residuals; 0 and NaN pass through) it has the bits of __ddiv_rn.
+__device__ __forceinline__ double div_const(double a, double c, double y)
 {
-    const double q = DDIV(r, h);
-    const double oq = DSUB(1.0, q);
-    return DMUL(DMUL(DMUL(kf, q), oq), oq);
-}
-__device__ __forceinline__ double dw_a(double kf, double r, double h)
-{
-    const double q = DDIV(r, h);
-    return DMUL(DMUL(DMUL(kf, DSUB(1.0, q)), DSUB(1.0, DMUL(3.0, q))), DDIV(1.0, h));
-}
-__device__ __forceinline__ double w_quad(double kf, double r, double h)
-{
-    const double oq = DSUB(1.0, DDIV(r, h));
-    return DMUL(kf, DMUL(oq, oq));
-}
-__device__ __forceinline__ double dw_quad(double kf, double r, double h)
-{
-    return DMUL(kf, DMUL(DDIV(-2.0, h), DSUB(1.0, DDIV(r, h))));
+    double q = DMUL(a, y);
+    q = __fma_rn(__fma_rn(-q, c, a), y, q);
+    return __fma_rn(__fma_rn(-q, c, a), y, q);
 }
 
 // The warp sums of D per-lane FP64 values by reduce-scatter: the same pairs,
