@@ -101,12 +101,13 @@ typedef struct mph_solve_stats {
     int status;
     int outer_iterations;    /* mixed form: FP64 refinement steps (0 for the FP64 form) */
     int inner_form;          /* operator of the CR iterations: 0 FP64 blocks, 1 FP32 blocks,
-                                2 FP32 pair terms (mixed form, factored, option inner_blocks 0) */
-    int inner_local_blocks;  /* inner_form 2: row blocks (512 fluid rows) whose neighbours' values are
-                                staged in shared memory, and the rest, which gather by column */
+                                2 FP32 without blocks (mixed form, factored, option inner_blocks 0) */
+    int inner_local_blocks;  /* inner_form 2: blocks of fluid rows (64, 128 or 256 by the particle count; 512 with
+                                mg_depth >= 0) whose neighbours' values are staged in shared memory, and the
+                                rest, which gather by column */
     int inner_gather_blocks;
     long long inner_local_cols;  /* distinct neighbour columns summed over the staged row blocks */
-    int inner_ct_local_blocks;   /* particle blocks (256) of the transposed P-list apply staging s */
+    int inner_ct_local_blocks;   /* particle blocks of the transposed apply staging s */
     int inner_reserved;          /* 0 */
 } mph_solve_stats;
 
@@ -238,13 +239,15 @@ int mph_case_set_solver(mph_case* c, double outer_rel_residual, double inner_rel
  *   "mixed_extra_sweeps" 0 (default) .. 8: mixed form only, extra level-0
  *   smoothing sweeps before and after the rest of its V-cycle.
  *   "inner_blocks" 0 (default) / 1: factored mixed form only.  0: the inner
- *   FP32 operator runs on the sliced FP32 pair terms and P-lists and no
- *   blocks are written (CsrCofA export then fails with MPH_ERR_STATE; the
+ *   FP32 operator is inertia and C Lambda C^T evaluated from the P-lists (the
+ *   viscous pairs are left to the FP64 outer residual) or, with mg_depth >= 0
+ *   and in domains over about 1900 RadiusP wide, runs on the sliced FP32 pair
+ *   terms and P-lists; no blocks are written (CsrCofA export then fails with MPH_ERR_STATE; the
  *   block columns CsrIndA still export).  1: FP32 blocks are assembled and
  *   the inner SpMV runs on them.
- *   "inner_local" 1 (default) / 0: pair-term inner operator only.  1: each
- *   block of rows (particles, for the transposed P-lists) whose distinct
- *   neighbours fit stages their s in shared memory; 0: every block gathers s
+ *   "inner_local" 1 (default) / 0: inner operator without blocks only.  1: each
+ *   block of rows (particles, for the transposed apply) whose distinct
+ *   neighbours fit stages their values in shared memory; 0: every block gathers s
  *   by column.  Both give the same bits. */
 int mph_case_set_option(mph_case* c, const char* name, double value);
 /* More options (no counterpart in the reference):
@@ -281,7 +284,8 @@ int mph_case_set_option(mph_case* c, const char* name, double value);
  *   main.cpp:4122), k the V-cycle cut after its first k levels.
  *   "mg_coarsest" 1 .. 8 (default 4): mixed form only, sweeps of a coarsest
  *   level run grid-wide (the reference's 4, main.cpp:4216).
- *   "pair_pack" 1 (default) / 0: pair-term inner operator only.  Slot records
+ *   "pair_pack" 1 (default) / 0: pair-term inner operator only (as the options
+ *   "pair_block", "ct_block", "pair_recompute" and "split_apply").  Slot records
  *   of 6 bytes (g as 11/11/10-bit fixed point of its slice's scale, and a
  *   2-byte block-local index) or 8 bytes (g in FP16 and the index).
  *   "pair_recompute" 0 (default) / 1: pair-term inner operator only; 1

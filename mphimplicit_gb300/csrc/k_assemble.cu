@@ -36,6 +36,11 @@ __global__ void k_max_int(const int* __restrict__ v, int n, int* __restrict__ ou
     if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
+void launch_max_int(mph_case* c, const int* v, int n, int* out)
+{
+    { k_max_int<<<grid_for(n, 256), 256, 0, c->stream>>>(v, n, out); MPH_COUNT_LAUNCH(); }
+}
+
 template <int D>
 __global__ void __launch_bounds__(128) k_matrix_c(DevParams P, const double* __restrict__ pos, const int* __restrict__ ncp,
                                                   const long long* __restrict__ nptrP, const int* __restrict__ nindP,
@@ -414,7 +419,7 @@ int launch_assemble(mph_case* c)
     // of four without per-slot bounds tests
     { k_slice_width<<<grid_for((long long)c->nslices * 32, 256), 256, 0, c->stream>>>(Nf, c->d.nfc, c->d.swidth, 4); MPH_COUNT_LAUNCH(); }
     MPH_CUDA(cudaMemsetAsync(c->d.dmax, 0, sizeof(int), c->stream));
-    { k_max_int<<<grid_for(c->nslices, 256), 256, 0, c->stream>>>(c->d.swidth, c->nslices, c->d.dmax); MPH_COUNT_LAUNCH(); }
+    launch_max_int(c, c->d.swidth, c->nslices, c->d.dmax);
     MPH_TRY(launch_scan_i32_to_i64(c, c->d.swidth, c->d.sptr, c->nslices));
     long long h_slots = 0;
     int h_width = 0;
@@ -428,6 +433,7 @@ int launch_assemble(mph_case* c)
     // form unless its inner operator runs on the pair terms
     c->step_factored = factored_applies(c);
     c->step_pairs = c->step_factored && !c->inner_blocks && c->visc_nonneg;
+    c->step_pen = pen_applies(c);
     {
         long long cap = c->d.cap_slots;
         void* p = c->d.acol;
@@ -500,7 +506,7 @@ int launch_assemble(mph_case* c)
         // mixed form: FP64 pair terms and b, transposed P-lists (the factored
         // FP64 operator), then FP32 blocks only
         MPH_TRY(build_ct(c));
-        if (c->step_pairs) MPH_TRY(launch_ct_slices(c));
+        if (c->step_pairs && !c->step_pen) MPH_TRY(launch_ct_slices(c));
         MPH_TRY(launch_pair_terms(c));
     }
     // the pair path of the point-Jacobi mixed form has all it needs (b and

@@ -228,12 +228,12 @@ k_pair_terms(DevParams P, const int* __restrict__ type, const double* __restrict
             const double pk = pvec[k];
 #pragma unroll
             for (int r = 0; r < D; ++r) sumv[r] -= cval[(pb + a) * D + r] * pk;
-            if (cvl32) {   // lambda_k C_ik for the FP32 inner operator
+            if (cvl32 || dinv) {   // lambda_k C_ik: the stored FP32 inner operator, the diagonal
                 const double lam = P.lambda[type[k]];
 #pragma unroll
                 for (int r = 0; r < D; ++r) {
                     const float cl = (float)(cval[(pb + a) * D + r] * lam);
-                    cvl32[(pb + a) * D + r] = cl;
+                    if (cvl32) cvl32[(pb + a) * D + r] = cl;
                     dpd[r] += cl * (float)cval[(pb + a) * D + r];
                 }
             }
@@ -1337,68 +1337,12 @@ static void apply32(mph_case* c, const float* x, float* y, int cap)
 
 void launch_apply32(mph_case* c, const float* x, float* y, int cap)
 {
+    if (c->step_pen) {   // the point-Jacobi form's own operator (k_penalty.cu; x and y are its s and y)
+        launch_pen_operator(c, cap);
+        return;
+    }
     if (c->dim == 2) apply32<2>(c, x, y, cap);
     else apply32<3>(c, x, y, cap);
-}
-
-// ---- the operator over the cases of a batch ------------------------------------------
-template <int D>
-__global__ void __launch_bounds__(MPH_CT_BLOCK) k_batch_ct32(const BatchCase* __restrict__ cs, const int* __restrict__ b0, int nc)
-{
-    const int c = batch_case_of(b0, nc, (int)blockIdx.x);
-    const BatchCase& B = cs[c];
-    const int lb = (int)blockIdx.x - b0[c];
-    if (B.ct_loc)
-        ct_apply32_body<D, true>(lb, B.N, B.ctsptr, B.ct_cnt, B.ctsval, B.s32, B.tct32, B.scal, B.flags, B.cap, B.ctuniq, B.ctucount);
-    else
-        ct_apply32_body<D, false>(lb, B.N, B.ctsptr, B.ct_cnt, B.ctsval, B.s32, B.tct32, B.scal, B.flags, B.cap, nullptr, nullptr);
-}
-
-template <int D, bool PACK>
-__global__ void __launch_bounds__(MPH_PAIR_BLOCK, 2) k_batch_visc32(const BatchCase* __restrict__ cs, const int* __restrict__ b0, int nc)
-{
-    const int c = batch_case_of(b0, nc, (int)blockIdx.x);
-    const BatchCase& B = cs[c];
-    const int lb = (int)blockIdx.x - b0[c];
-    if (B.vp_loc)
-        visc_pen32_body<D, true, PACK, true>(lb, B.vp_nb, B.Nf, B.nfc, B.sptr, B.acol, B.grec16, B.grec32, B.lcol16, B.pscale, B.sdiag32,
-                                             B.ncp, B.psptr, B.psval, B.tct32, B.s32, B.y32, B.scal, B.flags, B.partials, B.counter,
-                                             B.uniq, B.ucount);
-    else
-        visc_pen32_body<D, false, PACK, true>(lb, B.vp_nb, B.Nf, B.nfc, B.sptr, B.acol, B.grec16, B.grec32, B.lcol16, B.pscale,
-                                              B.sdiag32, B.ncp, B.psptr, B.psval, B.tct32, B.s32, B.y32, B.scal, B.flags, B.partials,
-                                              B.counter, nullptr, nullptr);
-}
-
-// the transposed apply and the viscous kernel of one batched CR iteration
-// (ct_b0 / vp_b0: their block starts; shared memory: the batch's largest)
-void launch_batch_operator(const BatchCase* cs, const int* ct_b0, const int* vp_b0, int nc, int dim, bool pack, int pair_block,
-                           int ct_block, int vp_smem, int ct_smem, int ct_blocks, int vp_blocks, cudaStream_t st)
-{
-    static std::once_flag once;
-    std::call_once(once, [] {   // fixed maxima (host threads of other batches would race on per-launch values)
-        cudaFuncSetAttribute(k_batch_ct32<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUMax * 2 * (int)sizeof(float));
-        cudaFuncSetAttribute(k_batch_ct32<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUMax * 4 * (int)sizeof(float));
-        cudaFuncSetAttribute(k_batch_visc32<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUMax * 2 * (int)sizeof(float));
-        cudaFuncSetAttribute(k_batch_visc32<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUMax * 2 * (int)sizeof(float));
-        cudaFuncSetAttribute(k_batch_visc32<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUMax * 4 * (int)sizeof(float));
-        cudaFuncSetAttribute(k_batch_visc32<3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUMax * 4 * (int)sizeof(float));
-    });
-    if (ct_blocks > 0) {
-        if (dim == 2) k_batch_ct32<2><<<ct_blocks, ct_block, ct_smem, st>>>(cs, ct_b0, nc);
-        else k_batch_ct32<3><<<ct_blocks, ct_block, ct_smem, st>>>(cs, ct_b0, nc);
-        MPH_COUNT_LAUNCH();
-    }
-    if (vp_blocks > 0) {
-        if (dim == 2) {
-            if (pack) k_batch_visc32<2, true><<<vp_blocks, pair_block, vp_smem, st>>>(cs, vp_b0, nc);
-            else k_batch_visc32<2, false><<<vp_blocks, pair_block, vp_smem, st>>>(cs, vp_b0, nc);
-        } else {
-            if (pack) k_batch_visc32<3, true><<<vp_blocks, pair_block, vp_smem, st>>>(cs, vp_b0, nc);
-            else k_batch_visc32<3, false><<<vp_blocks, pair_block, vp_smem, st>>>(cs, vp_b0, nc);
-        }
-        MPH_COUNT_LAUNCH();
-    }
 }
 
 // ---- level-0 multigrid stencils and D^-1 on the pair-term path --------------------
@@ -1971,9 +1915,11 @@ int launch_pair_terms(mph_case* c)
     if (!d.x32) MPH_CUDA(cudaMalloc((void**)&d.x32, (size_t)P.Nf * c->dim * 2 * sizeof(float)));
     if (!d.tct32) MPH_CUDA(cudaMalloc((void**)&d.tct32, (size_t)(P.N + 1) * sizeof(float)));
     long long ncv = 0;   // C values of the fluid rows, FP32 copy for the inner operator
-    MPH_CUDA(cudaMemcpyAsync(&ncv, d.nptrP + P.Nf, sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
-    MPH_CUDA(cudaStreamSynchronize(c->stream));
-    ncv *= c->dim;
+    if (!c->step_pen || fused) {
+        MPH_CUDA(cudaMemcpyAsync(&ncv, d.nptrP + P.Nf, sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
+        MPH_CUDA(cudaStreamSynchronize(c->stream));
+        ncv *= c->dim;
+    }
     if (ncv > d.cap_cval32) {
         if (d.cval32) cudaFree(d.cval32);
         d.cval32 = nullptr;
@@ -1981,7 +1927,7 @@ int launch_pair_terms(mph_case* c)
         MPH_CUDA(cudaMalloc((void**)&d.cval32, (size_t)(ncv + ncv / 8 + 1024) * sizeof(float)));
         d.cap_cval32 = ncv + ncv / 8 + 1024;
     }
-    { k_cval_f32<<<grid_for(ncv, 256), 256, 0, c->stream>>>(ncv, d.cval, d.cval32); MPH_COUNT_LAUNCH(); }
+    if (!c->step_pen) { k_cval_f32<<<grid_for(ncv, 256), 256, 0, c->stream>>>(ncv, d.cval, d.cval32); MPH_COUNT_LAUNCH(); }
     float* sdiag = nullptr;
     double* sdiag64 = nullptr;
     float* cvl = nullptr;
@@ -1990,13 +1936,15 @@ int launch_pair_terms(mph_case* c)
         if (!d.sdiag32) MPH_CUDA(cudaMalloc((void**)&d.sdiag32, (size_t)P.Nf * 8 * sizeof(float)));
         if (!d.sdiag64) MPH_CUDA(cudaMalloc((void**)&d.sdiag64, (size_t)P.Nf * 8 * sizeof(double)));
         sdiag64 = d.sdiag64;
-        MPH_TRY(grow_f(&d.cvl32, &d.cap_cvl32, ncv));
         sdiag = d.sdiag32;
-        cvl = d.cvl32;
+        if (!c->step_pen || fused) {
+            MPH_TRY(grow_f(&d.cvl32, &d.cap_cvl32, ncv));
+            cvl = d.cvl32;
+        }
         if (!d.pscale) MPH_CUDA(cudaMalloc((void**)&d.pscale, (size_t)((P.Nf + 31) / 32 + 1) * sizeof(float)));
         if (!fused) {
             MPH_CUDA(cudaMemsetAsync(d.pscale, 0, (size_t)((P.Nf + 31) / 32 + 1) * sizeof(float), c->stream));
-            if (!c->pair_recompute)
+            if (!c->pair_recompute && !c->step_pen)
                 gmax = reinterpret_cast<unsigned*>(d.pscale);   // slice maxima, turned into scales by the slicing
         }
     }
@@ -2131,6 +2079,17 @@ int launch_pairs_to_slices(mph_case* c)
     const DevParams& P = c->dp;
     const int D = c->dim;
     if (c->nslices == 0) return MPH_OK;
+    if (c->step_pen) {   // the outer residual's layout only: FP32 g and columns
+        MPH_TRY(grow_f(&d.pes32, &d.cap_pes32, c->nslots * D));
+        if (!pair_fused(c)) {
+            if (D == 2) k_list_to_slices<2, true><<<c->nslices, 256, 0, c->stream>>>(P.Nf, d.sptr, d.nfc, d.nptr, d.nind, d.pe32, nullptr,
+                                                                                    d.acol, d.pes32, nullptr, d.pscale, nullptr);
+            else k_list_to_slices<3, true><<<c->nslices, 256, 0, c->stream>>>(P.Nf, d.sptr, d.nfc, d.nptr, d.nind, d.pe32, nullptr,
+                                                                             d.acol, d.pes32, nullptr, d.pscale, nullptr);
+            MPH_COUNT_LAUNCH();
+        }
+        return launch_pen_lists(c);
+    }
     MPH_TRY(ensure_pair_records(c));
     const bool lrec = c->pair_recompute || c->pair_pack;   // records without the index half
     if (!d.psptr) {

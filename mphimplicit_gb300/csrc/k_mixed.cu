@@ -439,6 +439,14 @@ static void pq_precond(mph_case* c, cudaStream_t st, int n, unsigned rb, const f
     vcycle_mixed(c, q32, u32, scal + kSQU32);
 }
 
+// The squared reduction of the recursive residual a phase asks for: not below
+// what the inner operator leaves of the true one (k_penalty.cu).
+static double inner_target2(const mph_case* c)
+{
+    const double t = c->step_pen ? std::max(c->tol_inner, std::min(c->pen_tol, 0.1)) : c->tol_inner;
+    return t * t;
+}
+
 static void fill_mixed_stats(mph_case* c, int total_inner, int outer, const double* hs, bool bad, double tol_out2)
 {
     c->stats.iterations = total_inner;
@@ -501,7 +509,7 @@ static int device_solve(mph_case* c, double* hs, int* hflags)
     V *r32 = vec, *z32 = vec + (size_t)n, *s32 = vec + 2 * (size_t)n, *y32 = vec + 3 * (size_t)n;
     V *p32 = vec + 4 * (size_t)n, *q32 = vec + 5 * (size_t)n, *u32 = vec + 6 * (size_t)n;
     const double tol_out2 = c->tol_outer * c->tol_outer;
-    const double tol_in2 = c->tol_inner * c->tol_inner;
+    const double tol_in2 = inner_target2(c);
     const int cap = n;
     const int loop_cap = std::min(cap, kDeviceLoopMax);
     const size_t nvs = (size_t)c->dp.N * (D == 2 ? 2 : 4);
@@ -585,9 +593,13 @@ static int device_solve(mph_case* c, double* hs, int* hflags)
                     k_spmv32<D, 1, V><<<gs, 128, 0, s3>>>(Nf, d.nfc, d.sptr, d.acol, d.aval32, s32, y32, scal, flags, cap, part, counter);
                     MPH_COUNT_LAUNCH();
                 }
-                pq_precond(c, s3, n, rb, s32, y32, p32, q32, u32);
-                { k_xrs32<V, true><<<rb, kReduceThreads, 0, s3>>>(n, z32, r32, s32, p32, q32, u32, scal, flags, part, counter, loop_cap,
-                                                             1, h_in); MPH_COUNT_LAUNCH(); }
+                if (c->step_pen) {
+                    launch_pen_vectors(c, loop_cap, true, h_in);
+                } else {
+                    pq_precond(c, s3, n, rb, s32, y32, p32, q32, u32);
+                    { k_xrs32<V, true><<<rb, kReduceThreads, 0, s3>>>(n, z32, r32, s32, p32, q32, u32, scal, flags, part, counter, loop_cap,
+                                                                 1, h_in); MPH_COUNT_LAUNCH(); }
+                }
                 l_iter = t_launch_count - li0;
                 cudaGraph_t gi = nullptr;
                 if (cudaStreamEndCapture(s3, &gi) != cudaSuccess) fail_capture(fail(MPH_ERR_CUDA, "end of the CR iteration capture"));
@@ -683,7 +695,7 @@ struct MixedRun {
         q32 = vec + 5 * (size_t)n;
         u32 = vec + 6 * (size_t)n;
         tol_out2 = c->tol_outer * c->tol_outer;
-        tol_in2 = c->tol_inner * c->tol_inner;
+        tol_in2 = inner_target2(c);
         cap = n;
     }
 
@@ -819,6 +831,12 @@ static int mixed_solve_t(mph_case* c)
         }
         if (ev_end) cudaEventRecordWithFlags(ev_end, st, cudaEventRecordExternal);   // profiled graph: the operator's end
         else if (e) prof_begin(c, 0, &e[1]);
+        if (c->step_pen) {       // profiled graph: the vectors, the preconditioner among them
+            if (ev_v0) cudaEventRecordWithFlags(ev_v0, st, cudaEventRecordExternal);
+            launch_pen_vectors(c, cap, false, 0);
+            if (ev_v1) cudaEventRecordWithFlags(ev_v1, st, cudaEventRecordExternal);
+            return;
+        }
         if (mixed_jacobi(c)) {   // profiled graph: the update fused with the preconditioner
             if (ev_v0) cudaEventRecordWithFlags(ev_v0, st, cudaEventRecordExternal);
             pq_precond(c, st, n, rb, s32, y32, p32, q32, u32);
@@ -905,52 +923,20 @@ static int mixed_solve_t(mph_case* c)
 // The cases of mph_batch_step that run the point-Jacobi mixed form on the pair
 // path solve together: each case's start, phase tests, updates and FP64
 // residuals are its own (MixedRun, on its stream), while the CR iterations of
-// a refinement phase are four launches over all the cases still iterating
-// (each block runs the single-case kernel body on its case, with the
-// single-case block decomposition), so a case's bits are those it gets alone.
-__global__ void k_batch_pq32(const BatchCase* __restrict__ cs, const int* __restrict__ b0, int nc)
-{
-    const int c = batch_case_of(b0, nc, (int)blockIdx.x);
-    const BatchCase& B = cs[c];
-    pq_jacobi32_body<float>((int)blockIdx.x - b0[c], B.el_nb, B.n, B.s32, B.y32, B.p32, B.q32, B.invD, B.u32, B.scal, B.flags,
-                            B.partials, B.counter);
-}
-
-__global__ void k_batch_xrs32(const BatchCase* __restrict__ cs, const int* __restrict__ b0, int nc)
-{
-    const int c = batch_case_of(b0, nc, (int)blockIdx.x);
-    const BatchCase& B = cs[c];
-    xrs32_body<float, false>((int)blockIdx.x - b0[c], B.el_nb, B.n, B.z32, B.r32, B.s32, B.p32, B.q32, B.u32, B.scal, B.flags,
-                             B.partials, B.counter);
-}
-
-// the cases' solver flags, gathered for one read
-__global__ void k_batch_flags(const BatchCase* __restrict__ cs, int nc, int* __restrict__ out)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < nc * kFlagCount) out[t] = cs[t / kFlagCount].flags[t % kFlagCount];
-}
-
-void launch_batch_iteration(const BatchCase* cs, const int* b0, int nc, int dim, bool pack, int pair_block, int ct_block,
-                            int vp_smem, int ct_smem, const int* nblocks, cudaStream_t st)
-{
-    launch_batch_operator(cs, b0, b0 + (nc + 1), nc, dim, pack, pair_block, ct_block, vp_smem, ct_smem, nblocks[0], nblocks[1], st);
-    if (nblocks[2] > 0) {
-        { k_batch_pq32<<<nblocks[2], kReduceThreads, 0, st>>>(cs, b0 + 2 * (nc + 1), nc); MPH_COUNT_LAUNCH(); }
-        { k_batch_xrs32<<<nblocks[2], kReduceThreads, 0, st>>>(cs, b0 + 2 * (nc + 1), nc); MPH_COUNT_LAUNCH(); }
-    }
-}
-
+// a refinement phase are three launches over all the cases still iterating
+// (k_penalty.cu: each block runs the single-case kernel body on its case, with
+// the single-case block decomposition), so a case's bits are those it gets
+// alone.
 bool batch_solve_eligible(const mph_case* c)
 {
     return c->batch_solve && c->precision == MPH_PRECISION_MIXED && c->stage == 6 && c->step_pairs && mixed_jacobi(c) &&
-           !c->pair_recompute && !c->split_apply && !c->device_loop && !c->prof.on && c->dp.Nf > 0 && c->nslices > 0;
+           c->step_pen && !c->device_loop && !c->prof.on && c->dp.Nf > 0 && c->nslices > 0;
 }
 
 // The batched solve's device table, flag buffers, stream and events, per
 // host thread (one batch at a time per thread).
 struct BatchBuffers {
-    BatchCase* tab = nullptr;
+    void* tab = nullptr;
     int* b0 = nullptr;
     int* flags = nullptr;
     int* hflags = nullptr;
@@ -977,7 +963,7 @@ struct BatchBuffers {
         tab = nullptr;
         b0 = flags = hflags = nullptr;
         cap = 0;
-        MPH_CUDA(cudaMalloc((void**)&tab, (size_t)nc * sizeof(BatchCase)));
+        MPH_CUDA(cudaMalloc(&tab, (size_t)nc * batch_pen_bytes()));
         MPH_CUDA(cudaMalloc((void**)&b0, (size_t)3 * (nc + 1) * sizeof(int)));
         MPH_CUDA(cudaMalloc((void**)&flags, (size_t)nc * kFlagCount * sizeof(int)));
         MPH_CUDA(cudaMallocHost((void**)&hflags, (size_t)nc * kFlagCount * sizeof(int)));
@@ -990,7 +976,7 @@ static thread_local BatchBuffers t_batch;
 using ParFor = std::function<void(int, const std::function<int(int)>&)>;
 
 template <int D>
-static int batched_solve_t(std::vector<mph_case*>& cs, bool pack, int pair_block, int ct_block, const ParFor& par)
+static int batched_solve_t(std::vector<mph_case*>& cs, int rows, int W, const ParFor& par)
 {
     const int nc = (int)cs.size();
     BatchBuffers& tb = t_batch;
@@ -1010,57 +996,14 @@ static int batched_solve_t(std::vector<mph_case*>& cs, bool pack, int pair_block
         return runs[k].start();
     }));
     for (int k = 0; k < nc; ++k) chunk = std::max(chunk, cs[k]->chunk);
-    std::vector<BatchCase> tab(nc);
-    int vp_smem = 0, ct_smem = 0;
+    std::vector<char> tab((size_t)nc * batch_pen_bytes());
+    std::vector<int> blocks(3 * nc);   // the cases' block counts of the iteration's launches
+    int umax = 0;
     for (int k = 0; k < nc; ++k) {
-        mph_case* c = cs[k];
-        DeviceState& d = c->d;
-        MixedRun<D>& R = runs[k];
-        BatchCase& B = tab[k];
-        B.N = c->dp.N;
-        B.Nf = c->dp.Nf;
-        B.n = R.n;
-        B.cap = R.cap;
-        B.ct_loc = c->loc_ct_smem != 0;
-        B.vp_loc = c->loc_smem != 0;
-        B.ct_nb = (int)grid_for(c->dp.N, ct_block);
-        B.vp_nb = (int)grid_for(c->dp.Nf, pair_block);
-        B.el_nb = R.rb;
-        B.ctsptr = d.ctsptr;
-        B.ct_cnt = d.ct_cnt;
-        B.ctsval = (const float4*)d.ctsval;
-        B.tct32 = d.tct32;
-        B.ctuniq = d.ctuniq;
-        B.ctucount = d.ctucount;
-        B.nfc = d.nfc;
-        B.sptr = d.sptr;
-        B.acol = d.acol;
-        B.grec16 = d.grec16;
-        B.grec32 = d.grec32;
-        B.lcol16 = d.lcol16;
-        B.pscale = d.pscale;
-        B.sdiag32 = d.sdiag32;
-        B.ncp = d.ncp;
-        B.psptr = d.psptr;
-        B.psval = (const float4*)d.psval;
-        B.uniq = d.uniq;
-        B.ucount = d.ucount;
-        B.s32 = R.s32;
-        B.y32 = R.y32;
-        B.p32 = R.p32;
-        B.q32 = R.q32;
-        B.u32 = R.u32;
-        B.z32 = R.z32;
-        B.r32 = R.r32;
-        B.invD = d.v32 + 7 * (size_t)R.n;
-        B.scal = R.scal;
-        B.flags = R.flags;
-        B.partials = R.part;
-        B.counter = R.counter;
-        vp_smem = std::max(vp_smem, c->loc_smem);
-        ct_smem = std::max(ct_smem, c->loc_ct_smem);
+        batch_pen_fill(cs[k], runs[k].cap, tab.data(), k, &blocks[3 * k]);
+        umax = std::max(umax, cs[k]->pen_umax);
     }
-    MPH_CUDA(cudaMemcpyAsync(tb.tab, tab.data(), (size_t)nc * sizeof(BatchCase), cudaMemcpyHostToDevice, tb.st));
+    MPH_CUDA(cudaMemcpyAsync(tb.tab, tab.data(), tab.size(), cudaMemcpyHostToDevice, tb.st));
     std::vector<char> active(nc, 1);
     std::vector<int> b0(3 * (nc + 1));
     for (;;) {
@@ -1080,11 +1023,8 @@ static int batched_solve_t(std::vector<mph_case*>& cs, bool pack, int pair_block
             b0[k] = nb[0];
             b0[(nc + 1) + k] = nb[1];
             b0[2 * (nc + 1) + k] = nb[2];
-            if (active[k]) {
-                nb[0] += tab[k].ct_nb;
-                nb[1] += tab[k].vp_nb;
-                nb[2] += tab[k].el_nb;
-            }
+            if (active[k])
+                for (int l = 0; l < 3; ++l) nb[l] += blocks[3 * k + l];
         }
         b0[nc] = nb[0];
         b0[2 * nc + 1] = nb[1];
@@ -1099,8 +1039,8 @@ static int batched_solve_t(std::vector<mph_case*>& cs, bool pack, int pair_block
         bool all = false;
         while (!all) {
             for (int it = 0; it < chunk; ++it)
-                launch_batch_iteration(tb.tab, tb.b0, nc, D, pack, pair_block, ct_block, vp_smem, ct_smem, nb, tb.st);
-            { k_batch_flags<<<grid_for((long long)nc * kFlagCount, 256), 256, 0, tb.st>>>(tb.tab, nc, tb.flags); MPH_COUNT_LAUNCH(); }
+                launch_batch_pen(tb.tab, tb.b0, nc, D, rows, W, umax, nb, tb.st);
+            launch_batch_flags(tb.tab, nc, tb.flags, tb.st);
             MPH_CUDA(cudaMemcpyAsync(tb.hflags, tb.flags, (size_t)nc * kFlagCount * sizeof(int), cudaMemcpyDeviceToHost, tb.st));
             MPH_CUDA(cudaStreamSynchronize(tb.st));
             all = true;
@@ -1130,8 +1070,8 @@ static int batched_solve_t(std::vector<mph_case*>& cs, bool pack, int pair_block
     });
 }
 
-// Solve the eligible cases of a batch together, in groups of one dimension,
-// record format and block widths (the cases' stage must be 6).
+// Solve the eligible cases of a batch together, in groups of one dimension
+// and block shape (the cases' stage must be 6).
 int batched_mixed_solve(std::vector<mph_case*>& cases, const ParFor& par)
 {
     std::vector<char> taken(cases.size(), 0);
@@ -1141,14 +1081,12 @@ int batched_mixed_solve(std::vector<mph_case*>& cases, const ParFor& par)
         std::vector<mph_case*> g;
         for (size_t b = a; b < cases.size(); ++b) {
             mph_case* c = cases[b];
-            if (taken[b] || c->dim != c0->dim || c->pair_pack != c0->pair_pack || c->pair_block != c0->pair_block ||
-                c->ct_block != c0->ct_block)
-                continue;
+            if (taken[b] || c->dim != c0->dim || c->pen_rows != c0->pen_rows || c->pen_w != c0->pen_w) continue;
             taken[b] = 1;
             g.push_back(c);
         }
-        if (c0->dim == 2) MPH_TRY(batched_solve_t<2>(g, c0->pair_pack, c0->pair_block, c0->ct_block, par));
-        else MPH_TRY(batched_solve_t<3>(g, c0->pair_pack, c0->pair_block, c0->ct_block, par));
+        if (c0->dim == 2) MPH_TRY(batched_solve_t<2>(g, c0->pen_rows, c0->pen_w, par));
+        else MPH_TRY(batched_solve_t<3>(g, c0->pen_rows, c0->pen_w, par));
     }
     return MPH_OK;
 }

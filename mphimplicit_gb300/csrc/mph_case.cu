@@ -176,7 +176,9 @@ static int derive(mph_case* c, const mph_particles* parts)
         P.inert32[t] = (float)(P.density[t] * P.vol / P.vol / P.dt);
         P.lambda32[t] = (float)P.lambda[t];
         for (int u = 0; u < kTypeCount; ++u) P.vm32[t][u] = (float)(P.visc * P.muij[t][u]);
+        P.pen_lam32[t] = (float)(P.lambda[t] * (-P.kfp * P.m2h_rp));
     }
+    P.pen_w32 = (float)(-P.kfp * P.m2h_rp);
     P.wdA32 = (float)(-P.kfv * P.m2h_rv);
     // the pair terms of the FP32 inner operator are stored as sqrt(f) e, which
     // needs f >= 0 for every pair of types
@@ -197,15 +199,20 @@ static int derive(mph_case* c, const mph_particles* parts)
         }
         const int range = (int)std::ceil(P.rV / l0);
         const int rz = two_d ? 0 : range;
-        double fsum = 0.0;
+        double fsum = 0.0;   // for unit viscosity
         for (int ix = -range; ix <= range; ++ix)
             for (int iy = -range; iy <= range; ++iy)
                 for (int iz = -rz; iz <= rz; ++iz) {
                     if (ix == 0 && iy == 0 && iz == 0) continue;
                     const double r = l0 * std::sqrt((double)(ix * ix + iy * iy + iz * iz));
-                    if (r < P.rV) fsum += P.visc * mu_max * P.kfv * (2.0 / P.rV) * (1.0 - r / P.rV) / r;
+                    if (r < P.rV) fsum += P.visc * P.kfv * (2.0 / P.rV) * (1.0 - r / P.rV) / r;
                 }
-        c->visc_ratio = 4.0 * fsum / (rho_min / P.dt);
+        c->visc_ratio = 4.0 * (fsum * mu_max) / (rho_min / P.dt);
+        // the inner operator of the point-Jacobi form keeps 0.6 of a row's
+        // viscous diagonal (fsum mu / dim) and leaves the rest, at most about
+        // 0.7 of it, to the outer residual
+        for (int t = 0; t < kTypeCount; ++t) P.pen_diag32[t] = (float)(P.inert64[t] + 0.6 * fsum * std::fabs(P.mu[t]) / c->dim);
+        c->pen_tol = 0.7 * fsum * mu_max / c->dim / (rho_min / P.dt);
     }
     // walls (initializeWall main.cpp:1023-1062; theta = |omega|^2 as written there)
     for (int t = 0; t < 4; ++t)
@@ -247,6 +254,22 @@ static int derive(mph_case* c, const mph_particles* parts)
         P.dw[d] = dmax[d] - P.dmin[d];
         P.hw[d] = 0.5 * P.dw[d];
         P.wsafe[d] = 0.75 * P.dw[d];
+    }
+    // fixed-point positions in units of RadiusP / 2^e, e = 22 (a separation
+    // within RadiusP is then an FP32 integer) or less where the domain is too
+    // wide for 31 bits (k_penalty.cu uses them down to e = 20)
+    {
+        double wide = 0.0;
+        for (int d = 0; d < c->dim; ++d) wide = std::max(wide, P.dw[d]);
+        int e = 22;
+        while (e > 1 && std::ldexp(wide / P.rP, e) > 2.0e9) --e;
+        P.fix_scale = std::ldexp(1.0, e) / P.rP;
+        P.fix_inv = (float)std::ldexp(1.0, -e);
+        for (int d = 0; d < c->dim; ++d) {
+            const double w = std::nearbyint(P.dw[d] * P.fix_scale);
+            P.fix_w[d] = w < 2.0e9 ? (int)w : 0;
+            P.fix_h[d] = P.fix_w[d] / 2;
+        }
     }
     double cnt[3];
     cnt[0] = std::floor((dmax[0] - P.dmin[0]) / P.maxR);
@@ -377,7 +400,7 @@ int case_alloc_particles(mph_case* c)
     MPH_TRY(dalloc(c, &d.p, n));
     MPH_TRY(dalloc(c, &d.q, n));
     MPH_TRY(dalloc(c, &d.u, n));
-    MPH_TRY(dalloc(c, &d.partials, (size_t)std::max<size_t>(kReduceBlocks, Nf / 32 + 64)));
+    MPH_TRY(dalloc(c, &d.partials, (size_t)std::max<size_t>(kReduceBlocks, Nf / 16 + 64)));   // three values a 64-row block
     MPH_TRY(dalloc(c, &d.scal, 32));
     MPH_TRY(dalloc(c, &d.flags, kFlagCount));
     MPH_TRY(dalloc(c, &d.bbox, 8));
@@ -509,11 +532,14 @@ int stage_neighbors(mph_case* c)
     int pon = prof_begin(c, 3, &pe);
     launch_neighbor_count(c);
     if (pon) prof_end(c, 3, pe);
+    MPH_CUDA(cudaMemsetAsync(c->d.dmax + 1, 0, sizeof(int), c->stream));
+    launch_max_int(c, c->d.ncp, N, c->d.dmax + 1);   // longest P-list
     MPH_TRY(launch_scan_i32_to_i64(c, c->d.nc, c->d.nptr, N));
     MPH_TRY(launch_scan_i32_to_i64(c, c->d.ncp, c->d.nptrP, N));
     long long tot[2];
     MPH_CUDA(cudaMemcpyAsync(&tot[0], c->d.nptr + N, sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
     MPH_CUDA(cudaMemcpyAsync(&tot[1], c->d.nptrP + N, sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
+    MPH_CUDA(cudaMemcpyAsync(&c->pmax, c->d.dmax + 1, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     MPH_CUDA(cudaStreamSynchronize(c->stream));
     c->nnb = tot[0];
     c->nnbP = tot[1];
@@ -693,7 +719,7 @@ int case_destroy(mph_case* c)
                     (void*)d.tct32, (void*)d.pes32, (void*)d.sdiag32, (void*)d.sdiag64, (void*)d.cvl32, (void*)d.psptr, (void*)d.ctsptr,
                     (void*)d.pswidth, (void*)d.ctswidth, (void*)d.pscol, (void*)d.ctscol, (void*)d.psval, (void*)d.ctsval,
                     (void*)d.grec16, (void*)d.grec32, (void*)d.pscale, (void*)d.lcol16, (void*)d.uniq, (void*)d.ucount,
-                    (void*)d.ctuniq, (void*)d.ctucount, (void*)d.wkey, (void*)d.wval, (void*)d.ccell,
+                    (void*)d.ctuniq, (void*)d.ctucount, (void*)d.ipos, (void*)d.pidx, (void*)d.pgroups, (void*)d.puniq, (void*)d.pucount, (void*)d.wkey, (void*)d.wval, (void*)d.ccell,
                     (void*)d.io3, (void*)d.vprev, (void*)d.vprev_alt, (void*)d.sort_cnt, (void*)d.sort_off, d.scan_tmp})
         if (p) cudaFree(p);
     for (auto& p : c->prof.pending) {

@@ -65,6 +65,11 @@ struct DevParams {
     float lambda32[kTypeCount];
     float vm32[kTypeCount][kTypeCount];        // FP32 visc * muij, -kfv * m2h_rv, 1/h, rV^2 (pair terms)
     float wdA32, inv_rv32, rV2_32;
+    double fix_scale;                          // fixed-point positions: units a length (2^e / RadiusP), 2^-e, and the
+    float fix_inv;                             // domain's width and half width in units
+    int fix_w[3], fix_h[3];
+    float pen_diag32[kTypeCount];              // inner operator of the point-Jacobi form: its diagonal, lambda kfp 2/RadiusP,
+    float pen_lam32[kTypeCount], pen_w32;      // and kfp 2/RadiusP
     int exact_only;                            // 1: skip the FP32 pre-classification
     int surface;                               // 1 if any CofA != 0
 };
@@ -162,6 +167,14 @@ struct DeviceState {
     long long cap_ctuniq = 0;
     int* ctucount = nullptr;
     long long cap_ctucount = 0;
+    // inner operator of the point-Jacobi mixed form (k_penalty.cu): fixed-point
+    // positions with the type, the P-lists' 2-byte ranks, words a row of each
+    // slice, the row blocks' distinct columns and their counts (statistics
+    // after the blocks)
+    int4* ipos = nullptr;
+    uint2* pidx = nullptr;
+    long long cap_pidx = 0;
+    int *pgroups = nullptr, *puniq = nullptr, *pucount = nullptr;
     int* ccell = nullptr;              // packed cell coordinates of every particle (pair path)
     double* io3 = nullptr;             // host-layout staging, 2 x N x 3 doubles (state upload, field download)
     double *vprev = nullptr, *vprev_alt = nullptr;   // mixed form, option "extrapolate": start velocities of the two previous
@@ -281,6 +294,11 @@ struct mph_case {
     bool step_pairs = false;            // this step's FP32 inner operator runs on the sliced pair terms
     cudaEvent_t gev[128] = {};          // event pairs of a profiled CR graph chunk (operators, then V-cycles)
     bool level0_done = false;           // this step's level-0 multigrid stencils were written by the assembly
+    bool step_pen = false;              // this step's inner CR runs on k_penalty.cu's operator
+    int pmax = 0;                       // longest P-list of the current lists
+    int pen_rows = 0, pen_w = 0;        // its rows a block and threads a row
+    int pen_pw4 = 0, pen_umax = 0;      // 8-byte words a row has room for; largest staged count (rounded up)
+    double pen_tol = 0.0;               // what a refinement phase leaves at least (the viscous part outside the operator)
     int loc_smem = 0;                   // shared memory of k_visc_pen32's staged s (0: gathers by column)
     int loc_cap = 0;                    // staged neighbours a block of the pair-term operator has room for
     int loc_ct_smem = 0;                // shared memory of k_ct_apply32's staged s (0: gathers by column)
@@ -374,6 +392,7 @@ int launch_counting_sort(mph_case* c);
 void launch_cell_ranges_and_permute(mph_case* c);
 void launch_fluid_bbox(mph_case* c);
 void launch_neighbor_count(mph_case* c);
+void launch_max_int(mph_case* c, const int* v, int n, int* out);
 int launch_scan_i32_to_i64(mph_case* c, const int* in, long long* out, int n);
 int launch_slice_ptr(mph_case* c, int rows, const int* counts, int* width, long long* ptr, long long* total);
 void launch_neighbor_fill(mph_case* c);
@@ -386,31 +405,19 @@ int launch_assemble(mph_case* c);
 int launch_assemble_cells(mph_case* c, int kmax_rows, bool mix, bool* done);
 int build_ct(mph_case* c);
 bool factored_applies(const mph_case* c);
-// One case of a CR iteration launched over several cases (the batched
-// solve): the case's arrays and its share of each launch.  A block finds its
-// case from the launches' block starts and runs the single-case kernel body
-// with its block index inside the case, so each case's arithmetic, and its
-// reductions' order, are the single-case launch's.
-struct BatchCase {
-    int N, Nf, n, cap;                 // particles, fluid rows, vector length, iteration cap
-    int ct_loc, vp_loc;                // the case's blocks stage s (shared memory of the transposed / viscous kernel)
-    int ct_nb, vp_nb, el_nb;           // the case's block counts: transposed apply, viscous kernel, vector kernels
-    const long long* ctsptr; const int* ct_cnt; const float4* ctsval; float* tct32; const int* ctuniq; const int* ctucount;
-    const int* nfc; const long long* sptr; const int* acol; const unsigned short* grec16; const unsigned* grec32;
-    const unsigned short* lcol16; const float* pscale; const float* sdiag32; const int* ncp; const long long* psptr;
-    const float4* psval; const int* uniq; const int* ucount;
-    float *s32, *y32, *p32, *q32, *u32, *z32, *r32;
-    const float* invD;
-    double* scal; int* flags; double* partials; unsigned* counter;
-};
-// one FP32 CR iteration over the cases of a batch (all in the point-Jacobi
-// mixed form on the pair path, one dimension, one record format and one
-// pair / transposed block width): four launches on `st`; b0 holds the three
-// launches' block starts per case (3 x (ncases + 1) ints, device)
-void launch_batch_iteration(const BatchCase* cases_dev, const int* b0_dev, int ncases, int dim, bool pack, int pair_block,
-                            int ct_block, int vp_smem, int ct_smem, const int* nblocks, cudaStream_t st);
-void launch_batch_operator(const BatchCase* cs, const int* ct_b0, const int* vp_b0, int nc, int dim, bool pack, int pair_block,
-                           int ct_block, int vp_smem, int ct_smem, int ct_blocks, int vp_blocks, cudaStream_t st);
+// k_penalty.cu: the inner operator of the point-Jacobi mixed form, its lists
+// and vectors, and the same over the cases of a batch (a block finds its case
+// from the launches' block starts and runs the single-case kernel body with
+// its block index inside the case, so each case's arithmetic, and its
+// reductions' order, are the single-case launch's)
+bool pen_applies(const mph_case* c);
+int launch_pen_lists(mph_case* c);
+void launch_pen_operator(mph_case* c, int cap);
+void launch_pen_vectors(mph_case* c, int cap, bool use_cond, cudaGraphConditionalHandle cond);
+size_t batch_pen_bytes();
+void batch_pen_fill(const mph_case* c, int cap, void* table, int k, int* nb);
+void launch_batch_pen(const void* table, const int* b0, int nc, int dim, int rows, int W, int umax, const int* nb, cudaStream_t st);
+void launch_batch_flags(const void* table, int nc, int* out, cudaStream_t st);
 // par(n, f): run f(0) .. f(n-1) (the batch's host worker pool); the per-case
 // host parts of the batched solve (phase tests, updates) run through it
 int batched_mixed_solve(std::vector<mph_case*>& cases, const std::function<void(int, const std::function<int(int)>&)>& par);
