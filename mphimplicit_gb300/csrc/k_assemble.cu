@@ -127,6 +127,15 @@ __global__ void __launch_bounds__(128) k_vector_p(DevParams P, const int* __rest
 }
 
 
+// the source vector p of every particle (DevParams and lists of this step)
+void launch_vector_p(mph_case* c)
+{
+    DeviceState& d = c->d;
+    const unsigned g = grid_for(c->dp.N, 128);
+    if (c->dim == 2) { k_vector_p<2><<<g, 128, 0, c->stream>>>(c->dp, d.type, d.pos, d.vel, d.vsp, d.ncp, d.nptrP, d.nindP, d.pvec); MPH_COUNT_LAUNCH(); }
+    else { k_vector_p<3><<<g, 128, 0, c->stream>>>(c->dp, d.type, d.pos, d.vel, d.vsp, d.ncp, d.nptrP, d.nindP, d.pvec); MPH_COUNT_LAUNCH(); }
+}
+
 template <int D>
 __device__ __forceinline__ void flush_part(double* __restrict__ prow, int slot, const double (&acc)[D][D], bool add)
 {
@@ -412,8 +421,32 @@ int launch_assemble(mph_case* c)
     const DevParams& P = c->dp;
     const int Nf = P.Nf;
     const int D = c->dim;
-    // slice pointers
     c->nslices = (Nf + 31) / 32;
+    // the form of this step's system decides which block arrays exist: FP64
+    // blocks unless the FP64 operator is factored, FP32 blocks for the mixed
+    // form unless its inner operator runs without blocks
+    c->step_factored = factored_applies(c);
+    c->step_pairs = c->step_factored && !c->inner_blocks && c->visc_nonneg;
+    c->step_pen = pen_applies(c);
+    const bool need64 = !c->step_factored, need32 = c->precision == MPH_PRECISION_MIXED && !c->step_pairs;
+    if (!need64 && c->d.aval) {   // a form change (option) since the last step: release what is unused
+        cudaFree(c->d.aval);
+        c->d.aval = nullptr;
+        c->d.cap_aval = 0;
+    }
+    if (!need32 && c->d.aval32) {
+        cudaFree(c->d.aval32);
+        c->d.aval32 = nullptr;
+        c->d.cap_aval32 = 0;
+    }
+    if (c->step_pen) {
+        cudaEvent_t pe = nullptr;
+        const int pon = prof_begin(c, 2, &pe);
+        MPH_TRY(launch_pen_assemble(c));
+        if (pon) prof_end(c, 2, pe);
+        return MPH_OK;
+    }
+    // slice pointers
     // the fluid rows' slices padded to a multiple of 4 slots (zero padding
     // records): the pair-term operator then loops over whole slices in steps
     // of four without per-slot bounds tests
@@ -428,19 +461,12 @@ int launch_assemble(mph_case* c)
     MPH_CUDA(cudaStreamSynchronize(c->stream));
     const int kmax_rows = h_width / 32;   // longest fluid row
     c->nslots = h_slots;
-    // the form of this step's system decides which block arrays exist: FP64
-    // blocks unless the FP64 operator is factored, FP32 blocks for the mixed
-    // form unless its inner operator runs on the pair terms
-    c->step_factored = factored_applies(c);
-    c->step_pairs = c->step_factored && !c->inner_blocks && c->visc_nonneg;
-    c->step_pen = pen_applies(c);
     {
         long long cap = c->d.cap_slots;
         void* p = c->d.acol;
         MPH_TRY(ensure(&p, &cap, h_slots, sizeof(int)));
         c->d.acol = (int*)p;
         c->d.cap_slots = cap;
-        const bool need64 = !c->step_factored, need32 = c->precision == MPH_PRECISION_MIXED && !c->step_pairs;
         if (need64 && cap > c->d.cap_aval) {
             if (c->d.aval) cudaFree(c->d.aval);
             c->d.aval = nullptr;
@@ -455,16 +481,6 @@ int launch_assemble(mph_case* c)
             MPH_CUDA(cudaMalloc(&c->d.aval32, (size_t)cap * D * D * sizeof(float)));
             c->d.cap_aval32 = cap;
         }
-        if (!need64 && c->d.aval) {   // a form change (option) since the last step: release what is unused
-            cudaFree(c->d.aval);
-            c->d.aval = nullptr;
-            c->d.cap_aval = 0;
-        }
-        if (!need32 && c->d.aval32) {
-            cudaFree(c->d.aval32);
-            c->d.aval32 = nullptr;
-            c->d.cap_aval32 = 0;
-        }
     }
     // C values for the fluid rows (aligned with the P-list)
     long long h_cn = 0;
@@ -476,7 +492,6 @@ int launch_assemble(mph_case* c)
         c->d.cval = (double*)p;
     }
     const unsigned gf = grid_for(Nf, 128);
-    const unsigned ga = grid_for(P.N, 128);
     Level0Map M{};
     const mph::LevelGeom& g0 = c->lv[0];
     M.S = 1;
@@ -490,11 +505,10 @@ int launch_assemble(mph_case* c)
     }
     if (D == 2) {
         { k_matrix_c<2><<<gf, 128, 0, c->stream>>>(P, c->d.pos, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.cval); MPH_COUNT_LAUNCH(); }
-        { k_vector_p<2><<<ga, 128, 0, c->stream>>>(P, c->d.type, c->d.pos, c->d.vel, c->d.vsp, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.pvec); MPH_COUNT_LAUNCH(); }
     } else {
         { k_matrix_c<3><<<gf, 128, 0, c->stream>>>(P, c->d.pos, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.cval); MPH_COUNT_LAUNCH(); }
-        { k_vector_p<3><<<ga, 128, 0, c->stream>>>(P, c->d.type, c->d.pos, c->d.vel, c->d.vsp, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.pvec); MPH_COUNT_LAUNCH(); }
     }
+    launch_vector_p(c);
     // A: the cell-block kernel where it applies; the per-row kernel for the
     // rows of cells it flags (or for every row when it does not apply)
     cudaEvent_t pe = nullptr;
@@ -506,7 +520,7 @@ int launch_assemble(mph_case* c)
         // mixed form: FP64 pair terms and b, transposed P-lists (the factored
         // FP64 operator), then FP32 blocks only
         MPH_TRY(build_ct(c));
-        if (c->step_pairs && !c->step_pen) MPH_TRY(launch_ct_slices(c));
+        if (c->step_pairs) MPH_TRY(launch_ct_slices(c));
         MPH_TRY(launch_pair_terms(c));
     }
     // the pair path of the point-Jacobi mixed form has all it needs (b and

@@ -483,7 +483,7 @@ int build_ct(mph_case* c)
     } else {
         { k_ct_place<3><<<grid_for(tot, 256), 256, 0, c->stream>>>(tot, dv.ct_ptr, (const int3*)dv.ct_tmp, dv.cval, dv.ct_j, dv.ct_v); MPH_COUNT_LAUNCH(); }
     }
-    if (c->step_factored && !c->step_pen) {   // FP32 copy for the FP32 cell-block kernel and the stored inner operator
+    if (c->step_factored) {   // FP32 copy for the FP32 cell-block kernel and the stored inner operator
         MPH_TRY(grow_bytes((void**)&dv.ct_v32, &dv.cap_ct_v32, tot * D * (long long)sizeof(float)));
         { k_to_f32<<<grid_for(tot * D, 256), 256, 0, c->stream>>>(tot * D, dv.ct_v, dv.ct_v32); MPH_COUNT_LAUNCH(); }
     }

@@ -30,6 +30,7 @@
 #include <mutex>
 
 #include "mph_device.cuh"
+#include "mph_pairs.cuh"
 #include "mph_solver.cuh"
 
 namespace mph {
@@ -90,59 +91,6 @@ constexpr int kXs3 = MPH_XS3;
 // inertia term, so its FP32 rounding moves A x by ~1e-10 of |b| (the host
 // keeps the factored form off when that bound would reach 1e-2 of the outer
 // tolerance).  Inertia and C p stay FP64.
-// (e, f) of the pair (i, j) in FP32, as every pair-term kernel evaluates it
-// (one function, so that they agree bit for bit): x_j - x_i from the
-// two-float positions (the high parts of nearby positions subtract with one
-// FP32 rounding at most, so q is within about one FP32 ulp of the FP64
-// difference, with no FP64 arithmetic); the exact minimum image only when a
-// component is not well inside a quarter of the domain width (a periodic
-// image, which also sets *wrap).  e = q / |q|, f = visc mu_ij w'(|q|) / |q|
-// within RadiusV, else 0 (main.cpp:2261-2289).
-template <int D>
-__device__ __forceinline__ void pair_ef(const DevParams& P, int i, int j, int ti, const float* hi, const float* li,
-                                        const int* __restrict__ type, const double* __restrict__ pos,
-                                        const float* __restrict__ pos32, const float* __restrict__ poslo32,
-                                        int* __restrict__ wrap, float* e, float& f)
-{
-    if (j != i) {
-        float hj[3], lj[3];
-        int tj;
-        if (D == 3) {   // the high part's w holds the type bits (k_permute)
-            const float4 h4 = reinterpret_cast<const float4*>(pos32)[j];
-            hj[0] = h4.x; hj[1] = h4.y; hj[2] = h4.z;
-            tj = __float_as_int(h4.w);
-        } else {
-            load_f32<D>(pos32, j, hj);
-            tj = type[j];
-        }
-        load_f32<D>(poslo32, j, lj);
-        float q32[3] = {0.f, 0.f, 0.f};
-        bool inner = true;
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-            q32[d] = (hj[d] - hi[d]) + (lj[d] - li[d]);
-            inner = inner && fabsf(q32[d]) < 0.48f * P.hw32[d];
-        }
-        if (!inner) {
-            *wrap = 1;   // the recomputing inner operator then takes the minimum image
-            double xi[3], xj[3], q[3];
-            load_vec<D>(pos, i, xi);
-            load_vec<D>(pos, j, xj);
-            sep_vec<D>(P, xj, xi, q);
-#pragma unroll
-            for (int d = 0; d < D; ++d) q32[d] = (float)q[d];
-        }
-        const float r2 = q32[0] * q32[0] + q32[1] * q32[1] + q32[2] * q32[2];
-        if (r2 != 0.f && P.rV2_32 - r2 > 0.f) {
-            const float inv = rsqrtf(r2);
-            const float wd = P.wdA32 * (1.f - (r2 * inv) * P.inv_rv32);
-            f = P.vm32[ti][tj] * wd * inv;
-#pragma unroll
-            for (int d = 0; d < D; ++d) e[d] = q32[d] * inv;
-        }
-    }
-}
-
 // The end of a fluid row in the pair-term kernels, from its warp's per-lane
 // partial sums: b_i = - C p + inertia v in FP64 (the lanes' sums by
 // reduce-scatter; lane 8 r in 3-D, 16 r in 2-D, writes component r) and, with
@@ -228,12 +176,12 @@ k_pair_terms(DevParams P, const int* __restrict__ type, const double* __restrict
             const double pk = pvec[k];
 #pragma unroll
             for (int r = 0; r < D; ++r) sumv[r] -= cval[(pb + a) * D + r] * pk;
-            if (cvl32 || dinv) {   // lambda_k C_ik: the stored FP32 inner operator, the diagonal
+            if (cvl32) {   // lambda_k C_ik for the FP32 inner operator
                 const double lam = P.lambda[type[k]];
 #pragma unroll
                 for (int r = 0; r < D; ++r) {
                     const float cl = (float)(cval[(pb + a) * D + r] * lam);
-                    if (cvl32) cvl32[(pb + a) * D + r] = cl;
+                    cvl32[(pb + a) * D + r] = cl;
                     dpd[r] += cl * (float)cval[(pb + a) * D + r];
                 }
             }
@@ -394,15 +342,16 @@ __global__ void __launch_bounds__(256) k_wall_terms64(DevParams P, const int* __
                                                       const double* __restrict__ vel, const int* __restrict__ nc,
                                                       const int* __restrict__ nfc, const long long* __restrict__ nptr,
                                                       const int* __restrict__ nind, double* __restrict__ bvec,
-                                                      float* __restrict__ sdiag32, double* __restrict__ sdiag64)
+                                                      float* __restrict__ sdiag32, double* __restrict__ sdiag64, bool wall_rows_only)
 {
     // a warp per fluid row, its lanes over the row's wall slots; the lane
     // sums meet in a fixed shuffle tree (deterministic)
     const int lane = threadIdx.x & 31;
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= P.Nf) return;
-    const int ti = type[i];
     const int n = nc[i], nf = nfc[i];
+    if (wall_rows_only && n == nf) return;   // warp-uniform
+    const int ti = type[i];
     double sd[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // xx xy xz yy yz zz
     double sw[3] = {0.0, 0.0, 0.0};
     // this lane's warp sum after the reduce-scatter: value lane >> 1 of
@@ -447,7 +396,10 @@ __global__ void __launch_bounds__(256) k_wall_terms64(DevParams P, const int* __
         const int t = lane >> 1;
         if ((lane & 1) == 0 && t >= 6 && t < 6 + D) bvec[(size_t)i * D + (t - 6)] += val;
     }
-    if (sdiag32) {   // lane 2 t writes component t: one FP32 conversion a lane
+    if (wall_rows_only) {
+        const int t = lane >> 1;
+        if ((lane & 1) == 0 && t < 6) sdiag64[(size_t)i * 8 + t] = val;
+    } else if (sdiag32) {   // lane 2 t writes component t: one FP32 conversion a lane
         const int t = lane >> 1;
         if ((lane & 1) == 0 && t < 6) {
             sdiag32[(size_t)i * 8 + t] = (float)val;
@@ -1881,6 +1833,17 @@ bool factored_applies(const mph_case* c)
     return pair_path || pert < 1.0e-2 * c->tol_outer;
 }
 
+// the wall slots of the fluid rows: into b, and the wall part of the viscous
+// diagonal (wall_rows_only: sdiag64 of the rows that have wall slots, no more)
+void launch_wall_terms(mph_case* c, float* sdiag32, double* sdiag64, bool wall_rows_only)
+{
+    DeviceState& d = c->d;
+    const DevParams& P = c->dp;
+    const unsigned g = grid_for((long long)P.Nf * 32, 256);
+    if (c->dim == 2) { k_wall_terms64<2><<<g, 256, 0, c->stream>>>(P, d.type, d.pos, d.vel, d.nc, d.nfc, d.nptr, d.nind, d.bvec, sdiag32, sdiag64, wall_rows_only); MPH_COUNT_LAUNCH(); }
+    else { k_wall_terms64<3><<<g, 256, 0, c->stream>>>(P, d.type, d.pos, d.vel, d.nc, d.nfc, d.nptr, d.nind, d.bvec, sdiag32, sdiag64, wall_rows_only); MPH_COUNT_LAUNCH(); }
+}
+
 template <int D>
 static void pair_slices_launch(mph_case* c)
 {
@@ -1915,11 +1878,9 @@ int launch_pair_terms(mph_case* c)
     if (!d.x32) MPH_CUDA(cudaMalloc((void**)&d.x32, (size_t)P.Nf * c->dim * 2 * sizeof(float)));
     if (!d.tct32) MPH_CUDA(cudaMalloc((void**)&d.tct32, (size_t)(P.N + 1) * sizeof(float)));
     long long ncv = 0;   // C values of the fluid rows, FP32 copy for the inner operator
-    if (!c->step_pen || fused) {
-        MPH_CUDA(cudaMemcpyAsync(&ncv, d.nptrP + P.Nf, sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
-        MPH_CUDA(cudaStreamSynchronize(c->stream));
-        ncv *= c->dim;
-    }
+    MPH_CUDA(cudaMemcpyAsync(&ncv, d.nptrP + P.Nf, sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
+    MPH_CUDA(cudaStreamSynchronize(c->stream));
+    ncv *= c->dim;
     if (ncv > d.cap_cval32) {
         if (d.cval32) cudaFree(d.cval32);
         d.cval32 = nullptr;
@@ -1927,7 +1888,7 @@ int launch_pair_terms(mph_case* c)
         MPH_CUDA(cudaMalloc((void**)&d.cval32, (size_t)(ncv + ncv / 8 + 1024) * sizeof(float)));
         d.cap_cval32 = ncv + ncv / 8 + 1024;
     }
-    if (!c->step_pen) { k_cval_f32<<<grid_for(ncv, 256), 256, 0, c->stream>>>(ncv, d.cval, d.cval32); MPH_COUNT_LAUNCH(); }
+    { k_cval_f32<<<grid_for(ncv, 256), 256, 0, c->stream>>>(ncv, d.cval, d.cval32); MPH_COUNT_LAUNCH(); }
     float* sdiag = nullptr;
     double* sdiag64 = nullptr;
     float* cvl = nullptr;
@@ -1937,14 +1898,12 @@ int launch_pair_terms(mph_case* c)
         if (!d.sdiag64) MPH_CUDA(cudaMalloc((void**)&d.sdiag64, (size_t)P.Nf * 8 * sizeof(double)));
         sdiag64 = d.sdiag64;
         sdiag = d.sdiag32;
-        if (!c->step_pen || fused) {
-            MPH_TRY(grow_f(&d.cvl32, &d.cap_cvl32, ncv));
-            cvl = d.cvl32;
-        }
+        MPH_TRY(grow_f(&d.cvl32, &d.cap_cvl32, ncv));
+        cvl = d.cvl32;
         if (!d.pscale) MPH_CUDA(cudaMalloc((void**)&d.pscale, (size_t)((P.Nf + 31) / 32 + 1) * sizeof(float)));
         if (!fused) {
             MPH_CUDA(cudaMemsetAsync(d.pscale, 0, (size_t)((P.Nf + 31) / 32 + 1) * sizeof(float), c->stream));
-            if (!c->pair_recompute && !c->step_pen)
+            if (!c->pair_recompute)
                 gmax = reinterpret_cast<unsigned*>(d.pscale);   // slice maxima, turned into scales by the slicing
         }
     }
@@ -1953,18 +1912,16 @@ int launch_pair_terms(mph_case* c)
     // the mixed form without grid levels takes D^-1 from here (no level-0 pass)
     double* dinv = c->step_pairs && mixed_jacobi(c) ? d.invDiag : nullptr;
     const unsigned g = std::min<long long>(((long long)P.Nf + kPtWarps - 1) / kPtWarps, 152LL * 128 / kPtWarps);
-    const unsigned gw = grid_for((long long)P.Nf * 32, 256);
     if (c->dim == 2) {
         if (fused) pair_slices_launch<2>(c);
         else { k_pair_terms<2><<<g, kPtWarps * 32, 0, c->stream>>>(P, d.type, d.pos, d.pos32, d.poslo32, d.vel, d.nc, d.nptr, d.nind, d.nfc, d.ncp, d.nptrP,
                                                                     d.nindP, d.cval, d.pvec, d.pe32, d.bvec, cvl, gmax, d.wrap32, dinv); MPH_COUNT_LAUNCH(); }
-        { k_wall_terms64<2><<<gw, 256, 0, c->stream>>>(P, d.type, d.pos, d.vel, d.nc, d.nfc, d.nptr, d.nind, d.bvec, sdiag, sdiag64); MPH_COUNT_LAUNCH(); }
     } else {
         if (fused) pair_slices_launch<3>(c);
         else { k_pair_terms<3><<<g, kPtWarps * 32, 0, c->stream>>>(P, d.type, d.pos, d.pos32, d.poslo32, d.vel, d.nc, d.nptr, d.nind, d.nfc, d.ncp, d.nptrP,
                                                                     d.nindP, d.cval, d.pvec, d.pe32, d.bvec, cvl, gmax, d.wrap32, dinv); MPH_COUNT_LAUNCH(); }
-        { k_wall_terms64<3><<<gw, 256, 0, c->stream>>>(P, d.type, d.pos, d.vel, d.nc, d.nfc, d.nptr, d.nind, d.bvec, sdiag, sdiag64); MPH_COUNT_LAUNCH(); }
     }
+    launch_wall_terms(c, sdiag, sdiag64, false);
     return MPH_OK;
 }
 
@@ -2079,17 +2036,6 @@ int launch_pairs_to_slices(mph_case* c)
     const DevParams& P = c->dp;
     const int D = c->dim;
     if (c->nslices == 0) return MPH_OK;
-    if (c->step_pen) {   // the outer residual's layout only: FP32 g and columns
-        MPH_TRY(grow_f(&d.pes32, &d.cap_pes32, c->nslots * D));
-        if (!pair_fused(c)) {
-            if (D == 2) k_list_to_slices<2, true><<<c->nslices, 256, 0, c->stream>>>(P.Nf, d.sptr, d.nfc, d.nptr, d.nind, d.pe32, nullptr,
-                                                                                    d.acol, d.pes32, nullptr, d.pscale, nullptr);
-            else k_list_to_slices<3, true><<<c->nslices, 256, 0, c->stream>>>(P.Nf, d.sptr, d.nfc, d.nptr, d.nind, d.pe32, nullptr,
-                                                                             d.acol, d.pes32, nullptr, d.pscale, nullptr);
-            MPH_COUNT_LAUNCH();
-        }
-        return launch_pen_lists(c);
-    }
     MPH_TRY(ensure_pair_records(c));
     const bool lrec = c->pair_recompute || c->pair_pack;   // records without the index half
     if (!d.psptr) {

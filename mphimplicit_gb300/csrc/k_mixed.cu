@@ -391,6 +391,7 @@ int mixed_prepare(mph_case* c)
         MPH_CUDA(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
         MPH_CUDA(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
     }
+    if (c->step_pen) return MPH_OK;   // the assembly wrote the FP32 D^-1
     if (mixed_jacobi(c)) {   // point Jacobi: the FP32 D^-1 only
         const long long nv = (long long)c->dp.Nf * c->dim;
         if (!d.v32) MPH_CUDA(cudaMalloc((void**)&d.v32, (size_t)nv * 8 * sizeof(float)));
@@ -543,7 +544,9 @@ static int device_solve(mph_case* c, double* hs, int* hflags)
         int st_ = MPH_OK;
         auto fail_capture = [&](int e) { st_ = e; };
         auto residual = [&]() {
-            if (c->step_factored) {
+            if (c->step_pen) {
+                launch_pen_start_residual(c);
+            } else if (c->step_factored) {
                 launch_resid_factored(c, d.x, d.r, scal + kSRR);
             } else {
                 k_resid64<D><<<gs, 128, 0, c->stream>>>(Nf, d.nfc, d.sptr, d.acol, d.aval, d.x, d.bvec, d.r, part, counter,
@@ -575,9 +578,13 @@ static int device_solve(mph_case* c, double* hs, int* hflags)
         if (st_ == MPH_OK) {
             c->stream = s2;
             { k_phase_begin<<<1, 32, 0, s2>>>(scal, flags, h_in); MPH_COUNT_LAUNCH(); }
-            { k_to32<V><<<rb, kReduceThreads, 0, s2>>>(n, d.r, r32, z32, 1.0, scal, part, counter, scal + kSScale); MPH_COUNT_LAUNCH(); }
-            { k_phase_tol<<<1, 32, 0, s2>>>(scal, tol_in2, tol_out2); MPH_COUNT_LAUNCH(); }
-            vcycle_mixed(c, r32, s32, scal + kSQU32);   // s = M r
+            if (c->step_pen) {
+                launch_pen_phase(c, 1.0, scal + kSScale, tol_in2, tol_out2);
+            } else {
+                { k_to32<V><<<rb, kReduceThreads, 0, s2>>>(n, d.r, r32, z32, 1.0, scal, part, counter, scal + kSScale); MPH_COUNT_LAUNCH(); }
+                { k_phase_tol<<<1, 32, 0, s2>>>(scal, tol_in2, tol_out2); MPH_COUNT_LAUNCH(); }
+                vcycle_mixed(c, r32, s32, scal + kSQU32);   // s = M r
+            }
             cudaGraph_t body_in = nullptr;
             e = add_while_node(s2, h_in, &body_in);
             if (e != MPH_OK) fail_capture(e);
@@ -605,8 +612,12 @@ static int device_solve(mph_case* c, double* hs, int* hflags)
                 if (cudaStreamEndCapture(s3, &gi) != cudaSuccess) fail_capture(fail(MPH_ERR_CUDA, "end of the CR iteration capture"));
             }
             c->stream = s2;
-            { k_refine<V><<<rb, kReduceThreads, 0, s2>>>(n, d.x, z32, 1.0, scal + kSScale, flags); MPH_COUNT_LAUNCH(); }
-            residual();
+            if (c->step_pen) {
+                launch_pen_refine(c, 1.0, scal + kSScale, flags);
+            } else {
+                { k_refine<V><<<rb, kReduceThreads, 0, s2>>>(n, d.x, z32, 1.0, scal + kSScale, flags); MPH_COUNT_LAUNCH(); }
+                residual();
+            }
             { k_outer_check<<<1, 32, 0, s2>>>(scal, flags, tol_out2, c->max_outer, cap, h_out); MPH_COUNT_LAUNCH(); }
             cudaGraph_t go = nullptr;
             if (cudaStreamEndCapture(s2, &go) != cudaSuccess) fail_capture(fail(MPH_ERR_CUDA, "end of the phase capture"));
@@ -728,7 +739,8 @@ struct MixedRun {
         { k_x0<D><<<rb, kReduceThreads, 0, st>>>(Nf, d.type, d.vel, d.force, d.bvec, d.x, c->dp, vprev, nvs, have, c->extrapolate,
                                                  part, counter, scal + kSRR0); MPH_COUNT_LAUNCH(); }
         c->prev_valid = vprev ? std::min(c->prev_valid + 1, c->extrapolate) : 0;
-        residual();
+        if (c->step_pen) launch_pen_start_residual(c);
+        else residual();
         return MPH_OK;
     }
 
@@ -748,7 +760,13 @@ struct MixedRun {
         if (hs[kSRR] / hs[kSRR0] < tol_out2 || outer >= c->max_outer || hs[kSRR] == 0.0) return MPH_OK;
         if (outer > 0 && host_flags[kFlagIter] >= cap) return MPH_OK;
         if (outer == 0) scale = std::sqrt(hs[kSRR]);
-        else MPH_CUDA(cudaMemsetAsync(flags + kFlagDone, 0, sizeof(int), st));
+        if (c->step_pen) {
+            ++outer;
+            launch_pen_phase(c, 1.0 / scale, nullptr, tol_in2, tol_out2);
+            *go = true;
+            return MPH_OK;
+        }
+        if (outer > 0) MPH_CUDA(cudaMemsetAsync(flags + kFlagDone, 0, sizeof(int), st));
         ++outer;
         { k_to32<V><<<rb, kReduceThreads, 0, st>>>(n, c->d.r, r32, z32, 1.0 / scale, scal, part, counter); MPH_COUNT_LAUNCH(); }
         { k_phase_tol<<<1, 32, 0, st>>>(scal, tol_in2, tol_out2); MPH_COUNT_LAUNCH(); }
@@ -766,8 +784,12 @@ struct MixedRun {
             bad = true;
             return MPH_OK;
         }
-        { k_refine<V><<<rb, kReduceThreads, 0, c->stream>>>(n, c->d.x, z32, scale); MPH_COUNT_LAUNCH(); }
-        residual();
+        if (c->step_pen) {
+            launch_pen_refine(c, scale, nullptr, nullptr);
+        } else {
+            { k_refine<V><<<rb, kReduceThreads, 0, c->stream>>>(n, c->d.x, z32, scale); MPH_COUNT_LAUNCH(); }
+            residual();
+        }
         *go = true;
         return MPH_OK;
     }

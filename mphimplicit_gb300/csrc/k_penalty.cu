@@ -43,6 +43,7 @@
 #include <type_traits>
 
 #include "mph_device.cuh"
+#include "mph_pairs.cuh"
 #include "mph_solver.cuh"
 
 namespace mph {
@@ -59,18 +60,37 @@ constexpr int kMaxPenRows = 256;   // threads of a row block (rows times threads
 // blocks of 599 on average: 9.12 ms staged, 9.34 gathered) gains little.
 static int pen_ucap(int rows) { return 4 * rows + 128; }
 
+// Fixed-point positions of the penalty operator (ipos, units of RadiusP /
+// 2^22 over the whole domain) and of the viscous pairs (vpos, RadiusP / 2^26
+// modulo 2^32: a pair's separation is exact while it is shorter than 32
+// RadiusP), both with the particle's type; and whether a pair can be a
+// periodic image: bits 0-2 of *wrap, a particle within MaxRadius of the
+// domain's lower face of an axis, bits 3-5 of the upper one.
 template <int D>
-__global__ void k_fixed_positions(DevParams P, const int* __restrict__ type, const double* __restrict__ pos, int4* __restrict__ ipos)
+__global__ void __launch_bounds__(256) k_fixed_positions(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
+                                                         int4* __restrict__ ipos, int4* __restrict__ vpos, int* __restrict__ wrap)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.N) return;
-    double x[3];
-    load_vec<D>(pos, i, x);
-    int u[3] = {0, 0, 0};
+    unsigned near = 0u;
+    if (i < P.N) {
+        double x[3];
+        load_vec<D>(pos, i, x);
+        int u[3] = {0, 0, 0}, v[3] = {0, 0, 0};
 #pragma unroll
-    for (int d = 0; d < D; ++d) u[d] = __double2int_rn((x[d] - P.dmin[d]) * P.fix_scale);
-    ipos[i] = make_int4(u[0], u[1], u[2], type[i]);
+        for (int d = 0; d < D; ++d) {
+            const double r = x[d] - P.dmin[d];
+            u[d] = __double2int_rn(r * P.fix_scale);
+            v[d] = (int)(unsigned)(unsigned long long)__double2ll_rn(r * P.vfix_scale);
+            near |= (r < P.maxR ? 1u << d : 0u) | (P.dw[d] - r < P.maxR ? 8u << d : 0u);
+        }
+        const int t = type[i];
+        ipos[i] = make_int4(u[0], u[1], u[2], t);
+        vpos[i] = make_int4(v[0], v[1], v[2], t);
+    }
+    near = __reduce_or_sync(0xffffffffu, near);
+    if (near && (threadIdx.x & 31) == 0) atomicOr((unsigned*)wrap, near);
 }
+__device__ __forceinline__ bool may_wrap(int w) { return (w & (w >> 3) & 7) != 0; }
 
 // The P-lists of a block of rows as 2-byte ranks among the block's distinct
 // columns: uniq[block][0 .. U) the columns in ascending order, idx the rank of
@@ -321,7 +341,8 @@ __device__ __forceinline__ void pen_t_body(const DevParams& P, const PenArgs& A,
     const int rows = blockDim.x, W = blockDim.y;
     const int tid = threadIdx.y * rows + threadIdx.x, nth = rows * W;
     const int i = lb * rows + threadIdx.x;
-    const int done = A.flags[kFlagDone], wrap = *A.wrap;
+    const int done = A.flags[kFlagDone];
+    const bool wrap = may_wrap(*A.wrap);
     PenPre R;
     pen_prefetch(A, lb, i, A.N, tid, nth, threadIdx.y, W, R);
     int4 pi = make_int4(0, 0, 0, 0);
@@ -440,7 +461,8 @@ __device__ __forceinline__ void pen_y_body(const DevParams& P, const PenArgs& A,
     extern __shared__ int4 pen_smem[];
     const int rows = blockDim.x, W = blockDim.y;
     const int tid = threadIdx.y * rows + threadIdx.x, nth = rows * W;
-    const int done = A.flags[kFlagDone], it = A.flags[kFlagIter], wrap = *A.wrap;
+    const int done = A.flags[kFlagDone], it = A.flags[kFlagIter];
+    const bool wrap = may_wrap(*A.wrap);
     if (done) return;   // block-uniform: set before this launch
     int4* sa = pen_smem;
     float v[3] = {0.f, 0.f, 0.f};
@@ -628,6 +650,323 @@ __global__ void __launch_bounds__(kReduceThreads) k_pen_vec(PenArgs A, int n, in
     pen_vec_body<COND>(A, (int)blockIdx.x, (int)gridDim.x, n, use_cond, cond);
 }
 
+// ---- the system: C, b and D^-1 -------------------------------------------------------
+// C of every particle's P-list (calculateMatrixC main.cpp:2462-2507; the wall
+// rows' C_kj = - C_jk of fluid j give C^T its wall rows without a transposed
+// list), and for the fluid rows in the same pass b = inertia v - C p (its wall
+// velocities follow in k_wall_terms64) and the FP32 D^-1.  Bound by the FP64
+// pipe: 1.47 ms on 1.3 million particles.  C, the transposed lists (0.69 ms),
+// b with the pair terms (2.06) and their slicing (1.04) took 5.0 ms in passes
+// of their own.
+template <int D>
+__global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
+                                                    const double* __restrict__ vel, const int* __restrict__ ncp,
+                                                    const long long* __restrict__ nptrP, const int* __restrict__ nindP,
+                                                    const double* __restrict__ pvec, double* __restrict__ cval,
+                                                    double* __restrict__ bvec, float* __restrict__ invD)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P.N) return;
+    const bool fluid = i < P.Nf;
+    double xi[3];
+    load_vec<D>(pos, i, xi);
+    const double rP2 = P.rP * P.rP;
+    const long long b = nptrP[i];
+    const int n = ncp[i];
+    double self[3] = {0, 0, 0}, cp[3] = {0, 0, 0};
+    float dp[3] = {0.f, 0.f, 0.f};
+    int selfk = 0;
+    for (int a = 0; a < n; ++a) {
+        const int j = nindP[b + a];
+        double cv[3] = {0, 0, 0};
+        if (j == i) {
+            selfk = a;
+        } else if (fluid || j < P.Nf) {
+            double xj[3], q[3];
+            load_vec<D>(pos, j, xj);
+            sep_vec<D>(P, xj, xi, q);
+            const double r2 = norm2_exact<D>(q);
+            if (r2_pos_below(r2, rP2)) {
+                const double inv = rsqrt(r2);
+                const double wd = -P.kfp * (P.m2h_rp * (1.0 - (r2 * inv) * P.inv_rp));
+                const double pj = fluid ? pvec[j] : 0.0;
+                const float lam = P.lambda32[type[j]];
+#pragma unroll
+                for (int r = 0; r < D; ++r) {
+                    cv[r] = (q[r] * inv) * wd;
+                    self[r] += cv[r];
+                    cp[r] += cv[r] * pj;
+                    dp[r] += (float)cv[r] * (float)cv[r] * lam;
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < D; ++r) cval[(b + a) * D + r] = cv[r];
+    }
+    if (!fluid) return;
+    const int ti = type[i];
+    const double pi = pvec[i];
+    double v[3];
+    load_vec<D>(vel, i, v);
+#pragma unroll
+    for (int r = 0; r < D; ++r) {
+        if (n > 0) cval[(b + selfk) * D + r] = self[r];
+        bvec[(size_t)i * D + r] = P.inert64[ti] * v[r] - (cp[r] + self[r] * pi);
+        const float dg = P.inert32[ti] + P.pen_vd[ti] + dp[r] + (float)self[r] * (float)self[r] * P.lambda32[ti];
+        invD[(size_t)i * D + r] = dg != 0.f ? 1.f / dg : 0.f;
+    }
+}
+
+// The diagonal with its row's own viscous pairs, as the other forms' D^-1 (a
+// reader's request only: the point-Jacobi form keeps the lattice's).
+template <int D>
+__global__ void __launch_bounds__(256) k_pen_diag(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
+                                                  const float* __restrict__ pos32, const float* __restrict__ poslo32,
+                                                  const int* __restrict__ nc, const long long* __restrict__ nptr,
+                                                  const int* __restrict__ nind, const int* __restrict__ ncp,
+                                                  const long long* __restrict__ nptrP, const int* __restrict__ nindP,
+                                                  const double* __restrict__ cval, int* __restrict__ unused, double* __restrict__ dinv)
+{
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= P.Nf) return;
+    const int ti = type[i];
+    float hi[3], li[3], t[3] = {0.f, 0.f, 0.f};
+    load_f32<D>(pos32, i, hi);
+    load_f32<D>(poslo32, i, li);
+    for (int k = lane; k < nc[i]; k += 32) {
+        float e[3] = {0.f, 0.f, 0.f}, f = 0.f;
+        pair_ef<D>(P, i, nind[nptr[i] + k], ti, hi, li, type, pos, pos32, poslo32, unused, e, f);
+#pragma unroll
+        for (int d = 0; d < D; ++d) t[d] += f * e[d] * e[d];
+    }
+    for (int a = lane; a < ncp[i]; a += 32)
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            const double c = cval[(nptrP[i] + a) * D + d];
+            t[d] += (float)(c * P.lambda[type[nindP[nptrP[i] + a]]]) * (float)c;
+        }
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t[d] += __shfl_xor_sync(0xffffffffu, t[d], o);
+        const float dg = P.inert32[ti] + t[d];
+        if (lane == 0) dinv[(size_t)i * D + d] = (double)(dg != 0.f ? 1.f / dg : 0.f);
+    }
+}
+
+// ---- the FP64 outer residual ------------------------------------------------------------
+// r = b - A x, with A x in three parts: inertia, C Lambda C^T and the wall
+// part of the viscous diagonal in FP64 from x, the fluid pairs
+// sum f e (e . (x_i - x_j)) added up in FP64 over the solve's corrections,
+// V x = V x_0 + sum scale V z.  The pairs are evaluated from the positions in
+// FP32 (coefficients and row sums as the stored pair terms had them): the
+// differences of x_0 in two floats, those of the FP32 corrections z exactly.
+//
+// x_0 as records (hi, lo), or the update x += scale z and z as records
+template <int D, bool FIRST>
+__global__ void __launch_bounds__(256) k_pen_pack(int Nf, double* __restrict__ x, const float* __restrict__ z, double scale,
+                                                  const double* __restrict__ scale_src, const int* __restrict__ flags,
+                                                  float4* __restrict__ rec)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= Nf) return;
+    if (!FIRST && flags && flags[kFlagBad]) return;   // the device-driven solve: a phase that met a NaN ends the solve
+    float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
+    const double sc = FIRST ? 0.0 : (scale_src ? *scale_src : scale);
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        const size_t k = (size_t)i * D + d;
+        if (FIRST) {
+            const double v = x[k];
+            h[d] = (float)v;
+            l[d] = (float)(v - (double)h[d]);
+        } else {
+            h[d] = z[k];
+            x[k] += sc * (double)h[d];
+        }
+    }
+    rec[i] = make_float4(h[0], h[1], h[2], 0.f);
+    if (FIRST) rec[Nf + i] = make_float4(l[0], l[1], l[2], 0.f);
+}
+
+// vacc_i (+)= scale sum over the fluid neighbours of f e (e . (x_i - x_j)),
+// L lanes a row over its neighbour list.  A pair is two 16-byte gathers (three
+// for x_0) and some 35 instructions; bound by the L1's gather rate.  Against
+// the stored FP32 g and columns (16 bytes a slot streamed, x in six 4-byte
+// gathers: 1.33 ms on 1.3 million particles with the P-part) it needs no pair
+// terms, which took three passes to build: 0.73 ms for x_0, 0.62 for z.
+template <int D, int L, bool FIRST>
+__global__ void __launch_bounds__(256) k_pen_visc(DevParams P, const int4* __restrict__ vpos, const int* __restrict__ nfc,
+                                                  const long long* __restrict__ nptr, const int* __restrict__ nind,
+                                                  const float4* __restrict__ rec, int* __restrict__ wrap,
+                                                  const int* __restrict__ type, const double* __restrict__ pos,
+                                                  const float* __restrict__ pos32, const float* __restrict__ poslo32, double scale,
+                                                  const double* __restrict__ scale_src, double* __restrict__ vacc)
+{
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / L, lane = threadIdx.x & (L - 1);
+    float y[3] = {0.f, 0.f, 0.f};
+    if (i < P.Nf) {
+        const int n = nfc[i];
+        const int* col = nind + nptr[i];
+        const float4 hi = rec[i];
+        const float4 li = FIRST ? rec[P.Nf + i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4* lo = rec + P.Nf;
+        if (!may_wrap(*wrap)) {
+            const int4 pi = vpos[i];
+            const float vm0 = pi.w ? P.pen_vm[1][0] : P.pen_vm[0][0], vm1 = pi.w ? P.pen_vm[1][1] : P.pen_vm[0][1];
+#pragma unroll 4
+            for (int k = lane; k < n; k += L) {
+                const int j = col[k];
+                const int4 pj = vpos[j];
+                const float4 h = rec[j];
+                const float q[3] = {(float)(pj.x - pi.x), (float)(pj.y - pi.y), D == 3 ? (float)(pj.z - pi.z) : 0.f};
+                float dx[3] = {hi.x - h.x, hi.y - h.y, D == 3 ? hi.z - h.z : 0.f};
+                if (FIRST) {
+                    const float4 l = lo[j];
+                    dx[0] += li.x - l.x;
+                    dx[1] += li.y - l.y;
+                    if (D == 3) dx[2] += li.z - l.z;
+                }
+                float r2 = q[0] * q[0] + q[1] * q[1];
+                if (D == 3) r2 += q[2] * q[2];
+                const float inv = rsqrtf(fmaxf(r2, 1.f));
+                // visc mu_ij w' / |q|, w' = (1 - |q| / RadiusV) up to the constants in vm; q / |q| twice
+                const float c = (pj.w ? vm1 : vm0) * fmaxf(inv - P.pen_vk, 0.f) * (inv * inv);
+                float dot = q[0] * dx[0] + q[1] * dx[1];
+                if (D == 3) dot += q[2] * dx[2];
+                const float t = c * dot;
+#pragma unroll
+                for (int d = 0; d < D; ++d) y[d] += t * q[d];
+            }
+        } else {   // periodic images: the general pair term
+            const int ti = type[i];
+            float ph[3], pl[3];
+            load_f32<D>(pos32, i, ph);
+            load_f32<D>(poslo32, i, pl);
+            for (int k = lane; k < n; k += L) {
+                const int j = col[k];
+                float e[3] = {0.f, 0.f, 0.f}, f = 0.f;
+                pair_ef<D>(P, i, j, ti, ph, pl, type, pos, pos32, poslo32, wrap + 1, e, f);
+                const float4 h = rec[j];
+                float dx[3] = {hi.x - h.x, hi.y - h.y, hi.z - h.z};
+                if (FIRST) {
+                    const float4 l = lo[j];
+                    dx[0] += li.x - l.x;
+                    dx[1] += li.y - l.y;
+                    dx[2] += li.z - l.z;
+                }
+                const float t = f * (e[0] * dx[0] + e[1] * dx[1] + e[2] * dx[2]);
+#pragma unroll
+                for (int d = 0; d < D; ++d) y[d] += t * e[d];
+            }
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) y[d] += __shfl_xor_sync(0xffffffffu, y[d], o);
+    if (i < P.Nf && lane < D) {
+        const float yl = lane == 0 ? y[0] : (lane == 1 ? y[1] : y[2]);
+        const size_t k = (size_t)i * D + lane;
+        vacc[k] = FIRST ? (double)yl : vacc[k] + (scale_src ? *scale_src : scale) * (double)yl;
+    }
+}
+
+// lambda_k t_k, t = C^T x in FP64 from the particle's own P-list:
+// C_jk = - C_kj (to the rounding of the minimum image), and C_kk for a fluid
+// row itself
+template <int D>
+__global__ void __launch_bounds__(128) k_pen_ct64(DevParams P, const int* __restrict__ type, const int* __restrict__ ncp,
+                                                  const long long* __restrict__ nptrP, const int* __restrict__ nindP,
+                                                  const double* __restrict__ cval, const double* __restrict__ x, double* __restrict__ t)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= P.N) return;
+    const long long b = nptrP[k];
+    const int n = ncp[k];
+    double s = 0.0;
+#pragma unroll 2
+    for (int a = 0; a < n; ++a) {
+        const int j = nindP[b + a];
+        if (j >= P.Nf) continue;
+        double v = 0.0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) v += cval[(b + a) * D + d] * x[(size_t)j * D + d];
+        s = j == k ? s + v : s - v;
+    }
+    t[k] = P.lambda[type[k]] * s;
+}
+
+template <int D>
+__global__ void __launch_bounds__(128) k_pen_resid(DevParams P, const int* __restrict__ type, const int* __restrict__ nc,
+                                                   const int* __restrict__ nfc, const int* __restrict__ ncp,
+                                                   const long long* __restrict__ nptrP, const int* __restrict__ nindP,
+                                                   const double* __restrict__ cval, const double* __restrict__ t,
+                                                   const double* __restrict__ sdiag64, const double* __restrict__ vacc,
+                                                   const double* __restrict__ x, const double* __restrict__ b, double* __restrict__ r,
+                                                   double* __restrict__ partials, unsigned* __restrict__ counter, double* __restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double acc = 0.0;
+    if (i < P.Nf) {
+        double xi[3] = {0.0, 0.0, 0.0}, y[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            xi[d] = x[(size_t)i * D + d];
+            y[d] = vacc[(size_t)i * D + d];
+        }
+        const long long pb = nptrP[i];
+        const int np = ncp[i];
+#pragma unroll 2
+        for (int a = 0; a < np; ++a) {
+            const double lt = t[nindP[pb + a]];
+#pragma unroll
+            for (int d = 0; d < D; ++d) y[d] += cval[(pb + a) * D + d] * lt;
+        }
+        if (nc[i] > nfc[i]) {   // wall neighbours: their part of the viscous diagonal
+            const double2* sp = reinterpret_cast<const double2*>(sdiag64 + (size_t)i * 8);
+            const double2 p = sp[0], q = sp[1], e = sp[2];   // (xx, xy), (xz, yy), (yz, zz)
+            y[0] += p.x * xi[0] + p.y * xi[1] + q.x * xi[2];
+            y[1] += p.y * xi[0] + q.y * xi[1] + e.x * xi[2];
+            y[2] += q.x * xi[0] + e.x * xi[1] + e.y * xi[2];
+        }
+        const double inert = P.inert64[type[i]];
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            const size_t k = (size_t)i * D + d;
+            const double rv = b[k] - (inert * xi[d] + y[d]);
+            r[k] = rv;
+            acc += rv * rv;
+        }
+    }
+    reduce_finalize(acc, partials, counter, out);
+}
+
+// Start of a refinement phase: r32 = r / scale, s = D^-1 r32, z = 0, the inner
+// reference norm (r32, r32), the phase's target (reduce it by tol_in, but no
+// further than half of what the outer test still asks for) and the done flag.
+__global__ void __launch_bounds__(kReduceThreads) k_pen_phase(int n, const double* __restrict__ r, const float* __restrict__ invD,
+                                                              float* __restrict__ s, float* __restrict__ z, double inv_scale,
+                                                              const double* __restrict__ scale_src, double tol_in2, double tol_out2,
+                                                              double* __restrict__ scal, int* __restrict__ flags,
+                                                              double* __restrict__ partials, unsigned* __restrict__ counter)
+{
+    const double sc = scale_src ? 1.0 / *scale_src : inv_scale;
+    float acc = 0.f;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const float v = (float)(r[k] * sc);
+        s[k] = invD[k] * v;
+        z[k] = 0.f;
+        acc += v * v;
+    }
+    if (reduce_finalize_last(acc, partials, counter, scal + kSIn0)) {
+        const double need = 0.25 * tol_out2 * scal[kSRR0] / scal[kSRR];
+        scal[kSTol2] = need > tol_in2 ? need : tol_in2;
+        scal[kSIn] = scal[kSIn0];
+        flags[kFlagDone] = 0;
+    }
+}
+
 // ---- host side ---------------------------------------------------------------------
 constexpr int kPenBlocks = 152 * kPenResident;   // blocks of k_pen_y: what is resident at once
 
@@ -645,7 +984,16 @@ static void pen_shape(int N, int* rows, int* W)
 
 // The positions' unit is RadiusP / 2^20 or finer (domains up to about 1900
 // RadiusP wide); in wider ones the stored operator's records are closer to C.
-bool pen_applies(const mph_case* c) { return c->step_pairs && mixed_jacobi(c) && c->dp.fix_inv <= 1.0f / 1048576.0f; }
+// (The viscous pairs' separations hold MaxRadius below 16 RadiusP.)
+bool pen_applies(const mph_case* c)
+{
+    const DevParams& P = c->dp;
+    if (!(c->step_pairs && mixed_jacobi(c) && P.fix_inv <= 1.0f / 1048576.0f && P.maxR <= 16.0 * P.rP)) return false;
+    for (int t = 0; t < 2; ++t)
+        for (int u = 0; u < 2; ++u)
+            if (!(P.pen_vm[t][u] <= 1.0e30f)) return false;   // unit systems far outside FP32's range
+    return true;
+}
 
 template <typename T>
 static int grow_t(T** p, long long* cap, long long need)
@@ -663,26 +1011,20 @@ static int grow_t(T** p, long long* cap, long long need)
 static int pen_smem_t(const mph_case* c) { return c->pen_umax * (c->dim == 3 ? 24 : 16); }
 static int pen_smem_y(const mph_case* c) { return c->pen_umax * 16; }
 
-// Fixed-point positions and the P-lists' ranks of this step (after the
-// neighbour stage; c->pmax is the longest P-list).
-int launch_pen_lists(mph_case* c)
+// The P-lists' ranks of this step (c->pmax is the longest P-list).
+static int launch_pen_lists(mph_case* c)
 {
     DeviceState& d = c->d;
     const DevParams& P = c->dp;
     pen_shape(P.N, &c->pen_rows, &c->pen_w);
     c->pen_pw4 = (c->pmax + 3) / 4;
     const int nsl = (P.N + 31) / 32, nb = (int)grid_for(P.N, c->pen_rows), ucap = pen_ucap(c->pen_rows);
-    if (!d.ipos) {
-        MPH_CUDA(cudaMalloc((void**)&d.ipos, (size_t)P.N * sizeof(int4)));
+    if (!d.pgroups) {
         MPH_CUDA(cudaMalloc((void**)&d.pgroups, (size_t)nsl * sizeof(int)));
         MPH_CUDA(cudaMalloc((void**)&d.puniq, (size_t)nb * ucap * sizeof(int)));
         MPH_CUDA(cudaMalloc((void**)&d.pucount, (size_t)(nb + 4) * sizeof(int)));
     }
-    if (!d.tct32) MPH_CUDA(cudaMalloc((void**)&d.tct32, (size_t)(P.N + 1) * sizeof(float)));
     MPH_TRY(grow_t(&d.pidx, &d.cap_pidx, (long long)nsl * c->pen_pw4 * 32));
-    const unsigned g = grid_for(P.N, 256);
-    if (c->dim == 2) { k_fixed_positions<2><<<g, 256, 0, c->stream>>>(P, d.type, d.pos, d.ipos); MPH_COUNT_LAUNCH(); }
-    else { k_fixed_positions<3><<<g, 256, 0, c->stream>>>(P, d.type, d.pos, d.ipos); MPH_COUNT_LAUNCH(); }
     c->pen_umax = 0;
     c->loc_blocks[0] = 0;
     c->loc_blocks[1] = (int)grid_for(P.Nf, c->pen_rows);
@@ -711,6 +1053,108 @@ int launch_pen_lists(mph_case* c)
     c->loc_blocks[1] -= h[2];
     c->loc_cols = (long long)(unsigned)h[3];
     return MPH_OK;
+}
+
+// The assembly stage of the point-Jacobi mixed form: no blocks, no pair terms,
+// no slices and no transposed lists.
+int launch_pen_assemble(mph_case* c)
+{
+    DeviceState& d = c->d;
+    const DevParams& P = c->dp;
+    cudaStream_t st = c->stream;
+    const size_t n = (size_t)P.Nf * c->dim;
+    c->nslots = 0;
+    c->level0_done = c->ct_ready = false;
+    if (!d.ipos) MPH_CUDA(cudaMalloc((void**)&d.ipos, (size_t)P.N * sizeof(int4)));
+    if (!d.vpos) MPH_CUDA(cudaMalloc((void**)&d.vpos, (size_t)P.N * sizeof(int4)));
+    if (!d.z4) MPH_CUDA(cudaMalloc((void**)&d.z4, (size_t)P.Nf * 2 * sizeof(float4)));
+    if (!d.vacc) MPH_CUDA(cudaMalloc((void**)&d.vacc, n * sizeof(double)));
+    if (!d.v32) MPH_CUDA(cudaMalloc((void**)&d.v32, n * 8 * sizeof(float)));
+    if (!d.tct) MPH_CUDA(cudaMalloc((void**)&d.tct, (size_t)(P.N + 1) * sizeof(double)));
+    if (!d.tct32) MPH_CUDA(cudaMalloc((void**)&d.tct32, (size_t)(P.N + 1) * sizeof(float)));
+    if (!d.sdiag64) MPH_CUDA(cudaMalloc((void**)&d.sdiag64, (size_t)P.Nf * 8 * sizeof(double)));
+    MPH_TRY(grow_t(&d.cval, &d.cap_cval, c->nnbP * c->dim));
+    MPH_CUDA(cudaMemsetAsync(d.wrap32, 0, 2 * sizeof(int), st));
+    launch_vector_p(c);
+    const unsigned g = grid_for(P.N, 256), gs = grid_for(P.N, 128);
+    float* invD = d.v32 + 7 * n;
+    if (c->dim == 2) {
+        { k_fixed_positions<2><<<g, 256, 0, st>>>(P, d.type, d.pos, d.ipos, d.vpos, d.wrap32); MPH_COUNT_LAUNCH(); }
+        { k_pen_system<2><<<gs, 128, 0, st>>>(P, d.type, d.pos, d.vel, d.ncp, d.nptrP, d.nindP, d.pvec, d.cval, d.bvec, invD); MPH_COUNT_LAUNCH(); }
+    } else {
+        { k_fixed_positions<3><<<g, 256, 0, st>>>(P, d.type, d.pos, d.ipos, d.vpos, d.wrap32); MPH_COUNT_LAUNCH(); }
+        { k_pen_system<3><<<gs, 128, 0, st>>>(P, d.type, d.pos, d.vel, d.ncp, d.nptrP, d.nindP, d.pvec, d.cval, d.bvec, invD); MPH_COUNT_LAUNCH(); }
+    }
+    launch_wall_terms(c, nullptr, d.sdiag64, true);
+    return launch_pen_lists(c);
+}
+
+// D^-1 as a reader gets it (FP64 array), from the current step's lists and C
+int pen_exact_diag(mph_case* c)
+{
+    DeviceState& d = c->d;
+    const unsigned g = grid_for((long long)c->dp.Nf * 32, 256);
+    if (c->dim == 2) k_pen_diag<2><<<g, 256, 0, c->stream>>>(c->dp, d.type, d.pos, d.pos32, d.poslo32, d.nc, d.nptr, d.nind, d.ncp, d.nptrP, d.nindP, d.cval, d.wrap32 + 1, d.invDiag);
+    else k_pen_diag<3><<<g, 256, 0, c->stream>>>(c->dp, d.type, d.pos, d.pos32, d.poslo32, d.nc, d.nptr, d.nind, d.ncp, d.nptrP, d.nindP, d.cval, d.wrap32 + 1, d.invDiag);
+    MPH_COUNT_LAUNCH();
+    MPH_CUDA(cudaGetLastError());
+    return MPH_OK;
+}
+
+// the viscous pairs' sum, C^T x and the residual, after k_pen_pack
+template <int D, int L, bool FIRST>
+static void pen_residual(mph_case* c, double scale, const double* scale_src)
+{
+    DeviceState& d = c->d;
+    const DevParams& P = c->dp;
+    cudaStream_t st = c->stream;
+    { k_pen_visc<D, L, FIRST><<<grid_for((long long)P.Nf * L, 256), 256, 0, st>>>(P, d.vpos, d.nfc, d.nptr, d.nind, d.z4, d.wrap32, d.type,
+                                                                                d.pos, d.pos32, d.poslo32, scale, scale_src, d.vacc); MPH_COUNT_LAUNCH(); }
+    { k_pen_ct64<D><<<grid_for(P.N, 128), 128, 0, st>>>(P, d.type, d.ncp, d.nptrP, d.nindP, d.cval, d.x, d.tct); MPH_COUNT_LAUNCH(); }
+    { k_pen_resid<D><<<grid_for(P.Nf, 128), 128, 0, st>>>(P, d.type, d.nc, d.nfc, d.ncp, d.nptrP, d.nindP, d.cval, d.tct, d.sdiag64, d.vacc,
+                                                          d.x, d.bvec, d.r, d.partials, (unsigned*)(d.flags + kFlagCounter), d.scal + kSRR); MPH_COUNT_LAUNCH(); }
+}
+
+// lanes a row of k_pen_visc: about 180 neighbours in 3-D, 37 in 2-D
+constexpr int kVisc3 = 16, kVisc2 = 8;
+
+// r = b - A x of the start value
+void launch_pen_start_residual(mph_case* c)
+{
+    DeviceState& d = c->d;
+    const int Nf = c->dp.Nf;
+    if (c->dim == 2) {
+        { k_pen_pack<2, true><<<grid_for(Nf, 256), 256, 0, c->stream>>>(Nf, d.x, nullptr, 0.0, nullptr, nullptr, d.z4); MPH_COUNT_LAUNCH(); }
+        pen_residual<2, kVisc2, true>(c, 0.0, nullptr);
+    } else {
+        { k_pen_pack<3, true><<<grid_for(Nf, 256), 256, 0, c->stream>>>(Nf, d.x, nullptr, 0.0, nullptr, nullptr, d.z4); MPH_COUNT_LAUNCH(); }
+        pen_residual<3, kVisc3, true>(c, 0.0, nullptr);
+    }
+}
+
+// x += scale z and the residual after a phase
+void launch_pen_refine(mph_case* c, double scale, const double* scale_src, const int* flags)
+{
+    DeviceState& d = c->d;
+    const int Nf = c->dp.Nf;
+    const float* z = d.v32 + (size_t)Nf * c->dim;
+    if (c->dim == 2) {
+        { k_pen_pack<2, false><<<grid_for(Nf, 256), 256, 0, c->stream>>>(Nf, d.x, z, scale, scale_src, flags, d.z4); MPH_COUNT_LAUNCH(); }
+        pen_residual<2, kVisc2, false>(c, scale, scale_src);
+    } else {
+        { k_pen_pack<3, false><<<grid_for(Nf, 256), 256, 0, c->stream>>>(Nf, d.x, z, scale, scale_src, flags, d.z4); MPH_COUNT_LAUNCH(); }
+        pen_residual<3, kVisc3, false>(c, scale, scale_src);
+    }
+}
+
+void launch_pen_phase(mph_case* c, double inv_scale, const double* scale_src, double tol_in2, double tol_out2)
+{
+    DeviceState& d = c->d;
+    const int n = c->dp.Nf * c->dim;
+    float* v = d.v32;
+    { k_pen_phase<<<std::min<int>(grid_for(n, kReduceThreads), kReduceBlocks), kReduceThreads, 0, c->stream>>>(
+          n, d.r, v + 7 * (size_t)n, v + 2 * (size_t)n, v + (size_t)n, inv_scale, scale_src, tol_in2, tol_out2, d.scal, d.flags, d.partials,
+          (unsigned*)(d.flags + kFlagCounter)); MPH_COUNT_LAUNCH(); }
 }
 
 static PenArgs pen_args(const mph_case* c, int cap)

@@ -211,6 +211,12 @@ static int derive(mph_case* c, const mph_particles* parts)
         // the inner operator of the point-Jacobi form keeps 0.6 of a row's
         // viscous diagonal (fsum mu / dim) and leaves the rest, at most about
         // 0.7 of it, to the outer residual
+        P.vfix_scale = std::ldexp(1.0, 26) / P.rP;
+        P.pen_vk = (float)(1.0 / (P.rV * P.vfix_scale));
+        for (int t = 0; t < 2; ++t) {
+            P.pen_vd[t] = (float)(fsum * std::fabs(P.mu[t]) / c->dim);
+            for (int u = 0; u < 2; ++u) P.pen_vm[t][u] = (float)(P.visc * P.muij[t][u] * (-P.kfv * P.m2h_rv) * P.vfix_scale);
+        }
         for (int t = 0; t < kTypeCount; ++t) P.pen_diag32[t] = (float)(P.inert64[t] + 0.6 * fsum * std::fabs(P.mu[t]) / c->dim);
         c->pen_tol = 0.7 * fsum * mu_max / c->dim / (rho_min / P.dt);
     }
@@ -362,7 +368,7 @@ int case_alloc_particles(mph_case* c)
     MPH_TRY(dalloc(c, &d.poslo32, N * VSn));
     if (c->dim == 2) MPH_TRY(dalloc(c, &d.pt32, N));
     else d.pt32 = reinterpret_cast<float4*>(d.pos32);   // its w holds the type bits
-    MPH_TRY(dalloc(c, &d.wrap32, 1));
+    MPH_TRY(dalloc(c, &d.wrap32, 2));
     MPH_TRY(dalloc(c, &d.type, N));
     MPH_TRY(dalloc(c, &d.id, N));
     MPH_TRY(dalloc(c, &d.type_alt, N));
@@ -719,7 +725,7 @@ int case_destroy(mph_case* c)
                     (void*)d.tct32, (void*)d.pes32, (void*)d.sdiag32, (void*)d.sdiag64, (void*)d.cvl32, (void*)d.psptr, (void*)d.ctsptr,
                     (void*)d.pswidth, (void*)d.ctswidth, (void*)d.pscol, (void*)d.ctscol, (void*)d.psval, (void*)d.ctsval,
                     (void*)d.grec16, (void*)d.grec32, (void*)d.pscale, (void*)d.lcol16, (void*)d.uniq, (void*)d.ucount,
-                    (void*)d.ctuniq, (void*)d.ctucount, (void*)d.ipos, (void*)d.pidx, (void*)d.pgroups, (void*)d.puniq, (void*)d.pucount, (void*)d.wkey, (void*)d.wval, (void*)d.ccell,
+                    (void*)d.ctuniq, (void*)d.ctucount, (void*)d.ipos, (void*)d.vpos, (void*)d.z4, (void*)d.vacc, (void*)d.pidx, (void*)d.pgroups, (void*)d.puniq, (void*)d.pucount, (void*)d.wkey, (void*)d.wval, (void*)d.ccell,
                     (void*)d.io3, (void*)d.vprev, (void*)d.vprev_alt, (void*)d.sort_cnt, (void*)d.sort_off, d.scan_tmp})
         if (p) cudaFree(p);
     for (auto& p : c->prof.pending) {
@@ -787,6 +793,17 @@ int case_profile(mph_case* c, int enable)
 int case_profile_read(mph_case* c, double* out, int n)
 {
     MPH_TRY(prof_collect(c));
+    // the point-Jacobi mixed form builds no slices: the count they would have
+    if (c->step_pen && c->nslots == 0) {
+        std::vector<int> nfc(c->dp.Nf);
+        MPH_CUDA(cudaMemcpyAsync(nfc.data(), c->d.nfc, nfc.size() * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        MPH_CUDA(cudaStreamSynchronize(c->stream));
+        for (int i = 0; i < c->dp.Nf; i += 32) {
+            int m = 0;
+            for (int k = i; k < std::min(i + 32, c->dp.Nf); ++k) m = std::max(m, nfc[k]);
+            c->nslots += 32 * ((m + 3) / 4 * 4);
+        }
+    }
     std::vector<double> v;
     for (int k = 0; k < 7; ++k) v.push_back(c->prof.stage_ms[k]);
     for (int k = 0; k < kProfKernels; ++k) v.push_back(c->prof.kern_ms[k]);

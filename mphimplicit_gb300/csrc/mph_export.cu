@@ -80,7 +80,10 @@ static int build_export(mph_case* c, const std::string& name, Out& o)
     if (name == "VirialStressAtParticle") return f64(d.virS, (size_t)N * 9);
     if (name == "VectorP") return f64(d.pvec, N);
     if (name == "VectorB") return f64(d.bvec, (size_t)Nf * D);
-    if (name == "InvDiagA") return f64(d.invDiag, (size_t)Nf * D);
+    if (name == "InvDiagA") {
+        if (c->step_pen) MPH_TRY(pen_exact_diag(c));   // the step itself keeps the FP32 D^-1 with the lattice's viscous part
+        return f64(d.invDiag, (size_t)Nf * D);
+    }
     if (name == "CellFluidParticleBegin" || name == "CellFluidParticleEnd" || name == "CellWallParticleBegin" ||
         name == "CellWallParticleEnd") {
         std::vector<int> b;
@@ -117,8 +120,14 @@ static int build_export(mph_case* c, const std::string& name, Out& o)
         std::vector<long long> sptr;
         std::vector<double> aval;
         MPH_TRY(d2h(c, nfc, d.nfc, Nf));
-        MPH_TRY(d2h(c, sptr, d.sptr, (size_t)c->nslices + 1));
-        MPH_TRY(d2h(c, acol, d.acol, (size_t)c->nslots));
+        std::vector<long long> nptr;
+        if (c->step_pen) {   // no slices: a row's columns are the fluid part of its neighbour list
+            MPH_TRY(d2h(c, nptr, d.nptr, (size_t)Nf + 1));
+            if (name == "CsrIndA") MPH_TRY(d2h(c, acol, d.nind, (size_t)nptr[Nf]));
+        } else {
+            MPH_TRY(d2h(c, sptr, d.sptr, (size_t)c->nslices + 1));
+            MPH_TRY(d2h(c, acol, d.acol, (size_t)c->nslots));
+        }
         if (name == "CsrCofA" && c->step_factored) {
             // mixed form with the factored FP64 operator: only FP32 blocks exist
             std::vector<float> a32;
@@ -140,12 +149,12 @@ static int build_export(mph_case* c, const std::string& name, Out& o)
         if (o.kind == 0) o.i32.resize(nnz); else o.f64.resize(nnz);
         long long w = 0;
         for (int i = 0; i < Nf; ++i) {
-            const long long base = sptr[i >> 5];
+            const long long base = c->step_pen ? nptr[i] : sptr[i >> 5];
             const int lane = i & 31;
             for (int r = 0; r < D; ++r)
                 for (int k = 0; k < nfc[i]; ++k)
                     for (int s = 0; s < D; ++s, ++w) {
-                        if (o.kind == 0) o.i32[w] = D * acol[base + (long long)k * 32 + lane] + s;
+                        if (o.kind == 0) o.i32[w] = D * acol[c->step_pen ? base + k : base + (long long)k * 32 + lane] + s;
                         else o.f64[w] = aval[base * D * D + ((long long)k * D * D + r * D + s) * 32 + lane];
                     }
         }

@@ -68,6 +68,9 @@ struct DevParams {
     double fix_scale;                          // fixed-point positions: units a length (2^e / RadiusP), 2^-e, and the
     float fix_inv;                             // domain's width and half width in units
     int fix_w[3], fix_h[3];
+    double vfix_scale;                         // the same for the viscous pairs: 2^26 / RadiusP, modulo 2^32
+    float pen_vm[2][2], pen_vk, pen_vd[2];     // visc mu_ij w' and 1/RadiusV of the fluid pairs in those units; the lattice's
+                                               // viscous diagonal of a fluid row
     float pen_diag32[kTypeCount];              // inner operator of the point-Jacobi form: its diagonal, lambda kfp 2/RadiusP,
     float pen_lam32[kTypeCount], pen_w32;      // and kfp 2/RadiusP
     int exact_only;                            // 1: skip the FP32 pre-classification
@@ -172,6 +175,9 @@ struct DeviceState {
     // slice, the row blocks' distinct columns and their counts (statistics
     // after the blocks)
     int4* ipos = nullptr;
+    int4* vpos = nullptr;
+    float4* z4 = nullptr;              // the solution or its last correction, a record a row (two where it is in two floats)
+    double* vacc = nullptr;            // viscous fluid pairs of A x, added up over the refinement phases
     uint2* pidx = nullptr;
     long long cap_pidx = 0;
     int *pgroups = nullptr, *puniq = nullptr, *pucount = nullptr;
@@ -402,6 +408,8 @@ void launch_density_full(mph_case* c);
 void ensure_density_a(mph_case* c);
 void launch_output_fields(mph_case* c);
 int launch_assemble(mph_case* c);
+void launch_vector_p(mph_case* c);
+void launch_wall_terms(mph_case* c, float* sdiag32, double* sdiag64, bool wall_rows_only);
 int launch_assemble_cells(mph_case* c, int kmax_rows, bool mix, bool* done);
 int build_ct(mph_case* c);
 bool factored_applies(const mph_case* c);
@@ -411,7 +419,11 @@ bool factored_applies(const mph_case* c);
 // its block index inside the case, so each case's arithmetic, and its
 // reductions' order, are the single-case launch's)
 bool pen_applies(const mph_case* c);
-int launch_pen_lists(mph_case* c);
+int launch_pen_assemble(mph_case* c);
+int pen_exact_diag(mph_case* c);
+void launch_pen_start_residual(mph_case* c);
+void launch_pen_refine(mph_case* c, double scale, const double* scale_src, const int* flags);
+void launch_pen_phase(mph_case* c, double inv_scale, const double* scale_src, double tol_in2, double tol_out2);
 void launch_pen_operator(mph_case* c, int cap);
 void launch_pen_vectors(mph_case* c, int cap, bool use_cond, cudaGraphConditionalHandle cond);
 size_t batch_pen_bytes();

@@ -135,6 +135,31 @@ __device__ __forceinline__ bool reduce_finalize_step(T v, double* __restrict__ p
     return reduce_finalize_step(v, partials, counter, out, it, (int)blockIdx.x, (int)gridDim.x);
 }
 
+// As reduce_finalize; returns true in thread 0 of the last block, after the store.
+template <typename T>
+__device__ __forceinline__ bool reduce_finalize_last(T v, double* __restrict__ partials, unsigned* __restrict__ counter,
+                                                     double* __restrict__ out)
+{
+    __shared__ bool last;
+    const double bs = block_sum(v);
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x] = bs;
+        __threadfence();
+        last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    double s = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) s += __ldcg(partials + b);
+    s = block_sum(s);
+    if (threadIdx.x == 0) {
+        *out = s;
+        *counter = 0u;
+    }
+    return threadIdx.x == 0;
+}
+
 // The case of launch block b: the last case whose first block is <= b (b0:
 // ncases + 1 block starts; a case without blocks is never found).
 __device__ __forceinline__ int batch_case_of(const int* __restrict__ b0, int ncases, int b)
