@@ -753,10 +753,14 @@ struct MixedRun {
         MPH_CUDA(cudaMemcpyAsync(hs, scal, sizeof(hs), cudaMemcpyDeviceToHost, st));
         MPH_CUDA(cudaMemcpyAsync(host_flags, flags, sizeof(host_flags), cudaMemcpyDeviceToHost, st));
         MPH_CUDA(cudaStreamSynchronize(st));
-        if (!(hs[kSRR] == hs[kSRR])) {
+        if (host_flags[kFlagStall]) return fail(MPH_ERR_CUDA, "the resident CR iteration's grid barrier ran out of time");
+        if (!(hs[kSRR] == hs[kSRR]) || (c->pen_resident && c->step_pen && host_flags[kFlagBad])) {
             bad = true;
             return MPH_OK;
         }
+        // a resident launch that ended at its iteration bound goes on in the
+        // same phase
+        if (c->step_pen && c->pen_resident && outer > 0 && !host_flags[kFlagDone]) --outer;
         if (hs[kSRR] / hs[kSRR0] < tol_out2 || outer >= c->max_outer || hs[kSRR] == 0.0) return MPH_OK;
         if (outer > 0 && host_flags[kFlagIter] >= cap) return MPH_OK;
         if (outer == 0) scale = std::sqrt(hs[kSRR]);
@@ -811,7 +815,7 @@ static int mixed_solve_t(mph_case* c)
 {
     using V = float;
     MPH_TRY(mixed_prepare(c));
-    if (c->device_loop && c->use_graphs && !c->prof.on) {
+    if (c->device_loop && c->use_graphs && !c->prof.on && !(c->step_pen && c->pen_resident)) {
         if (c->extrapolate && !c->d.vprev) {
             const size_t nvs0 = (size_t)c->dp.N * (D == 2 ? 2 : 4);
             MPH_CUDA(cudaMalloc((void**)&c->d.vprev, 2 * nvs0 * sizeof(double)));
@@ -871,6 +875,23 @@ static int mixed_solve_t(mph_case* c)
         }
         { k_xrs32<V, false><<<rb, kReduceThreads, 0, st>>>(n, z32, r32, s32, p32, q32, u32, scal, flags, part, counter); MPH_COUNT_LAUNCH(); }
     };
+    if (c->step_pen && c->pen_resident) {
+        // one launch a phase, and one read of the solve's state before each;
+        // with profiling on an event pair a phase counts for its iterations
+        for (;;) {
+            bool go = false;
+            const int it0 = host_flags[kFlagIter];
+            MPH_TRY(run.phase(&go));
+            if (c->prof.on && host_flags[kFlagIter] > it0) c->prof.kern_n[0] += host_flags[kFlagIter] - it0 - 1;   // the pair itself counts one
+            if (!go) break;
+            cudaEvent_t e0 = nullptr;
+            const int pon = prof_begin(c, 0, &e0);
+            MPH_TRY(launch_pen_resident(c, cap));
+            if (pon) prof_end(c, 0, e0);
+            launch_pen_refine(c, run.scale, nullptr, flags);
+        }
+        return run.finish();
+    }
     const int chunk = c->chunk;
     const bool graphs = c->use_graphs;
     // with profiling on, the captured chunk records a fixed event pair around
@@ -952,7 +973,7 @@ static int mixed_solve_t(mph_case* c)
 bool batch_solve_eligible(const mph_case* c)
 {
     return c->batch_solve && c->precision == MPH_PRECISION_MIXED && c->stage == 6 && c->step_pairs && mixed_jacobi(c) &&
-           c->step_pen && !c->device_loop && !c->prof.on && c->dp.Nf > 0 && c->nslices > 0;
+           c->step_pen && !c->pen_resident && !c->device_loop && !c->prof.on && c->dp.Nf > 0 && c->nslices > 0;
 }
 
 // The batched solve's device table, flag buffers, stream and events, per

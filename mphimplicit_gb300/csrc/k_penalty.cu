@@ -53,7 +53,11 @@ constexpr int kSAlpha = 25, kSBeta = 26, kSQUPrev = 27;   // this iteration's al
 __device__ __forceinline__ int rho_slot32(int it) { return 20 + (it & 1); }
 
 constexpr int kPlWords = 1 << 13;   // bitmap of a row block's columns: 2^18 particles, fluid and wall window together
-constexpr int kMaxPenRows = 256;   // threads of a row block (rows times threads a row)
+constexpr int kMaxPenRows = 256;   // threads of a row block (rows times threads a row) of the per-iteration kernels
+constexpr int kCrThreads = 512;    // of the resident iteration's blocks, two an SM
+constexpr int kCrBlocks = 2 * 152;
+constexpr int kCrMinRows = 192;    // rows a block at least (a solve of 15,000 particles: 2.01, 1.89, 2.00 ms with 128, 192, 256)
+constexpr int kCrSmem = 100 * 1024;   // dynamic: two blocks an SM with their 7 KB of static shared memory
 // Staged neighbours a block of `rows` rows has room for.  Blocks of a
 // 3.5-spacing cell order have about 2.8 (256 rows) to 3.9 (64) times their
 // rows of them, against some 20 slots a row; one with more (a solve of 211
@@ -101,7 +105,7 @@ __device__ __forceinline__ bool may_wrap(int w) { return (w & (w >> 3) & 7) != 0
 // two index windows, the fluid particles' and the walls' (walls follow the
 // fluid in the order).  ucount[block] = U, or -1 where the windows or U are
 // too large.
-__global__ void __launch_bounds__(kMaxPenRows) k_plist_ranks(int N, int Nf, int pw4, int ucap, const int* __restrict__ ncp,
+__global__ void __launch_bounds__(kCrThreads) k_plist_ranks(int N, int Nf, int pw4, int ucap, const int* __restrict__ ncp,
                                                              const long long* __restrict__ nptrP, const int* __restrict__ nindP,
                                                              uint2* __restrict__ idx, int* __restrict__ groups,
                                                              int* __restrict__ uniq, int* __restrict__ ucount)
@@ -650,6 +654,461 @@ __global__ void __launch_bounds__(kReduceThreads) k_pen_vec(PenArgs A, int n, in
     pen_vec_body<COND>(A, (int)blockIdx.x, (int)gridDim.x, n, use_cond, cond);
 }
 
+// ---- the resident iteration -----------------------------------------------------------
+// All CR iterations of a refinement phase in one cooperative kernel, for the
+// cases whose rows fit the chip at once (up to 155,648 particles).  Such a
+// case's iteration is not bound by anything a kernel does but by three
+// launches, their load chains and their last-block reductions (19 us on 15,000
+// particles, 33 on 126,000; resident 9 and 22, there bound by the conflicts of
+// the shared-memory gathers).  Here a block keeps its rows' neighbours' positions and ranks in
+// shared memory and its vectors in registers for the whole phase, and an
+// iteration crosses the grid's barrier twice:
+//
+//   after t    lambda t of every particle, and (r, r) of the vectors it came from
+//   after y    s, D^-1 y and D^-1 q of every row, and the dot products
+//
+// With alpha and beta known (every block adds the blocks' sums in the same
+// order) a block forms the new s of its own rows and of its staged neighbours
+// alike, s - alpha (D^-1 y + beta D^-1 q), so the new s needs no barrier of
+// its own.
+//
+// The sums across warps and blocks are in two floats (48 bits): an FP64
+// addition takes this part some hundred clocks, and the chain of them took 4
+// us an iteration; a warp's own terms are summed in FP32 as elsewhere.
+//
+// All blocks are resident (cooperative launch), so a wait ends; it is bounded
+// all the same, and a block whose wait runs out raises kFlagStall and leaves,
+// as the others then do.  A launch runs at most kCrMaxIter iterations.
+constexpr int kCrMaxIter = 4096;
+constexpr int kCrSpin = 1 << 21;
+
+struct PenCr {
+    float4* rec;                   // per row 3 records: s, a = D^-1 y, b = D^-1 q
+    float *v3, *v1;                // the blocks' (s, y), (y, a), (y, b) in two floats each; (r, r)
+    unsigned* count;               // arrivals of this launch's crossings
+};
+
+// two-float arithmetic (D. E. Knuth's two-sum; T. J. Dekker)
+struct F2 { float h, l; };
+__device__ __forceinline__ F2 f2_fast(float h, float l)   // |h| >= |l|
+{
+    const float s = __fadd_rn(h, l);
+    return {s, __fadd_rn(l, -__fadd_rn(s, -h))};
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b)
+{
+    const float s = __fadd_rn(a.h, b.h), t = __fadd_rn(s, -a.h);
+    const float e = __fadd_rn(__fadd_rn(a.h, -__fadd_rn(s, -t)), __fadd_rn(b.h, -t));
+    return f2_fast(s, __fadd_rn(e, __fadd_rn(a.l, b.l)));
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b)
+{
+    const float p = __fmul_rn(a.h, b.h);
+    return f2_fast(p, __fadd_rn(__fmaf_rn(a.h, b.h, -p), __fmaf_rn(a.h, b.l, __fmul_rn(a.l, b.h))));
+}
+__device__ __forceinline__ F2 f2_div(F2 a, F2 b)
+{
+    const float q = __fdiv_rn(a.h, b.h);
+    const float r = __fadd_rn(__fmaf_rn(-q, b.h, a.h), __fmaf_rn(-q, b.l, a.l));
+    return f2_fast(q, __fdiv_rn(r, b.h));
+}
+__device__ __forceinline__ F2 f2_of(double v)
+{
+    const float h = (float)v;
+    return {h, (float)(v - (double)h)};
+}
+__device__ __forceinline__ F2 f2_warp_sum(F2 v, int from)
+{
+    for (int o = from; o > 0; o >>= 1)
+        v = f2_add(v, F2{__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o)});
+    return v;
+}
+
+// The grid's crossing number `epoch`: this block's nv values (mine, shared
+// memory) are out, and whatever the block's threads wrote before it can be
+// read (through L2) by every block after it.  The arrivals are counted (the
+// count only grows during a launch) and one thread a block waits for them; a
+// word per block and value that every block polls instead was slower (nb^2
+// polls).
+__device__ __forceinline__ bool cr_cross(unsigned* count, float* vals, const float* mine, int nv, unsigned epoch, int lb, int nb, int tid,
+                                         int* flags)
+{
+    __shared__ int ok_s;
+    __syncthreads();
+    if (tid < 32) {
+        if (tid < nv) vals[(size_t)lb * nv + tid] = mine[tid];
+        __syncwarp();
+        if (tid == 0) {
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+            const unsigned target = epoch * (unsigned)nb;
+            unsigned v = 0;
+            int n = 0;
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+            } while ((int)(v - target) < 0 && ++n < kCrSpin);
+            ok_s = (int)(v - target) >= 0;
+            if (!ok_s) flags[kFlagStall] = 1;
+        }
+    }
+    __syncthreads();
+    return ok_s != 0;
+}
+
+// the sum over the blocks of one two-float value (stride: floats a block), by one warp
+__device__ __forceinline__ F2 cr_sum(const float* vals, int stride, int nb, int lane)
+{
+    constexpr int K = (kCrBlocks + 31) / 32;
+    float2 v[K];
+#pragma unroll
+    for (int u = 0; u < K; ++u) {
+        const int k = lane + 32 * u;
+        v[u] = k < nb ? __ldcg(reinterpret_cast<const float2*>(vals + (size_t)k * stride)) : make_float2(0.f, 0.f);
+    }
+    F2 s{v[0].x, v[0].y};
+#pragma unroll
+    for (int u = 1; u < K; ++u)
+        if (32 * u < nb) s = f2_add(s, F2{v[u].x, v[u].y});
+    return f2_warp_sum(s, 16);
+}
+
+// the new s of a row, own or staged: the same two operations everywhere
+__device__ __forceinline__ float cr_new_s(float s, float a, float b, float alpha, float beta)
+{
+    return __fmaf_rn(-alpha, __fmaf_rn(beta, b, a), s);
+}
+
+// a row's published records (zeros for a wall), and the new s from them
+struct CrRec { float4 r[3]; };
+template <int D>
+__device__ __forceinline__ CrRec cr_load(const float4* rec, int j, int Nf)
+{
+    CrRec R;
+    R.r[0] = R.r[1] = R.r[2] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (j >= 0 && j < Nf) {
+#pragma unroll
+        for (int u = 0; u < D; ++u) R.r[u] = __ldcg(rec + 3 * (size_t)j + u);
+    }
+    return R;
+}
+template <int D>
+__device__ __forceinline__ void cr_combine(const CrRec& R, float alpha, float beta, float* v)
+{
+    if (D == 3) {
+        v[0] = cr_new_s(R.r[0].x, R.r[1].x, R.r[2].x, alpha, beta);
+        v[1] = cr_new_s(R.r[0].y, R.r[1].y, R.r[2].y, alpha, beta);
+        v[2] = cr_new_s(R.r[0].z, R.r[1].z, R.r[2].z, alpha, beta);
+    } else {   // s, a in the first record
+        v[0] = cr_new_s(R.r[0].x, R.r[0].z, R.r[1].x, alpha, beta);
+        v[1] = cr_new_s(R.r[0].y, R.r[0].w, R.r[1].y, alpha, beta);
+        v[2] = 0.f;
+    }
+}
+
+template <int D>
+__device__ __forceinline__ void cr_publish(float4* rec, int i, const float* s, const float* a, const float* b)
+{
+    if (D == 3) {
+        rec[3 * (size_t)i] = make_float4(s[0], s[1], s[2], 0.f);
+        rec[3 * (size_t)i + 1] = make_float4(a[0], a[1], a[2], 0.f);
+        rec[3 * (size_t)i + 2] = make_float4(b[0], b[1], b[2], 0.f);
+    } else {
+        rec[3 * (size_t)i] = make_float4(s[0], s[1], a[0], a[1]);
+        rec[3 * (size_t)i + 1] = make_float4(b[0], b[1], 0.f, 0.f);
+    }
+}
+
+template <int D>
+__global__ void __launch_bounds__(kCrThreads, 2) k_pen_cr(DevParams P, PenArgs A, PenCr C)
+{
+    extern __shared__ int4 pen_smem[];
+    __shared__ float wred[3][kCrThreads / 32];
+    __shared__ float part[kCrThreads * D];
+    __shared__ F2 sum_s[3];
+    __shared__ float val_s[6];
+    __shared__ float ab_s[2];
+    __shared__ F2 rr_s;
+    __shared__ int stop_s;
+    const int rows = blockDim.x, W = blockDim.y, w = threadIdx.y;
+    const int tid = w * rows + threadIdx.x, nth = rows * W, lane = tid & 31, warp = tid >> 5;
+    const int lb = blockIdx.x, nb = gridDim.x;
+    const int i = lb * rows + threadIdx.x;
+    unsigned epoch = 0;
+    int4* sa = pen_smem;                                                 // position, and s (2-D) or its first component
+    float2* sb = reinterpret_cast<float2*>(pen_smem + A.umax);           // 3-D: the other two
+    float* st = reinterpret_cast<float*>(sb + (D == 3 ? A.umax : 0));    // lambda t
+    int* ul = reinterpret_cast<int*>(st + A.umax);                       // the staged columns
+    uint2* words = reinterpret_cast<uint2*>(ul + A.umax);                // the rows' ranks, word by word
+    const bool wrap = may_wrap(*A.wrap);
+    // what the phase keeps
+    const int U = A.ucount ? A.ucount[lb] : -1;
+    const int n = i < A.N ? A.ncp[i] : 0;
+    for (int k = tid; k < U; k += nth) {
+        const int j = A.uniq[(size_t)lb * A.ucap + k];
+        ul[k] = j;
+        sa[k] = A.ipos[j];
+    }
+    const int j0 = tid < U ? ul[tid] : -1;   // the thread's first staged neighbour
+    int ng = 0;
+    if (U >= 0 && n > 0) {
+        ng = A.groups[i >> 5];
+        const uint2* ip = A.idx + ((long long)(i >> 5) * A.pw4) * 32 + (i & 31);
+        for (int g = w; g < ng; g += W) words[(size_t)g * rows + threadIdx.x] = ip[(long long)g * 32];
+    }
+    const int4 pi = i < A.N ? A.ipos[i] : make_int4(0, 0, 0, 0);
+    const int um[3] = {pi.x - kMagic, pi.y - kMagic, pi.z - kMagic};
+    const bool fluid = i < A.Nf, mine = w == 0 && fluid;
+    int it = A.flags[kFlagIter];
+    const int it_end = it + kCrMaxIter;
+    const F2 stop_rr = f2_of(A.scal[kSTol2] * A.scal[kSIn0]);
+    // thread 0's: (s, y) and (q, D^-1 q) of the last iteration
+    F2 rho = f2_of(A.scal[rho_slot32(it - 1)]), qu = f2_of(A.scal[kSQUPrev]);
+    const float m = P.pen_diag32[pi.w], lam = P.pen_lam32[pi.w];
+    float s[3] = {0.f, 0.f, 0.f}, a[3] = {0.f, 0.f, 0.f}, b[3] = {0.f, 0.f, 0.f};
+    float p[3] = {0.f, 0.f, 0.f}, z[3] = {0.f, 0.f, 0.f}, dv[3] = {0.f, 0.f, 0.f};
+    if (mine) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            const size_t k = (size_t)i * D + d;
+            s[d] = A.s[k];
+            z[d] = A.z[k];
+            dv[d] = A.invD[k];
+            if (it > 0) {
+                p[d] = A.p[k];
+                b[d] = A.q[k];   // D^-1 q, as this kernel leaves it
+            }
+        }
+        const float zero[3] = {0.f, 0.f, 0.f};
+        cr_publish<D>(C.rec, i, s, zero, zero);
+    }
+    // the row's slots: staged records by rank, or columns
+    auto slots = [&](auto&& term) {
+        if (U >= 0) {
+            for (int g = w; g < ng; g += W) {
+                const uint2 v = words[(size_t)g * rows + threadIdx.x];
+                term((int)(v.x & 0xffffu));
+                term((int)(v.x >> 16));
+                term((int)(v.y & 0xffffu));
+                term((int)(v.y >> 16));
+            }
+        } else {
+            const int* col = A.nindP + (i < A.N ? A.nptrP[i] : 0);
+            for (int g = w; 4 * g < n; g += W)
+                for (int k = 4 * g; k < min(n, 4 * g + 4); ++k) term(col[k]);
+        }
+    };
+    float alpha = 0.f, beta = 0.f;
+    bool first = true;
+    if (tid < 6) val_s[tid] = 0.f;
+    bool ok = cr_cross(C.count, C.v3, val_s, 6, ++epoch, lb, nb, tid, A.flags);   // every row's s is out
+    // a crossing's first loads: the thread's first neighbour's records, while
+    // alpha and beta are formed
+    CrRec pre = cr_load<D>(C.rec, j0, A.Nf);
+    while (ok) {
+        // the new vectors of the own row (not before the phase's first iteration)
+        if (!first) {
+            float rs = 0.f;
+            if (mine) {
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    p[d] = beta * p[d] + s[d];
+                    z[d] += alpha * p[d];
+                    s[d] = cr_new_s(s[d], a[d], b[d], alpha, beta);
+                    b[d] = __fmaf_rn(beta, b[d], a[d]);
+                    const float r = dv[d] != 0.f ? __fdividef(s[d], dv[d]) : 0.f;
+                    rs += r * r;
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o);
+            if (lane == 0) wred[0][warp] = rs;
+            ++it;
+        }
+        // the new s of the staged neighbours
+        auto put = [&](int k, const CrRec& R) {
+            float v[3];
+            cr_combine<D>(R, alpha, beta, v);
+            if (D == 3) {
+                sa[k].w = __float_as_int(v[0]);
+                sb[k] = make_float2(v[1], v[2]);
+            } else {
+                sa[k].z = __float_as_int(v[0]);
+                sa[k].w = __float_as_int(v[1]);
+            }
+        };
+        if (tid < U) put(tid, pre);
+#pragma unroll 2
+        for (int k = tid + nth; k < U; k += nth) put(k, cr_load<D>(C.rec, ul[k], A.Nf));
+        float si[3] = {s[0], s[1], s[2]};
+        if (W > 1 && w > 0 && fluid && n > 0) cr_combine<D>(cr_load<D>(C.rec, i, A.Nf), alpha, beta, si);
+        __syncthreads();
+        if (!first && warp == 0) {
+            const F2 v = f2_warp_sum(F2{lane < (nth >> 5) ? wred[0][lane] : 0.f, 0.f}, 8);
+            if (lane == 0) {
+                val_s[0] = v.h;
+                val_s[1] = v.l;
+            }
+        }
+        // lambda t
+        float acc = 0.f;
+        if (n > 0) {
+            auto sum = [&](auto WR) {
+                auto one = [&](const int* uj, const float* sj) {
+                    float dq[3];
+                    const float cf = pen_coef<D, decltype(WR)::value>(P, um, uj, dq);
+                    float dot = __fmul_rn(dq[0], __fadd_rn(si[0], -sj[0]));
+                    dot = __fmaf_rn(dq[1], __fadd_rn(si[1], -sj[1]), dot);
+                    if (D == 3) dot = __fmaf_rn(dq[2], __fadd_rn(si[2], -sj[2]), dot);
+                    acc = __fmaf_rn(cf, dot, acc);
+                };
+                slots([&](int k) {
+                    if (U >= 0) {
+                        const int4 pj = sa[k];
+                        const int uj[3] = {pj.x, pj.y, pj.z};
+                        if (D == 3) {
+                            const float2 v = sb[k];
+                            const float sj[3] = {__int_as_float(pj.w), v.x, v.y};
+                            one(uj, sj);
+                        } else {
+                            const float sj[3] = {__int_as_float(pj.z), __int_as_float(pj.w), 0.f};
+                            one(uj, sj);
+                        }
+                    } else {
+                        const int4 pj = A.ipos[k];
+                        const int uj[3] = {pj.x, pj.y, pj.z};
+                        float sj[3];
+                        cr_combine<D>(cr_load<D>(C.rec, k, A.Nf), alpha, beta, sj);
+                        one(uj, sj);
+                    }
+                });
+            };
+            if (wrap) sum(std::true_type());
+            else sum(std::false_type());
+        }
+        float ti = acc;
+        if (W > 1) {   // the row's partial sums in the order of w
+            part[tid] = acc;
+            __syncthreads();
+            ti = part[threadIdx.x];
+            for (int v = 1; v < W; ++v) ti += part[v * rows + threadIdx.x];
+        }
+        ti = n > 0 ? lam * ti : 0.f;
+        if (w == 0 && i < A.N) A.t[i] = ti;
+        // every particle's lambda t (and every block's (r, r)) is out
+        if (!(ok = cr_cross(C.count, C.v1, val_s, 2, ++epoch, lb, nb, tid, A.flags))) break;
+        if (!first && warp == (nth >> 5) - 1) {   // the stop test
+            const F2 v = cr_sum(C.v1, 2, nb, lane);
+            if (lane == 0) {
+                const bool bad = !(v.h == v.h);
+                const bool below = __fadd_rn(__fadd_rn(v.h, -stop_rr.h), __fadd_rn(v.l, -stop_rr.l)) < 0.f;
+                rr_s = v;
+                stop_s = (it >= A.cap || below || bad) ? (bad ? 3 : 1) : (it >= it_end ? 2 : 0);
+            }
+        }
+#pragma unroll 2
+        for (int k = tid; k < U; k += nth) st[k] = __ldcg(A.t + ul[k]);
+        __syncthreads();
+        if (!first && stop_s) break;   // the same in every block
+        first = false;
+        // y = M s
+        float y[3] = {0.f, 0.f, 0.f};
+        if (fluid && n > 0) {
+            auto sum = [&](auto WR) {
+                auto one = [&](const int* uj, float tj) {
+                    float dq[3];
+                    const float cf = __fmul_rn(pen_coef<D, decltype(WR)::value>(P, um, uj, dq), __fadd_rn(tj, ti));
+#pragma unroll
+                    for (int d = 0; d < D; ++d) y[d] = __fmaf_rn(cf, dq[d], y[d]);
+                };
+                slots([&](int k) {
+                    const int4 pj = U >= 0 ? sa[k] : A.ipos[k];
+                    const int uj[3] = {pj.x, pj.y, pj.z};
+                    one(uj, U >= 0 ? st[k] : __ldcg(A.t + k));
+                });
+            };
+            if (wrap) sum(std::true_type());
+            else sum(std::false_type());
+        }
+        if (W > 1) {
+#pragma unroll
+            for (int d = 0; d < D; ++d) part[tid * D + d] = y[d];
+            __syncthreads();
+            if (w == 0)
+                for (int v = 1; v < W; ++v)
+#pragma unroll
+                    for (int d = 0; d < D; ++d) y[d] += part[(v * rows + threadIdx.x) * D + d];
+        }
+        float v[3] = {0.f, 0.f, 0.f};
+        if (mine) {
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                y[d] = __fmaf_rn(m, s[d], __fmul_rn(P.pen_w32, y[d]));
+                a[d] = dv[d] * y[d];
+                v[0] += s[d] * y[d];
+                v[1] += a[d] * y[d];
+                v[2] += b[d] * y[d];
+            }
+            cr_publish<D>(C.rec, i, s, a, b);
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
+            if (lane == 0) wred[c][warp] = v[c];
+        }
+        __syncthreads();
+        if (warp < 3) {
+            const F2 x = f2_warp_sum(F2{lane < (nth >> 5) ? wred[warp][lane] : 0.f, 0.f}, 8);
+            if (lane == 0) {
+                val_s[2 * warp] = x.h;
+                val_s[2 * warp + 1] = x.l;
+            }
+        }
+        // every row's s, a, b and every block's dot products are out
+        if (!(ok = cr_cross(C.count, C.v3, val_s, 6, ++epoch, lb, nb, tid, A.flags))) break;
+        pre = cr_load<D>(C.rec, j0, A.Nf);
+        if (warp < 3) {
+            const F2 v = cr_sum(C.v3 + 2 * warp, 6, nb, lane);
+            if (lane == 0) sum_s[warp] = v;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            const F2 x[3] = {sum_s[0], sum_s[1], sum_s[2]};
+            // beta = rho / rho', (q, D^-1 q) = (y, a) + beta (2 (y, b) + beta (q', D^-1 q')), alpha = rho / (q, D^-1 q)
+            F2 be{0.f, 0.f}, nq = x[1];
+            if (it > 0) {
+                be = f2_div(x[0], rho);
+                nq = f2_add(nq, f2_mul(be, f2_add(F2{2.f * x[2].h, 2.f * x[2].l}, f2_mul(be, qu))));
+            }
+            rho = x[0];
+            qu = nq;
+            ab_s[0] = f2_div(rho, qu).h;
+            ab_s[1] = be.h;
+        }
+        __syncthreads();
+        alpha = ab_s[0];
+        beta = ab_s[1];
+    }
+    if (mine) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            const size_t k = (size_t)i * D + d;
+            A.z[k] = z[d];
+            A.p[k] = p[d];
+            A.q[k] = b[d];
+        }
+    }
+    if (lb == 0 && tid == 0) {
+        A.flags[kFlagIter] = it;
+        if (ok) {
+            A.scal[rho_slot32(it - 1)] = (double)rho.h + (double)rho.l;
+            A.scal[kSQUPrev] = (double)qu.h + (double)qu.l;
+            A.scal[kSIn] = (double)rr_s.h + (double)rr_s.l;
+            if (stop_s != 2) A.flags[kFlagDone] = 1;   // 2: the launch's bound, the phase goes on
+            if (stop_s == 3) A.flags[kFlagBad] = 1;
+        }
+    }
+}
+
 // ---- the system: C, b and D^-1 -------------------------------------------------------
 // C of every particle's P-list (calculateMatrixC main.cpp:2462-2507; the wall
 // rows' C_kj = - C_jk of fluid j give C^T its wall rows without a transposed
@@ -960,6 +1419,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_pen_phase(int n, const doubl
         acc += v * v;
     }
     if (reduce_finalize_last(acc, partials, counter, scal + kSIn0)) {
+
         const double need = 0.25 * tol_out2 * scal[kSRR0] / scal[kSRR];
         scal[kSTol2] = need > tol_in2 ? need : tol_in2;
         scal[kSIn] = scal[kSIn0];
@@ -970,16 +1430,48 @@ __global__ void __launch_bounds__(kReduceThreads) k_pen_phase(int n, const doubl
 // ---- host side ---------------------------------------------------------------------
 constexpr int kPenBlocks = 152 * kPenResident;   // blocks of k_pen_y: what is resident at once
 
-// Rows a block and threads a row.  A large case takes 256 rows a block (a
-// row's share of the staged neighbours falls with the block: 5.2, 4.5 and 4.2
-// times the rows of 128, 256 and 512); a small one fewer rows and four threads
-// a row, so that its blocks reach every SM and a row's words are not one
-// chain.
-static void pen_shape(int N, int* rows, int* W)
+// Shared memory of the resident iteration for `umax` staged neighbours
+static size_t cr_smem(const mph_case* c, int rows, int umax)
 {
-    if (N > 152 * 512) { *rows = 256; *W = 1; }
-    else if (N > 152 * 192) { *rows = 128; *W = 2; }
-    else { *rows = 64; *W = 4; }
+    return (size_t)umax * (c->dim == 3 ? 32 : 24) + (size_t)rows * ((c->pmax + 3) / 4) * sizeof(uint2) + 16;
+}
+
+// Blocks of the resident iteration that the device holds at once (0: none)
+static int cr_capacity(int dim)
+{
+    static std::once_flag once;
+    static int cap[2] = {0, 0};
+    std::call_once(once, [] {
+        int dev = 0, sms = 0, coop = 0, nb[2] = {0, 0};
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+        cudaFuncSetAttribute(k_pen_cr<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCrSmem);
+        cudaFuncSetAttribute(k_pen_cr<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCrSmem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[0], k_pen_cr<2>, kCrThreads, kCrSmem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[1], k_pen_cr<3>, kCrThreads, kCrSmem);
+        for (int k = 0; k < 2; ++k) cap[k] = coop ? sms * nb[k] : 0;
+    });
+    return std::min(cap[dim - 2], kCrBlocks);
+}
+
+// Rows a block and threads a row.  Up to 155,648 particles the iteration is
+// resident: up to 512 threads a block, the rows spread evenly over at most two
+// blocks an SM (the choice does not depend on what a step's blocks stage, so
+// that staged and gathering runs keep one order of sums).  Beyond, and for
+// lists too long for shared memory, 256 rows a block in the per-iteration
+// kernels (a row's share of the staged neighbours falls with the block), or
+// fewer and several threads a row where the blocks would not reach every SM.
+static void pen_shape(mph_case* c)
+{
+    const int N = c->dp.N;
+    const int cap = cr_capacity(c->dim);
+    const int rows = std::max(kCrMinRows, cap > 0 ? ((N + cap - 1) / cap + 31) / 32 * 32 : 0);
+    c->pen_resident = rows <= kCrThreads && (long long)rows * cap >= N && cr_smem(c, rows, (pen_ucap(rows) + 127) / 128 * 128) <= kCrSmem;
+    if (c->pen_resident) { c->pen_rows = rows; c->pen_w = kCrThreads / rows; }
+    else if (N > 152 * 512) { c->pen_rows = 256; c->pen_w = 1; }
+    else if (N > 152 * 192) { c->pen_rows = 128; c->pen_w = 2; }
+    else { c->pen_rows = 64; c->pen_w = 4; }
 }
 
 // The positions' unit is RadiusP / 2^20 or finer (domains up to about 1900
@@ -1016,13 +1508,15 @@ static int launch_pen_lists(mph_case* c)
 {
     DeviceState& d = c->d;
     const DevParams& P = c->dp;
-    pen_shape(P.N, &c->pen_rows, &c->pen_w);
+    pen_shape(c);
     c->pen_pw4 = (c->pmax + 3) / 4;
     const int nsl = (P.N + 31) / 32, nb = (int)grid_for(P.N, c->pen_rows), ucap = pen_ucap(c->pen_rows);
-    if (!d.pgroups) {
-        MPH_CUDA(cudaMalloc((void**)&d.pgroups, (size_t)nsl * sizeof(int)));
-        MPH_CUDA(cudaMalloc((void**)&d.puniq, (size_t)nb * ucap * sizeof(int)));
-        MPH_CUDA(cudaMalloc((void**)&d.pucount, (size_t)(nb + 4) * sizeof(int)));
+    if (!d.pgroups) MPH_CUDA(cudaMalloc((void**)&d.pgroups, (size_t)nsl * sizeof(int)));
+    MPH_TRY(grow_t(&d.puniq, &d.cap_puniq, (long long)nb * ucap));
+    MPH_TRY(grow_t(&d.pucount, &d.cap_pucount, nb + 4));
+    if (c->pen_resident && !d.cr_rec) {
+        MPH_CUDA(cudaMalloc((void**)&d.cr_rec, (size_t)P.Nf * 3 * sizeof(float4)));
+        MPH_CUDA(cudaMalloc((void**)&d.cr_vals, (size_t)(8 * kCrBlocks + 32) * sizeof(float)));
     }
     MPH_TRY(grow_t(&d.pidx, &d.cap_pidx, (long long)nsl * c->pen_pw4 * 32));
     c->pen_umax = 0;
@@ -1189,6 +1683,26 @@ static PenArgs pen_args(const mph_case* c, int cap)
     A.partials = d.partials;
     A.counter = (unsigned*)(d.flags + kFlagCounter);
     return A;
+}
+
+// The phase's iterations in one cooperative launch
+int launch_pen_resident(mph_case* c, int cap)
+{
+    DeviceState& d = c->d;
+    PenArgs A = pen_args(c, cap);
+    const int nb = (int)grid_for(A.N, c->pen_rows);
+    PenCr C{};
+    C.rec = d.cr_rec;
+    C.v3 = d.cr_vals;
+    C.v1 = d.cr_vals + 6 * kCrBlocks;
+    C.count = (unsigned*)(d.cr_vals + 8 * kCrBlocks);
+    MPH_CUDA(cudaMemsetAsync(C.count, 0, sizeof(unsigned), c->stream));
+    const dim3 blk(c->pen_rows, c->pen_w);
+    void* args[] = {&c->dp, &A, &C};
+    const size_t smem = cr_smem(c, c->pen_rows, c->pen_umax);
+    MPH_CUDA(cudaLaunchCooperativeKernel(c->dim == 2 ? (const void*)k_pen_cr<2> : (const void*)k_pen_cr<3>, dim3(nb), blk, args, smem, c->stream));
+    MPH_COUNT_LAUNCH();
+    return MPH_OK;
 }
 
 // y = M s and the iteration's scalars (two launches), then the vectors (one)

@@ -725,7 +725,7 @@ int case_destroy(mph_case* c)
                     (void*)d.tct32, (void*)d.pes32, (void*)d.sdiag32, (void*)d.sdiag64, (void*)d.cvl32, (void*)d.psptr, (void*)d.ctsptr,
                     (void*)d.pswidth, (void*)d.ctswidth, (void*)d.pscol, (void*)d.ctscol, (void*)d.psval, (void*)d.ctsval,
                     (void*)d.grec16, (void*)d.grec32, (void*)d.pscale, (void*)d.lcol16, (void*)d.uniq, (void*)d.ucount,
-                    (void*)d.ctuniq, (void*)d.ctucount, (void*)d.ipos, (void*)d.vpos, (void*)d.z4, (void*)d.vacc, (void*)d.pidx, (void*)d.pgroups, (void*)d.puniq, (void*)d.pucount, (void*)d.wkey, (void*)d.wval, (void*)d.ccell,
+                    (void*)d.ctuniq, (void*)d.ctucount, (void*)d.ipos, (void*)d.cr_rec, (void*)d.cr_vals, (void*)d.vpos, (void*)d.z4, (void*)d.vacc, (void*)d.pidx, (void*)d.pgroups, (void*)d.puniq, (void*)d.pucount, (void*)d.wkey, (void*)d.wval, (void*)d.ccell,
                     (void*)d.io3, (void*)d.vprev, (void*)d.vprev_alt, (void*)d.sort_cnt, (void*)d.sort_off, d.scan_tmp})
         if (p) cudaFree(p);
     for (auto& p : c->prof.pending) {

@@ -179,7 +179,9 @@ struct DeviceState {
     float4* z4 = nullptr;              // the solution or its last correction, a record a row (two where it is in two floats)
     double* vacc = nullptr;            // viscous fluid pairs of A x, added up over the refinement phases
     uint2* pidx = nullptr;
-    long long cap_pidx = 0;
+    long long cap_pidx = 0, cap_puniq = 0, cap_pucount = 0;
+    float* cr_vals = nullptr;          // its blocks' sums, and the count of the grid's crossings
+    float4* cr_rec = nullptr;          // the resident iteration's published vectors, three records a row
     int *pgroups = nullptr, *puniq = nullptr, *pucount = nullptr;
     int* ccell = nullptr;              // packed cell coordinates of every particle (pair path)
     double* io3 = nullptr;             // host-layout staging, 2 x N x 3 doubles (state upload, field download)
@@ -303,6 +305,7 @@ struct mph_case {
     bool step_pen = false;              // this step's inner CR runs on k_penalty.cu's operator
     int pmax = 0;                       // longest P-list of the current lists
     int pen_rows = 0, pen_w = 0;        // its rows a block and threads a row
+    bool pen_resident = false;          // a phase's CR iterations in one cooperative kernel (the case's rows fit the chip at once)
     int pen_pw4 = 0, pen_umax = 0;      // 8-byte words a row has room for; largest staged count (rounded up)
     double pen_tol = 0.0;               // what a refinement phase leaves at least (the viscous part outside the operator)
     int loc_smem = 0;                   // shared memory of k_visc_pen32's staged s (0: gathers by column)
@@ -424,6 +427,7 @@ int pen_exact_diag(mph_case* c);
 void launch_pen_start_residual(mph_case* c);
 void launch_pen_refine(mph_case* c, double scale, const double* scale_src, const int* flags);
 void launch_pen_phase(mph_case* c, double inv_scale, const double* scale_src, double tol_in2, double tol_out2);
+int launch_pen_resident(mph_case* c, int cap);
 void launch_pen_operator(mph_case* c, int cap);
 void launch_pen_vectors(mph_case* c, int cap, bool use_cond, cudaGraphConditionalHandle cond);
 size_t batch_pen_bytes();

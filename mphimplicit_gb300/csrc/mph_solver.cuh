@@ -18,7 +18,7 @@ enum {
     kSOuterRes = 8, kSOuterRes0 = 9, kSScalarCount = 16
 };
 // int flag slots
-enum { kFlagDone = 0, kFlagIter = 1, kFlagCap = 2, kFlagBad = 3, kFlagCounter = 4, kFlagOuter = 5, kFlagCount = 8 };
+enum { kFlagDone = 0, kFlagIter = 1, kFlagCap = 2, kFlagBad = 3, kFlagCounter = 4, kFlagOuter = 5, kFlagStall = 6, kFlagCount = 8 };
 
 constexpr int kReduceBlocks = 1216;   // 152 SMs x 8 blocks: bound on the partials count
 constexpr int kGraphChunk = 8;        // CR iterations per captured graph chunk (FP64 form; the mixed form's option "chunk")
