@@ -8,6 +8,8 @@
 // lies inside a conservative band around MaxRadius^2 or RadiusP^2 is decided
 // by the reference's exact FP64 expression.  The band is derived from the
 // coordinate magnitudes at case creation (or the FP32 step is disabled).
+#include <algorithm>
+
 #include "mph_device.cuh"
 
 namespace mph {
@@ -434,6 +436,109 @@ int launch_scan_i32_to_i64(mph_case* c, const int* in, long long* out, int n)
     { k_scan_reduce<<<nb, kScanThreads, 0, c->stream>>>(in, n, bsum); MPH_COUNT_LAUNCH(); }
     { k_scan_blocks<<<1, kScanThreads, 0, c->stream>>>(bsum, nb); MPH_COUNT_LAUNCH(); }
     { k_scan_apply<<<nb, kScanThreads, 0, c->stream>>>(in, n, bsum, out); MPH_COUNT_LAUNCH(); }
+    return MPH_OK;
+}
+
+// The same for the two neighbour lists in one go (nc -> nptr, ncp -> nptrP:
+// grid row 0 and 1), with totals[0], [1] the list lengths and totals[2] the
+// longest P-list: three launches instead of eight and one read.
+struct ScanLists {
+    const int* in[2];
+    long long* out[2];
+    long long* bsum[2];
+    long long* totals;
+    int* bmax;
+};
+__global__ void __launch_bounds__(kScanThreads) k_scan2_reduce(ScanLists A, int n)
+{
+    const int a = blockIdx.y;
+    const long long b0 = (long long)blockIdx.x * kScanChunk;
+    long long s = 0;
+    int mx = 0;
+    for (int k = 0; k < kScanPer; ++k) {
+        const long long idx = b0 + (long long)k * kScanThreads + threadIdx.x;
+        const int v = idx < n ? A.in[a][idx] : 0;
+        s += v;
+        mx = max(mx, v);
+    }
+    long long tot;
+    block_excl_scan(s, &tot);
+    if (a == 1) {
+        __shared__ int wm[kScanThreads / 32];
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = mx;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < kScanThreads / 32; ++w) mx = max(mx, wm[w]);
+            A.bmax[blockIdx.x] = mx;
+        }
+    }
+    if (threadIdx.x == 0) A.bsum[a][blockIdx.x] = tot;
+}
+__global__ void __launch_bounds__(kScanThreads) k_scan2_blocks(ScanLists A, int nb)
+{
+    const int a = blockIdx.x;
+    long long carry = 0;
+    int mx = 0;
+    for (int base = 0; base < nb; base += kScanThreads) {
+        const int k = base + threadIdx.x;
+        const long long v = k < nb ? A.bsum[a][k] : 0;
+        long long tot;
+        const long long ex = block_excl_scan(v, &tot);
+        if (k < nb) A.bsum[a][k] = carry + ex;
+        carry += tot;
+        if (a == 1 && k < nb) mx = max(mx, A.bmax[k]);
+    }
+    if (a == 1) {
+        __shared__ int wm[kScanThreads / 32];
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = mx;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < kScanThreads / 32; ++w) mx = max(mx, wm[w]);
+            A.totals[2] = mx;
+        }
+    }
+    if (threadIdx.x == 0) A.totals[a] = carry;
+}
+__global__ void __launch_bounds__(kScanThreads) k_scan2_apply(ScanLists A, int n)
+{
+    const int a = blockIdx.y;
+    const long long b0 = (long long)blockIdx.x * kScanChunk;
+    int v[kScanPer];
+    long long s = 0;
+    for (int k = 0; k < kScanPer; ++k) {
+        const long long idx = b0 + (long long)threadIdx.x * kScanPer + k;
+        v[k] = idx < n ? A.in[a][idx] : 0;
+        s += v[k];
+    }
+    long long tot;
+    long long run = block_excl_scan(s, &tot) + A.bsum[a][blockIdx.x];
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.out[a][0] = 0;
+    for (int k = 0; k < kScanPer; ++k) {
+        const long long idx = b0 + (long long)threadIdx.x * kScanPer + k;
+        run += v[k];
+        if (idx < n) A.out[a][idx + 1] = run;
+    }
+}
+int launch_scan_lists(mph_case* c, int n)
+{
+    DeviceState& d = c->d;
+    const int nb = std::max(1, (n + kScanChunk - 1) / kScanChunk);
+    const size_t need = (size_t)(3 * nb + 3) * sizeof(long long);
+    if (need > d.scan_tmp_bytes) {
+        if (d.scan_tmp) cudaFree(d.scan_tmp);
+        d.scan_tmp = nullptr;
+        d.scan_tmp_bytes = 0;
+        MPH_CUDA(cudaMalloc(&d.scan_tmp, need * 2));
+        d.scan_tmp_bytes = need * 2;
+    }
+    long long* t = (long long*)d.scan_tmp;
+    const ScanLists A{{d.nc, d.ncp}, {d.nptr, d.nptrP}, {t, t + nb + 1}, d.totals, (int*)(t + 2 * nb + 2)};
+    const dim3 g(nb, 2);
+    { k_scan2_reduce<<<g, kScanThreads, 0, c->stream>>>(A, n); MPH_COUNT_LAUNCH(); }
+    { k_scan2_blocks<<<2, kScanThreads, 0, c->stream>>>(A, nb); MPH_COUNT_LAUNCH(); }
+    { k_scan2_apply<<<g, kScanThreads, 0, c->stream>>>(A, n); MPH_COUNT_LAUNCH(); }
     return MPH_OK;
 }
 

@@ -56,7 +56,10 @@ constexpr int kPlWords = 1 << 13;   // bitmap of a row block's columns: 2^18 par
 constexpr int kMaxPenRows = 256;   // threads of a row block (rows times threads a row) of the per-iteration kernels
 constexpr int kCrThreads = 512;    // of the resident iteration's blocks, two an SM
 constexpr int kCrBlocks = 2 * 152;
-constexpr int kCrMinRows = 192;    // rows a block at least (a solve of 15,000 particles: 2.01, 1.89, 2.00 ms with 128, 192, 256)
+#ifndef MPH_CR_MIN
+#define MPH_CR_MIN 192
+#endif
+constexpr int kCrMinRows = MPH_CR_MIN;    // rows a block at least (a solve of 15,000 particles: 2.01, 1.89, 2.00 ms with 128, 192, 256)
 constexpr int kCrSmem = 100 * 1024;   // dynamic: two blocks an SM with their 7 KB of static shared memory
 // Staged neighbours a block of `rows` rows has room for.  Blocks of a
 // 3.5-spacing cell order have about 2.8 (256 rows) to 3.9 (64) times their
@@ -1568,7 +1571,6 @@ int launch_pen_assemble(mph_case* c)
     if (!d.tct32) MPH_CUDA(cudaMalloc((void**)&d.tct32, (size_t)(P.N + 1) * sizeof(float)));
     if (!d.sdiag64) MPH_CUDA(cudaMalloc((void**)&d.sdiag64, (size_t)P.Nf * 8 * sizeof(double)));
     MPH_TRY(grow_t(&d.cval, &d.cap_cval, c->nnbP * c->dim));
-    MPH_CUDA(cudaMemsetAsync(d.wrap32, 0, 2 * sizeof(int), st));
     launch_vector_p(c);
     const unsigned g = grid_for(P.N, 256), gs = grid_for(P.N, 128);
     float* invD = d.v32 + 7 * n;

@@ -510,16 +510,12 @@ int stage_cellsort(mph_case* c)
     if (c->cell_sort) MPH_TRY(launch_counting_sort(c));
     else launch_bitonic_sort(c);
     launch_cell_ranges_and_permute(c);
-    const int init[8] = {c->dp.cc[0], c->dp.cc[1], c->dp.cc[2], 0, 0, 0, 0, 0};
-    MPH_CUDA(cudaMemcpyAsync(c->d.bbox, init, sizeof(init), cudaMemcpyHostToDevice, c->stream));
     launch_fluid_bbox(c);
-    int hb[8];
-    int ends[2];
+    int hb[8];   // the fluid's cell box, the ends of the fluid and the wall particles
     MPH_CUDA(cudaMemcpyAsync(hb, c->d.bbox, sizeof(hb), cudaMemcpyDeviceToHost, c->stream));
-    MPH_CUDA(cudaMemcpyAsync(&ends[0], c->d.bucket + c->dp.T, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    MPH_CUDA(cudaMemcpyAsync(&ends[1], c->d.bucket + 2 * c->dp.T, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     MPH_CUDA(cudaStreamSynchronize(c->stream));
     MPH_CUDA(cudaGetLastError());
+    const int* ends = hb + 6;
     c->fB = 0;
     c->fE = ends[0];
     c->wB = ends[0];
@@ -538,15 +534,12 @@ int stage_neighbors(mph_case* c)
     int pon = prof_begin(c, 3, &pe);
     launch_neighbor_count(c);
     if (pon) prof_end(c, 3, pe);
-    MPH_CUDA(cudaMemsetAsync(c->d.dmax + 1, 0, sizeof(int), c->stream));
-    launch_max_int(c, c->d.ncp, N, c->d.dmax + 1);   // longest P-list
-    MPH_TRY(launch_scan_i32_to_i64(c, c->d.nc, c->d.nptr, N));
-    MPH_TRY(launch_scan_i32_to_i64(c, c->d.ncp, c->d.nptrP, N));
-    long long tot[2];
-    MPH_CUDA(cudaMemcpyAsync(&tot[0], c->d.nptr + N, sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
-    MPH_CUDA(cudaMemcpyAsync(&tot[1], c->d.nptrP + N, sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
-    MPH_CUDA(cudaMemcpyAsync(&c->pmax, c->d.dmax + 1, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    // the row pointers of both lists, and on the host their totals and the longest P-list
+    MPH_TRY(launch_scan_lists(c, N));
+    long long tot[3];
+    MPH_CUDA(cudaMemcpyAsync(tot, c->d.totals, sizeof(tot), cudaMemcpyDeviceToHost, c->stream));
     MPH_CUDA(cudaStreamSynchronize(c->stream));
+    c->pmax = (int)tot[2];
     c->nnb = tot[0];
     c->nnbP = tot[1];
     void* p = c->d.nind;

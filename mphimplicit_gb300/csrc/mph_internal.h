@@ -402,6 +402,7 @@ void launch_cell_ranges_and_permute(mph_case* c);
 void launch_fluid_bbox(mph_case* c);
 void launch_neighbor_count(mph_case* c);
 void launch_max_int(mph_case* c, const int* v, int n, int* out);
+int launch_scan_lists(mph_case* c, int n);
 int launch_scan_i32_to_i64(mph_case* c, const int* in, long long* out, int n);
 int launch_slice_ptr(mph_case* c, int rows, const int* counts, int* width, long long* ptr, long long* total);
 void launch_neighbor_fill(mph_case* c);
