@@ -16,7 +16,10 @@
 // V-cycle: levels with many rows run as grid-wide kernels: one fused Jacobi
 //         kernel per smoothing sweep (S_new = S + invD (Q - A S)), a residual
 //         kernel before each restriction, and the restriction (child sums).
-//         Every level from the first one with at most kCtaRows rows down to
+//         In the FP64 form the levels from the first one with at most
+//         kTailRows rows on are applied as one matrix (k_mg_tail_apply).  In
+//         the mixed form
+//         every level from the first one with at most kCtaRows rows down to
 //         the coarsest and back runs inside one cluster of kClusterCtas
 //         1024-thread blocks (one per SM), its sweeps separated by cluster
 //         barriers, so the small levels cost one launch and read their
@@ -274,7 +277,57 @@ __device__ __forceinline__ int row_parent(const LevelK& S_, const LevelK& L, int
     return grid_index(L, (p[0] + S_.mn[0]) / 2 - L.mn[0], (p[1] + S_.mn[1]) / 2 - L.mn[1], (p[2] + S_.mn[2]) / 2 - L.mn[2]) * D + rD;
 }
 
+__host__ __device__ inline bool full_stencil(const LevelK& L, int D)
+{
+    return L.st[0] == 3 && L.st[1] == 3 && L.st[2] == (D == 3 ? 3 : 1);
+}
+
 // ---- grid-wide V-cycle kernels ------------------------------------------------------
+// FP64 sweeps of levels with the full 3^D stencil: four threads a row, every
+// fourth stencil cell each, their sums added by shuffles.  Such a sweep is
+// bound by a row's chain of FP64 multiply-adds (their latency is beyond 100
+// clocks here, and a level has few rows: 24,000 threads with 81 terms each on
+// 216,000 particles, 25 us a sweep); four chains a row are a quarter as long
+// with four times the threads in flight.  The threads of a stencil part hold 8 consecutive
+// rows, so their loads stay 64-byte segments.
+// RESID: out = Q - A S;  else out = S + invD (Q - A S).
+template <int D, bool RESID>
+__global__ void __launch_bounds__(128) k_mg_sweep64(LevelK L, const double* __restrict__ cofT, const double* __restrict__ invd,
+                                                    const double* __restrict__ Q, const double* __restrict__ Sin,
+                                                    double* __restrict__ out, const int* __restrict__ flags)
+{
+    if (flags[kFlagDone]) return;
+    constexpr int NC = D == 3 ? 27 : 9;
+    const int lane = threadIdx.x & 31, part = lane >> 3;
+    const int row = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 8 + (lane & 7);
+    double sum = 0.0;
+    if (row < L.rows) {
+        int p[3];
+        grid_coords(L, row / D, p);
+#pragma unroll
+        for (int u = 0; u < (NC + 3) / 4; ++u) {
+            const int cell = part + 4 * u;
+            if (cell < NC) {
+                int q[3] = {p[0] + (D == 3 ? cell / 9 : cell / 3) - 1, p[1] + (D == 3 ? (cell / 3) % 3 : cell % 3) - 1,
+                            p[2] + (D == 3 ? cell % 3 - 1 : 0)};
+#pragma unroll
+                for (int d = 0; d < D; ++d) q[d] += q[d] < 0 ? L.cnt[d] : (q[d] >= L.cnt[d] ? -L.cnt[d] : 0);
+                const double* cp = cofT + (size_t)cell * D * L.rows + row;
+                const double* sp = Sin + (size_t)grid_index(L, q[0], q[1], q[2]) * D;
+#pragma unroll
+                for (int sD = 0; sD < D; ++sD) sum += -cp[(size_t)sD * L.rows] * sp[sD];
+            }
+        }
+    }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+    if (row < L.rows && part == 0) {
+        const double r = Q[row] + sum;
+        if (RESID) out[row] = r;
+        else out[row] = Sin[row] + invd[row] * r;
+    }
+}
+
 template <int D, typename T>
 __global__ void k_mg_jacobi(LevelK L, const T* __restrict__ cofT, const T* __restrict__ invd, const T* __restrict__ Q,
                             const T* __restrict__ Sin, T* __restrict__ Sout, const int* __restrict__ flags)
@@ -349,11 +402,6 @@ __device__ __forceinline__ void sweep3_rows(const LevelK& L, const float* __rest
             else out[row] = Sin[row] + invd[row] * r;
         }
     }
-}
-
-__host__ __device__ inline bool full_stencil(const LevelK& L, int D)
-{
-    return L.st[0] == 3 && L.st[1] == 3 && L.st[2] == (D == 3 ? 3 : 1);
 }
 
 // one warp of 10 rows per launch slot (the grid covers the level once)
@@ -644,6 +692,170 @@ k_mg_small_levels(CoarseArgs<T> A, const int* __restrict__ flags)
         A.Sfine[row] = A.Sfine[row] + cur[A.first][row_parent<D>(S_, A.L[A.first], row)];
 }
 
+// ---- the FP64 form's small levels as one matrix ---------------------------------------
+// From the first level with at most kTailRows rows on (restriction below it,
+// smoothing, coarsest sweeps, prolongation), a V-cycle is one linear map S = M Q
+// of that level's right-hand side.  Smoothing the small levels takes some 40
+// dependent sweeps of few rows, each a barrier apart and bound by FP64
+// latency or by the FP64 units of the few SMs that take part; as a matrix
+// they are one pass of n^2 multiply-adds spread over the whole chip.  M is
+// built once a solve, a block a column: the sweeps on the unit vector, in the
+// sweeps' own order (the cells' coefficients stay in L2 meanwhile); a solve's
+// values move by rounding only (1e-16).  A solve of 10,000 particles in 2-D
+// (578 rows, 57 cycles) took 7.4 ms with one cluster kernel for the small
+// levels (81 us of a 132 us iteration) and takes 3.2; of 216,000 in 3-D (375
+// rows, 75 cycles; with k_mg_sweep64) 82 and 62.
+// Up to 1024 rows: M is 8 MB and its build some 5e8 multiply-adds (about a
+// millisecond in 3-D, less than a dozen cycles of sweeps); eight times the
+// rows, the next level up in 3-D, would be 64 times both.
+constexpr int kTailRows = 1024;
+constexpr int kTailTotal = 2 * kTailRows + 256;   // rows of all its levels (each at most half the last, and one cell an axis)
+constexpr int kTailThreads = 256;
+
+struct TailArgs {
+    int first, depth;
+    LevelK L[kMaxLevels];
+    const double* cof[kMaxLevels];
+    const double* invd[kMaxLevels];
+    int off[kMaxLevels];              // a level's first row among the vectors in shared memory
+    int total;                        // rows of all levels
+};
+
+template <int D>
+__global__ void __launch_bounds__(kTailThreads) k_mg_tail_columns(const __grid_constant__ TailArgs A, double* __restrict__ M)
+{
+    extern __shared__ double tail_smem[];
+    double *Q = tail_smem, *S = Q + A.total, *S2 = S + A.total, *R = S2 + A.total;
+    const int col = blockIdx.x, n = A.L[A.first].rows;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    auto sweeps = [&](int l, int count) {   // an even or odd number: the result is left in S
+        const LevelK& L = A.L[l];
+        const int o = A.off[l];
+        for (int k = 0; k < count; ++k) {
+            for (int row = tid; row < L.rows; row += nt)
+                S2[o + row] = S[o + row] + A.invd[l][row] * row_residual<D, double, true>(L, A.cof[l], Q + o, S + o, row);
+            __syncthreads();
+            for (int row = tid; row < L.rows; row += nt) S[o + row] = S2[o + row];   // read again by the same thread's row only after the barrier
+            __syncthreads();
+        }
+    };
+    for (int l = A.first; l < A.depth; ++l) {
+        const LevelK& L = A.L[l];
+        const int o = A.off[l];
+        for (int row = tid; row < L.rows; row += nt) {
+            const double q = l == A.first ? (row == col ? 1.0 : 0.0) : row_restrict<D, double>(A.L[l - 1], L, R + A.off[l - 1], row);
+            Q[o + row] = q;
+            S[o + row] = A.invd[l][row] * q;
+        }
+        __syncthreads();
+        sweeps(l, l == 0 ? 1 : l == A.depth - 1 ? 4 : 2);
+        if (l < A.depth - 1) {
+            for (int row = tid; row < L.rows; row += nt) R[o + row] = row_residual<D, double, true>(L, A.cof[l], Q + o, S + o, row);
+            __syncthreads();
+        }
+    }
+    for (int l = A.depth - 1; l > A.first; --l) {
+        const LevelK& F = A.L[l - 1];
+        for (int row = tid; row < F.rows; row += nt) S[A.off[l - 1] + row] += S[A.off[l] + row_parent<D>(F, A.L[l], row)];
+        __syncthreads();
+        sweeps(l - 1, l == 1 ? 2 : 3);
+    }
+    for (int row = tid; row < n; row += nt) M[(size_t)row * n + col] = S[row];
+}
+
+// S = M Q of the tail's first level L, two warps a row, four rows a block.
+// RESTRICT: Q = R r of the finer level F, formed by every block for itself (a
+// launch less), and S is added to the finer level's S (each of a row's
+// children has that one parent); else Q as given and S stored.
+template <int D, bool RESTRICT>
+__global__ void __launch_bounds__(kTailThreads) k_mg_tail_apply(LevelK F, LevelK L, const double* __restrict__ M,
+                                                                const double* __restrict__ in, double* __restrict__ S,
+                                                                const int* __restrict__ flags)
+{
+    if (flags[kFlagDone]) return;
+    __shared__ double q[kTailRows];
+    __shared__ double half[kTailThreads / 32];
+    const int n = L.rows, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int row = threadIdx.x; row < n; row += blockDim.x) q[row] = RESTRICT ? row_restrict<D, double>(F, L, in, row) : in[row];
+    __syncthreads();
+    const int row = blockIdx.x * (kTailThreads / 64) + (warp >> 1);
+    double a = 0.0, b = 0.0;
+    if (row < n) {
+        const double* m = M + (size_t)row * n;
+        int c = (warp & 1) * 32 + lane;
+        for (; c + 64 < n; c += 128) {
+            a += m[c] * q[c];
+            b += m[c + 64] * q[c + 64];
+        }
+        if (c < n) a += m[c] * q[c];
+    }
+    a += b;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane == 0) half[warp] = a;
+    __syncthreads();
+    if ((warp & 1) || row >= n) return;
+    const double s = half[warp] + half[warp + 1];
+    if (!RESTRICT) {
+        if (lane == 0) S[row] = s;
+        return;
+    }
+    int p[3], fm[3], fM[3];
+    grid_coords(L, row / D, p);
+    child_range(F, L, p, fm, fM);
+    const int dx = lane & 1, dy = (lane >> 1) & 1, dz = lane >> 2;
+    if (dx >= fm[0] && dx < 2 - fM[0] && dy >= fm[1] && dy < 2 - fM[1] && dz >= fm[2] && dz < 2 - fM[2]) {
+        const int g = grid_index(F, 2 * (p[0] + L.mn[0]) + dx - F.mn[0], 2 * (p[1] + L.mn[1]) + dy - F.mn[1],
+                                 2 * (p[2] + L.mn[2]) + dz - F.mn[2]);
+        S[g * D + row % D] += s;
+    }
+}
+
+// the tail's first level (depth: none)
+static int tail_first(const mph_case* c)
+{
+    int total = 0, first = c->depth;
+    while (first > 0 && c->lv[first - 1].rows <= kTailRows && total + c->lv[first - 1].rows <= kTailTotal) total += c->lv[--first].rows;
+    return first;
+}
+
+// its matrix, before a solve's first V-cycle
+int build_mg_tail(mph_case* c)
+{
+    const int first = tail_first(c);
+    if (first >= c->depth) return MPH_OK;
+    const int n = c->lv[first].rows;
+    if ((long long)n * n > c->d.cap_mg_tail) {
+        if (c->d.mg_tail) cudaFree(c->d.mg_tail);
+        c->d.mg_tail = nullptr;
+        c->d.cap_mg_tail = 0;
+        const long long want = std::min<long long>((long long)n * n + (long long)n * n / 2, (long long)kTailRows * kTailRows);
+        MPH_CUDA(cudaMalloc((void**)&c->d.mg_tail, (size_t)want * sizeof(double)));
+        c->d.cap_mg_tail = want;
+    }
+    TailArgs A{};
+    A.first = first;
+    A.depth = c->depth;
+    for (int l = 0; l < c->depth; ++l) {
+        A.L[l] = level_k(c, l);
+        A.cof[l] = c->d.mg_cof + c->lv[l].off_cof;
+        A.invd[l] = c->d.mg_invd + c->lv[l].off_vec;
+        A.off[l] = A.total;
+        if (l >= first) A.total += A.L[l].rows;
+    }
+    const int smem = 4 * A.total * (int)sizeof(double);
+    static std::once_flag once;
+    std::call_once(once, [] {   // the largest any case can need
+        const int smax = 4 * kTailTotal * (int)sizeof(double);
+        cudaFuncSetAttribute(k_mg_tail_columns<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax);
+        cudaFuncSetAttribute(k_mg_tail_columns<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax);
+    });
+    if (c->dim == 2) { k_mg_tail_columns<2><<<n, kTailThreads, smem, c->stream>>>(A, c->d.mg_tail); MPH_COUNT_LAUNCH(); }
+    else { k_mg_tail_columns<3><<<n, kTailThreads, smem, c->stream>>>(A, c->d.mg_tail); MPH_COUNT_LAUNCH(); }
+    MPH_CUDA(cudaGetLastError());
+    return MPH_OK;
+}
+
 // ---- host-side V-cycle -----------------------------------------------------------
 template <int D, typename T, typename TQ>
 static void vcycle_t(mph_case* c, const TQ* q, TQ* u, const TQ* invDiag, const T* cof, const T* invd, T* Qp, T* Sa, T* Sb,
@@ -672,10 +884,14 @@ static void vcycle_t(mph_case* c, const TQ* q, TQ* u, const TQ* invDiag, const T
     T* cur[kMaxLevels];
     T* oth[kMaxLevels];
     for (int l = 0; l < depth; ++l) { cur[l] = Sa + ov(l); oth[l] = Sb + ov(l); }
-    // first level handled by the single-block kernel (>= 1), or depth if none
+    // first level of the small levels' kernel, or depth if none
     int first = depth;
-    for (int l = 1; l < depth; ++l)
-        if (L[l].rows <= kCtaRows) { first = l; break; }
+    if (mixed) {
+        for (int l = 1; l < depth; ++l)
+            if (L[l].rows <= kCtaRows) { first = l; break; }
+    } else {
+        first = tail_first(c);
+    }
     // FP32 levels with the full stencil: the three-threads-a-row sweep
     auto split = [&](int l) { return std::is_same<T, float>::value && full_stencil(L[l], D); };
     auto grid3 = [&](int l) { return (unsigned)((L[l].rows + 39) / 40); };   // 4 warps of 10 rows a block
@@ -686,6 +902,10 @@ static void vcycle_t(mph_case* c, const TQ* q, TQ* u, const TQ* invDiag, const T
                 T* t = cur[l]; cur[l] = oth[l]; oth[l] = t;
                 return;
             }
+        } else if (full_stencil(L[l], D)) {
+            { k_mg_sweep64<D, false><<<grid_for((long long)L[l].rows * 4, 128), 128, 0, st>>>(L[l], cof + oc(l), invd + ov(l), Qp + ov(l), cur[l], oth[l], flags); MPH_COUNT_LAUNCH(); }
+            T* t = cur[l]; cur[l] = oth[l]; oth[l] = t;
+            return;
         }
         { k_mg_jacobi<D, T><<<grid_for(L[l].rows, 128), 128, 0, st>>>(L[l], cof + oc(l), invd + ov(l), Qp + ov(l), cur[l], oth[l],
                                                                        flags); MPH_COUNT_LAUNCH(); }
@@ -697,13 +917,17 @@ static void vcycle_t(mph_case* c, const TQ* q, TQ* u, const TQ* invDiag, const T
                 { k_mg_sweep3<D, true><<<grid3(l), 128, 0, st>>>(L[l], cof + oc(l), nullptr, Qp + ov(l), cur[l], Rp + ov(l), flags); MPH_COUNT_LAUNCH(); }
                 return;
             }
+        } else if (full_stencil(L[l], D)) {
+            { k_mg_sweep64<D, true><<<grid_for((long long)L[l].rows * 4, 128), 128, 0, st>>>(L[l], cof + oc(l), nullptr, Qp + ov(l), cur[l], Rp + ov(l), flags); MPH_COUNT_LAUNCH(); }
+            return;
         }
         { k_mg_residual<D, T><<<grid_for(L[l].rows, 128), 128, 0, st>>>(L[l], cof + oc(l), Qp + ov(l), cur[l], Rp + ov(l), flags); MPH_COUNT_LAUNCH(); }
     };
     // down, grid-wide levels
     { k_mg_p2g<D, T, TQ><<<grid_for(L[0].rows, 128), 128, 0, st>>>(c->dp, L[0], c->d.bucket, q, invd + ov(0), Qp + ov(0),
                                                                    cur[0], flags); MPH_COUNT_LAUNCH(); }
-    for (int k = 0; k < 1 + extra0; ++k) jacobi(0);      // level 0: 2 updates (+ extra0)
+    if (first > 0)
+        for (int k = 0; k < 1 + extra0; ++k) jacobi(0);      // level 0: 2 updates (+ extra0)
     for (int l = 1; l < first; ++l) {
         residual(l - 1);
         { k_mg_restrict<D, T><<<grid_for(L[l].rows, 128), 128, 0, st>>>(L[l - 1], L[l], Rp + ov(l - 1), invd + ov(l), Qp + ov(l),
@@ -712,37 +936,41 @@ static void vcycle_t(mph_case* c, const TQ* q, TQ* u, const TQ* invDiag, const T
         for (int k = 0; k < sweeps; ++k) jacobi(l);
     }
     if (first < depth) {
-        residual(first - 1);
-        CoarseArgs<T> A;
-        A.first = first;
-        A.depth = depth;
-        for (int l = 0; l < depth; ++l) {
-            A.L[l] = L[l];
-            A.cof[l] = cof + oc(l);
-            A.invd[l] = invd + ov(l);
-            A.Q[l] = Qp + ov(l);
-            A.Sa[l] = Sa + ov(l);
-            A.Sb[l] = Sb + ov(l);
-            A.R[l] = Rp + ov(l);
-        }
-        A.Sfine = cur[first - 1];
-        A.pre = pre;
-        A.post = post;
-        A.dense = -1;
-        A.dinv = nullptr;
+        if (first > 0) residual(first - 1);
         if constexpr (std::is_same<T, float>::value) {
+            CoarseArgs<T> A;
+            A.first = first;
+            A.depth = depth;
+            for (int l = 0; l < depth; ++l) {
+                A.L[l] = L[l];
+                A.cof[l] = cof + oc(l);
+                A.invd[l] = invd + ov(l);
+                A.Q[l] = Qp + ov(l);
+                A.Sa[l] = Sa + ov(l);
+                A.Sb[l] = Sb + ov(l);
+                A.R[l] = Rp + ov(l);
+            }
+            A.Sfine = cur[first - 1];
+            A.pre = pre;
+            A.post = post;
+            A.dense = -1;
+            A.dinv = nullptr;
             if (c->dense_level >= first && c->dense_level < depth) {
                 A.dense = c->dense_level;
                 A.dinv = c->d.mg_dinv32;
             }
+            if (kClusterCtas > 8) {
+                static std::once_flag once;
+                std::call_once(once, [] {
+                    cudaFuncSetAttribute(k_mg_small_levels<D, T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+                });
+            }
+            { k_mg_small_levels<D, T><<<kClusterCtas, kCtaThreads, 0, st>>>(A, flags); MPH_COUNT_LAUNCH(); }
+        } else {
+            const unsigned g = grid_for(L[first].rows, kTailThreads / 64);
+            if (first > 0) { k_mg_tail_apply<D, true><<<g, kTailThreads, 0, st>>>(L[first - 1], L[first], c->d.mg_tail, Rp + ov(first - 1), cur[first - 1], flags); MPH_COUNT_LAUNCH(); }
+            else { k_mg_tail_apply<D, false><<<g, kTailThreads, 0, st>>>(L[0], L[0], c->d.mg_tail, Qp + ov(0), cur[0], flags); MPH_COUNT_LAUNCH(); }
         }
-        if (kClusterCtas > 8) {
-            static std::once_flag once;
-            std::call_once(once, [] {
-                cudaFuncSetAttribute(k_mg_small_levels<D, T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            });
-        }
-        { k_mg_small_levels<D, T><<<kClusterCtas, kCtaThreads, 0, st>>>(A, flags); MPH_COUNT_LAUNCH(); }
     }
     // up, grid-wide levels: the block kernel already prolongated into level
     // first-1; without it the coarsest level is prolongated here
@@ -758,7 +986,8 @@ static void vcycle_t(mph_case* c, const TQ* q, TQ* u, const TQ* invDiag, const T
         for (int k = 0; k < post; ++k) jacobi(l);
         prolong(l);
     }
-    for (int k = 0; k < 2 + extra0; ++k) jacobi(0);      // level 0 post-smoothing
+    if (first > 0)
+        for (int k = 0; k < 2 + extra0; ++k) jacobi(0);      // level 0 post-smoothing
     const int blocks = std::min<int>(grid_for(c->dp.Nf, 256), kReduceBlocks);
     { k_mg_g2p_dot<D, T, TQ><<<blocks, 256, 0, st>>>(c->dp, L[0], c->d.key, invDiag, q, cur[0], u, c->d.partials,
                                                      (unsigned*)(c->d.flags + kFlagCounter), dot_out, flags); MPH_COUNT_LAUNCH(); }

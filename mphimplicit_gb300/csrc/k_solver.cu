@@ -179,6 +179,7 @@ static int cr_solve_t(mph_case* c)
 
     { k_cr_init<D><<<rb, kReduceThreads, 0, st>>>(Nf, c->d.type, c->d.vel, c->d.force, c->d.bvec, c->d.x, c->dp.density[0],
                                                 c->dp.density[1], c->dp.vol, c->dp.dt, part, counter, scal + kSRR0); MPH_COUNT_LAUNCH(); }
+    MPH_TRY(build_mg_tail(c));
     vcycle_fp64(c, c->d.bvec, c->d.s, scal + kSRS0);
     { k_spmv<D, 0><<<gs, 128, 0, st>>>(Nf, c->d.nfc, c->d.sptr, c->d.acol, c->d.aval, c->d.x, c->d.bvec, c->d.r, scal, flags, 0,
                                      tol2, part, counter, scal + kSRR); MPH_COUNT_LAUNCH(); }

@@ -204,6 +204,8 @@ struct DeviceState {
     float *mg_cof32 = nullptr, *mg_invd32 = nullptr;
     float* mg_dinv32 = nullptr;     // mixed form: dense inverse of the exactly solved coarse level
     long long cap_mg_dinv32 = 0;
+    double* mg_tail = nullptr;      // FP64 form: the small levels' matrix of this solve
+    long long cap_mg_tail = 0;
     float *mg_q32 = nullptr, *mg_s32 = nullptr, *mg_r32 = nullptr, *mg_res32 = nullptr;
     float* v32 = nullptr;           // mixed form: 7 FP32 CR vectors + FP32 D^-1, each D*Nf
     long long cap_mg_cof = 0, cap_mg_vec = 0, cap_mg_cof32 = 0, cap_mg_vec32 = 0;

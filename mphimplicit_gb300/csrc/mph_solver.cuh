@@ -255,6 +255,7 @@ int capture_graph(mph_case* c, cudaGraphExec_t* exec, unsigned long long* sig_sl
     return MPH_OK;
 }
 
+int build_mg_tail(mph_case* c);
 void vcycle_fp64(mph_case* c, const double* q, double* u, double* dot_out);
 void vcycle_mixed(mph_case* c, const float* q, float* u, double* dot_out);
 
