@@ -231,11 +231,14 @@ int mph_case_set_solver(mph_case* c, double outer_rel_residual, double inner_rel
  *   are recorded on a private side stream of the case and launched on the
  *   case stream.  A step waits on the host for its solver flags, so mph_step
  *   must not be called while the case stream is being captured.
- *   "factored" 1 (default) / 0: mixed form only.  1: where 2 RadiusP <
+ *   "factored" 1 (default) / 0: mixed form.  1: where 2 RadiusP <
  *   MaxRadius, the FP64 operator of the outer residual is applied in factored
  *   form (viscous pair terms + C Lambda C^T through the transposed P-lists)
  *   and only FP32 blocks are assembled; CsrCofA then exports the FP32 blocks.
- *   0: FP64 blocks are assembled and copied to FP32.
+ *   0: FP64 blocks are assembled and copied to FP32.  FP64 form, 3-D: 1
+ *   also lets the solve apply A in parts (FP64 C Lambda C^T over the P-lists,
+ *   the pairs in two floats) where its viscous part is at most a tenth of the
+ *   inertia; 0 applies the stored blocks.
  *   "mixed_extra_sweeps" 0 (default) .. 8: mixed form only, extra level-0
  *   smoothing sweeps before and after the rest of its V-cycle.
  *   "inner_blocks" 0 (default) / 1: factored mixed form only.  0: the inner

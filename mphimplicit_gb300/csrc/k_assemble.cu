@@ -42,12 +42,12 @@ void launch_max_int(mph_case* c, const int* v, int n, int* out)
 }
 
 template <int D>
-__global__ void __launch_bounds__(128) k_matrix_c(DevParams P, const double* __restrict__ pos, const int* __restrict__ ncp,
+__global__ void __launch_bounds__(128) k_matrix_c(DevParams P, int rows, const double* __restrict__ pos, const int* __restrict__ ncp,
                                                   const long long* __restrict__ nptrP, const int* __restrict__ nindP,
                                                   double* __restrict__ cval)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.Nf) return;
+    if (i >= rows) return;
     double xi[3];
     load_vec<D>(pos, i, xi);
     const double rP2 = P.rP * P.rP;
@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(128) k_matrix_c(DevParams P, const double* __r
 #pragma unroll
         for (int r = 0; r < D; ++r) cval[(b + a) * D + r] = cv[r];
     }
+    if (i >= P.Nf) return;   // a wall's own slot meets no fluid row
 #pragma unroll
     for (int r = 0; r < D; ++r) cval[(b + selfk) * D + r] = self[r];
 }
@@ -428,6 +429,7 @@ int launch_assemble(mph_case* c)
     c->step_factored = factored_applies(c);
     c->step_pairs = c->step_factored && !c->inner_blocks && c->visc_nonneg;
     c->step_pen = pen_applies(c);
+    c->step_f64 = f64_parts_apply(c);
     const bool need64 = !c->step_factored, need32 = c->precision == MPH_PRECISION_MIXED && !c->step_pairs;
     if (!need64 && c->d.aval) {   // a form change (option) since the last step: release what is unused
         cudaFree(c->d.aval);
@@ -486,6 +488,8 @@ int launch_assemble(mph_case* c)
     long long h_cn = 0;
     MPH_CUDA(cudaMemcpyAsync(&h_cn, c->d.nptrP + Nf, sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
     MPH_CUDA(cudaStreamSynchronize(c->stream));
+    const int crows = c->step_f64 ? P.N : Nf;   // the operator in parts reads C^T from every particle's own row
+    if (c->step_f64) h_cn = c->nnbP;
     {
         void* p = c->d.cval;
         MPH_TRY(ensure(&p, &c->d.cap_cval, h_cn * D, sizeof(double)));
@@ -504,9 +508,9 @@ int launch_assemble(mph_case* c)
         if (d < D && g0.cnt[d] < 3) M.folded = 1;
     }
     if (D == 2) {
-        { k_matrix_c<2><<<gf, 128, 0, c->stream>>>(P, c->d.pos, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.cval); MPH_COUNT_LAUNCH(); }
+        { k_matrix_c<2><<<grid_for(crows, 128), 128, 0, c->stream>>>(P, crows, c->d.pos, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.cval); MPH_COUNT_LAUNCH(); }
     } else {
-        { k_matrix_c<3><<<gf, 128, 0, c->stream>>>(P, c->d.pos, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.cval); MPH_COUNT_LAUNCH(); }
+        { k_matrix_c<3><<<grid_for(crows, 128), 128, 0, c->stream>>>(P, crows, c->d.pos, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.cval); MPH_COUNT_LAUNCH(); }
     }
     launch_vector_p(c);
     // A: the cell-block kernel where it applies; the per-row kernel for the

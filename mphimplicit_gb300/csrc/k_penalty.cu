@@ -45,6 +45,7 @@
 #include "mph_device.cuh"
 #include "mph_pairs.cuh"
 #include "mph_solver.cuh"
+#include "mph_twofloat.cuh"
 
 namespace mph {
 
@@ -690,42 +691,6 @@ struct PenCr {
     float *v3, *v1;                // the blocks' (s, y), (y, a), (y, b) in two floats each; (r, r)
     unsigned* count;               // arrivals of this launch's crossings
 };
-
-// two-float arithmetic (D. E. Knuth's two-sum; T. J. Dekker)
-struct F2 { float h, l; };
-__device__ __forceinline__ F2 f2_fast(float h, float l)   // |h| >= |l|
-{
-    const float s = __fadd_rn(h, l);
-    return {s, __fadd_rn(l, -__fadd_rn(s, -h))};
-}
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b)
-{
-    const float s = __fadd_rn(a.h, b.h), t = __fadd_rn(s, -a.h);
-    const float e = __fadd_rn(__fadd_rn(a.h, -__fadd_rn(s, -t)), __fadd_rn(b.h, -t));
-    return f2_fast(s, __fadd_rn(e, __fadd_rn(a.l, b.l)));
-}
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b)
-{
-    const float p = __fmul_rn(a.h, b.h);
-    return f2_fast(p, __fadd_rn(__fmaf_rn(a.h, b.h, -p), __fmaf_rn(a.h, b.l, __fmul_rn(a.l, b.h))));
-}
-__device__ __forceinline__ F2 f2_div(F2 a, F2 b)
-{
-    const float q = __fdiv_rn(a.h, b.h);
-    const float r = __fadd_rn(__fmaf_rn(-q, b.h, a.h), __fmaf_rn(-q, b.l, a.l));
-    return f2_fast(q, __fdiv_rn(r, b.h));
-}
-__device__ __forceinline__ F2 f2_of(double v)
-{
-    const float h = (float)v;
-    return {h, (float)(v - (double)h)};
-}
-__device__ __forceinline__ F2 f2_warp_sum(F2 v, int from)
-{
-    for (int o = from; o > 0; o >>= 1)
-        v = f2_add(v, F2{__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o)});
-    return v;
-}
 
 // The grid's crossing number `epoch`: this block's nv values (mine, shared
 // memory) are out, and whatever the block's threads wrote before it can be

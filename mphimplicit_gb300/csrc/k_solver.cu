@@ -11,14 +11,12 @@
 //   v = x
 //
 // Kernels per iteration: sliced-ELL block SpMV with the (s,y) dot and the
-// convergence test; p/q update; the V-cycle (its last kernel forms (q,u));
+// convergence test (in 3-D the operator in parts of k_f64op.cu, two kernels); p/q update; the V-cycle (its last kernel forms (q,u));
 // x/r/s update with the (r,r) dot.  All scalars stay on the device.
 #include "mph_device.cuh"
 #include "mph_solver.cuh"
 
 namespace mph {
-
-__host__ __device__ __forceinline__ int rho_slot(int it) { return kSRho + 8 + (it & 1); }   // two alternating slots
 
 template <int D>
 __global__ void k_cr_init(int Nf, const int* __restrict__ type, const double* __restrict__ vel, const double* __restrict__ force,
@@ -43,8 +41,13 @@ __global__ void k_cr_init(int Nf, const int* __restrict__ type, const double* __
 // the rho slot of iteration it = flags[kFlagIter], after the convergence test
 // of that iteration, rr/rr0 < tol2 (out is unused).  The reference's test is
 // rr/rr0 < 1e-12 (main.cpp:4346), i.e. tol2 = (1e-6)^2.
+// A slice of 32 rows a block, four warps of it every fourth block column
+// each: a row's chain of FP64 multiply-adds and column loads a quarter as
+// long (10,000 rows in 2-D are 313 warps, two an SM).
+constexpr int kSpmvSplit = 4;
+
 template <int D, int MODE>
-__global__ void __launch_bounds__(128) k_spmv(int Nf, const int* __restrict__ nfc, const long long* __restrict__ sptr,
+__global__ void __launch_bounds__(32 * kSpmvSplit) k_spmv(int Nf, const int* __restrict__ nfc, const long long* __restrict__ sptr,
                                               const int* __restrict__ acol, const double* __restrict__ aval,
                                               const double* __restrict__ xin, const double* __restrict__ b,
                                               double* __restrict__ yout, double* __restrict__ scal, int* __restrict__ flags,
@@ -53,30 +56,27 @@ __global__ void __launch_bounds__(128) k_spmv(int Nf, const int* __restrict__ nf
 {
     constexpr int DD = D * D;
     if (MODE == 1) {
-        if (flags[kFlagDone]) return;
-        const int it = flags[kFlagIter];
-        const double rr = scal[kSRR], rr0 = scal[kSRR0];
-        const bool bad = !(rr == rr);   // NaN residual
-        if (it >= cap || rr / rr0 < tol2 || bad) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const int stop = cr_stop(scal, flags, cap, tol2);
+        if (stop) {
+            if (stop > 1 && blockIdx.x == 0 && threadIdx.x == 0) {
                 flags[kFlagDone] = 1;
-                if (bad) flags[kFlagBad] = 1;
+                if (stop == 3) flags[kFlagBad] = 1;
             }
             return;
         }
-        out = scal + rho_slot(it);
+        out = scal + cr_rho_slot(flags[kFlagIter]);
     }
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
     double acc = 0.0;
+    double y[3] = {0.0, 0.0, 0.0};
     if (i < Nf) {
-        const int lane = i & 31;
         const long long base = sptr[i >> 5];
         const int* cp = acol + base + lane;
         const double* vp = aval + base * DD + lane;
-        double y[3] = {0.0, 0.0, 0.0};
         const int n = nfc[i];
-#pragma unroll 2
-        for (int k = 0; k < n; ++k) {
+#pragma unroll 4
+        for (int k = w; k < n; k += kSpmvSplit) {
             const int col = cp[(long long)k * 32];
             double xv[3];
 #pragma unroll
@@ -86,6 +86,17 @@ __global__ void __launch_bounds__(128) k_spmv(int Nf, const int* __restrict__ nf
 #pragma unroll
                 for (int s = 0; s < D; ++s) y[r] += vp[((long long)k * DD + r * D + s) * 32] * xv[s];
         }
+    }
+    __shared__ double part[kSpmvSplit - 1][D][32];
+    if (w > 0)
+#pragma unroll
+        for (int r = 0; r < D; ++r) part[w - 1][r][lane] = y[r];
+    __syncthreads();
+    if (w == 0 && i < Nf) {
+#pragma unroll
+        for (int v = 0; v < kSpmvSplit - 1; ++v)
+#pragma unroll
+            for (int r = 0; r < D; ++r) y[r] += part[v][r][lane];
 #pragma unroll
         for (int r = 0; r < D; ++r) {
             const size_t k = (size_t)i * D + r;
@@ -114,7 +125,10 @@ __global__ void k_update_pq(int n, const double* __restrict__ s, const double* _
         }
         return;
     }
-    const double beta = scal[rho_slot(it)] / scal[rho_slot(it - 1)];
+    __shared__ double beta_s;   // the quotient once a block: in every thread it took two thirds of the kernel
+    if (threadIdx.x == 0) beta_s = scal[cr_rho_slot(it)] / scal[cr_rho_slot(it - 1)];
+    __syncthreads();
+    const double beta = beta_s;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         p[k] = beta * p[k] + s[k];
         q[k] = beta * q[k] + y[k];
@@ -129,8 +143,10 @@ __global__ void k_update_xrs(int n, double* __restrict__ x, double* __restrict__
                              unsigned* __restrict__ counter)
 {
     if (flags[kFlagDone]) return;
-    const int it = flags[kFlagIter];
-    const double alpha = scal[rho_slot(it)] / scal[kSQU];
+    __shared__ double alpha_s;
+    if (threadIdx.x == 0) alpha_s = scal[cr_rho_slot(flags[kFlagIter])] / scal[kSQU];
+    __syncthreads();
+    const double alpha = alpha_s;
     double acc = 0.0;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         x[k] += alpha * p[k];
@@ -170,7 +186,7 @@ static int cr_solve_t(mph_case* c)
     unsigned* counter = (unsigned*)(flags + kFlagCounter);
     double* part = c->d.partials;
     const int rb = std::min<int>(grid_for(n, kReduceThreads), kReduceBlocks);
-    const unsigned gs = grid_for(Nf, 128);
+    const unsigned gs = grid_for(Nf, 32);
     // stop test ||r||/||b|| < tol_outer on squared norms (1e-6 by default, the
     // reference's constant; mph_case_set_solver tightens it)
     const double tol2 = c->tol_outer == 1.0e-6 ? 1.0e-12 : c->tol_outer * c->tol_outer;
@@ -180,10 +196,22 @@ static int cr_solve_t(mph_case* c)
     { k_cr_init<D><<<rb, kReduceThreads, 0, st>>>(Nf, c->d.type, c->d.vel, c->d.force, c->d.bvec, c->d.x, c->dp.density[0],
                                                 c->dp.density[1], c->dp.vol, c->dp.dt, part, counter, scal + kSRR0); MPH_COUNT_LAUNCH(); }
     MPH_TRY(build_mg_tail(c));
+    // the operator in parts where it applies and its records fit, else the stored blocks
+    bool parts = false;
+    if constexpr (D == 3) {
+        if (c->step_f64) MPH_TRY(f64_parts_build(c, &parts));
+    }
     vcycle_fp64(c, c->d.bvec, c->d.s, scal + kSRS0);
-    { k_spmv<D, 0><<<gs, 128, 0, st>>>(Nf, c->d.nfc, c->d.sptr, c->d.acol, c->d.aval, c->d.x, c->d.bvec, c->d.r, scal, flags, 0,
-                                     tol2, part, counter, scal + kSRR); MPH_COUNT_LAUNCH(); }
+    if (parts) {
+        launch_f64_pack(c, c->d.x);
+        launch_f64_apply(c, 0, c->d.x, c->d.r, 0, tol2, scal + kSRR);
+    } else {
+        k_spmv<D, 0><<<gs, 32 * kSpmvSplit, 0, st>>>(Nf, c->d.nfc, c->d.sptr, c->d.acol, c->d.aval, c->d.x, c->d.bvec, c->d.r, scal, flags, 0,
+                                         tol2, part, counter, scal + kSRR);
+        MPH_COUNT_LAUNCH();
+    }
     vcycle_fp64(c, c->d.r, c->d.s, scal + kSQU);
+    if (parts) launch_f64_pack(c, c->d.s);
 
     // One CR iteration; the iteration index lives in flags[kFlagIter], so the
     // same launch sequence serves every iteration (and can be replayed as a
@@ -191,15 +219,24 @@ static int cr_solve_t(mph_case* c)
     const int cap = n;   // the reference iterates at most N = D*Nf times
     auto iteration = [&, c](cudaEvent_t* e) {
         cudaStream_t st = c->stream;   // the capture stream while a graph is recorded
-        { k_spmv<D, 1><<<gs, 128, 0, st>>>(Nf, c->d.nfc, c->d.sptr, c->d.acol, c->d.aval, c->d.s, nullptr, c->d.y, scal, flags,
-                                         cap, tol2, part, counter, nullptr); MPH_COUNT_LAUNCH(); }
+        if (parts) {
+            launch_f64_apply(c, 1, c->d.s, c->d.y, cap, tol2, nullptr);
+        } else {
+            k_spmv<D, 1><<<gs, 32 * kSpmvSplit, 0, st>>>(Nf, c->d.nfc, c->d.sptr, c->d.acol, c->d.aval, c->d.s, nullptr, c->d.y, scal, flags,
+                                             cap, tol2, part, counter, nullptr);
+            MPH_COUNT_LAUNCH();
+        }
         if (e) prof_begin(c, 0, &e[1]);
         { k_update_pq<<<rb, kReduceThreads, 0, st>>>(n, c->d.s, c->d.y, c->d.p, c->d.q, scal, flags); MPH_COUNT_LAUNCH(); }
         if (e) prof_begin(c, 1, &e[2]);
         vcycle_fp64(c, c->d.q, c->d.u, scal + kSQU);
         if (e) prof_begin(c, 1, &e[3]);
-        { k_update_xrs<<<rb, kReduceThreads, 0, st>>>(n, c->d.x, c->d.r, c->d.s, c->d.p, c->d.q, c->d.u, scal, flags, part,
-                                                    counter); MPH_COUNT_LAUNCH(); }
+        if (parts) {
+            launch_f64_update_xrs(c, rb);
+        } else {
+            k_update_xrs<<<rb, kReduceThreads, 0, st>>>(n, c->d.x, c->d.r, c->d.s, c->d.p, c->d.q, c->d.u, scal, flags, part, counter);
+            MPH_COUNT_LAUNCH();
+        }
     };
     const int chunk = 8;
     int host_flags[kFlagCount];
@@ -210,7 +247,7 @@ static int cr_solve_t(mph_case* c)
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> timed;
     const bool graphs = c->use_graphs && !c->prof.on;
     if (graphs) {
-        MPH_TRY(capture_graph(c, &c->cr_exec, &c->cr_sig, graph_signature(c, tol2, cap), [&] {
+        MPH_TRY(capture_graph(c, &c->cr_exec, &c->cr_sig, graph_signature(c, tol2, parts ? -cap : cap), [&] {
             for (int k = 0; k < chunk; ++k) iteration(nullptr);
         }, &c->cr_launches));
     }

@@ -206,6 +206,10 @@ struct DeviceState {
     long long cap_mg_dinv32 = 0;
     double* mg_tail = nullptr;      // FP64 form: the small levels' matrix of this solve
     long long cap_mg_tail = 0;
+    float2* f64g = nullptr;         // FP64 form: the pairs' records of the operator in parts (three a slot)
+    long long cap_f64g = 0;
+    int* f64type = nullptr;         // the particles' types of this solve
+    float4* f64rec = nullptr;       // and the CR direction's (float4, then float2 a row)
     float *mg_q32 = nullptr, *mg_s32 = nullptr, *mg_r32 = nullptr, *mg_res32 = nullptr;
     float* v32 = nullptr;           // mixed form: 7 FP32 CR vectors + FP32 D^-1, each D*Nf
     long long cap_mg_cof = 0, cap_mg_vec = 0, cap_mg_cof32 = 0, cap_mg_vec32 = 0;
@@ -304,6 +308,8 @@ struct mph_case {
     bool step_pairs = false;            // this step's FP32 inner operator runs on the sliced pair terms
     cudaEvent_t gev[128] = {};          // event pairs of a profiled CR graph chunk (operators, then V-cycles)
     bool level0_done = false;           // this step's level-0 multigrid stencils were written by the assembly
+    bool step_f64 = false;              // this step's FP64 solve may run on k_f64op.cu's operator in parts
+    long long f64_slots = 0;            // slots the pair records have room for (their two arrays' split)
     bool step_pen = false;              // this step's inner CR runs on k_penalty.cu's operator
     int pmax = 0;                       // longest P-list of the current lists
     int pen_rows = 0, pen_w = 0;        // its rows a block and threads a row
@@ -418,6 +424,7 @@ void launch_vector_p(mph_case* c);
 void launch_wall_terms(mph_case* c, float* sdiag32, double* sdiag64, bool wall_rows_only);
 int launch_assemble_cells(mph_case* c, int kmax_rows, bool mix, bool* done);
 int build_ct(mph_case* c);
+bool f64_parts_apply(const mph_case* c);
 bool factored_applies(const mph_case* c);
 // k_penalty.cu: the inner operator of the point-Jacobi mixed form, its lists
 // and vectors, and the same over the cases of a batch (a block finds its case

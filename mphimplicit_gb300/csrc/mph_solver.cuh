@@ -20,6 +20,8 @@ enum {
 // int flag slots
 enum { kFlagDone = 0, kFlagIter = 1, kFlagCap = 2, kFlagBad = 3, kFlagCounter = 4, kFlagOuter = 5, kFlagStall = 6, kFlagCount = 8 };
 
+__host__ __device__ __forceinline__ int cr_rho_slot(int it) { return kSRho + 8 + (it & 1); }   // FP64 form: two alternating slots
+
 constexpr int kReduceBlocks = 1216;   // 152 SMs x 8 blocks: bound on the partials count
 constexpr int kGraphChunk = 8;        // CR iterations per captured graph chunk (FP64 form; the mixed form's option "chunk")
 constexpr int kMaxGraphChunk = 32;
@@ -63,6 +65,22 @@ __device__ __forceinline__ double block_sum(float v)
         for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
     }
     return d;   // valid in thread 0
+}
+
+// The convergence test of an iteration's application by one thread of
+// the block: an FP64 quotient in every thread took some 50 us of
+// the FP64 units' time over the 2.4 million of k_f64_parts.  0: go on, 1: done
+// before, 2: stop, 3: stop with a NaN.
+__device__ __forceinline__ int cr_stop(const double* __restrict__ scal, const int* __restrict__ flags, int cap, double tol2)
+{
+    __shared__ int stop_s;
+    if (threadIdx.x == 0) {
+        const double rr = scal[kSRR];
+        const bool bad = !(rr == rr);
+        stop_s = flags[kFlagDone] ? 1 : bad ? 3 : (flags[kFlagIter] >= cap || rr / scal[kSRR0] < tol2) ? 2 : 0;
+    }
+    __syncthreads();
+    return stop_s;
 }
 
 // Store this block's partial; the last block reduces all partials in block
@@ -256,6 +274,11 @@ int capture_graph(mph_case* c, cudaGraphExec_t* exec, unsigned long long* sig_sl
 }
 
 int build_mg_tail(mph_case* c);
+bool f64_parts_apply(const mph_case* c);
+int f64_parts_build(mph_case* c, bool* ok);
+void launch_f64_pack(mph_case* c, const double* s);
+void launch_f64_apply(mph_case* c, int mode, const double* x, double* y, int cap, double tol2, double* out);
+void launch_f64_update_xrs(mph_case* c, int blocks);
 void vcycle_fp64(mph_case* c, const double* q, double* u, double* dot_out);
 void vcycle_mixed(mph_case* c, const float* q, float* u, double* dot_out);
 
