@@ -18,6 +18,7 @@
 // default outer tolerance is the reference's ||r||/||b|| < 1e-6;
 // mph_case_set_solver tightens it (e.g. 1e-10).
 #include <algorithm>
+#include <cstring>
 
 #include "mph_device.cuh"
 #include "mph_solver.cuh"
@@ -345,7 +346,8 @@ __global__ void k_store_velocity_m(int Nf, const double* __restrict__ x, double*
 template <int D>
 __global__ void k_x0(int Nf, const int* __restrict__ type, const double* __restrict__ vel, const double* __restrict__ force,
                      const double* __restrict__ b, double* __restrict__ x, DevParams P, double* __restrict__ vprev, size_t nvs,
-                     int have, int keep, double* __restrict__ partials, unsigned* __restrict__ counter, double* __restrict__ out)
+                     int have, int keep, float4* __restrict__ rec, double* __restrict__ partials, unsigned* __restrict__ counter,
+                     double* __restrict__ out)
 {
     double acc = 0.0;
     const int n = Nf * D;
@@ -364,6 +366,11 @@ __global__ void k_x0(int Nf, const int* __restrict__ type, const double* __restr
             vprev[a] = vn;
         }
         x[k] = x0;
+        if (rec) {   // x0 in two floats, for the viscous pairs of the first residual
+            const float h = (float)x0;
+            reinterpret_cast<float*>(rec + i)[r] = h;
+            reinterpret_cast<float*>(rec + Nf + i)[r] = (float)(x0 - (double)h);
+        }
         acc += b[k] * b[k];
     }
     reduce_finalize(acc, partials, counter, out);
@@ -561,7 +568,7 @@ static int device_solve(mph_case* c, double* hs, int* hflags)
         cudaMemsetAsync(scal, 0, 32 * sizeof(double), s1);
         cudaMemsetAsync(flags, 0, kFlagCount * sizeof(int), s1);
         { k_x0<D><<<rb, kReduceThreads, 0, s1>>>(Nf, d.type, d.vel, d.force, d.bvec, d.x, c->dp, vprev, nvs, have, c->extrapolate,
-                                                 part, counter, scal + kSRR0); MPH_COUNT_LAUNCH(); }
+                                                 c->step_pen ? d.z4 : nullptr, part, counter, scal + kSRR0); MPH_COUNT_LAUNCH(); }
         residual();
         { k_outer_check<<<1, 32, 0, s1>>>(scal, flags, tol_out2, c->max_outer, cap, h_out); MPH_COUNT_LAUNCH(); }
         cudaGraph_t body_out = nullptr;
@@ -726,8 +733,7 @@ struct MixedRun {
     {
         DeviceState& d = c->d;
         cudaStream_t st = c->stream;
-        MPH_CUDA(cudaMemsetAsync(scal, 0, 32 * sizeof(double), st));
-        MPH_CUDA(cudaMemsetAsync(flags, 0, kFlagCount * sizeof(int), st));
+        MPH_CUDA(cudaMemsetAsync(scal, 0, kSolveStateBytes, st));   // the flags lie behind the scalars
         const size_t nvs = (size_t)c->dp.N * (D == 2 ? 2 : 4);
         if (c->extrapolate && !d.vprev) {
             MPH_CUDA(cudaMalloc((void**)&d.vprev, 2 * nvs * sizeof(double)));
@@ -737,7 +743,7 @@ struct MixedRun {
         double* vprev = c->extrapolate ? d.vprev : nullptr;
         const int have = std::min(c->prev_valid, c->extrapolate);
         { k_x0<D><<<rb, kReduceThreads, 0, st>>>(Nf, d.type, d.vel, d.force, d.bvec, d.x, c->dp, vprev, nvs, have, c->extrapolate,
-                                                 part, counter, scal + kSRR0); MPH_COUNT_LAUNCH(); }
+                                                 c->step_pen ? d.z4 : nullptr, part, counter, scal + kSRR0); MPH_COUNT_LAUNCH(); }
         c->prev_valid = vprev ? std::min(c->prev_valid + 1, c->extrapolate) : 0;
         if (c->step_pen) launch_pen_start_residual(c);
         else residual();
@@ -750,9 +756,11 @@ struct MixedRun {
     {
         *go = false;
         cudaStream_t st = c->stream;
-        MPH_CUDA(cudaMemcpyAsync(hs, scal, sizeof(hs), cudaMemcpyDeviceToHost, st));
-        MPH_CUDA(cudaMemcpyAsync(host_flags, flags, sizeof(host_flags), cudaMemcpyDeviceToHost, st));
+        char state[kSolveStateBytes];
+        MPH_CUDA(cudaMemcpyAsync(state, scal, sizeof(state), cudaMemcpyDeviceToHost, st));
         MPH_CUDA(cudaStreamSynchronize(st));
+        std::memcpy(hs, state, sizeof(hs));
+        std::memcpy(host_flags, state + sizeof(hs), sizeof(host_flags));
         if (host_flags[kFlagStall]) return fail(MPH_ERR_CUDA, "the resident CR iteration's grid barrier ran out of time");
         if (!(hs[kSRR] == hs[kSRR]) || (c->pen_resident && c->step_pen && host_flags[kFlagBad])) {
             bad = true;
@@ -798,10 +806,15 @@ struct MixedRun {
         return MPH_OK;
     }
 
-    int finish()
+    // stored: the velocity array holds x already, and hs the solve's last state
+    int finish(bool stored = false)
     {
         cudaStream_t st = c->stream;
         const int total_inner = host_flags[kFlagIter];
+        if (stored) {
+            fill_mixed_stats(c, total_inner, outer, hs, bad, tol_out2);
+            return MPH_OK;
+        }
         { k_store_velocity_m<D><<<grid_for(n, 256), 256, 0, st>>>(Nf, c->d.x, c->d.vel); MPH_COUNT_LAUNCH(); }
         MPH_CUDA(cudaMemcpyAsync(hs, scal, sizeof(hs), cudaMemcpyDeviceToHost, st));
         MPH_CUDA(cudaStreamSynchronize(st));
@@ -886,11 +899,12 @@ static int mixed_solve_t(mph_case* c)
             if (!go) break;
             cudaEvent_t e0 = nullptr;
             const int pon = prof_begin(c, 0, &e0);
-            MPH_TRY(launch_pen_resident(c, cap));
+            MPH_TRY(launch_pen_resident(c, cap, run.scale));
             if (pon) prof_end(c, 0, e0);
-            launch_pen_refine(c, run.scale, nullptr, flags);
+            launch_pen_residual(c, run.scale);
         }
-        return run.finish();
+        // a phase leaves the velocities (not one that met a NaN), and its end was read above
+        return run.finish(run.outer > 0 && !run.bad);
     }
     const int chunk = c->chunk;
     const bool graphs = c->use_graphs;

@@ -57,10 +57,13 @@ constexpr int kPlWords = 1 << 13;   // bitmap of a row block's columns: 2^18 par
 constexpr int kMaxPenRows = 256;   // threads of a row block (rows times threads a row) of the per-iteration kernels
 constexpr int kCrThreads = 512;    // of the resident iteration's blocks, two an SM
 constexpr int kCrBlocks = 2 * 152;
-#ifndef MPH_CR_MIN
-#define MPH_CR_MIN 192
-#endif
-constexpr int kCrMinRows = MPH_CR_MIN;    // rows a block at least (a solve of 15,000 particles: 2.01, 1.89, 2.00 ms with 128, 192, 256)
+// Rows a block at least.  A solve alone is fastest on many blocks (15,000
+// particles in 3-D: 2.01, 1.89, 2.00 ms with 128, 192, 256; 17,000 in 2-D,
+// where a row is a fifth of the work: 1.00, 1.04, 1.08 with 192, 256, 384),
+// but the blocks of a solve hold their SMs until it ends: an ensemble of 64
+// two-dimensional cases on their streams takes 52.9, 46.3, 37.9 and 37.5 ms
+// with 192, 256, 384 and 512.
+constexpr int kCrMinRows3 = 192, kCrMinRows2 = 384;
 constexpr int kCrSmem = 100 * 1024;   // dynamic: two blocks an SM with their 7 KB of static shared memory
 // Staged neighbours a block of `rows` rows has room for.  Blocks of a
 // 3.5-spacing cell order have about 2.8 (256 rows) to 3.9 (64) times their
@@ -690,6 +693,11 @@ struct PenCr {
     float4* rec;                   // per row 3 records: s, a = D^-1 y, b = D^-1 q
     float *v3, *v1;                // the blocks' (s, y), (y, a), (y, b) in two floats each; (r, r)
     unsigned* count;               // arrivals of this launch's crossings
+    // the phase's end: x += scale z, z as records for the residual, the
+    // velocity array
+    double scale;
+    double *x, *vel;
+    float4* z4;
 };
 
 // The grid's crossing number `epoch`: this block's nv values (mine, shared
@@ -1064,6 +1072,16 @@ __global__ void __launch_bounds__(kCrThreads, 2) k_pen_cr(DevParams P, PenArgs A
             A.p[k] = p[d];
             A.q[k] = b[d];
         }
+        if (ok && stop_s != 3) {   // not after a NaN
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                const size_t k = (size_t)i * D + d;
+                const double v = C.x[k] + C.scale * (double)z[d];
+                C.x[k] = v;
+                C.vel[(size_t)i * (D == 2 ? 2 : 4) + d] = v;
+            }
+            C.z4[i] = make_float4(z[0], z[1], z[2], 0.f);
+        }
     }
     if (lb == 0 && tid == 0) {
         A.flags[kFlagIter] = it;
@@ -1189,31 +1207,48 @@ __global__ void __launch_bounds__(256) k_pen_diag(DevParams P, const int* __rest
 // FP32 (coefficients and row sums as the stored pair terms had them): the
 // differences of x_0 in two floats, those of the FP32 corrections z exactly.
 //
-// x_0 as records (hi, lo), or the update x += scale z and z as records
-template <int D, bool FIRST>
+// (x_0 comes as records (hi, lo) from k_x0.)  The update x += scale z, and z as records:
+template <int D>
 __global__ void __launch_bounds__(256) k_pen_pack(int Nf, double* __restrict__ x, const float* __restrict__ z, double scale,
                                                   const double* __restrict__ scale_src, const int* __restrict__ flags,
                                                   float4* __restrict__ rec)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= Nf) return;
-    if (!FIRST && flags && flags[kFlagBad]) return;   // the device-driven solve: a phase that met a NaN ends the solve
-    float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
-    const double sc = FIRST ? 0.0 : (scale_src ? *scale_src : scale);
+    if (flags && flags[kFlagBad]) return;   // the device-driven solve: a phase that met a NaN ends the solve
+    float h[3] = {0.f, 0.f, 0.f};
+    const double sc = scale_src ? *scale_src : scale;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
         const size_t k = (size_t)i * D + d;
-        if (FIRST) {
-            const double v = x[k];
-            h[d] = (float)v;
-            l[d] = (float)(v - (double)h[d]);
-        } else {
-            h[d] = z[k];
-            x[k] += sc * (double)h[d];
-        }
+        h[d] = z[k];
+        x[k] += sc * (double)h[d];
     }
     rec[i] = make_float4(h[0], h[1], h[2], 0.f);
-    if (FIRST) rec[Nf + i] = make_float4(l[0], l[1], l[2], 0.f);
+}
+
+// lambda_k t_k, t = C^T x in FP64 from the particle's own P-list:
+// C_jk = - C_kj (to the rounding of the minimum image), and C_kk for a fluid
+// row itself
+template <int D>
+__device__ __forceinline__ void pen_ct64(const DevParams& P, int k, const int* __restrict__ type, const int* __restrict__ ncp,
+                                         const long long* __restrict__ nptrP, const int* __restrict__ nindP,
+                                         const double* __restrict__ cval, const double* __restrict__ x, double* __restrict__ t)
+{
+    if (k >= P.N) return;
+    const long long b = nptrP[k];
+    const int n = ncp[k];
+    double s = 0.0;
+#pragma unroll 2
+    for (int a = 0; a < n; ++a) {
+        const int j = nindP[b + a];
+        if (j >= P.Nf) continue;
+        double v = 0.0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) v += cval[(b + a) * D + d] * x[(size_t)j * D + d];
+        s = j == k ? s + v : s - v;
+    }
+    t[k] = P.lambda[type[k]] * s;
 }
 
 // vacc_i (+)= scale sum over the fluid neighbours of f e (e . (x_i - x_j)),
@@ -1222,15 +1257,23 @@ __global__ void __launch_bounds__(256) k_pen_pack(int Nf, double* __restrict__ x
 // the stored FP32 g and columns (16 bytes a slot streamed, x in six 4-byte
 // gathers: 1.33 ms on 1.3 million particles with the P-part) it needs no pair
 // terms, which took three passes to build: 0.73 ms for x_0, 0.62 for z.
+// The launch's first nbT blocks form lambda t of C^T x meanwhile (pen_ct64).
 template <int D, int L, bool FIRST>
-__global__ void __launch_bounds__(256) k_pen_visc(DevParams P, const int4* __restrict__ vpos, const int* __restrict__ nfc,
+__global__ void __launch_bounds__(256) k_pen_visc(DevParams P, int nbT, const int4* __restrict__ vpos, const int* __restrict__ nfc,
                                                   const long long* __restrict__ nptr, const int* __restrict__ nind,
                                                   const float4* __restrict__ rec, int* __restrict__ wrap,
                                                   const int* __restrict__ type, const double* __restrict__ pos,
                                                   const float* __restrict__ pos32, const float* __restrict__ poslo32, double scale,
-                                                  const double* __restrict__ scale_src, double* __restrict__ vacc)
+                                                  const double* __restrict__ scale_src, double* __restrict__ vacc,
+                                                  const int* __restrict__ ncp, const long long* __restrict__ nptrP,
+                                                  const int* __restrict__ nindP, const double* __restrict__ cval,
+                                                  const double* __restrict__ x, double* __restrict__ t)
 {
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / L, lane = threadIdx.x & (L - 1);
+    if ((int)blockIdx.x < nbT) {
+        pen_ct64<D>(P, blockIdx.x * blockDim.x + threadIdx.x, type, ncp, nptrP, nindP, cval, x, t);
+        return;
+    }
+    const int i = ((blockIdx.x - nbT) * blockDim.x + threadIdx.x) / L, lane = threadIdx.x & (L - 1);
     float y[3] = {0.f, 0.f, 0.f};
     if (i < P.Nf) {
         const int n = nfc[i];
@@ -1299,31 +1342,6 @@ __global__ void __launch_bounds__(256) k_pen_visc(DevParams P, const int4* __res
     }
 }
 
-// lambda_k t_k, t = C^T x in FP64 from the particle's own P-list:
-// C_jk = - C_kj (to the rounding of the minimum image), and C_kk for a fluid
-// row itself
-template <int D>
-__global__ void __launch_bounds__(128) k_pen_ct64(DevParams P, const int* __restrict__ type, const int* __restrict__ ncp,
-                                                  const long long* __restrict__ nptrP, const int* __restrict__ nindP,
-                                                  const double* __restrict__ cval, const double* __restrict__ x, double* __restrict__ t)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= P.N) return;
-    const long long b = nptrP[k];
-    const int n = ncp[k];
-    double s = 0.0;
-#pragma unroll 2
-    for (int a = 0; a < n; ++a) {
-        const int j = nindP[b + a];
-        if (j >= P.Nf) continue;
-        double v = 0.0;
-#pragma unroll
-        for (int d = 0; d < D; ++d) v += cval[(b + a) * D + d] * x[(size_t)j * D + d];
-        s = j == k ? s + v : s - v;
-    }
-    t[k] = P.lambda[type[k]] * s;
-}
-
 template <int D>
 __global__ void __launch_bounds__(128) k_pen_resid(DevParams P, const int* __restrict__ type, const int* __restrict__ nc,
                                                    const int* __restrict__ nfc, const int* __restrict__ ncp,
@@ -1376,8 +1394,10 @@ __global__ void __launch_bounds__(kReduceThreads) k_pen_phase(int n, const doubl
                                                               float* __restrict__ s, float* __restrict__ z, double inv_scale,
                                                               const double* __restrict__ scale_src, double tol_in2, double tol_out2,
                                                               double* __restrict__ scal, int* __restrict__ flags,
-                                                              double* __restrict__ partials, unsigned* __restrict__ counter)
+                                                              double* __restrict__ partials, unsigned* __restrict__ counter,
+                                                              unsigned* __restrict__ crossings)
 {
+    if (crossings && blockIdx.x == 0 && threadIdx.x == 0) *crossings = 0u;   // of the resident launch that follows
     const double sc = scale_src ? 1.0 / *scale_src : inv_scale;
     float acc = 0.f;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
@@ -1434,7 +1454,7 @@ static void pen_shape(mph_case* c)
 {
     const int N = c->dp.N;
     const int cap = cr_capacity(c->dim);
-    const int rows = std::max(kCrMinRows, cap > 0 ? ((N + cap - 1) / cap + 31) / 32 * 32 : 0);
+    const int rows = std::max(c->dim == 2 ? kCrMinRows2 : kCrMinRows3, cap > 0 ? ((N + cap - 1) / cap + 31) / 32 * 32 : 0);
     c->pen_resident = rows <= kCrThreads && (long long)rows * cap >= N && cr_smem(c, rows, (pen_ucap(rows) + 127) / 128 * 128) <= kCrSmem;
     if (c->pen_resident) { c->pen_rows = rows; c->pen_w = kCrThreads / rows; }
     else if (N > 152 * 512) { c->pen_rows = 256; c->pen_w = 1; }
@@ -1529,7 +1549,10 @@ int launch_pen_assemble(mph_case* c)
     c->level0_done = c->ct_ready = false;
     if (!d.ipos) MPH_CUDA(cudaMalloc((void**)&d.ipos, (size_t)P.N * sizeof(int4)));
     if (!d.vpos) MPH_CUDA(cudaMalloc((void**)&d.vpos, (size_t)P.N * sizeof(int4)));
-    if (!d.z4) MPH_CUDA(cudaMalloc((void**)&d.z4, (size_t)P.Nf * 2 * sizeof(float4)));
+    if (!d.z4) {   // components that a record does not use stay zero
+        MPH_CUDA(cudaMalloc((void**)&d.z4, (size_t)P.Nf * 2 * sizeof(float4)));
+        MPH_CUDA(cudaMemsetAsync(d.z4, 0, (size_t)P.Nf * 2 * sizeof(float4), st));
+    }
     if (!d.vacc) MPH_CUDA(cudaMalloc((void**)&d.vacc, n * sizeof(double)));
     if (!d.v32) MPH_CUDA(cudaMalloc((void**)&d.v32, n * 8 * sizeof(float)));
     if (!d.tct) MPH_CUDA(cudaMalloc((void**)&d.tct, (size_t)(P.N + 1) * sizeof(double)));
@@ -1569,9 +1592,10 @@ static void pen_residual(mph_case* c, double scale, const double* scale_src)
     DeviceState& d = c->d;
     const DevParams& P = c->dp;
     cudaStream_t st = c->stream;
-    { k_pen_visc<D, L, FIRST><<<grid_for((long long)P.Nf * L, 256), 256, 0, st>>>(P, d.vpos, d.nfc, d.nptr, d.nind, d.z4, d.wrap32, d.type,
-                                                                                d.pos, d.pos32, d.poslo32, scale, scale_src, d.vacc); MPH_COUNT_LAUNCH(); }
-    { k_pen_ct64<D><<<grid_for(P.N, 128), 128, 0, st>>>(P, d.type, d.ncp, d.nptrP, d.nindP, d.cval, d.x, d.tct); MPH_COUNT_LAUNCH(); }
+    const unsigned nbT = grid_for(P.N, 256);
+    { k_pen_visc<D, L, FIRST><<<nbT + grid_for((long long)P.Nf * L, 256), 256, 0, st>>>(
+          P, (int)nbT, d.vpos, d.nfc, d.nptr, d.nind, d.z4, d.wrap32, d.type, d.pos, d.pos32, d.poslo32, scale, scale_src, d.vacc,
+          d.ncp, d.nptrP, d.nindP, d.cval, d.x, d.tct); MPH_COUNT_LAUNCH(); }
     { k_pen_resid<D><<<grid_for(P.Nf, 128), 128, 0, st>>>(P, d.type, d.nc, d.nfc, d.ncp, d.nptrP, d.nindP, d.cval, d.tct, d.sdiag64, d.vacc,
                                                           d.x, d.bvec, d.r, d.partials, (unsigned*)(d.flags + kFlagCounter), d.scal + kSRR); MPH_COUNT_LAUNCH(); }
 }
@@ -1579,18 +1603,18 @@ static void pen_residual(mph_case* c, double scale, const double* scale_src)
 // lanes a row of k_pen_visc: about 180 neighbours in 3-D, 37 in 2-D
 constexpr int kVisc3 = 16, kVisc2 = 8;
 
-// r = b - A x of the start value
+// r = b - A x of the start value (its records are in z4, k_x0)
 void launch_pen_start_residual(mph_case* c)
 {
-    DeviceState& d = c->d;
-    const int Nf = c->dp.Nf;
-    if (c->dim == 2) {
-        { k_pen_pack<2, true><<<grid_for(Nf, 256), 256, 0, c->stream>>>(Nf, d.x, nullptr, 0.0, nullptr, nullptr, d.z4); MPH_COUNT_LAUNCH(); }
-        pen_residual<2, kVisc2, true>(c, 0.0, nullptr);
-    } else {
-        { k_pen_pack<3, true><<<grid_for(Nf, 256), 256, 0, c->stream>>>(Nf, d.x, nullptr, 0.0, nullptr, nullptr, d.z4); MPH_COUNT_LAUNCH(); }
-        pen_residual<3, kVisc3, true>(c, 0.0, nullptr);
-    }
+    if (c->dim == 2) pen_residual<2, kVisc2, true>(c, 0.0, nullptr);
+    else pen_residual<3, kVisc3, true>(c, 0.0, nullptr);
+}
+
+// the residual after a resident phase, which has updated x and left z in z4
+void launch_pen_residual(mph_case* c, double scale)
+{
+    if (c->dim == 2) pen_residual<2, kVisc2, false>(c, scale, nullptr);
+    else pen_residual<3, kVisc3, false>(c, scale, nullptr);
 }
 
 // x += scale z and the residual after a phase
@@ -1600,13 +1624,15 @@ void launch_pen_refine(mph_case* c, double scale, const double* scale_src, const
     const int Nf = c->dp.Nf;
     const float* z = d.v32 + (size_t)Nf * c->dim;
     if (c->dim == 2) {
-        { k_pen_pack<2, false><<<grid_for(Nf, 256), 256, 0, c->stream>>>(Nf, d.x, z, scale, scale_src, flags, d.z4); MPH_COUNT_LAUNCH(); }
+        { k_pen_pack<2><<<grid_for(Nf, 256), 256, 0, c->stream>>>(Nf, d.x, z, scale, scale_src, flags, d.z4); MPH_COUNT_LAUNCH(); }
         pen_residual<2, kVisc2, false>(c, scale, scale_src);
     } else {
-        { k_pen_pack<3, false><<<grid_for(Nf, 256), 256, 0, c->stream>>>(Nf, d.x, z, scale, scale_src, flags, d.z4); MPH_COUNT_LAUNCH(); }
+        { k_pen_pack<3><<<grid_for(Nf, 256), 256, 0, c->stream>>>(Nf, d.x, z, scale, scale_src, flags, d.z4); MPH_COUNT_LAUNCH(); }
         pen_residual<3, kVisc3, false>(c, scale, scale_src);
     }
 }
+
+static unsigned* cr_count(const mph_case* c) { return (unsigned*)(c->d.cr_vals + 8 * kCrBlocks); }
 
 void launch_pen_phase(mph_case* c, double inv_scale, const double* scale_src, double tol_in2, double tol_out2)
 {
@@ -1615,7 +1641,7 @@ void launch_pen_phase(mph_case* c, double inv_scale, const double* scale_src, do
     float* v = d.v32;
     { k_pen_phase<<<std::min<int>(grid_for(n, kReduceThreads), kReduceBlocks), kReduceThreads, 0, c->stream>>>(
           n, d.r, v + 7 * (size_t)n, v + 2 * (size_t)n, v + (size_t)n, inv_scale, scale_src, tol_in2, tol_out2, d.scal, d.flags, d.partials,
-          (unsigned*)(d.flags + kFlagCounter)); MPH_COUNT_LAUNCH(); }
+          (unsigned*)(d.flags + kFlagCounter), c->pen_resident ? cr_count(c) : nullptr); MPH_COUNT_LAUNCH(); }
 }
 
 static PenArgs pen_args(const mph_case* c, int cap)
@@ -1653,7 +1679,7 @@ static PenArgs pen_args(const mph_case* c, int cap)
 }
 
 // The phase's iterations in one cooperative launch
-int launch_pen_resident(mph_case* c, int cap)
+int launch_pen_resident(mph_case* c, int cap, double scale)
 {
     DeviceState& d = c->d;
     PenArgs A = pen_args(c, cap);
@@ -1662,8 +1688,11 @@ int launch_pen_resident(mph_case* c, int cap)
     C.rec = d.cr_rec;
     C.v3 = d.cr_vals;
     C.v1 = d.cr_vals + 6 * kCrBlocks;
-    C.count = (unsigned*)(d.cr_vals + 8 * kCrBlocks);
-    MPH_CUDA(cudaMemsetAsync(C.count, 0, sizeof(unsigned), c->stream));
+    C.count = cr_count(c);   // zeroed by k_pen_phase
+    C.scale = scale;
+    C.x = d.x;
+    C.vel = d.vel;
+    C.z4 = d.z4;
     const dim3 blk(c->pen_rows, c->pen_w);
     void* args[] = {&c->dp, &A, &C};
     const size_t smem = cr_smem(c, c->pen_rows, c->pen_umax);

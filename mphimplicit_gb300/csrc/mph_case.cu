@@ -407,8 +407,8 @@ int case_alloc_particles(mph_case* c)
     MPH_TRY(dalloc(c, &d.q, n));
     MPH_TRY(dalloc(c, &d.u, n));
     MPH_TRY(dalloc(c, &d.partials, (size_t)std::max<size_t>(kReduceBlocks, Nf / 16 + 64)));   // three values a 64-row block
-    MPH_TRY(dalloc(c, &d.scal, 32));
-    MPH_TRY(dalloc(c, &d.flags, kFlagCount));
+    MPH_TRY(dalloc(c, &d.scal, 32 + kFlagCount * sizeof(int) / sizeof(double)));
+    d.flags = reinterpret_cast<int*>(d.scal + 32);   // one read brings both
     MPH_TRY(dalloc(c, &d.bbox, 8));
     MPH_TRY(dalloc(c, &d.totals, 8));
     MPH_TRY(dalloc(c, &d.dmax, 4));

@@ -437,7 +437,8 @@ int pen_exact_diag(mph_case* c);
 void launch_pen_start_residual(mph_case* c);
 void launch_pen_refine(mph_case* c, double scale, const double* scale_src, const int* flags);
 void launch_pen_phase(mph_case* c, double inv_scale, const double* scale_src, double tol_in2, double tol_out2);
-int launch_pen_resident(mph_case* c, int cap);
+int launch_pen_resident(mph_case* c, int cap, double scale);
+void launch_pen_residual(mph_case* c, double scale);
 void launch_pen_operator(mph_case* c, int cap);
 void launch_pen_vectors(mph_case* c, int cap, bool use_cond, cudaGraphConditionalHandle cond);
 size_t batch_pen_bytes();

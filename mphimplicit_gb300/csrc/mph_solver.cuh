@@ -22,6 +22,8 @@ enum { kFlagDone = 0, kFlagIter = 1, kFlagCap = 2, kFlagBad = 3, kFlagCounter = 
 
 __host__ __device__ __forceinline__ int cr_rho_slot(int it) { return kSRho + 8 + (it & 1); }   // FP64 form: two alternating slots
 
+constexpr size_t kSolveStateBytes = 32 * sizeof(double) + kFlagCount * sizeof(int);   // scalars, then flags
+
 constexpr int kReduceBlocks = 1216;   // 152 SMs x 8 blocks: bound on the partials count
 constexpr int kGraphChunk = 8;        // CR iterations per captured graph chunk (FP64 form; the mixed form's option "chunk")
 constexpr int kMaxGraphChunk = 32;
