@@ -2,7 +2,7 @@
 //
 //   k_density       : calculateDensityA + calculateGravityCenter +
 //                     calculateDensityP (main.cpp:1737, 1767, 1903) in one
-//                     neighbour pass; every sum keeps the reference's order
+//                     neighbour pass, in the list's order
 //   k_pressure_a_*  : calculatePressureA (main.cpp:1801)
 //   k_diffuse       : calculateDiffuseInterface (main.cpp:1851)
 //   k_accelerate    : calculatePhysicalCoefficients' mass (main.cpp:1710),
@@ -18,12 +18,28 @@
 
 namespace mph {
 
+// sqrt(v) of v >= 0 from the reciprocal square root: v y and one residual
+// correction (P. Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000", 1990), within a hair of half a unit in the last place
+__device__ __forceinline__ double sqrt_by_rsqrt(double v)
+{
+    if (__double_as_longlong(v) == 0) return 0.0;
+    const double y = rsqrt(v), r = v * y;
+    return __fma_rn(__fma_rn(-r, r, v), 0.5 * y, r);
+}
+
 // The density pass is bound by the FP64 pipe (about 180 neighbours a particle
-// in 3-D, all of them inside the radii): its divisions are all by constants
-// of the case, so they go through div_const (5 FP64 operations with the bits
-// of the quotient), q = r / RadiusA serves both weights (RadiusG is RadiusA),
-// and the radius tests compare bit patterns on the integer pipe.  Every value
-// keeps its bits.  9.69 -> 6.42 ms on 326,592 particles.
+// in 3-D, all of them inside the radii).  The weights' constants stand before
+// the sums, w_a = kf t (1 - t)^2 and w = kf (1 - t)^2 with t = r / RadiusA
+// (RadiusG is RadiusA, main.cpp:236-307, 888), so a pair is one root, one
+// 1 - t, two products for the density and a product and three multiply-adds
+// for the gravity centre: some 37 FP64 operations where the reference's terms
+// one by one took 80, with roundings left out accordingly.  The sums run in
+// pieces of 32 neighbours, which keeps their own roundings below those of one
+// long sum.  The radius tests compare bit patterns on the integer pipe.
+// 326,592 particles: 6.42 -> 2.79 ms; 71,300: 1.84 -> 0.80.
+constexpr int kDensityRun = 32;
+
 template <int D>
 __global__ void __launch_bounds__(128) k_density(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
                                                  const int* __restrict__ nc, const long long* __restrict__ nptr,
@@ -39,34 +55,41 @@ __global__ void __launch_bounds__(128) k_density(DevParams P, const int* __restr
     double sa = 0.0, sp = 0.0, sg[3] = {0.0, 0.0, 0.0};
     const long long b = nptr[i];
     const int n = nc[i];
-    for (int k = 0; k < n; ++k) {
-        const int j = nind[b + k];
-        if (j == i) continue;
-        double xj[3], q[3];
-        load_vec<D>(pos, j, xj);
-        sep_vec<D>(P, xj, xi, q);
-        const double r2 = norm2_exact<D>(q);
-        const bool inA = r2_within(r2, rA2), inP = r2_within(r2, rP2);   // RadiusG = RadiusA (main.cpp:888)
-        if (!(inA || inP)) continue;
-        const double r = __dsqrt_rn(r2);
-        if (inA) {
-            const double ratio = P.ratio[ti][type[j]];
-            const double t = div_const(r, P.rA, P.inv_ra);
-            const double oq = DSUB(1.0, t);
-            // w_a and w_quad with their common quotient (main.cpp:236-307)
-            sa = DADD(sa, DMUL(ratio, DMUL(DMUL(DMUL(P.kfa, t), oq), oq)));
-            const double w = DMUL(ratio, DMUL(P.kfg, DMUL(oq, oq)));
+    for (int k0 = 0; k0 < n; k0 += kDensityRun) {
+        double ra = 0.0, rp = 0.0, rg[3] = {0.0, 0.0, 0.0};
+        for (int k = k0; k < min(n, k0 + kDensityRun); ++k) {
+            const int j = nind[b + k];
+            if (j == i) continue;
+            double xj[3], q[3];
+            load_vec<D>(pos, j, xj);
+            sep_vec<D>(P, xj, xi, q);
+            const double r2 = norm2_fma<D>(q);
+            const bool inA = r2_within(r2, rA2), inP = r2_within(r2, rP2);
+            if (!(inA || inP)) continue;
+            const double r = sqrt_by_rsqrt(r2);
+            if (inA) {
+                const double ratio = P.ratio[ti][type[j]];
+                const double oq = __fma_rn(-r, P.inv_ra_lo, __fma_rn(-r, P.inv_ra, 1.0)), w = ratio * (oq * oq);
+                ra += r * w;
 #pragma unroll
-            for (int d = 0; d < D; ++d) sg[d] = DADD(sg[d], DMUL(div_const(DMUL(q[d], w), P.R2g, P.inv_R2g), P.rG));
+                for (int d = 0; d < D; ++d) rg[d] += w * q[d];
+            }
+            if (inP) {
+                const double oq = __fma_rn(-r, P.inv_rp, 1.0);
+                rp += oq * oq;
+            }
         }
-        if (inP) {
-            const double oq = DSUB(1.0, div_const(r, P.rP, P.inv_rp));
-            sp = DADD(sp, DMUL(P.kfp, DMUL(oq, oq)));
-        }
+        sa += ra;
+        sp += rp;
+#pragma unroll
+        for (int d = 0; d < D; ++d) sg[d] += rg[d];
     }
-    densA[i] = sa;
+    densA[i] = sa * (P.kfa * P.inv_ra);
+    const double cg = P.kfg * P.rG / P.R2g;
+#pragma unroll
+    for (int d = 0; d < D; ++d) sg[d] *= cg;
     store_vec<D>(gcen, i, sg);
-    vsp[i] = DSUB(sp, P.N0p);
+    vsp[i] = __fma_rn(P.kfp, sp, -P.N0p);
 }
 
 __global__ void k_pressure_a(DevParams P, const int* __restrict__ type, const double* __restrict__ densA, double* __restrict__ presA)
@@ -307,8 +330,9 @@ __global__ void __launch_bounds__(128) k_output_forces(DevParams P, const int* _
 }
 
 // calculateDensityP alone over the P-list.  The P-list holds exactly the
-// pairs with r^2 <= RadiusP^2, in the full list's order, so the sum is
-// bit-identical to the full-list pass.
+// pairs with r^2 <= RadiusP^2, in the full list's order (the sum differs from
+// the full-list pass's by the rounding of its pieces).  As k_density: 37 FP64
+// operations a pair became 28; 340 -> 243 us on 374,000 particles.
 template <int D>
 __global__ void __launch_bounds__(128) k_density_p(DevParams P, const double* __restrict__ pos, const int* __restrict__ ncp,
                                                    const long long* __restrict__ nptrP, const int* __restrict__ nindP,
@@ -328,13 +352,13 @@ __global__ void __launch_bounds__(128) k_density_p(DevParams P, const double* __
         double xj[3], q[3];
         load_vec<D>(pos, j, xj);
         sep_vec<D>(P, xj, xi, q);
-        const double r2 = norm2_exact<D>(q);
-        if (r2_within(r2, rP2)) {
-            const double oq = DSUB(1.0, div_const(__dsqrt_rn(r2), P.rP, P.inv_rp));   // w_quad
-            sp = DADD(sp, DMUL(P.kfp, DMUL(oq, oq)));
+        const double r2 = norm2_fma<D>(q);
+        if (r2_within(r2, rP2)) {   // w_quad
+            const double oq = __fma_rn(-sqrt_by_rsqrt(r2), P.inv_rp, 1.0);
+            sp += oq * oq;
         }
     }
-    vsp[i] = DSUB(sp, P.N0p);
+    vsp[i] = __fma_rn(P.kfp, sp, -P.N0p);
 }
 
 static void launch_density_p(mph_case* c)

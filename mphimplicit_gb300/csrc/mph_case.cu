@@ -165,7 +165,7 @@ static int derive(mph_case* c, const mph_particles* parts)
     P.inv_rp = 1.0 / P.rP;
     P.m2h_rp = -2.0 / P.rP;
     P.inv_ra = 1.0 / P.rA;
-    P.inv_R2g = 1.0 / P.R2g;
+    P.inv_ra_lo = std::fma(-P.rA, P.inv_ra, 1.0) / P.rA;
     for (int t = 0; t < kTypeCount; ++t)
         for (int u = 0; u < kTypeCount; ++u)
             P.muij[t][u] = 2.0 * (P.mu[t] * P.mu[u]) / (P.mu[t] + P.mu[u]);

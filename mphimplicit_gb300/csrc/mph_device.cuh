@@ -68,6 +68,14 @@ __device__ __forceinline__ double norm2_exact(const double* q)
 }
 
 template <int D>
+__device__ __forceinline__ double norm2_fma(const double* q)
+{
+    double s = __fma_rn(q[1], q[1], q[0] * q[0]);
+    if (D == 3) s = __fma_rn(q[2], q[2], s);
+    return s;
+}
+
+template <int D>
 __device__ __forceinline__ void load_vec(const double* __restrict__ a, int i, double* v)
 {
     if (D == 2) {
@@ -107,20 +115,6 @@ __device__ __forceinline__ void sep_vec(const DevParams& P, const double* xj, co
 {
 #pragma unroll
     for (int d = 0; d < D; ++d) q[d] = sep_exact(xj[d], xi[d], P.hw[d], P.dw[d], P.wsafe[d]);
-}
-
-// a / c rounded to nearest for a constant c > 0, with y = 1 / c rounded to
-// nearest: a first quotient and two residual corrections (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000", 1990:
-// the first correction gives a quotient within one unit in the last place,
-// the second the correctly rounded one).  Five FP64 operations; for the
-// lengths and weights it serves (normal numbers, no over- or underflow in the
-// residuals; 0 and NaN pass through) it has the bits of __ddiv_rn.
-__device__ __forceinline__ double div_const(double a, double c, double y)
-{
-    double q = DMUL(a, y);
-    q = __fma_rn(__fma_rn(-q, c, a), y, q);
-    return __fma_rn(__fma_rn(-q, c, a), y, q);
 }
 
 // The warp sums of D per-lane FP64 values by reduce-scatter: the same pairs,

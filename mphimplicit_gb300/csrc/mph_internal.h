@@ -56,7 +56,7 @@ struct DevParams {
     double gravity[3];
     double visc;                               // 8 (2D) or 10 (3D)
     double inv_rv, m2h_rv, inv_rp, m2h_rp;     // 1/h and -2/h of the V and P kernels (assembly)
-    double inv_ra, inv_R2g;                    // 1/h of the A and G kernels, 1/R2g
+    double inv_ra, inv_ra_lo;                  // 1/RadiusA and its remainder
     double muij[kTypeCount][kTypeCount];       // harmonic mean 2 mu_i mu_j / (mu_i + mu_j)
     double inert64[kTypeCount];                // density * vol / vol / dt in that order (the reference's inertia), once
     float maxR2_lo, maxR2_hi, rP2_lo, rP2_hi;  // FP32 pre-classification band
