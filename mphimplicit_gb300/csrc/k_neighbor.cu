@@ -151,9 +151,16 @@ __global__ void __launch_bounds__(128) k_neighbors(DevParams P, int rx, int ry, 
 // on every axis) needs no minimum-image correction in FP32.  A bucket with
 // more than kNbMaxP particles, a pass with more than kNbCap candidates, a walk
 // of more than 27 cells or the exact-only mode runs the per-thread walk.
-constexpr int kNbThreads = 256;
-constexpr int kNbCap = 1536;
+//
+// In 2-D a cell has about 10 particles and 90 candidates, so the blocks are
+// small and many: 64 threads and room for 512 candidates (30 KB of shared
+// memory a block of eight warps held an SM to seven blocks and left their
+// start and staging latencies uncovered).  Both passes on 735,000 particles 1.0 -> 0.63
+// ms (0.71 with 128 threads).  In 3-D, 30 and 810: 256 threads, 1536.
+template <int D> constexpr int kNbThreads = D == 2 ? 64 : 256;   // at least two warps: one a pass reads the walk's buckets
+template <int D> constexpr int kNbCap = D == 2 ? 512 : 1536;
 constexpr int kNbMaxP = 256;
+static_assert(kNbThreads<2> >= 64 && kNbThreads<3> >= 64, "a warp for each of the two passes");
 
 // The FP32 squared distance of a staged candidate (the minimum image only
 // for a walk that wraps), as classify computes it.
@@ -191,15 +198,15 @@ __device__ __forceinline__ int classify_exact(const DevParams& P, const double* 
 }
 
 template <int D, bool FILL>
-__global__ void __launch_bounds__(kNbThreads) k_neighbors_cells(DevParams P, int rx, int ry, int rz, int wB, int wE,
+__global__ void __launch_bounds__(kNbThreads<D>) k_neighbors_cells(DevParams P, int rx, int ry, int rz, int wB, int wE,
                                                                 const int* __restrict__ key, const int* __restrict__ bucket,
                                                                 const double* __restrict__ pos, const float* __restrict__ pos32,
                                                                 int* __restrict__ nc, int* __restrict__ nfc, int* __restrict__ ncp,
                                                                 const long long* __restrict__ nptr, const long long* __restrict__ nptrP,
                                                                 int* __restrict__ nind, int* __restrict__ nindP)
 {
-    __shared__ float4 spos[kNbCap];
-    __shared__ int sj[kNbCap];
+    __shared__ float4 spos[kNbCap<D>];
+    __shared__ int sj[kNbCap<D>];
     __shared__ int coff[2][28];
     __shared__ int cbeg[2][27];
     __shared__ int sn0[kNbMaxP], snp0[kNbMaxP];
@@ -246,7 +253,7 @@ __global__ void __launch_bounds__(kNbThreads) k_neighbors_cells(DevParams P, int
             if (lane == 0) coff[pass][0] = 0;
         }
         __syncthreads();
-        slow = coff[0][ncell] > kNbCap || coff[1][ncell] > kNbCap;
+        slow = coff[0][ncell] > kNbCap<D> || coff[1][ncell] > kNbCap<D>;
     }
     if (slow) {   // the same for every thread of the block
         for (int i = r0 + tid; i < r1; i += blockDim.x)
@@ -559,10 +566,10 @@ static void launch_neighbors_cells(mph_case* c, const int* r)
     const unsigned g = (unsigned)(2 * c->dp.T);
     DeviceState& d = c->d;
     if (c->dim == 2)
-        k_neighbors_cells<2, FILL><<<g, kNbThreads, 0, c->stream>>>(c->dp, r[0], r[1], r[2], c->wB, c->wE, d.key, d.bucket, d.pos, d.pos32,
+        k_neighbors_cells<2, FILL><<<g, kNbThreads<2>, 0, c->stream>>>(c->dp, r[0], r[1], r[2], c->wB, c->wE, d.key, d.bucket, d.pos, d.pos32,
                                                                     d.nc, d.nfc, d.ncp, d.nptr, d.nptrP, d.nind, d.nindP);
     else
-        k_neighbors_cells<3, FILL><<<g, kNbThreads, 0, c->stream>>>(c->dp, r[0], r[1], r[2], c->wB, c->wE, d.key, d.bucket, d.pos, d.pos32,
+        k_neighbors_cells<3, FILL><<<g, kNbThreads<3>, 0, c->stream>>>(c->dp, r[0], r[1], r[2], c->wB, c->wE, d.key, d.bucket, d.pos, d.pos32,
                                                                     d.nc, d.nfc, d.ncp, d.nptr, d.nptrP, d.nind, d.nindP);
     MPH_COUNT_LAUNCH();
 }
