@@ -10,6 +10,8 @@
 // coordinate magnitudes at case creation (or the FP32 step is disabled).
 #include <algorithm>
 
+#include <type_traits>
+
 #include "mph_device.cuh"
 
 namespace mph {
@@ -152,6 +154,11 @@ __global__ void __launch_bounds__(128) k_neighbors(DevParams P, int rx, int ry, 
 // more than kNbMaxP particles, a pass with more than kNbCap candidates, a walk
 // of more than 27 cells or the exact-only mode runs the per-thread walk.
 //
+// The walk is bound by the integer pipe, some 45 instructions a chunk of 32
+// candidates in its first form; the bands are now tested by ballots, the
+// candidate's index rides in its record and the wrap is decided outside the
+// loop: both passes on 1.3 million particles 4.7 -> 4.0 ms.
+//
 // In 2-D a cell has about 10 particles and 90 candidates, so the blocks are
 // small and many: 64 threads and room for 512 candidates (30 KB of shared
 // memory a block of eight warps held an SM to seven blocks and left their
@@ -164,24 +171,16 @@ static_assert(kNbThreads<2> >= 64 && kNbThreads<3> >= 64, "a warp for each of th
 
 // The FP32 squared distance of a staged candidate (the minimum image only
 // for a walk that wraps), as classify computes it.
-template <int D>
-__device__ __forceinline__ float d2_staged(const DevParams& P, bool wrap, const float* xi32, const float4 pj)
+template <int D, bool WRAP>
+__device__ __forceinline__ float d2_staged(const DevParams& P, const float* xi32, const float4 pj)
 {
-    float a = pj.x - xi32[0], b = pj.y - xi32[1];
-    if (D == 2) {
-        if (wrap) {
-            a = a > P.hw32[0] ? a - P.w32[0] : (a < -P.hw32[0] ? a + P.w32[0] : a);
-            b = b > P.hw32[1] ? b - P.w32[1] : (b < -P.hw32[1] ? b + P.w32[1] : b);
-        }
-        return a * a + b * b;
-    }
-    float e = pj.z - xi32[2];
-    if (wrap) {
+    float a = pj.x - xi32[0], b = pj.y - xi32[1], e = D == 3 ? pj.z - xi32[2] : 0.f;
+    if (WRAP) {
         a = a > P.hw32[0] ? a - P.w32[0] : (a < -P.hw32[0] ? a + P.w32[0] : a);
         b = b > P.hw32[1] ? b - P.w32[1] : (b < -P.hw32[1] ? b + P.w32[1] : b);
-        e = e > P.hw32[2] ? e - P.w32[2] : (e < -P.hw32[2] ? e + P.w32[2] : e);
+        if (D == 3) e = e > P.hw32[2] ? e - P.w32[2] : (e < -P.hw32[2] ? e + P.w32[2] : e);
     }
-    return a * a + b * b + e * e;
+    return D == 3 ? a * a + b * b + e * e : a * a + b * b;
 }
 
 // The reference's FP64 decision for a pair inside the FP32 band.
@@ -206,7 +205,6 @@ __global__ void __launch_bounds__(kNbThreads<D>) k_neighbors_cells(DevParams P, 
                                                                 int* __restrict__ nind, int* __restrict__ nindP)
 {
     __shared__ float4 spos[kNbCap<D>];
-    __shared__ int sj[kNbCap<D>];
     __shared__ int coff[2][28];
     __shared__ int cbeg[2][27];
     __shared__ int sn0[kNbMaxP], snp0[kNbMaxP];
@@ -264,8 +262,7 @@ __global__ void __launch_bounds__(kNbThreads<D>) k_neighbors_cells(DevParams P, 
         const int F = coff[pass][ncell];
         // candidates F.. up to a multiple of 32: far away, never neighbours
         for (int k = F + tid; k < ((F + 31) & ~31); k += blockDim.x) {
-            spos[k] = make_float4(1e18f, 1e18f, 1e18f, 0.f);
-            sj[k] = -1;
+            spos[k] = make_float4(1e18f, 1e18f, 1e18f, __int_as_float(-1));
         }
         for (int t = wl; t < ncell; t += nw) {
             const int beg = cbeg[pass][t], off = coff[pass][t], cnt = coff[pass][t + 1] - off;
@@ -278,8 +275,8 @@ __global__ void __launch_bounds__(kNbThreads<D>) k_neighbors_cells(DevParams P, 
                 } else {
                     pj = reinterpret_cast<const float4*>(pos32)[j];
                 }
+                pj.w = __int_as_float(j);
                 spos[off + k] = pj;
-                sj[off + k] = j;
             }
         }
         __syncthreads();
@@ -300,32 +297,35 @@ __global__ void __launch_bounds__(kNbThreads<D>) k_neighbors_cells(DevParams P, 
             float xi32[3] = {0.f, 0.f, 0.f};
             load_xi32<D>(pos32, i, xi32);
             const unsigned lt = (1u << lane) - 1u;
-            for (int c0 = 0; c0 < F; c0 += 32) {
-                const int c = c0 + lane;
-                // FP32 first: far (> the band above MaxRadius^2), or inside
-                // MaxRadius and clear of the RadiusP band; the rest exactly
-                const float d2 = d2_staged<D>(P, wrap, xi32, spos[c]);
-                const bool inM = d2 < P.maxR2_lo, inP = d2 < P.rP2_lo;
-                const bool sure = d2 > P.maxR2_hi || (inM && (inP || d2 > P.rP2_hi));
-                bool m = sure && inM, pp = sure && inP;
-                if (__any_sync(full, !sure)) {
-                    if (!sure) {
-                        const int cl = classify_exact<D>(P, pos, i, sj[c]);
-                        m = cl & 1;
-                        pp = (cl & 2) != 0;
+            auto walk = [&](auto WR) {
+                for (int c0 = 0; c0 < F; c0 += 32) {
+                    // FP32 first: below the band around a squared radius in,
+                    // above it out; a chunk with a candidate inside a band
+                    // (the two ballots differ) asks exactly
+                    const float4 pj = spos[c0 + lane];
+                    const float d2 = d2_staged<D, decltype(WR)::value>(P, xi32, pj);
+                    unsigned bm = __ballot_sync(full, d2 < P.maxR2_lo), bp = __ballot_sync(full, d2 < P.rP2_lo);
+                    const unsigned hm = __ballot_sync(full, !(d2 > P.maxR2_hi)), hp = __ballot_sync(full, !(d2 > P.rP2_hi));
+                    if ((bm ^ hm) | (bp ^ hp)) {
+                        bool m = (bm >> lane) & 1u, pp = (bp >> lane) & 1u;
+                        if ((((bm ^ hm) | (bp ^ hp)) >> lane) & 1u) {
+                            const int cl = classify_exact<D>(P, pos, i, __float_as_int(pj.w));
+                            m = cl & 1;
+                            pp = (cl & 2) != 0;
+                        }
+                        bm = __ballot_sync(full, m);
+                        bp = __ballot_sync(full, pp);
                     }
-                }
-                const unsigned bm = __ballot_sync(full, m), bp = __ballot_sync(full, pp);
-                if (FILL) {
-                    if (bm) {
-                        const int j = sj[c];
-                        if (m) outM[n + __popc(bm & lt)] = j;
-                        if (pp) outP[np + __popc(bp & lt)] = j;
+                    if (FILL) {
+                        if ((bm >> lane) & 1u) outM[n + __popc(bm & lt)] = __float_as_int(pj.w);
+                        if ((bp >> lane) & 1u) outP[np + __popc(bp & lt)] = __float_as_int(pj.w);
                     }
+                    n += __popc(bm);
+                    np += __popc(bp);
                 }
-                n += __popc(bm);
-                np += __popc(bp);
-            }
+            };
+            if (wrap) walk(std::true_type());
+            else walk(std::false_type());
             if (lane == 0) {
                 if (pass == 0) {
                     sn0[pi] = n;
