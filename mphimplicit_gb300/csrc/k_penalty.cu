@@ -63,6 +63,7 @@ constexpr int kCrBlocks = 2 * 152;
 // but the blocks of a solve hold their SMs until it ends: an ensemble of 64
 // two-dimensional cases on their streams takes 52.9, 46.3, 37.9 and 37.5 ms
 // with 192, 256, 384 and 512.
+constexpr int kCrAhead = 3;        // staged neighbours a thread loads while alpha and beta are formed, in blocks alone on their SM
 constexpr int kCrMinRows3 = 192, kCrMinRows2 = 384;
 constexpr int kCrSmem = 100 * 1024;   // dynamic: two blocks an SM with their 7 KB of static shared memory
 // Staged neighbours a block of `rows` rows has room for.  Blocks of a
@@ -793,8 +794,8 @@ __device__ __forceinline__ void cr_publish(float4* rec, int i, const float* s, c
     }
 }
 
-template <int D>
-__global__ void __launch_bounds__(kCrThreads, 2) k_pen_cr(DevParams P, PenArgs A, PenCr C)
+template <int D, int PF>
+__global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams P, PenArgs A, PenCr C)
 {
     extern __shared__ int4 pen_smem[];
     __shared__ float wred[3][kCrThreads / 32];
@@ -823,7 +824,9 @@ __global__ void __launch_bounds__(kCrThreads, 2) k_pen_cr(DevParams P, PenArgs A
         ul[k] = j;
         sa[k] = A.ipos[j];
     }
-    const int j0 = tid < U ? ul[tid] : -1;   // the thread's first staged neighbour
+    int j0[PF];   // the thread's first staged neighbours
+#pragma unroll
+    for (int u = 0; u < PF; ++u) j0[u] = tid + u * nth < U ? ul[tid + u * nth] : -1;
     int ng = 0;
     if (U >= 0 && n > 0) {
         ng = A.groups[i >> 5];
@@ -878,7 +881,9 @@ __global__ void __launch_bounds__(kCrThreads, 2) k_pen_cr(DevParams P, PenArgs A
     bool ok = cr_cross(C.count, C.v3, val_s, 6, ++epoch, lb, nb, tid, A.flags);   // every row's s is out
     // a crossing's first loads: the thread's first neighbour's records, while
     // alpha and beta are formed
-    CrRec pre = cr_load<D>(C.rec, j0, A.Nf);
+    CrRec pre[PF];
+#pragma unroll
+    for (int u = 0; u < PF; ++u) pre[u] = cr_load<D>(C.rec, j0[u], A.Nf);
     while (ok) {
         // the new vectors of the own row (not before the phase's first iteration)
         if (!first) {
@@ -911,9 +916,11 @@ __global__ void __launch_bounds__(kCrThreads, 2) k_pen_cr(DevParams P, PenArgs A
                 sa[k].w = __float_as_int(v[1]);
             }
         };
-        if (tid < U) put(tid, pre);
+#pragma unroll
+        for (int u = 0; u < PF; ++u)
+            if (tid + u * nth < U) put(tid + u * nth, pre[u]);
 #pragma unroll 2
-        for (int k = tid + nth; k < U; k += nth) put(k, cr_load<D>(C.rec, ul[k], A.Nf));
+        for (int k = tid + PF * nth; k < U; k += nth) put(k, cr_load<D>(C.rec, ul[k], A.Nf));
         float si[3] = {s[0], s[1], s[2]};
         if (W > 1 && w > 0 && fluid && n > 0) cr_combine<D>(cr_load<D>(C.rec, i, A.Nf), alpha, beta, si);
         __syncthreads();
@@ -1041,7 +1048,8 @@ __global__ void __launch_bounds__(kCrThreads, 2) k_pen_cr(DevParams P, PenArgs A
         }
         // every row's s, a, b and every block's dot products are out
         if (!(ok = cr_cross(C.count, C.v3, val_s, 6, ++epoch, lb, nb, tid, A.flags))) break;
-        pre = cr_load<D>(C.rec, j0, A.Nf);
+#pragma unroll
+        for (int u = 0; u < PF; ++u) pre[u] = cr_load<D>(C.rec, j0[u], A.Nf);
         if (warp < 3) {
             const F2 v = cr_sum(C.v3 + 2 * warp, 6, nb, lane);
             if (lane == 0) sum_s[warp] = v;
@@ -1434,11 +1442,12 @@ static int cr_capacity(int dim)
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        cudaFuncSetAttribute(k_pen_cr<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCrSmem);
-        cudaFuncSetAttribute(k_pen_cr<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCrSmem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[0], k_pen_cr<2>, kCrThreads, kCrSmem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[1], k_pen_cr<3>, kCrThreads, kCrSmem);
-        for (int k = 0; k < 2; ++k) cap[k] = coop ? sms * nb[k] : 0;
+        const void* f[4] = {(const void*)k_pen_cr<2, 1>, (const void*)k_pen_cr<3, 1>, (const void*)k_pen_cr<2, kCrAhead>, (const void*)k_pen_cr<3, kCrAhead>};
+        for (const void* k : f) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCrSmem);
+        for (int k = 0; k < 2; ++k) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[k], f[k], kCrThreads, kCrSmem);
+            cap[k] = coop ? sms * nb[k] : 0;
+        }
     });
     return std::min(cap[dim - 2], kCrBlocks);
 }
@@ -1696,7 +1705,11 @@ int launch_pen_resident(mph_case* c, int cap, double scale)
     const dim3 blk(c->pen_rows, c->pen_w);
     void* args[] = {&c->dp, &A, &C};
     const size_t smem = cr_smem(c, c->pen_rows, c->pen_umax);
-    MPH_CUDA(cudaLaunchCooperativeKernel(c->dim == 2 ? (const void*)k_pen_cr<2> : (const void*)k_pen_cr<3>, dim3(nb), blk, args, smem, c->stream));
+    // a block an SM and the device to itself: the form with more registers
+    const bool alone = nb <= kCrBlocks / 2 && !c->shared_gpu;
+    const void* f = c->dim == 2 ? (alone ? (const void*)k_pen_cr<2, kCrAhead> : (const void*)k_pen_cr<2, 1>)
+                                : (alone ? (const void*)k_pen_cr<3, kCrAhead> : (const void*)k_pen_cr<3, 1>);
+    MPH_CUDA(cudaLaunchCooperativeKernel(f, dim3(nb), blk, args, smem, c->stream));
     MPH_COUNT_LAUNCH();
     return MPH_OK;
 }

@@ -110,6 +110,8 @@ int batch_step(mph_case** cases, int ncases, int nsteps, int workers)
         c->stream = c->own_stream;
         borrowed[k] = 1;
     }
+    if (ncases > 1)
+        for (int k = 0; k < ncases; ++k) cases[k]->shared_gpu = true;
     const int nw = workers > 0 ? std::min(workers, ncases) : default_workers(ncases);
     std::vector<int> status(ncases, MPH_OK);
     std::vector<std::string> msg(ncases);
@@ -203,8 +205,10 @@ int batch_step(mph_case** cases, int ncases, int nsteps, int workers)
                 msg[k] = "the solve did not converge";
             }
     }
-    for (int k = 0; k < ncases; ++k)
+    for (int k = 0; k < ncases; ++k) {
+        cases[k]->shared_gpu = false;
         if (borrowed[k]) cases[k]->stream = nullptr;
+    }
     int last = MPH_OK;
     for (int k = 0; k < ncases; ++k) {
         if (status[k] == MPH_OK) continue;
@@ -323,6 +327,7 @@ struct mph_server {
                         st = mph_case_set_option(r->c, r->options[k].first.c_str(), r->options[k].second);
                 }
                 if (st == MPH_OK) {
+                    r->c->shared_gpu = true;
                     const auto a = Clock::now();
                     st = mph::case_step(r->c, 1);
                     const float ms = std::chrono::duration<float, std::milli>(Clock::now() - a).count();

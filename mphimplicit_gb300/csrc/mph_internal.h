@@ -310,6 +310,7 @@ struct mph_case {
     bool level0_done = false;           // this step's level-0 multigrid stencils were written by the assembly
     bool step_f64 = false;              // this step's FP64 solve may run on k_f64op.cu's operator in parts
     long long f64_slots = 0;            // slots the pair records have room for (their two arrays' split)
+    bool shared_gpu = false;            // other cases step on this GPU meanwhile (a batch of several, a server)
     bool step_pen = false;              // this step's inner CR runs on k_penalty.cu's operator
     int pmax = 0;                       // longest P-list of the current lists
     int pen_rows = 0, pen_w = 0;        // its rows a block and threads a row

@@ -22,11 +22,21 @@ __device__ __forceinline__ F2 f2_mul(F2 a, F2 b)
     const float p = __fmul_rn(a.h, b.h);
     return f2_fast(p, __fadd_rn(__fmaf_rn(a.h, b.h, -p), __fmaf_rn(a.h, b.l, __fmul_rn(a.l, b.h))));
 }
+// a / b: a first quotient by the approximate reciprocal and two residual
+// corrections (Newton's method), without the FP32 division's own chain
 __device__ __forceinline__ F2 f2_div(F2 a, F2 b)
 {
-    const float q = __fdiv_rn(a.h, b.h);
+    const float m = fabsf(b.h);
+    if (!(m > 1e-30f && m < 1e30f)) {   // the reciprocal would leave FP32's normal range
+        const float q = __fdiv_rn(a.h, b.h);
+        const float r = __fadd_rn(__fmaf_rn(-q, b.h, a.h), __fmaf_rn(-q, b.l, a.l));
+        return f2_fast(q, __fdiv_rn(r, b.h));
+    }
+    const float y = __fdividef(1.f, b.h);
+    const float q0 = __fmul_rn(a.h, y);
+    const float q = __fmaf_rn(__fmaf_rn(-q0, b.h, a.h), y, q0);
     const float r = __fadd_rn(__fmaf_rn(-q, b.h, a.h), __fmaf_rn(-q, b.l, a.l));
-    return f2_fast(q, __fdiv_rn(r, b.h));
+    return f2_fast(q, __fmul_rn(r, y));
 }
 __device__ __forceinline__ F2 f2_of(double v)
 {
