@@ -1463,8 +1463,16 @@ static void pen_shape(mph_case* c)
 {
     const int N = c->dp.N;
     const int cap = cr_capacity(c->dim);
-    const int rows = std::max(c->dim == 2 ? kCrMinRows2 : kCrMinRows3, cap > 0 ? ((N + cap - 1) / cap + 31) / 32 * 32 : 0);
-    c->pen_resident = rows <= kCrThreads && (long long)rows * cap >= N && cr_smem(c, rows, (pen_ucap(rows) + 127) / 128 * 128) <= kCrSmem;
+    int rows = std::max(c->dim == 2 ? kCrMinRows2 : kCrMinRows3, cap > 0 ? ((N + cap - 1) / cap + 31) / 32 * 32 : 0);
+    // as long as the rows fit, one block an SM: half the blocks at a crossing
+    // and twice the registers (k_pen_resident's kCrAhead).  A step of 33,600
+    // particles in 3-D 2.44 -> 2.03 ms, 57,000 2.61 -> 2.42, 71,000 3.03 ->
+    // 2.75; 2-D the same either way.  (One block of up to 1024 threads an SM
+    // beyond 77,824 particles, with the registers of two: no difference.)
+    const int one = ((N + kCrBlocks / 2 - 1) / (kCrBlocks / 2) + 31) / 32 * 32;
+    auto fits = [c](int r) { return r <= kCrThreads && cr_smem(c, r, (pen_ucap(r) + 127) / 128 * 128) <= (size_t)kCrSmem; };
+    if (cap == kCrBlocks && one > rows && fits(one)) rows = one;
+    c->pen_resident = fits(rows) && (long long)rows * cap >= N;
     if (c->pen_resident) { c->pen_rows = rows; c->pen_w = kCrThreads / rows; }
     else if (N > 152 * 512) { c->pen_rows = 256; c->pen_w = 1; }
     else if (N > 152 * 192) { c->pen_rows = 128; c->pen_w = 2; }
