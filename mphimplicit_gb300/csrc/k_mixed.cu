@@ -401,9 +401,9 @@ int mixed_prepare(mph_case* c)
     if (c->step_pen) return MPH_OK;   // the assembly wrote the FP32 D^-1
     if (mixed_jacobi(c)) {   // point Jacobi: the FP32 D^-1 only
         const long long nv = (long long)c->dp.Nf * c->dim;
-        if (!d.v32) MPH_CUDA(cudaMalloc((void**)&d.v32, (size_t)nv * 8 * sizeof(float)));
+        if (!d.v32) MPH_CUDA(cudaMalloc((void**)&d.v32, vec32_stride(nv) * 8 * sizeof(float)));
         c->dense_level = -1;
-        { k_convert<double, float><<<grid_for(nv, 256), 256, 0, c->stream>>>(nv, d.invDiag, d.v32 + 7 * nv); MPH_COUNT_LAUNCH(); }
+        { k_convert<double, float><<<grid_for(nv, 256), 256, 0, c->stream>>>(nv, d.invDiag, d.v32 + 7 * vec32_stride(nv)); MPH_COUNT_LAUNCH(); }
         return MPH_OK;
     }
     MPH_TRY(grow_f(&d.mg_cof32, &d.cap_mg_cof32, c->mg_cof_total));
@@ -418,12 +418,12 @@ int mixed_prepare(mph_case* c)
     }
     const long long nv = (long long)c->dp.Nf * c->dim;
     if (!d.v32) {
-        MPH_CUDA(cudaMalloc((void**)&d.v32, (size_t)nv * 8 * sizeof(float)));
+        MPH_CUDA(cudaMalloc((void**)&d.v32, vec32_stride(nv) * 8 * sizeof(float)));
     }
     cudaStream_t st = c->stream;
     { k_convert<double, float><<<grid_for(c->mg_cof_total, 256), 256, 0, st>>>(c->mg_cof_total, d.mg_cof, d.mg_cof32); MPH_COUNT_LAUNCH(); }
     { k_convert<double, float><<<grid_for(c->mg_rows_total, 256), 256, 0, st>>>(c->mg_rows_total, d.mg_invd, d.mg_invd32); MPH_COUNT_LAUNCH(); }
-    { k_convert<double, float><<<grid_for(nv, 256), 256, 0, st>>>(nv, d.invDiag, d.v32 + 7 * nv); MPH_COUNT_LAUNCH(); }
+    { k_convert<double, float><<<grid_for(nv, 256), 256, 0, st>>>(nv, d.invDiag, d.v32 + 7 * vec32_stride(nv)); MPH_COUNT_LAUNCH(); }
     return mixed_dense_coarse(c);
 }
 
@@ -438,7 +438,7 @@ static void pq_precond(mph_case* c, cudaStream_t st, int n, unsigned rb, const f
     double* scal = d.scal;
     const int* flags = d.flags;
     if (mixed_jacobi(c)) {
-        const float* invD = d.v32 + 7 * (size_t)c->dp.Nf * c->dim;
+        const float* invD = d.v32 + 7 * vec32_stride((long long)c->dp.Nf * c->dim);
         { k_pq_jacobi32<float><<<rb, kReduceThreads, 0, st>>>(n, s32, y32, p32, q32, invD, u32, scal, flags, d.partials,
                                                               (unsigned*)(d.flags + kFlagCounter)); MPH_COUNT_LAUNCH(); }
         return;
@@ -514,8 +514,9 @@ static int device_solve(mph_case* c, double* hs, int* hflags)
     const int rb = std::min<int>(grid_for(n, kReduceThreads), kReduceBlocks);
     const unsigned gs = grid_for(Nf, 128);
     V* vec = d.v32;
-    V *r32 = vec, *z32 = vec + (size_t)n, *s32 = vec + 2 * (size_t)n, *y32 = vec + 3 * (size_t)n;
-    V *p32 = vec + 4 * (size_t)n, *q32 = vec + 5 * (size_t)n, *u32 = vec + 6 * (size_t)n;
+    const size_t ns = vec32_stride(n);
+    V *r32 = vec, *z32 = vec + ns, *s32 = vec + 2 * ns, *y32 = vec + 3 * ns;
+    V *p32 = vec + 4 * ns, *q32 = vec + 5 * ns, *u32 = vec + 6 * ns;
     const double tol_out2 = c->tol_outer * c->tol_outer;
     const double tol_in2 = inner_target2(c);
     const int cap = n;
@@ -706,12 +707,13 @@ struct MixedRun {
         gs = grid_for(Nf, 128);
         V* vec = d.v32;
         r32 = vec;
-        z32 = vec + (size_t)n;
-        s32 = vec + 2 * (size_t)n;
-        y32 = vec + 3 * (size_t)n;
-        p32 = vec + 4 * (size_t)n;
-        q32 = vec + 5 * (size_t)n;
-        u32 = vec + 6 * (size_t)n;
+        const size_t ns = vec32_stride(n);
+        z32 = vec + ns;
+        s32 = vec + 2 * ns;
+        y32 = vec + 3 * ns;
+        p32 = vec + 4 * ns;
+        q32 = vec + 5 * ns;
+        u32 = vec + 6 * ns;
         tol_out2 = c->tol_outer * c->tol_outer;
         tol_in2 = inner_target2(c);
         cap = n;

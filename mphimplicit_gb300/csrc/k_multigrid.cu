@@ -1041,7 +1041,7 @@ int mixed_dense_coarse(mph_case* c)
 void vcycle_mixed(mph_case* c, const float* q, float* u, double* dot_out)
 {
     DeviceState& d = c->d;
-    const float* invDiag32 = d.v32 + 7 * (size_t)c->dp.Nf * c->dim;
+    const float* invDiag32 = d.v32 + 7 * vec32_stride((long long)c->dp.Nf * c->dim);
     if (c->dim == 2)
         vcycle_t<2, float, float>(c, q, u, invDiag32, d.mg_cof32, d.mg_invd32, d.mg_q32, d.mg_s32, d.mg_r32, d.mg_res32, dot_out,
                                   c->mixed_extra_sweeps);

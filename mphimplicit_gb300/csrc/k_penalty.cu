@@ -623,17 +623,40 @@ __device__ __forceinline__ void pen_vec_body(const PenArgs& A, int lb, int nb, i
     }
     const float alpha = ab[0], beta = ab[1];
     float acc = 0.f;
-    for (int k = lb * blockDim.x + threadIdx.x; k < n; k += nb * blockDim.x) {
-        const float s = A.s[k], y = A.y[k], d = A.invD[k];
-        const float p = it == 0 ? s : beta * A.p[k] + s;
-        const float q = it == 0 ? y : beta * A.q[k] + y;
+    auto one = [&](float& s, float y, float d, float& p, float& q, float& z) {
+        p = it == 0 ? s : beta * p + s;
+        q = it == 0 ? y : beta * q + y;
+        z += alpha * p;
+        s = s - alpha * (d * q);
+        const float r = d != 0.f ? __fdividef(s, d) : 0.f;
+        acc += r * r;
+    };
+    // four components a thread (the vectors are 16-byte aligned), the last n mod 4 one by one
+    for (int k = lb * blockDim.x + threadIdx.x; k < (n >> 2); k += nb * blockDim.x) {
+        float4 s = reinterpret_cast<float4*>(A.s)[k], z = reinterpret_cast<float4*>(A.z)[k];
+        const float4 y = reinterpret_cast<const float4*>(A.y)[k], d = reinterpret_cast<const float4*>(A.invD)[k];
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p;
+        if (it > 0) {
+            p = reinterpret_cast<float4*>(A.p)[k];
+            q = reinterpret_cast<float4*>(A.q)[k];
+        }
+        one(s.x, y.x, d.x, p.x, q.x, z.x);
+        one(s.y, y.y, d.y, p.y, q.y, z.y);
+        one(s.z, y.z, d.z, p.z, q.z, z.z);
+        one(s.w, y.w, d.w, p.w, q.w, z.w);
+        reinterpret_cast<float4*>(A.s)[k] = s;
+        reinterpret_cast<float4*>(A.z)[k] = z;
+        reinterpret_cast<float4*>(A.p)[k] = p;
+        reinterpret_cast<float4*>(A.q)[k] = q;
+    }
+    if (lb == 0 && (int)threadIdx.x < (n & 3)) {
+        const int k = (n & ~3) + threadIdx.x;
+        float s = A.s[k], z = A.z[k], p = it > 0 ? A.p[k] : 0.f, q = it > 0 ? A.q[k] : 0.f;
+        one(s, A.y[k], A.invD[k], p, q, z);
+        A.s[k] = s;
+        A.z[k] = z;
         A.p[k] = p;
         A.q[k] = q;
-        A.z[k] += alpha * p;
-        const float sn = s - alpha * (d * q);
-        A.s[k] = sn;
-        const float r = d != 0.f ? __fdividef(sn, d) : 0.f;
-        acc += r * r;
     }
     const bool last = reduce_finalize_step(acc, A.partials, A.counter, A.scal + kSIn, A.flags + kFlagIter, lb, nb);
     if (last) {
@@ -1571,14 +1594,14 @@ int launch_pen_assemble(mph_case* c)
         MPH_CUDA(cudaMemsetAsync(d.z4, 0, (size_t)P.Nf * 2 * sizeof(float4), st));
     }
     if (!d.vacc) MPH_CUDA(cudaMalloc((void**)&d.vacc, n * sizeof(double)));
-    if (!d.v32) MPH_CUDA(cudaMalloc((void**)&d.v32, n * 8 * sizeof(float)));
+    if (!d.v32) MPH_CUDA(cudaMalloc((void**)&d.v32, vec32_stride(n) * 8 * sizeof(float)));
     if (!d.tct) MPH_CUDA(cudaMalloc((void**)&d.tct, (size_t)(P.N + 1) * sizeof(double)));
     if (!d.tct32) MPH_CUDA(cudaMalloc((void**)&d.tct32, (size_t)(P.N + 1) * sizeof(float)));
     if (!d.sdiag64) MPH_CUDA(cudaMalloc((void**)&d.sdiag64, (size_t)P.Nf * 8 * sizeof(double)));
     MPH_TRY(grow_t(&d.cval, &d.cap_cval, c->nnbP * c->dim));
     launch_vector_p(c);
     const unsigned g = grid_for(P.N, 256), gs = grid_for(P.N, 128);
-    float* invD = d.v32 + 7 * n;
+    float* invD = d.v32 + 7 * vec32_stride(n);
     if (c->dim == 2) {
         { k_fixed_positions<2><<<g, 256, 0, st>>>(P, d.type, d.pos, d.ipos, d.vpos, d.wrap32); MPH_COUNT_LAUNCH(); }
         { k_pen_system<2><<<gs, 128, 0, st>>>(P, d.type, d.pos, d.vel, d.ncp, d.nptrP, d.nindP, d.pvec, d.cval, d.bvec, invD); MPH_COUNT_LAUNCH(); }
@@ -1639,7 +1662,7 @@ void launch_pen_refine(mph_case* c, double scale, const double* scale_src, const
 {
     DeviceState& d = c->d;
     const int Nf = c->dp.Nf;
-    const float* z = d.v32 + (size_t)Nf * c->dim;
+    const float* z = d.v32 + vec32_stride((long long)Nf * c->dim);
     if (c->dim == 2) {
         { k_pen_pack<2><<<grid_for(Nf, 256), 256, 0, c->stream>>>(Nf, d.x, z, scale, scale_src, flags, d.z4); MPH_COUNT_LAUNCH(); }
         pen_residual<2, kVisc2, false>(c, scale, scale_src);
@@ -1657,7 +1680,7 @@ void launch_pen_phase(mph_case* c, double inv_scale, const double* scale_src, do
     const int n = c->dp.Nf * c->dim;
     float* v = d.v32;
     { k_pen_phase<<<std::min<int>(grid_for(n, kReduceThreads), kReduceBlocks), kReduceThreads, 0, c->stream>>>(
-          n, d.r, v + 7 * (size_t)n, v + 2 * (size_t)n, v + (size_t)n, inv_scale, scale_src, tol_in2, tol_out2, d.scal, d.flags, d.partials,
+          n, d.r, v + 7 * vec32_stride(n), v + 2 * vec32_stride(n), v + vec32_stride(n), inv_scale, scale_src, tol_in2, tol_out2, d.scal, d.flags, d.partials,
           (unsigned*)(d.flags + kFlagCounter), c->pen_resident ? cr_count(c) : nullptr); MPH_COUNT_LAUNCH(); }
 }
 
@@ -1681,12 +1704,13 @@ static PenArgs pen_args(const mph_case* c, int cap)
     A.ncp = d.ncp;
     A.nindP = d.nindP;
     A.nptrP = d.nptrP;
-    A.z = d.v32 + n;
-    A.s = d.v32 + 2 * n;
-    A.y = d.v32 + 3 * n;
-    A.p = d.v32 + 4 * n;
-    A.q = d.v32 + 5 * n;
-    A.invD = d.v32 + 7 * n;
+    const size_t ns = vec32_stride(n);
+    A.z = d.v32 + ns;
+    A.s = d.v32 + 2 * ns;
+    A.y = d.v32 + 3 * ns;
+    A.p = d.v32 + 4 * ns;
+    A.q = d.v32 + 5 * ns;
+    A.invD = d.v32 + 7 * ns;
     A.t = d.tct32;
     A.scal = d.scal;
     A.flags = d.flags;
@@ -1722,6 +1746,8 @@ int launch_pen_resident(mph_case* c, int cap, double scale)
     return MPH_OK;
 }
 
+static unsigned vec_blocks(int n) { return std::min<unsigned>(grid_for(n / 4 + 1, kReduceThreads), kReduceBlocks); }
+
 // y = M s and the iteration's scalars (two launches), then the vectors (one)
 void launch_pen_operator(mph_case* c, int cap)
 {
@@ -1741,7 +1767,7 @@ void launch_pen_vectors(mph_case* c, int cap, bool use_cond, cudaGraphConditiona
 {
     const PenArgs A = pen_args(c, cap);
     const int n = A.Nf * c->dim;
-    const unsigned rb = std::min<int>(grid_for(n, kReduceThreads), kReduceBlocks);
+    const unsigned rb = vec_blocks(n);
     if (use_cond) { k_pen_vec<true><<<rb, kReduceThreads, 0, c->stream>>>(A, n, 1, cond); MPH_COUNT_LAUNCH(); }
     else { k_pen_vec<false><<<rb, kReduceThreads, 0, c->stream>>>(A, n, 0, cond); MPH_COUNT_LAUNCH(); }
 }
@@ -1788,7 +1814,7 @@ void batch_pen_fill(const mph_case* c, int cap, void* table, int k, int* nb)
     B.t_nb = nb[0] = (int)grid_for(c->dp.N, c->pen_rows);
     B.y_nrb = (int)grid_for(c->dp.Nf, c->pen_rows);
     B.y_nb = nb[1] = std::min(B.y_nrb, kPenBlocks);
-    B.v_nb = nb[2] = std::min<int>(grid_for(B.n, kReduceThreads), kReduceBlocks);
+    B.v_nb = nb[2] = (int)vec_blocks(B.n);
 }
 
 // One CR iteration of the cases that still iterate (b0: the block starts of

@@ -246,6 +246,10 @@ struct Profile {
 }  // namespace mph
 
 // Opaque handle of the C ABI.
+// The mixed form's FP32 vectors lie in one buffer at this distance (16-byte
+// aligned each)
+inline size_t vec32_stride(long long n) { return ((size_t)n + 3) & ~(size_t)3; }
+
 struct mph_case {
     int dim = 3;
     int precision = MPH_PRECISION_FP64;
