@@ -50,7 +50,8 @@
 namespace mph {
 
 constexpr int kSIn0 = 16, kSIn = 17, kSTol2 = 23;         // as in k_mixed.cu
-constexpr int kSAlpha = 25, kSBeta = 26, kSQUPrev = 27;   // this iteration's alpha and beta, (q, D^-1 q) of the last one
+constexpr int kSAlpha = 25, kSQUPrev = 27;   // this iteration's alpha and beta (two floats), (q, D^-1 q) of the last one
+constexpr int kSStop = 28;                   // the phase's target (r, r) in two floats
 __device__ __forceinline__ int rho_slot32(int it) { return 20 + (it & 1); }
 
 constexpr int kPlWords = 1 << 13;   // bitmap of a row block's columns: 2^18 particles, fluid and wall window together
@@ -273,6 +274,70 @@ struct PenArgs {
     unsigned* counter;
 };
 
+// Sums over the grid of NC values a thread (256 threads a block): FP32 in a
+// warp, two floats beyond, in one order.  Thread 0 of the last block to arrive
+// gets them (true).  Two floats because an FP64 addition is some hundred
+// clocks long here and the chains of these sums, and of the quotients made
+// from them, stood at the end of two kernels an iteration (12 us of vectors
+// took 4 to stream).
+template <int NC>
+__device__ __forceinline__ bool grid_sums(const float* v, const PenArgs& A, int lb, int nb, int tid, F2* out)
+{
+    constexpr int NW = 8;   // warps
+    __shared__ float ws[NC][NW];
+    __shared__ F2 wf[NC][NW];
+    __shared__ bool last;
+    const int lane = tid & 31, wid = tid >> 5;
+    float2* parts = reinterpret_cast<float2*>(A.partials);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        float x = v[c];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (lane == 0) ws[c][wid] = x;
+    }
+    __syncthreads();
+    const int c = min(lane >> 3, NC - 1), w = lane & 7;   // eight lanes a value
+    if (wid == 0) {
+        const F2 x = f2_warp_sum(F2{ws[c][w], 0.f}, NW / 2);
+        if (w == 0 && (lane >> 3) < NC) __stcg(parts + (size_t)NC * lb + c, make_float2(x.h, x.l));
+        __syncwarp();
+        if (lane == 0) {
+            __threadfence();
+            last = atomicAdd(A.counter, 1u) == (unsigned)nb - 1;
+        }
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    constexpr int K = (kReduceBlocks + 255) / 256;
+    float2 p[K][NC];
+#pragma unroll
+    for (int u = 0; u < K; ++u)
+#pragma unroll
+        for (int d = 0; d < NC; ++d) {
+            const int k = tid + 256 * u;
+            p[u][d] = k < nb ? __ldcg(parts + (size_t)NC * k + d) : make_float2(0.f, 0.f);
+        }
+#pragma unroll
+    for (int d = 0; d < NC; ++d) {
+        F2 x{p[0][d].x, p[0][d].y};
+#pragma unroll
+        for (int u = 1; u < K; ++u)
+            if (256 * u < nb) x = f2_add(x, F2{p[u][d].x, p[u][d].y});
+        x = f2_warp_sum(x, 16);
+        if (lane == 0) wf[d][wid] = x;
+    }
+    __syncthreads();
+    if (wid != 0) return false;
+    const F2 x = f2_warp_sum(wf[c][w], NW / 2);
+#pragma unroll
+    for (int d = 0; d < NC; ++d)
+        out[d] = F2{__shfl_sync(0xffffffffu, x.h, 8 * d), __shfl_sync(0xffffffffu, x.l, 8 * d)};
+    if (lane == 0) *A.counter = 0u;
+    return lane == 0;
+}
+
 // What a thread has in flight before its block's neighbours are staged: the
 // first columns it stages and the first words of its row.  Their loads do not
 // wait for the block's count or the row's length (both buffers have room for
@@ -434,32 +499,6 @@ __device__ __forceinline__ void pen_t_body(const DevParams& P, const PenArgs& A,
     if (i < A.N) A.t[i] = R.n > 0 ? P.pen_lam32[pi.w] * acc : 0.f;
 }
 
-// Sums over the block of three FP32 values a thread: FP32 within a warp, FP64
-// across the warps, as block_sum.
-__device__ __forceinline__ void block_sum3(float (&v)[3], double (&out)[3])
-{
-    __shared__ double ws[3][32];
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int nw = (blockDim.x * blockDim.y + 31) >> 5;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_down_sync(0xffffffffu, v[c], o);
-        if (lane == 0) ws[c][wid] = (double)v[c];
-    }
-    __syncthreads();
-    if (wid == 0) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            double d = lane < nw ? ws[c][lane] : 0.0;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
-            out[c] = d;
-        }
-    }
-    __syncthreads();
-}
-
 // y = M s, and the iteration's scalars: rho = (s, y), and with
 // q <- y + beta q the product (q, D^-1 q) from (y, D^-1 y), (y, D^-1 q) and
 // the last iteration's, so that one vector kernel can follow with alpha and
@@ -553,50 +592,18 @@ __device__ __forceinline__ void pen_y_body(const DevParams& P, const PenArgs& A,
             }
         }
     }
-    double b[3];
-    block_sum3(v, b);
-    __shared__ bool last;
-    if (tid == 0) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) A.partials[3 * (size_t)lb0 + c] = b[c];
-        __threadfence();
-        last = atomicAdd(A.counter, 1u) == (unsigned)nb - 1;
+    F2 x[3];
+    if (!grid_sums<3>(v, A, lb0, nb, tid, x)) return;
+    float2* scal2 = reinterpret_cast<float2*>(A.scal);   // these slots hold two floats here
+    F2 be{0.f, 0.f}, qu = x[1];
+    if (it > 0) {
+        const float2 rp = scal2[rho_slot32(it - 1)], qp = scal2[kSQUPrev];
+        be = f2_div(x[0], F2{rp.x, rp.y});
+        qu = f2_add(qu, f2_mul(be, f2_add(F2{2.f * x[2].h, 2.f * x[2].l}, f2_mul(be, F2{qp.x, qp.y}))));
     }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    double sum[3] = {0.0, 0.0, 0.0};
-#pragma unroll 4
-    for (int k = tid; k < nb; k += nth)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) sum[c] += __ldcg(A.partials + 3 * (size_t)k + c);
-    __shared__ double ws[3][32];
-    const int lane = tid & 31, wid = tid >> 5, nwarp = (nth + 31) >> 5;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum[c] += __shfl_down_sync(0xffffffffu, sum[c], o);
-        if (lane == 0) ws[c][wid] = sum[c];
-    }
-    __syncthreads();
-    if (tid == 0) {
-        double r[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            r[c] = ws[c][0];
-            for (int w = 1; w < nwarp; ++w) r[c] += ws[c][w];
-        }
-        *A.counter = 0u;
-        double beta = 0.0, qu = r[1];
-        if (it > 0) {
-            beta = r[0] / A.scal[rho_slot32(it - 1)];
-            qu += beta * (2.0 * r[2] + beta * A.scal[kSQUPrev]);
-        }
-        A.scal[rho_slot32(it)] = r[0];
-        A.scal[kSQUPrev] = qu;
-        A.scal[kSBeta] = beta;
-        A.scal[kSAlpha] = r[0] / qu;
-    }
+    scal2[rho_slot32(it)] = make_float2(x[0].h, x[0].l);
+    scal2[kSQUPrev] = make_float2(qu.h, qu.l);
+    scal2[kSAlpha] = make_float2(f2_div(x[0], qu).h, be.h);
 }
 
 // p = s + beta p, q = y + beta q, z += alpha p, s -= alpha D^-1 q, and (r, r)
@@ -611,8 +618,9 @@ __device__ __forceinline__ void pen_vec_body(const PenArgs& A, int lb, int nb, i
     __shared__ float ab[2];
     if (threadIdx.x == 0) {
         it_s = A.flags[kFlagDone] ? -1 : A.flags[kFlagIter];
-        ab[0] = (float)A.scal[kSAlpha];
-        ab[1] = (float)A.scal[kSBeta];
+        const float2 v = reinterpret_cast<const float2*>(A.scal)[kSAlpha];
+        ab[0] = v.x;
+        ab[1] = v.y;
     }
     __syncthreads();
     const int it = it_s;
@@ -658,15 +666,18 @@ __device__ __forceinline__ void pen_vec_body(const PenArgs& A, int lb, int nb, i
         A.p[k] = p;
         A.q[k] = q;
     }
-    const bool last = reduce_finalize_step(acc, A.partials, A.counter, A.scal + kSIn, A.flags + kFlagIter, lb, nb);
-    if (last) {
-        const double rr = A.scal[kSIn], rr0 = A.scal[kSIn0];
-        const bool bad = !(rr == rr);
-        const bool stop = it + 1 >= A.cap || rr / rr0 < A.scal[kSTol2] || bad;
+    F2 rr;
+    if (grid_sums<1>(&acc, A, lb, nb, threadIdx.x, &rr)) {
+        const float2 t = reinterpret_cast<const float2*>(A.scal)[kSStop];
+        const bool bad = !(rr.h == rr.h);
+        const bool below = __fadd_rn(__fadd_rn(rr.h, -t.x), __fadd_rn(rr.l, -t.y)) < 0.f;
+        const bool stop = it + 1 >= A.cap || below || bad;
+        A.flags[kFlagIter] = it + 1;   // every block has read it (they all took their tickets)
         if (stop) {
             A.flags[kFlagDone] = 1;
             if (bad) A.flags[kFlagBad] = 1;
         }
+        A.scal[kSIn] = (double)rr.h + (double)rr.l;
         if constexpr (COND)
             if (use_cond) cudaGraphSetConditional(cond, stop ? 0u : 1u);
     }
@@ -1440,7 +1451,10 @@ __global__ void __launch_bounds__(kReduceThreads) k_pen_phase(int n, const doubl
     if (reduce_finalize_last(acc, partials, counter, scal + kSIn0)) {
 
         const double need = 0.25 * tol_out2 * scal[kSRR0] / scal[kSRR];
-        scal[kSTol2] = need > tol_in2 ? need : tol_in2;
+        const double tol2 = need > tol_in2 ? need : tol_in2;
+        scal[kSTol2] = tol2;
+        const F2 stop = f2_of(tol2 * scal[kSIn0]);
+        reinterpret_cast<float2*>(scal)[kSStop] = make_float2(stop.h, stop.l);
         scal[kSIn] = scal[kSIn0];
         flags[kFlagDone] = 0;
     }
