@@ -260,14 +260,26 @@ __global__ void k_bucket_order(int nb, const long long* __restrict__ off, int* _
 }
 
 // ---- bucket starts, permutation -------------------------------------------
-// bucket[b] = first sorted position whose key >= b, b in [0, 2T]
+// bucket[b] = first sorted position whose key >= b, b in [0, 2T].  A run of
+// empty cells (the free space of a dam: tens of thousands) is filled by the
+// warp together; by the one thread at its edge it took 171 us of a 5.7 ms
+// step on 735,000 particles in 2-D.
 __global__ void k_bucket_starts(const int* __restrict__ key, int N, int T, int* __restrict__ bucket)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > N) return;
-    const int lo = (i == 0) ? 0 : key[i - 1] + 1;
-    const int hi = (i == N) ? 2 * T : key[i];
-    for (int b = lo; b <= hi; ++b) bucket[b] = i;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    int lo = 1, hi = 0;
+    if (i <= N) {
+        lo = (i == 0) ? 0 : key[i - 1] + 1;
+        hi = (i == N) ? 2 * T : key[i];
+    }
+    const bool wide = hi - lo >= 4;
+    if (!wide)
+        for (int b = lo; b <= hi; ++b) bucket[b] = i;
+    for (unsigned m = __ballot_sync(0xffffffffu, wide); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        const int l = __shfl_sync(0xffffffffu, lo, src), h = __shfl_sync(0xffffffffu, hi, src), v = __shfl_sync(0xffffffffu, i, src);
+        for (int b = l + lane; b <= h; b += 32) bucket[b] = v;
+    }
 }
 
 template <int D>
