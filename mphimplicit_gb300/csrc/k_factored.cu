@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(256) k_wall_terms64(DevParams P, const int* __
                                                       const double* __restrict__ vel, const int* __restrict__ nc,
                                                       const int* __restrict__ nfc, const long long* __restrict__ nptr,
                                                       const int* __restrict__ nind, double* __restrict__ bvec,
-                                                      float* __restrict__ sdiag32, double* __restrict__ sdiag64, bool wall_rows_only)
+                                                      float* __restrict__ sdiag32, double* __restrict__ sdiag64)
 {
     // a warp per fluid row, its lanes over the row's wall slots; the lane
     // sums meet in a fixed shuffle tree (deterministic)
@@ -350,7 +350,6 @@ __global__ void __launch_bounds__(256) k_wall_terms64(DevParams P, const int* __
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= P.Nf) return;
     const int n = nc[i], nf = nfc[i];
-    if (wall_rows_only && n == nf) return;   // warp-uniform
     const int ti = type[i];
     double sd[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // xx xy xz yy yz zz
     double sw[3] = {0.0, 0.0, 0.0};
@@ -396,10 +395,7 @@ __global__ void __launch_bounds__(256) k_wall_terms64(DevParams P, const int* __
         const int t = lane >> 1;
         if ((lane & 1) == 0 && t >= 6 && t < 6 + D) bvec[(size_t)i * D + (t - 6)] += val;
     }
-    if (wall_rows_only) {
-        const int t = lane >> 1;
-        if ((lane & 1) == 0 && t < 6) sdiag64[(size_t)i * 8 + t] = val;
-    } else if (sdiag32) {   // lane 2 t writes component t: one FP32 conversion a lane
+    if (sdiag32) {   // lane 2 t writes component t: one FP32 conversion a lane
         const int t = lane >> 1;
         if ((lane & 1) == 0 && t < 6) {
             sdiag32[(size_t)i * 8 + t] = (float)val;
@@ -1834,14 +1830,14 @@ bool factored_applies(const mph_case* c)
 }
 
 // the wall slots of the fluid rows: into b, and the wall part of the viscous
-// diagonal (wall_rows_only: sdiag64 of the rows that have wall slots, no more)
-void launch_wall_terms(mph_case* c, float* sdiag32, double* sdiag64, bool wall_rows_only)
+// diagonal
+void launch_wall_terms(mph_case* c, float* sdiag32, double* sdiag64)
 {
     DeviceState& d = c->d;
     const DevParams& P = c->dp;
     const unsigned g = grid_for((long long)P.Nf * 32, 256);
-    if (c->dim == 2) { k_wall_terms64<2><<<g, 256, 0, c->stream>>>(P, d.type, d.pos, d.vel, d.nc, d.nfc, d.nptr, d.nind, d.bvec, sdiag32, sdiag64, wall_rows_only); MPH_COUNT_LAUNCH(); }
-    else { k_wall_terms64<3><<<g, 256, 0, c->stream>>>(P, d.type, d.pos, d.vel, d.nc, d.nfc, d.nptr, d.nind, d.bvec, sdiag32, sdiag64, wall_rows_only); MPH_COUNT_LAUNCH(); }
+    if (c->dim == 2) { k_wall_terms64<2><<<g, 256, 0, c->stream>>>(P, d.type, d.pos, d.vel, d.nc, d.nfc, d.nptr, d.nind, d.bvec, sdiag32, sdiag64); MPH_COUNT_LAUNCH(); }
+    else { k_wall_terms64<3><<<g, 256, 0, c->stream>>>(P, d.type, d.pos, d.vel, d.nc, d.nfc, d.nptr, d.nind, d.bvec, sdiag32, sdiag64); MPH_COUNT_LAUNCH(); }
 }
 
 template <int D>
@@ -1921,7 +1917,7 @@ int launch_pair_terms(mph_case* c)
         else { k_pair_terms<3><<<g, kPtWarps * 32, 0, c->stream>>>(P, d.type, d.pos, d.pos32, d.poslo32, d.vel, d.nc, d.nptr, d.nind, d.nfc, d.ncp, d.nptrP,
                                                                     d.nindP, d.cval, d.pvec, d.pe32, d.bvec, cvl, gmax, d.wrap32, dinv); MPH_COUNT_LAUNCH(); }
     }
-    launch_wall_terms(c, sdiag, sdiag64, false);
+    launch_wall_terms(c, sdiag, sdiag64);
     return MPH_OK;
 }
 

@@ -1141,8 +1141,8 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
 // C of every particle's P-list (calculateMatrixC main.cpp:2462-2507; the wall
 // rows' C_kj = - C_jk of fluid j give C^T its wall rows without a transposed
 // list), and for the fluid rows in the same pass b = inertia v - C p (its wall
-// velocities follow in k_wall_terms64) and the FP32 D^-1.  Bound by the FP64
-// pipe: 1.47 ms on 1.3 million particles.  C, the transposed lists (0.69 ms),
+// velocities follow in k_pen_wall) and the FP32 D^-1.  Bound by the FP64
+// pipe: 1.2 ms on 1.3 million particles.  C, the transposed lists (0.69 ms),
 // b with the pair terms (2.06) and their slicing (1.04) took 5.0 ms in passes
 // of their own.
 template <int D>
@@ -1157,7 +1157,7 @@ __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __re
     const bool fluid = i < P.Nf;
     double xi[3];
     load_vec<D>(pos, i, xi);
-    const double rP2 = P.rP * P.rP;
+    const double rP2 = P.rP * P.rP, K = -P.kfp * P.m2h_rp;
     const long long b = nptrP[i];
     const int n = ncp[i];
     double self[3] = {0, 0, 0}, cp[3] = {0, 0, 0};
@@ -1172,15 +1172,15 @@ __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __re
             double xj[3], q[3];
             load_vec<D>(pos, j, xj);
             sep_vec<D>(P, xj, xi, q);
-            const double r2 = norm2_exact<D>(q);
+            const double r2 = norm2_fma<D>(q);
             if (r2_pos_below(r2, rP2)) {
-                const double inv = rsqrt(r2);
-                const double wd = -P.kfp * (P.m2h_rp * (1.0 - (r2 * inv) * P.inv_rp));
+                // w' / r = kf (-2 / RadiusP) (1 - r / RadiusP) / r
+                const double f = K * (rsqrt(r2) - P.inv_rp);
                 const double pj = fluid ? pvec[j] : 0.0;
                 const float lam = P.lambda32[type[j]];
 #pragma unroll
                 for (int r = 0; r < D; ++r) {
-                    cv[r] = (q[r] * inv) * wd;
+                    cv[r] = q[r] * f;
                     self[r] += cv[r];
                     cp[r] += cv[r] * pj;
                     dp[r] += (float)cv[r] * (float)cv[r] * lam;
@@ -1202,6 +1202,70 @@ __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __re
         const float dg = P.inert32[ti] + P.pen_vd[ti] + dp[r] + (float)self[r] * (float)self[r] * P.lambda32[ti];
         invD[(size_t)i * D + r] = dg != 0.f ? 1.f / dg : 0.f;
     }
+}
+
+// The wall slots of the fluid rows in FP64 (main.cpp:2274-2303): the wall part
+// of the row's viscous diagonal block (rows with wall slots only) and, with
+// the wall velocities, into b; L threads a row.  f = visc mu_ij kf' (1/r -
+// 1/RadiusV), and every term is one factor f / r^2 of q (x) q.  A warp a row
+// took 0.61 ms on 1.3 million particles, most of it rows without any slots
+// and sums over the warp; the assembly stage takes 2.26 ms there with 16
+// threads a row, 2.32 with 4, which leave 15 slots in line a thread (0.18 ms
+// on 15,000 particles, 0.15 with 16).  In 2-D a row has a dozen: 8.
+template <int D, int L>
+__global__ void __launch_bounds__(128) k_pen_wall(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
+                                                  const double* __restrict__ vel, const int* __restrict__ nc,
+                                                  const int* __restrict__ nfc, const long long* __restrict__ nptr,
+                                                  const int* __restrict__ nind, double* __restrict__ bvec, double* __restrict__ sdiag64)
+{
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / L, part = threadIdx.x % L;
+    const int nf = i < P.Nf ? nfc[i] : 0, n = i < P.Nf ? nc[i] : 0;
+    if (!__any_sync(0xffffffffu, n > nf)) return;   // none of the warp's rows
+    double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};      // xx xy xz yy yz zz, then b's
+    if (n > nf) {
+        const int ti = type[i];
+        const long long nb = nptr[i];
+        const double rV2 = P.rV * P.rV, K = -P.kfv * P.m2h_rv * P.visc;
+        double xi[3];
+        load_vec<D>(pos, i, xi);
+        for (int k = nf + part; k < n; k += L) {
+            const int j = nind[nb + k];
+            double xj[3], vj[3], q[3] = {0.0, 0.0, 0.0}, qv = 0.0, fq[3] = {0.0, 0.0, 0.0};
+            load_vec<D>(pos, j, xj);
+            sep_vec<D>(P, xj, xi, q);
+            const double r2 = norm2_fma<D>(q);
+            if (!r2_pos_below(r2, rV2)) continue;
+            load_vec<D>(vel, j, vj);
+            const double inv = rsqrt(r2);
+            const double f = (K * P.muij[ti][type[j]]) * (inv - P.inv_rv) * (inv * inv);
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                qv += q[d] * vj[d];
+                fq[d] = f * q[d];
+            }
+#pragma unroll
+            for (int d = 0; d < D; ++d) v[6 + d] += fq[d] * qv;
+            v[0] += fq[0] * q[0];
+            v[1] += fq[0] * q[1];
+            v[3] += fq[1] * q[1];
+            if (D == 3) {
+                v[2] += fq[0] * q[2];
+                v[4] += fq[1] * q[2];
+                v[5] += fq[2] * q[2];
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+        if (D == 2 && (t == 2 || t == 4 || t == 5 || t == 8)) continue;
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) v[t] += __shfl_xor_sync(0xffffffffu, v[t], o);
+    }
+    if (n == nf || part != 0) return;
+#pragma unroll
+    for (int t = 0; t < 6; ++t) sdiag64[(size_t)i * 8 + t] = v[t];
+#pragma unroll
+    for (int d = 0; d < D; ++d) bvec[(size_t)i * D + d] += v[6 + d];
 }
 
 // The diagonal with its row's own viscous pairs, as the other forms' D^-1 (a
@@ -1623,7 +1687,12 @@ int launch_pen_assemble(mph_case* c)
         { k_fixed_positions<3><<<g, 256, 0, st>>>(P, d.type, d.pos, d.ipos, d.vpos, d.wrap32); MPH_COUNT_LAUNCH(); }
         { k_pen_system<3><<<gs, 128, 0, st>>>(P, d.type, d.pos, d.vel, d.ncp, d.nptrP, d.nindP, d.pvec, d.cval, d.bvec, invD); MPH_COUNT_LAUNCH(); }
     }
-    launch_wall_terms(c, nullptr, d.sdiag64, true);
+    auto walls = [&](auto kern, int lanes) {
+        kern<<<grid_for((long long)P.Nf * lanes, 128), 128, 0, st>>>(P, d.type, d.pos, d.vel, d.nc, d.nfc, d.nptr, d.nind, d.bvec, d.sdiag64);
+        MPH_COUNT_LAUNCH();
+    };
+    if (c->dim == 2) walls(k_pen_wall<2, 8>, 8);
+    else walls(k_pen_wall<3, 16>, 16);
     return launch_pen_lists(c);
 }
 

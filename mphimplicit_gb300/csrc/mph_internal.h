@@ -426,7 +426,7 @@ void ensure_density_a(mph_case* c);
 void launch_output_fields(mph_case* c);
 int launch_assemble(mph_case* c);
 void launch_vector_p(mph_case* c);
-void launch_wall_terms(mph_case* c, float* sdiag32, double* sdiag64, bool wall_rows_only);
+void launch_wall_terms(mph_case* c, float* sdiag32, double* sdiag64);
 int launch_assemble_cells(mph_case* c, int kmax_rows, bool mix, bool* done);
 int build_ct(mph_case* c);
 bool f64_parts_apply(const mph_case* c);
