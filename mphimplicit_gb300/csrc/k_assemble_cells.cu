@@ -165,7 +165,7 @@ k_assemble_cells(DevParams P, CellMap M, int rx, int ry, int rz, int mwords, int
         const int w = x >> 5, b = x & 31;
         return wpre[w] + __popc(mask[w] & ((1u << b) - 1u));
     };
-    const double rV2 = P.rV * P.rV;
+    const double rV2 = P.rV * P.rV, visc = -P.kfv * P.m2h_rv * P.visc;
 
     for (int i = r0 + warp; i < r1; i += kAsmWarps) {
         const int n = nc[i], nf = nfc[i];
@@ -232,27 +232,24 @@ k_assemble_cells(DevParams P, CellMap M, int rx, int ry, int rz, int mwords, int
             double xj[3], q[3];
             load_vec<D>(pos, j, xj);
             sep_vec<D>(P, xj, xi, q);
-            const double r2 = norm2_exact<D>(q);
+            const double r2 = norm2_fma<D>(q);
             if (!r2_pos_below(r2, rV2)) continue;
+            // f e (x) e = F q (x) q, F = visc mu_ij kf' (1/r - 1/RadiusV) / r^2
             const double inv = rsqrt(r2);
-            const double wd = -P.kfv * (P.m2h_rv * (1.0 - (r2 * inv) * P.inv_rv));
-            const double f = P.visc * P.muij[ti][type[j]] * wd * inv;
-            double e[3];
-#pragma unroll
-            for (int d = 0; d < D; ++d) e[d] = q[d] * inv;
+            const double F = (visc * P.muij[ti][type[j]]) * (inv - P.inv_rv) * (inv * inv);
             const bool fluid = k < nf;
             double vj[3];
             if (!fluid) load_vec<D>(vel, j, vj);
-            // the block f e (x) e is symmetric: the upper triangle is formed once
-            // (f e_r first, then times e_s) and mirrored
-            double fe[3];
+            // the block is symmetric: the upper triangle is formed once
+            // (F q_r first, then times q_s) and mirrored
+            double fq[3];
 #pragma unroll
-            for (int r = 0; r < D; ++r) fe[r] = f * e[r];
+            for (int r = 0; r < D; ++r) fq[r] = F * q[r];
 #pragma unroll
             for (int r = 0; r < D; ++r)
 #pragma unroll
                 for (int s = r; s < D; ++s) {
-                    const double coef = fe[r] * e[s];
+                    const double coef = fq[r] * q[s];
                     selfc[r * D + s] += (T)coef;
                     if (fluid) {
                         acc[k * DD + r * D + s] = (T)-coef;
@@ -263,25 +260,45 @@ k_assemble_cells(DevParams P, CellMap M, int rx, int ry, int rz, int mwords, int
                     }
                 }
         }
-        // warp sums of the upper triangle, mirrored (the FP32 form sums all entries)
+        const long long pb = nptrP[i];
+        const int np = ncp[i];
+        double cp[3] = {0, 0, 0};   // C p (main.cpp:2574-2584)
+        if (MIX) {   // warp sums of every entry
 #pragma unroll
-        for (int r = 0; r < D; ++r)
+            for (int t = 0; t < DD; ++t)
 #pragma unroll
-            for (int s = 0; s < D; ++s) {
-                if (!MIX && s < r) continue;
+                for (int o = 16; o > 0; o >>= 1) selfc[t] += __shfl_xor_sync(0xffffffffu, selfc[t], o);
+        } else {
+            // warp sums of the upper triangle, of the wall velocities' part of b
+            // and of C p together by reduce-scatter (16 FP64 additions a lane
+            // where a butterfly a value takes 60); value t ends in lane 2 t
+            for (int a = lane; a < np; a += 32) {
+                const double pk = pvec[nindP[pb + a]];
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) selfc[r * D + s] += __shfl_xor_sync(0xffffffffu, selfc[r * D + s], o);
+                for (int r = 0; r < D; ++r) cp[r] += cval[(pb + a) * D + r] * pk;
             }
-        if (!MIX) {
+            constexpr int UT = D * (D + 1) / 2;
+            double v[16] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-            for (int r = 1; r < D; ++r)
+            for (int r = 0, m = 0; r < D; ++r)
 #pragma unroll
-                for (int s = 0; s < r; ++s) selfc[r * D + s] = selfc[s * D + r];
+                for (int s = r; s < D; ++s, ++m) v[m] = (double)selfc[r * D + s];
+#pragma unroll
+            for (int r = 0; r < D; ++r) {
+                v[UT + r] = sumv[r];
+                v[UT + D + r] = cp[r];
+            }
+            const double val = warp_reduce_scatter<16>(v, lane);
+#pragma unroll
+            for (int r = 0, m = 0; r < D; ++r)
+#pragma unroll
+                for (int s = r; s < D; ++s, ++m) selfc[r * D + s] = selfc[s * D + r] = (T)__shfl_sync(0xffffffffu, val, 2 * m);
+#pragma unroll
+            for (int r = 0; r < D; ++r) {
+                sumv[r] = __shfl_sync(0xffffffffu, val, 2 * (UT + r));
+                cp[r] = __shfl_sync(0xffffffffu, val, 2 * (UT + D + r));
+            }
         }
-#pragma unroll
-        for (int r = 0; r < D; ++r)
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sumv[r] += __shfl_xor_sync(0xffffffffu, sumv[r], o);
         const int self = __reduce_max_sync(0xffffffffu, myself);
         // inertia density/dt as the reference forms it, (rho*vol)/vol/dt,
         // formed once on the host (its FP32 rounding for the FP32 form)
@@ -319,20 +336,27 @@ k_assemble_cells(DevParams P, CellMap M, int rx, int ry, int rz, int mwords, int
             __syncwarp();
         };
         // 3. C Lambda C^T, one P-neighbour column at a time (main.cpp:2590-2641)
-        const long long pb = nptrP[i];
-        const int np = ncp[i];
+        int ka = 0;
+        T gl[3] = {T(0), T(0), T(0)};   // the lane's column of 32 and its C lambda, read by the others in turn
         for (int a = 0; a < np; ++a) {
-            const int k = nindP[pb + a];
-            T ga[3];
-            if (MIX) {
-                const float lam = P.lambda32[type[k]];
+            if ((a & 31) == 0) {
+                if (a + lane < np) {
+                    ka = nindP[pb + a + lane];
+                    if (MIX) {
+                        const float lam = P.lambda32[type[ka]];
 #pragma unroll
-                for (int r = 0; r < D; ++r) ga[r] = cval32[(pb + a) * D + r] * lam;
-            } else {
-                const double lam = P.lambda[type[k]];
+                        for (int r = 0; r < D; ++r) gl[r] = cval32[(pb + a + lane) * D + r] * lam;
+                    } else {
+                        const double lam = P.lambda[type[ka]];
 #pragma unroll
-                for (int r = 0; r < D; ++r) ga[r] = (T)(cval[(pb + a) * D + r] * lam);
+                        for (int r = 0; r < D; ++r) gl[r] = (T)(cval[(pb + a + lane) * D + r] * lam);
+                    }
+                }
             }
+            const int k = __shfl_sync(0xffffffffu, ka, a & 31);
+            T ga[3];
+#pragma unroll
+            for (int r = 0; r < D; ++r) ga[r] = __shfl_sync(0xffffffffu, gl[r], a & 31);
             const long long e0 = ctptr[k], e1 = ctptr[k + 1];
             for (long long e = e0 + lane; e < e1; e += 32) {
                 const int l = local_of(ct_j[e]);
@@ -353,26 +377,19 @@ k_assemble_cells(DevParams P, CellMap M, int rx, int ry, int rz, int mwords, int
             }
             __syncwarp();
         }
-        // 4. b: wall terms + inertia - C p (main.cpp:2318-2333, 2574-2584)
-        double cp[3] = {0, 0, 0};
-        for (int a = lane; a < (MIX ? 0 : np); a += 32) {
-            const double pk = pvec[nindP[pb + a]];
-#pragma unroll
-            for (int r = 0; r < D; ++r) cp[r] += cval[(pb + a) * D + r] * pk;
-        }
-#pragma unroll
-        for (int r = 0; r < D; ++r)
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) cp[r] += __shfl_xor_sync(0xffffffffu, cp[r], o);
-        if (lane == 0) {
-#pragma unroll
-            for (int r = 0; r < D; ++r) {
-                if (!MIX) bvec[(size_t)i * D + r] = (sumv[r] + (double)inert * vi[r]) - cp[r];
-                const T dg = acc[self * DD + r * D + r];
-                invDiag[(size_t)i * D + r] = (double)(dg != T(0) ? T(1) / dg : T(0));
+        // 4. b: wall terms + inertia - C p (main.cpp:2318-2333, 2574-2584), and
+        // D^-1, a component a lane (one division, not D in line)
+        if (lane < D) {
+            if (!MIX) {
+                const double sv = lane == 0 ? sumv[0] : lane == 1 ? sumv[1] : sumv[2];
+                const double vl = lane == 0 ? vi[0] : lane == 1 ? vi[1] : vi[2];
+                const double cl = lane == 0 ? cp[0] : lane == 1 ? cp[1] : cp[2];
+                bvec[(size_t)i * D + lane] = (sv + (double)inert * vl) - cl;
             }
-            selfk_out[i] = self;
+            const T dg = acc[self * DD + lane * D + lane];
+            invDiag[(size_t)i * D + lane] = (double)(dg != T(0) ? T(1) / dg : T(0));
         }
+        if (lane == 0) selfk_out[i] = self;
         // 5. level-0 partial stencils: the row's blocks summed per neighbour cell
         for (int t = lane; t < nw * DD; t += 32) {
             const int s = t / DD, rs = t % DD;
