@@ -159,7 +159,7 @@ def precond_name(args, mixed: bool) -> str:
     if not mixed:
         return "multigrid V-cycle (the reference's)"
     if args.mg_depth < 0:
-        return "point Jacobi, fused with the CR vector update"
+        return "point Jacobi, in the CR vector update"
     return "multigrid V-cycle, " + ("every level" if args.mg_depth == 0 else f"{args.mg_depth} level(s)")
 
 
@@ -198,6 +198,43 @@ def pair_apply_bytes(prof, scal, dim, st=None, rec="pack"):
     if staged:
         vp += st["inner_local_cols"] * 4 + (st["inner_local_blocks"] + st["inner_gather_blocks"]) * 4
     return ct + vp
+
+
+def pen_apply_bytes(prof, scal, dim, st=None):
+    """Algorithmic bytes of one application of the point-Jacobi mixed form's
+    inner operator, inertia + C Lambda C^T from the P-lists (k_pen_t + k_pen_y,
+    or an iteration's share of the resident k_pen_cr): a 2-byte rank per P-list
+    slot, the lists of every particle for t and of the fluid rows for y;
+    positions (16 bytes a particle) in both; s read in both, t written and
+    read, y, D^-1 and q; the row blocks' distinct columns (4 bytes each)."""
+    nf = int(scal["FluidParticleEnd"])
+    n = int(scal["ParticleCount"])
+    pslots = scal["NonzeroCountC"] / dim
+    cols = 4 * (st or {}).get("inner_local_cols", 0)
+    return 2 * prof["nnbP"] + 2 * pslots + 2 * 16 * n + (2 + 3) * 4 * dim * nf + 8 * n + 2 * cols
+
+
+def f64_parts_bytes(prof, scal, dim):
+    """Algorithmic bytes of one application of the 3-D FP64 form's operator in
+    parts (k_f64_parts + k_f64_rows): a 24-byte pair record and a column per
+    fluid slot, the direction's 24-byte records, C (3 doubles) and a column per
+    P-slot of every particle for t and of the fluid rows for y, t, the pair
+    part written and read, x and y."""
+    nf = int(scal["FluidParticleEnd"])
+    n = int(scal["ParticleCount"])
+    slots = scal["NonzeroCountA"] / (dim * dim)
+    pslots = scal["NonzeroCountC"] / dim
+    return slots * 28 + nf * 24 + (prof["nnbP"] + pslots) * 28 + 16 * n + nf * (48 + 48)
+
+
+def assemble_pen_bytes(prof, scal, dim):
+    """Algorithmic bytes of the point-Jacobi mixed form's assembly stage: the
+    P-lists and the particle state read once; C (D doubles) and a 2-byte rank
+    per P-slot of every particle, b (D doubles) and D^-1 (D floats) per fluid
+    row written."""
+    nf = int(scal["FluidParticleEnd"])
+    n = int(scal["ParticleCount"])
+    return 4 * prof["nnbP"] + 64 * n + prof["nnbP"] * (8 * dim + 2) + nf * dim * 12 + 48 * n
 
 
 def assemble_bytes(prof, scal, dim):
@@ -429,10 +466,11 @@ def case_roofline(engine, params, parts, dim, args, steps: int = 3):
     g.close()
     n = max(prof["kern_n_spmv"], 1)
     avg = prof["kern_ms_spmv"] / 1000.0 / n
-    b = pair_apply_bytes(prof, scal, dim, st) if st.get("inner_form") == 2 else spmv_bytes(prof, scal, dim, 4)
+    pen = st.get("inner_form") == 2
+    b = pen_apply_bytes(prof, scal, dim, st) if pen else spmv_bytes(prof, scal, dim, 4)
     peak, kind = measured_peaks()
     return {"bound": "hbm", "achieved": b / avg / 1e9, "peak": peak, "unit": "GB/s", "frac": b / avg / 1e9 / peak,
-            "traffic": None, "kernel": "k_ct_apply32+k_visc_pen32" if st.get("inner_form") == 2 else "k_spmv32",
+            "traffic": None, "kernel": "k_pen_t+k_pen_y" if pen else "k_spmv32",
             "peak_source": kind, "algorithmic_bytes_per_launch": b, "avg_launch_ms": avg * 1000.0, "launches": n,
             "case": f"{parts.count} particles ({dim}D), run alone"}
 
@@ -890,7 +928,11 @@ def run_single(args, dist, rank, world, local):
     vb = 4 if prec == PRECISION_MIXED else 8
     pairs = st.get("inner_form") == 2
     rec = "recompute" if args.pair_recompute else ("pack" if args.pair_pack else "fp16")
-    kern = {"spmv": ("k_ct_apply32+k_visc_pen32" if rec != "recompute" else "k_ct_apply32+k_visc_rc32",
+    pen = pairs and args.mg_depth < 0   # the point-Jacobi form's own operator
+    parts64 = prec == PRECISION_FP64 and dim == 3 and not args.no_factored
+    kern = {"spmv": ("k_pen_t+k_pen_y", lambda p_, s_, d_: pen_apply_bytes(p_, s_, d_, st)) if pen else
+                    ("k_f64_parts+k_f64_rows", f64_parts_bytes) if parts64 else
+                    ("k_ct_apply32+k_visc_pen32" if rec != "recompute" else "k_ct_apply32+k_visc_rc32",
                      lambda p_, s_, d_: pair_apply_bytes(p_, s_, d_, st, rec)) if pairs else
                     ("k_spmv32" if vb == 4 else "k_spmv", lambda p_, s_, d_: spmv_bytes(p_, s_, d_, vb)),
             "assemble_a": ("k_assemble_cells", assemble_bytes)}
@@ -904,13 +946,15 @@ def run_single(args, dist, rank, world, local):
                 "kernel": kern[dom][0], "peak_source": peak_kind,
                 "algorithmic_bytes_per_launch": bytes_per, "avg_launch_ms": avg_s * 1000.0, "launches": nlaunch}
     asm_ms = prof["stage_ms_assemble"] / psteps
-    asm_bytes = (assemble_pair_bytes(prof, scal, dim, case, jacobi=args.mg_depth < 0,
+    asm_bytes = (assemble_pen_bytes(prof, scal, dim) if pen else
+                 assemble_pair_bytes(prof, scal, dim, case, jacobi=args.mg_depth < 0,
                                      rec_bytes={"pack": 6, "fp16": 8, "recompute": 2}[rec]) if pairs
                  else assemble_bytes(prof, scal, dim))
     roofline_asm = {"bound": "hbm", "achieved": asm_bytes / (asm_ms / 1000.0) / 1e9, "peak": peak, "unit": "GB/s",
                     "frac": asm_bytes / (asm_ms / 1000.0) / 1e9 / peak, "stage": "assemble",
                     "algorithmic_bytes_per_step": asm_bytes, "ms_per_step": asm_ms, "peak_source": peak_kind,
-                    "form": "pair terms (mixed)" if pairs else "sliced-ELL blocks"}
+                    "form": "C, b and D^-1 (point-Jacobi mixed)" if pen else
+                    "pair terms (mixed)" if pairs else "sliced-ELL blocks"}
     case.close()
 
     cpu = None
@@ -960,13 +1004,13 @@ def run_single(args, dist, rank, world, local):
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": 1000.0 * total_s / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "f64" if prec == PRECISION_FP64 else
+        "dtype": "f64" if prec == PRECISION_FP64 else "f32-inner/f64-outer" if pen else
                  (f"f32-inner({ {'fp16': 'fp16', 'pack': '11/11/10-bit fixed-point', 'recompute': 'recomputed fp32'}[rec]} "
                   f"pair terms)/f64-outer" if pairs else "f32-inner/f64-outer"),
         "data": "synthetic",
         "config": {"workload": args.workload, "description": desc, "dim": dim, "particles": N, "fluid": Nf,
                    "precision": args.precision, "parallelism": "replicas" if world > 1 else "single",
-                   "l2": "inputs larger than L2 (the pair terms alone exceed 129 MB by ~50x)",
+                   "l2": "inputs larger than L2 (the neighbour lists alone exceed 129 MB by ~5x)",
                    "p50_step_ms": float(np.percentile(step_ms, 50)), "p99_step_ms": float(np.percentile(step_ms, 99)),
                    "outer_tol": tol, "cr_iterations": iters, "outer_refinements": outer_main,
                    "cr_start": {0: "v_n (the reference's)", 1: "linear extrapolation of the last start velocities",
