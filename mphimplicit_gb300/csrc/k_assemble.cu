@@ -83,14 +83,14 @@ __global__ void __launch_bounds__(128) k_matrix_c(DevParams P, int rows, const d
     for (int r = 0; r < D; ++r) cval[(b + selfk) * D + r] = self[r];
 }
 
-template <int D>
+template <int D, int L>
 __global__ void __launch_bounds__(128) k_vector_p(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
                                                   const double* __restrict__ vel, const double* __restrict__ vsp,
                                                   const int* __restrict__ ncp, const long long* __restrict__ nptrP,
                                                   const int* __restrict__ nindP, double* __restrict__ pvec)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.N) return;
+    const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) / L, part = threadIdx.x % L;
+    const int i = min(i0, P.N - 1);   // beyond the last row: its lists, no store
     const int ti = type[i];
     const double v0 = vsp[i];
     double p = 0.0;
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(128) k_vector_p(DevParams P, const int* __rest
     const double rP2 = P.rP * P.rP;
     double sum = 0.0;
     const long long b = nptrP[i];
-    for (int a = 0; a < ncp[i]; ++a) {
+    for (int a = part; a < ncp[i]; a += L) {
         const int j = nindP[b + a];
         if (j == i) continue;
         const bool wj = is_wall(type[j]);
@@ -124,7 +124,8 @@ __global__ void __launch_bounds__(128) k_vector_p(DevParams P, const int* __rest
             if (wj) sum += lam * (-e * wd) * vj[s];
         }
     }
-    pvec[i] = p + sum;
+    sum = row_sum<L>(sum);
+    if (i0 < P.N && part == 0) pvec[i] = p + sum;
 }
 
 
@@ -132,9 +133,13 @@ __global__ void __launch_bounds__(128) k_vector_p(DevParams P, const int* __rest
 void launch_vector_p(mph_case* c)
 {
     DeviceState& d = c->d;
-    const unsigned g = grid_for(c->dp.N, 128);
-    if (c->dim == 2) { k_vector_p<2><<<g, 128, 0, c->stream>>>(c->dp, d.type, d.pos, d.vel, d.vsp, d.ncp, d.nptrP, d.nindP, d.pvec); MPH_COUNT_LAUNCH(); }
-    else { k_vector_p<3><<<g, 128, 0, c->stream>>>(c->dp, d.type, d.pos, d.vel, d.vsp, d.ncp, d.nptrP, d.nindP, d.pvec); MPH_COUNT_LAUNCH(); }
+    const int L = plist_lanes(c->dp.N);
+    auto go = [&](auto kern) {
+        kern<<<grid_for((long long)c->dp.N * L, 128), 128, 0, c->stream>>>(c->dp, d.type, d.pos, d.vel, d.vsp, d.ncp, d.nptrP, d.nindP, d.pvec);
+        MPH_COUNT_LAUNCH();
+    };
+    if (c->dim == 2) L == 4 ? go(k_vector_p<2, 4>) : go(k_vector_p<2, 1>);
+    else L == 4 ? go(k_vector_p<3, 4>) : go(k_vector_p<3, 1>);
 }
 
 template <int D>

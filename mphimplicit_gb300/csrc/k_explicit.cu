@@ -333,20 +333,19 @@ __global__ void __launch_bounds__(128) k_output_forces(DevParams P, const int* _
 // pairs with r^2 <= RadiusP^2, in the full list's order (the sum differs from
 // the full-list pass's by the rounding of its pieces).  As k_density: 37 FP64
 // operations a pair became 28; 340 -> 243 us on 374,000 particles.
-template <int D>
+template <int D, int L>
 __global__ void __launch_bounds__(128) k_density_p(DevParams P, const double* __restrict__ pos, const int* __restrict__ ncp,
                                                    const long long* __restrict__ nptrP, const int* __restrict__ nindP,
                                                    double* __restrict__ vsp)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.N) return;
-    double xi[3];
-    load_vec<D>(pos, i, xi);
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / L, part = threadIdx.x % L;
+    double xi[3] = {0.0, 0.0, 0.0};
+    if (i < P.N) load_vec<D>(pos, i, xi);
     const double rP2 = DMUL(P.rP, P.rP);
     double sp = 0.0;
-    const long long b = nptrP[i];
-    const int n = ncp[i];
-    for (int k = 0; k < n; ++k) {
+    const long long b = i < P.N ? nptrP[i] : 0;
+    const int n = i < P.N ? ncp[i] : 0;
+    for (int k = part; k < n; k += L) {
         const int j = nindP[b + k];
         if (j == i) continue;
         double xj[3], q[3];
@@ -358,17 +357,20 @@ __global__ void __launch_bounds__(128) k_density_p(DevParams P, const double* __
             sp += oq * oq;
         }
     }
-    vsp[i] = __fma_rn(P.kfp, sp, -P.N0p);
+    sp = row_sum<L>(sp);
+    if (i < P.N && part == 0) vsp[i] = __fma_rn(P.kfp, sp, -P.N0p);
 }
 
 static void launch_density_p(mph_case* c)
 {
     const DevParams& P = c->dp;
-    const unsigned g = grid_for(P.N, 128);
-    if (c->dim == 2)
-        { k_density_p<2><<<g, 128, 0, c->stream>>>(P, c->d.pos, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.vsp); MPH_COUNT_LAUNCH(); }
-    else
-        { k_density_p<3><<<g, 128, 0, c->stream>>>(P, c->d.pos, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.vsp); MPH_COUNT_LAUNCH(); }
+    const int L = plist_lanes(P.N);
+    auto go = [&](auto kern) {
+        kern<<<grid_for((long long)P.N * L, 128), 128, 0, c->stream>>>(P, c->d.pos, c->d.ncp, c->d.nptrP, c->d.nindP, c->d.vsp);
+        MPH_COUNT_LAUNCH();
+    };
+    if (c->dim == 2) L == 4 ? go(k_density_p<2, 4>) : go(k_density_p<2, 1>);
+    else L == 4 ? go(k_density_p<3, 4>) : go(k_density_p<3, 1>);
 }
 
 // The full density pass (DensityA, GravityCenter, DensityP) and PressureA.

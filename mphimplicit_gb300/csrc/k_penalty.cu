@@ -29,8 +29,8 @@
 // by an addition to the bits of 1.5 2^23 (integer-to-float conversions run on
 // the quarter-rate pipe of the reciprocal square root).
 //
-// On 1,297,696 particles an application takes 98 us (k_pen_t 51, k_pen_y 47;
-// the viscous pairs and stored records: 398) and the vectors 22 us in one
+// On 1,297,696 particles an application takes 95 us (k_pen_t 51, k_pen_y 44;
+// the viscous pairs and stored records: 398) and the vectors 20 us in one
 // kernel (43 in two), with 142 CR iterations where there were 140.
 //
 // A block of rows stages its distinct neighbours (position with s, or with
@@ -701,8 +701,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_pen_vec(PenArgs A, int n, in
 // cases whose rows fit the chip at once (up to 155,648 particles).  Such a
 // case's iteration is not bound by anything a kernel does but by three
 // launches, their load chains and their last-block reductions (19 us on 15,000
-// particles, 33 on 126,000; resident 9 and 22, there bound by the conflicts of
-// the shared-memory gathers).  Here a block keeps its rows' neighbours' positions and ranks in
+// particles, 33 on 126,000; resident 8.2, and 20.5 on 147,000).  Here a block keeps its rows' neighbours' positions and ranks in
 // shared memory and its vectors in registers for the whole phase, and an
 // iteration crosses the grid's barrier twice:
 //
@@ -1145,25 +1144,25 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
 // pipe: 1.2 ms on 1.3 million particles.  C, the transposed lists (0.69 ms),
 // b with the pair terms (2.06) and their slicing (1.04) took 5.0 ms in passes
 // of their own.
-template <int D>
+template <int D, int L>
 __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
                                                     const double* __restrict__ vel, const int* __restrict__ ncp,
                                                     const long long* __restrict__ nptrP, const int* __restrict__ nindP,
                                                     const double* __restrict__ pvec, double* __restrict__ cval,
                                                     double* __restrict__ bvec, float* __restrict__ invD)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.N) return;
+    const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) / L, part = threadIdx.x % L;
+    const int i = min(i0, P.N - 1);
     const bool fluid = i < P.Nf;
     double xi[3];
     load_vec<D>(pos, i, xi);
     const double rP2 = P.rP * P.rP, K = -P.kfp * P.m2h_rp;
     const long long b = nptrP[i];
-    const int n = ncp[i];
+    const int n = i0 < P.N ? ncp[i] : 0;
     double self[3] = {0, 0, 0}, cp[3] = {0, 0, 0};
     float dp[3] = {0.f, 0.f, 0.f};
     int selfk = 0;
-    for (int a = 0; a < n; ++a) {
+    for (int a = part; a < n; a += L) {
         const int j = nindP[b + a];
         double cv[3] = {0, 0, 0};
         if (j == i) {
@@ -1190,7 +1189,14 @@ __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __re
 #pragma unroll
         for (int r = 0; r < D; ++r) cval[(b + a) * D + r] = cv[r];
     }
-    if (!fluid) return;
+#pragma unroll
+    for (int r = 0; r < D; ++r) {
+        self[r] = row_sum<L>(self[r]);
+        cp[r] = row_sum<L>(cp[r]);
+        dp[r] = row_sum<L>(dp[r]);
+    }
+    selfk = row_sum<L>(selfk);   // set by one lane
+    if (!fluid || i0 >= P.N || part != 0) return;
     const int ti = type[i];
     const double pi = pvec[i];
     double v[3];
@@ -1336,17 +1342,17 @@ __global__ void __launch_bounds__(256) k_pen_pack(int Nf, double* __restrict__ x
 // lambda_k t_k, t = C^T x in FP64 from the particle's own P-list:
 // C_jk = - C_kj (to the rounding of the minimum image), and C_kk for a fluid
 // row itself
-template <int D>
-__device__ __forceinline__ void pen_ct64(const DevParams& P, int k, const int* __restrict__ type, const int* __restrict__ ncp,
+template <int D, int L>
+__device__ __forceinline__ void pen_ct64(const DevParams& P, int tid, const int* __restrict__ type, const int* __restrict__ ncp,
                                          const long long* __restrict__ nptrP, const int* __restrict__ nindP,
                                          const double* __restrict__ cval, const double* __restrict__ x, double* __restrict__ t)
 {
-    if (k >= P.N) return;
-    const long long b = nptrP[k];
-    const int n = ncp[k];
+    const int k = tid / L, part = tid % L;
+    const long long b = k < P.N ? nptrP[k] : 0;
+    const int n = k < P.N ? ncp[k] : 0;
     double s = 0.0;
 #pragma unroll 2
-    for (int a = 0; a < n; ++a) {
+    for (int a = part; a < n; a += L) {
         const int j = nindP[b + a];
         if (j >= P.Nf) continue;
         double v = 0.0;
@@ -1354,7 +1360,8 @@ __device__ __forceinline__ void pen_ct64(const DevParams& P, int k, const int* _
         for (int d = 0; d < D; ++d) v += cval[(b + a) * D + d] * x[(size_t)j * D + d];
         s = j == k ? s + v : s - v;
     }
-    t[k] = P.lambda[type[k]] * s;
+    s = row_sum<L>(s);
+    if (k < P.N && part == 0) t[k] = P.lambda[type[k]] * s;
 }
 
 // vacc_i (+)= scale sum over the fluid neighbours of f e (e . (x_i - x_j)),
@@ -1362,9 +1369,10 @@ __device__ __forceinline__ void pen_ct64(const DevParams& P, int k, const int* _
 // for x_0) and some 35 instructions; bound by the L1's gather rate.  Against
 // the stored FP32 g and columns (16 bytes a slot streamed, x in six 4-byte
 // gathers: 1.33 ms on 1.3 million particles with the P-part) it needs no pair
-// terms, which took three passes to build: 0.73 ms for x_0, 0.62 for z.
+// terms, which took three passes to build: with C^T x in the same launch 0.93
+// ms for x_0, 0.82 for z.
 // The launch's first nbT blocks form lambda t of C^T x meanwhile (pen_ct64).
-template <int D, int L, bool FIRST>
+template <int D, int L, bool FIRST, int LT>
 __global__ void __launch_bounds__(256) k_pen_visc(DevParams P, int nbT, const int4* __restrict__ vpos, const int* __restrict__ nfc,
                                                   const long long* __restrict__ nptr, const int* __restrict__ nind,
                                                   const float4* __restrict__ rec, int* __restrict__ wrap,
@@ -1376,7 +1384,7 @@ __global__ void __launch_bounds__(256) k_pen_visc(DevParams P, int nbT, const in
                                                   const double* __restrict__ x, double* __restrict__ t)
 {
     if ((int)blockIdx.x < nbT) {
-        pen_ct64<D>(P, blockIdx.x * blockDim.x + threadIdx.x, type, ncp, nptrP, nindP, cval, x, t);
+        pen_ct64<D, LT>(P, blockIdx.x * blockDim.x + threadIdx.x, type, ncp, nptrP, nindP, cval, x, t);
         return;
     }
     const int i = ((blockIdx.x - nbT) * blockDim.x + threadIdx.x) / L, lane = threadIdx.x & (L - 1);
@@ -1448,7 +1456,7 @@ __global__ void __launch_bounds__(256) k_pen_visc(DevParams P, int nbT, const in
     }
 }
 
-template <int D>
+template <int D, int L>
 __global__ void __launch_bounds__(128) k_pen_resid(DevParams P, const int* __restrict__ type, const int* __restrict__ nc,
                                                    const int* __restrict__ nfc, const int* __restrict__ ncp,
                                                    const long long* __restrict__ nptrP, const int* __restrict__ nindP,
@@ -1457,22 +1465,26 @@ __global__ void __launch_bounds__(128) k_pen_resid(DevParams P, const int* __res
                                                    const double* __restrict__ x, const double* __restrict__ b, double* __restrict__ r,
                                                    double* __restrict__ partials, unsigned* __restrict__ counter, double* __restrict__ out)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double acc = 0.0;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / L, part = threadIdx.x % L;
+    double acc = 0.0, y[3] = {0.0, 0.0, 0.0};
     if (i < P.Nf) {
-        double xi[3] = {0.0, 0.0, 0.0}, y[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-            xi[d] = x[(size_t)i * D + d];
-            y[d] = vacc[(size_t)i * D + d];
-        }
         const long long pb = nptrP[i];
         const int np = ncp[i];
 #pragma unroll 2
-        for (int a = 0; a < np; ++a) {
+        for (int a = part; a < np; a += L) {
             const double lt = t[nindP[pb + a]];
 #pragma unroll
             for (int d = 0; d < D; ++d) y[d] += cval[(pb + a) * D + d] * lt;
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < D; ++d) y[d] = row_sum<L>(y[d]);
+    if (i < P.Nf && part == 0) {
+        double xi[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            xi[d] = x[(size_t)i * D + d];
+            y[d] += vacc[(size_t)i * D + d];
         }
         if (nc[i] > nfc[i]) {   // wall neighbours: their part of the viscous diagonal
             const double2* sp = reinterpret_cast<const double2*>(sdiag64 + (size_t)i * 8);
@@ -1566,7 +1578,7 @@ static void pen_shape(mph_case* c)
     const int cap = cr_capacity(c->dim);
     int rows = std::max(c->dim == 2 ? kCrMinRows2 : kCrMinRows3, cap > 0 ? ((N + cap - 1) / cap + 31) / 32 * 32 : 0);
     // as long as the rows fit, one block an SM: half the blocks at a crossing
-    // and twice the registers (k_pen_resident's kCrAhead).  A step of 33,600
+    // and twice the registers (kCrAhead).  A step of 33,600
     // particles in 3-D 2.44 -> 2.03 ms, 57,000 2.61 -> 2.42, 71,000 3.03 ->
     // 2.75; 2-D the same either way.  (One block of up to 1024 threads an SM
     // beyond 77,824 particles, with the registers of two: no difference.)
@@ -1678,14 +1690,19 @@ int launch_pen_assemble(mph_case* c)
     if (!d.sdiag64) MPH_CUDA(cudaMalloc((void**)&d.sdiag64, (size_t)P.Nf * 8 * sizeof(double)));
     MPH_TRY(grow_t(&d.cval, &d.cap_cval, c->nnbP * c->dim));
     launch_vector_p(c);
-    const unsigned g = grid_for(P.N, 256), gs = grid_for(P.N, 128);
+    const unsigned g = grid_for(P.N, 256);
     float* invD = d.v32 + 7 * vec32_stride(n);
+    const int L = plist_lanes(P.N);
+    auto system = [&](auto kern) {
+        kern<<<grid_for((long long)P.N * L, 128), 128, 0, st>>>(P, d.type, d.pos, d.vel, d.ncp, d.nptrP, d.nindP, d.pvec, d.cval, d.bvec, invD);
+        MPH_COUNT_LAUNCH();
+    };
     if (c->dim == 2) {
         { k_fixed_positions<2><<<g, 256, 0, st>>>(P, d.type, d.pos, d.ipos, d.vpos, d.wrap32); MPH_COUNT_LAUNCH(); }
-        { k_pen_system<2><<<gs, 128, 0, st>>>(P, d.type, d.pos, d.vel, d.ncp, d.nptrP, d.nindP, d.pvec, d.cval, d.bvec, invD); MPH_COUNT_LAUNCH(); }
+        L == 4 ? system(k_pen_system<2, 4>) : system(k_pen_system<2, 1>);
     } else {
         { k_fixed_positions<3><<<g, 256, 0, st>>>(P, d.type, d.pos, d.ipos, d.vpos, d.wrap32); MPH_COUNT_LAUNCH(); }
-        { k_pen_system<3><<<gs, 128, 0, st>>>(P, d.type, d.pos, d.vel, d.ncp, d.nptrP, d.nindP, d.pvec, d.cval, d.bvec, invD); MPH_COUNT_LAUNCH(); }
+        L == 4 ? system(k_pen_system<3, 4>) : system(k_pen_system<3, 1>);
     }
     auto walls = [&](auto kern, int lanes) {
         kern<<<grid_for((long long)P.Nf * lanes, 128), 128, 0, st>>>(P, d.type, d.pos, d.vel, d.nc, d.nfc, d.nptr, d.nind, d.bvec, d.sdiag64);
@@ -1709,18 +1726,25 @@ int pen_exact_diag(mph_case* c)
 }
 
 // the viscous pairs' sum, C^T x and the residual, after k_pen_pack
-template <int D, int L, bool FIRST>
-static void pen_residual(mph_case* c, double scale, const double* scale_src)
+template <int D, int L, bool FIRST, int LT>
+static void pen_residual_t(mph_case* c, double scale, const double* scale_src)
 {
     DeviceState& d = c->d;
     const DevParams& P = c->dp;
     cudaStream_t st = c->stream;
-    const unsigned nbT = grid_for(P.N, 256);
-    { k_pen_visc<D, L, FIRST><<<nbT + grid_for((long long)P.Nf * L, 256), 256, 0, st>>>(
+    const unsigned nbT = grid_for((long long)P.N * LT, 256);
+    { k_pen_visc<D, L, FIRST, LT><<<nbT + grid_for((long long)P.Nf * L, 256), 256, 0, st>>>(
           P, (int)nbT, d.vpos, d.nfc, d.nptr, d.nind, d.z4, d.wrap32, d.type, d.pos, d.pos32, d.poslo32, scale, scale_src, d.vacc,
           d.ncp, d.nptrP, d.nindP, d.cval, d.x, d.tct); MPH_COUNT_LAUNCH(); }
-    { k_pen_resid<D><<<grid_for(P.Nf, 128), 128, 0, st>>>(P, d.type, d.nc, d.nfc, d.ncp, d.nptrP, d.nindP, d.cval, d.tct, d.sdiag64, d.vacc,
+    { k_pen_resid<D, LT><<<grid_for((long long)P.Nf * LT, 128), 128, 0, st>>>(P, d.type, d.nc, d.nfc, d.ncp, d.nptrP, d.nindP, d.cval, d.tct, d.sdiag64, d.vacc,
                                                           d.x, d.bvec, d.r, d.partials, (unsigned*)(d.flags + kFlagCounter), d.scal + kSRR); MPH_COUNT_LAUNCH(); }
+}
+
+template <int D, int L, bool FIRST>
+static void pen_residual(mph_case* c, double scale, const double* scale_src)
+{
+    if (plist_lanes(c->dp.N) == 4) pen_residual_t<D, L, FIRST, 4>(c, scale, scale_src);
+    else pen_residual_t<D, L, FIRST, 1>(c, scale, scale_src);
 }
 
 // lanes a row of k_pen_visc: about 180 neighbours in 3-D, 37 in 2-D

@@ -75,6 +75,15 @@ __device__ __forceinline__ double norm2_fma(const double* q)
     return s;
 }
 
+// The sum of a value over the L lanes of a row (L a power of two; the same in all of them)
+template <int L, typename T>
+__device__ __forceinline__ T row_sum(T v)
+{
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 template <int D>
 __device__ __forceinline__ void load_vec(const double* __restrict__ a, int i, double* v)
 {
