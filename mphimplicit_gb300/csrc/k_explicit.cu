@@ -37,7 +37,7 @@ __device__ __forceinline__ double sqrt_by_rsqrt(double v)
 // one by one took 80, with roundings left out accordingly.  The sums run in
 // pieces of 32 neighbours, which keeps their own roundings below those of one
 // long sum.  The radius tests compare bit patterns on the integer pipe.
-// 326,592 particles: 6.42 -> 2.79 ms; 71,300: 1.84 -> 0.80.
+// 326,592 particles: 6.42 -> 2.79 ms; 71,200: 1.84 -> 0.80.
 constexpr int kDensityRun = 32;
 
 template <int D>
@@ -105,7 +105,7 @@ __global__ void k_pressure_a(DevParams P, const int* __restrict__ type, const do
 // one of h = ratio_ji g_j - ratio_ij g_i, with one reciprocal square root and
 // the constants' products formed once, about 60 FP64 operations a pair
 // against some 30 divisions with the terms formed one by one.  4.82 -> 1.31
-// ms on 71,300 particles.
+// ms on 71,200 particles.
 template <int D>
 __global__ void __launch_bounds__(128) k_surface_forces(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
                                                         const int* __restrict__ nc, const long long* __restrict__ nptr,
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(128) k_output_forces(DevParams P, const int* _
 // calculateDensityP alone over the P-list.  The P-list holds exactly the
 // pairs with r^2 <= RadiusP^2, in the full list's order (the sum differs from
 // the full-list pass's by the rounding of its pieces).  As k_density: 37 FP64
-// operations a pair became 28; 340 -> 243 us on 374,000 particles.
+// operations a pair became 28; 340 -> 243 us on 326,592 particles.
 template <int D, int L>
 __global__ void __launch_bounds__(128) k_density_p(DevParams P, const double* __restrict__ pos, const int* __restrict__ ncp,
                                                    const long long* __restrict__ nptrP, const int* __restrict__ nindP,

@@ -3,8 +3,8 @@
 // A = inertia + V + C Lambda C^T (calculateMatrixA main.cpp:2251-2335,
 // multiplyMatrixC main.cpp:2574-2642).  Stored as 3 x 3 blocks it takes 9
 // FP64 multiply-adds and 72 bytes a neighbour (about 170 a row in 3-D), and
-// the FP64 units bound it: 0.66 ms an application on 216,000 particles for
-// 2.7 GB of blocks.  In parts it takes 0.38:
+// the FP64 units bound it: 0.66 ms an application on 216,000 fluid particles for
+// 2.7 GB of blocks.  In parts it takes 0.35:
 //
 //   t_k = lambda_k sum_{j in P(k)} C_jk . s_j,  (C Lambda C^T s)_i = sum_{k in P(i)} C_ik t_k   FP64, over P-lists of about 20
 //   (V s)_i = sum_j g_ij (g_ij . (s_i - s_j)) + W_i s_i,   g = sqrt(f) q / |q|, W_i the wall slots' block
@@ -102,7 +102,7 @@ __device__ __forceinline__ F2 f2_rsqrt(F2 v)
 // RadiusV, f / inertia = A (1/r - 1), A = visc mu_ij kf 2 / RadiusV^2 / inertia
 // up to the sign (main.cpp:2261-2289), so g = sqrt(A (1/r - 1)) r_vec / r, from
 // the FP64 separation on in two floats: in FP64 throughout the kernel took
-// 3.6 ms on 216,000 particles, once a solve; it takes 2.4.  type_out: the types at an
+// 3.6 ms on 216,000 fluid particles, once a solve; it takes 2.4.  type_out: the types at an
 // address that stays from step to step (the particle arrays swap with their
 // alternates; the iteration's graph is replayed).
 __global__ void __launch_bounds__(128) k_f64_pairs(DevParams P, double inert, const int* __restrict__ type, const double* __restrict__ pos,
@@ -178,9 +178,10 @@ __global__ void __launch_bounds__(128) k_f64_pairs(DevParams P, double inert, co
 // itself), and the pairs' part of y, four threads (of four warps) a row.  A
 // pair streams 28 bytes, gathers 24 (the neighbour's record, mostly from L1
 // and L2) and takes about 90 FP32 instructions; the latency of column, then
-// record, bounds it.  On 216,000 particles 308 us with four threads a row
+// record, bounds it.  On 216,000 fluid particles 308 us with four threads a row
 // and eight pairs in flight (a thread a row: 438 with two, 350 with eight;
-// eight threads a row, 322), the stream of records alone some 160.
+// eight threads a row, 322; 288 with the stop test's quotient once a block),
+// the stream of records alone some 160.
 constexpr int kF64Lanes = 4;      // threads a row of t
 constexpr int kPairSplit = 4;     // and of the pairs
 constexpr int kPairUnroll = 8;

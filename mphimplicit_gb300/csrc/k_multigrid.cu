@@ -287,7 +287,7 @@ __host__ __device__ inline bool full_stencil(const LevelK& L, int D)
 // fourth stencil cell each, their sums added by shuffles.  Such a sweep is
 // bound by a row's chain of FP64 multiply-adds (their latency is beyond 100
 // clocks here, and a level has few rows: 24,000 threads with 81 terms each on
-// 216,000 particles, 25 us a sweep); four chains a row are a quarter as long
+// 326,592 particles, 25 us a sweep); four chains a row are a quarter as long
 // with four times the threads in flight.  The threads of a stencil part hold 8 consecutive
 // rows, so their loads stay 64-byte segments.
 // RESID: out = Q - A S;  else out = S + invD (Q - A S).
@@ -701,9 +701,9 @@ k_mg_small_levels(CoarseArgs<T> A, const int* __restrict__ flags)
 // they are one pass of n^2 multiply-adds spread over the whole chip.  M is
 // built once a solve, a block a column: the sweeps on the unit vector, in the
 // sweeps' own order (the cells' coefficients stay in L2 meanwhile); a solve's
-// values move by rounding only (1e-16).  A solve of 10,000 particles in 2-D
+// values move by rounding only (1e-16).  A solve of 12,000 particles in 2-D
 // (578 rows, 57 cycles) took 7.4 ms with one cluster kernel for the small
-// levels (81 us of a 132 us iteration) and takes 3.2; of 216,000 in 3-D (375
+// levels (81 us of a 132 us iteration) and takes 3.2; of 326,592 in 3-D (375
 // rows, 75 cycles; with k_mg_sweep64) 82 and 62.
 // Up to 1024 rows: M is 8 MB and its build some 5e8 multiply-adds (about a
 // millisecond in 3-D, less than a dozen cycles of sweeps); eight times the

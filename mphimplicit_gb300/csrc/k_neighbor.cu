@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(128) k_neighbors(DevParams P, int rx, int ry, 
 // In 2-D a cell has about 10 particles and 90 candidates, so the blocks are
 // small and many: 64 threads and room for 512 candidates (30 KB of shared
 // memory a block of eight warps held an SM to seven blocks and left their
-// start and staging latencies uncovered).  Both passes on 735,000 particles 1.0 -> 0.63
+// start and staging latencies uncovered).  Both passes on 412,000 particles 1.0 -> 0.63
 // ms (0.71 with 128 threads).  In 3-D, 30 and 810: 256 threads, 1536.
 template <int D> constexpr int kNbThreads = D == 2 ? 64 : 256;   // at least two warps: one a pass reads the walk's buckets
 template <int D> constexpr int kNbCap = D == 2 ? 512 : 1536;

@@ -104,8 +104,8 @@ __global__ void k_cell_keys(DevParams P, const double* __restrict__ pos, const i
 // back, so a pass costs one trip through shared memory and one barrier where
 // a stage of two 4-byte arrays each had one.  The stages above a tile run
 // three a launch in the same way, through global memory.  The whole cell-sort
-// stage on 1.3 million particles 0.90 -> 0.55 ms, on 17,000 0.165 -> 0.11.
-// Tiles of 2^12: 2^11, 2^13 and 2^14 took 0.121, 0.113 and 0.128 ms on 17,000
+// stage on 1.3 million particles 0.90 -> 0.55 ms, on 22,000 0.165 -> 0.11.
+// Tiles of 2^12: 2^11, 2^13 and 2^14 took 0.121, 0.113 and 0.128 ms on 22,000
 // (a tile is one block: larger ones leave SMs idle), 0.58, 0.57 and 0.52 on
 // 1.3 million.
 constexpr int kTileExp = 12;
@@ -263,7 +263,7 @@ __global__ void k_bucket_order(int nb, const long long* __restrict__ off, int* _
 // bucket[b] = first sorted position whose key >= b, b in [0, 2T].  A run of
 // empty cells (the free space of a dam: tens of thousands) is filled by the
 // warp together; by the one thread at its edge it took 171 us of a 5.7 ms
-// step on 735,000 particles in 2-D.
+// step on 412,000 particles in 2-D.
 __global__ void k_bucket_starts(const int* __restrict__ key, int N, int T, int* __restrict__ bucket)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;

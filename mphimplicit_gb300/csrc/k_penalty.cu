@@ -58,8 +58,8 @@ constexpr int kPlWords = 1 << 13;   // bitmap of a row block's columns: 2^18 par
 constexpr int kMaxPenRows = 256;   // threads of a row block (rows times threads a row) of the per-iteration kernels
 constexpr int kCrThreads = 512;    // of the resident iteration's blocks, two an SM
 constexpr int kCrBlocks = 2 * 152;
-// Rows a block at least.  A solve alone is fastest on many blocks (15,000
-// particles in 3-D: 2.01, 1.89, 2.00 ms with 128, 192, 256; 17,000 in 2-D,
+// Rows a block at least.  A solve alone is fastest on many blocks (22,000
+// particles in 3-D: 2.01, 1.89, 2.00 ms with 128, 192, 256; 12,000 in 2-D,
 // where a row is a fifth of the work: 1.00, 1.04, 1.08 with 192, 256, 384),
 // but the blocks of a solve hold their SMs until it ends: an ensemble of 64
 // two-dimensional cases on their streams takes 52.9, 46.3, 37.9 and 37.5 ms
@@ -700,10 +700,11 @@ __global__ void __launch_bounds__(kReduceThreads) k_pen_vec(PenArgs A, int n, in
 // All CR iterations of a refinement phase in one cooperative kernel, for the
 // cases whose rows fit the chip at once (up to 155,648 particles).  Such a
 // case's iteration is not bound by anything a kernel does but by three
-// launches, their load chains and their last-block reductions (19 us on 15,000
-// particles, 33 on 126,000; resident 8.2, and 20.5 on 147,000).  Here a block keeps its rows' neighbours' positions and ranks in
-// shared memory and its vectors in registers for the whole phase, and an
-// iteration crosses the grid's barrier twice:
+// launches, their load chains and their last-block reductions (19 us on 22,000
+// particles, 33 on 155,000; resident 8.2 and 20.5).  Here a block keeps its
+// rows' neighbours' positions and ranks in shared memory and its vectors in
+// registers for the whole phase, and an iteration crosses the grid's barrier
+// twice:
 //
 //   after t    lambda t of every particle, and (r, r) of the vectors it came from
 //   after y    s, D^-1 y and D^-1 q of every row, and the dot products
@@ -1217,7 +1218,7 @@ __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __re
 // took 0.61 ms on 1.3 million particles, most of it rows without any slots
 // and sums over the warp; the assembly stage takes 2.26 ms there with 16
 // threads a row, 2.32 with 4, which leave 15 slots in line a thread (0.18 ms
-// on 15,000 particles, 0.15 with 16).  In 2-D a row has a dozen: 8.
+// on 22,000 particles, 0.15 with 16).  In 2-D a row has a dozen: 8.
 template <int D, int L>
 __global__ void __launch_bounds__(128) k_pen_wall(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
                                                   const double* __restrict__ vel, const int* __restrict__ nc,

@@ -67,8 +67,14 @@ int case_footprint(const mph_params* prm, const mph_particles* parts, int dim, i
         b += (double)Nf * np * (D * 4.0 + 4.0) * 2.2 + (double)N * (8.0 * 16.0 + 8.0) + (double)Nf * 32.0;
         b += (double)Nf * 17.0 * 4.0;                         // block-local neighbour columns
         b += (double)N * 33.0 * 4.0 + (double)Nf * np * 2.0;   // the same for the transposed P-lists (blocks of 256)
+        // the point-Jacobi form has none of these, but C and ranks of every
+        // particle's P-list (a wall-heavy case), fixed-point positions and the
+        // residual's and the resident iteration's records
+        b += 1.13 * (double)N * np * (D * 8.0 + 2.0) + (double)N * 60.0 + (double)Nf * 130.0;
     } else {
         b += blocks * DD * 8.0;                               // FP64 blocks
+        if (precision != MPH_PRECISION_MIXED && dim == 3)     // the operator in parts: pair records, C of every P-list
+            b += 1.13 * (blocks * 24.0 + (double)N * np * D * 8.0) + (double)N * 12.0 + (double)Nf * 120.0;
         if (precision == MPH_PRECISION_MIXED) {
             b += 2.0 * blocks * DD * 4.0;                     // FP32 blocks, sliced and row-contiguous
             b += (double)Nf * nb * 16.0;                      // FP32 pair terms

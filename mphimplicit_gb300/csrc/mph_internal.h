@@ -252,9 +252,9 @@ inline size_t vec32_stride(long long n) { return ((size_t)n + 3) & ~(size_t)3; }
 
 // Threads a row of the P-list passes (density, p, C and b, C^T x, residual):
 // four where the rows alone leave the chip waiting on each row's chain of some
-// twenty dependent loads and FP64 operations (15,000 particles: assembly 0.157
+// twenty dependent loads and FP64 operations (22,000 particles: assembly 0.157
 // -> 0.131 ms, a solve 1.58 -> 1.55), one beyond, where the FP64 sums over a
-// row's threads cost more than they hide (147,000: a solve 3.79 and 3.92;
+// row's threads cost more than they hide (155,000: a solve 3.79 and 3.92;
 // 1.3 million: 22.5 and 23.8).
 inline int plist_lanes(int n) { return n <= 65536 ? 4 : 1; }
 
