@@ -844,12 +844,12 @@ int build_mg_tail(mph_case* c)
         if (l >= first) A.total += A.L[l].rows;
     }
     const int smem = 4 * A.total * (int)sizeof(double);
-    static std::once_flag once;
-    std::call_once(once, [] {   // the largest any case can need
+    if (!c->tail_attr) {   // once a case (a function's attributes belong to the device): the largest any case can need
         const int smax = 4 * kTailTotal * (int)sizeof(double);
-        cudaFuncSetAttribute(k_mg_tail_columns<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax);
-        cudaFuncSetAttribute(k_mg_tail_columns<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax);
-    });
+        if (c->dim == 2) MPH_CUDA(cudaFuncSetAttribute(k_mg_tail_columns<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+        else MPH_CUDA(cudaFuncSetAttribute(k_mg_tail_columns<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+        c->tail_attr = true;
+    }
     if (c->dim == 2) { k_mg_tail_columns<2><<<n, kTailThreads, smem, c->stream>>>(A, c->d.mg_tail); MPH_COUNT_LAUNCH(); }
     else { k_mg_tail_columns<3><<<n, kTailThreads, smem, c->stream>>>(A, c->d.mg_tail); MPH_COUNT_LAUNCH(); }
     MPH_CUDA(cudaGetLastError());

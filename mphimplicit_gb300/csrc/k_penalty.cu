@@ -1547,23 +1547,19 @@ static size_t cr_smem(const mph_case* c, int rows, int umax)
 }
 
 // Blocks of the resident iteration that the device holds at once (0: none)
-static int cr_capacity(int dim)
+static int cr_capacity(mph_case* c)
 {
-    static std::once_flag once;
-    static int cap[2] = {0, 0};
-    std::call_once(once, [] {
-        int dev = 0, sms = 0, coop = 0, nb[2] = {0, 0};
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        const void* f[4] = {(const void*)k_pen_cr<2, 1>, (const void*)k_pen_cr<3, 1>, (const void*)k_pen_cr<2, kCrAhead>, (const void*)k_pen_cr<3, kCrAhead>};
+    if (c->cr_cap < 0) {   // once a case: the attributes and the count belong to its device
+        int sms = 0, coop = 0, nb = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
+        const void* f[2] = {c->dim == 2 ? (const void*)k_pen_cr<2, 1> : (const void*)k_pen_cr<3, 1>,
+                            c->dim == 2 ? (const void*)k_pen_cr<2, kCrAhead> : (const void*)k_pen_cr<3, kCrAhead>};
         for (const void* k : f) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCrSmem);
-        for (int k = 0; k < 2; ++k) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[k], f[k], kCrThreads, kCrSmem);
-            cap[k] = coop ? sms * nb[k] : 0;
-        }
-    });
-    return std::min(cap[dim - 2], kCrBlocks);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f[0], kCrThreads, kCrSmem);
+        c->cr_cap = std::min(coop ? sms * nb : 0, kCrBlocks);
+    }
+    return c->cr_cap;
 }
 
 // Rows a block and threads a row.  Up to 155,648 particles the iteration is
@@ -1576,7 +1572,7 @@ static int cr_capacity(int dim)
 static void pen_shape(mph_case* c)
 {
     const int N = c->dp.N;
-    const int cap = cr_capacity(c->dim);
+    const int cap = cr_capacity(c);
     int rows = std::max(c->dim == 2 ? kCrMinRows2 : kCrMinRows3, cap > 0 ? ((N + cap - 1) / cap + 31) / 32 * 32 : 0);
     // as long as the rows fit, one block an SM: half the blocks at a crossing
     // and twice the registers (kCrAhead).  A step of 33,600
@@ -1645,15 +1641,14 @@ static int launch_pen_lists(mph_case* c)
     c->loc_ct_blocks = 0;
     if (!c->inner_local) return MPH_OK;
     const size_t smem = 2 * kPlWords * sizeof(unsigned);
-    static std::once_flag once;
-    std::call_once(once, [smem] {   // fixed maxima: host threads of a batch would race on per-launch values
-        cudaFuncSetAttribute(k_plist_ranks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (!c->pen_attr) {   // once a case; fixed maxima: host threads of a batch would race on per-launch values
         const int t = (pen_ucap(kMaxPenRows) + 256) * 24, y = (pen_ucap(kMaxPenRows) + 256) * 16;
-        cudaFuncSetAttribute(k_pen_t<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, t);
-        cudaFuncSetAttribute(k_pen_t<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, t);
-        cudaFuncSetAttribute(k_pen_y<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, y);
-        cudaFuncSetAttribute(k_pen_y<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, y);
-    });
+        const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        MPH_CUDA(cudaFuncSetAttribute(k_plist_ranks, a, (int)smem));
+        MPH_CUDA(c->dim == 2 ? cudaFuncSetAttribute(k_pen_t<2>, a, t) : cudaFuncSetAttribute(k_pen_t<3>, a, t));
+        MPH_CUDA(c->dim == 2 ? cudaFuncSetAttribute(k_pen_y<2>, a, y) : cudaFuncSetAttribute(k_pen_y<3>, a, y));
+        c->pen_attr = true;
+    }
     MPH_CUDA(cudaMemsetAsync(d.pucount + nb, 0, 4 * sizeof(int), c->stream));
     { k_plist_ranks<<<nb, c->pen_rows, smem, c->stream>>>(P.N, P.Nf, c->pen_pw4, ucap, d.ncp, d.nptrP, d.nindP, d.pidx, d.pgroups,
                                                          d.puniq, d.pucount); MPH_COUNT_LAUNCH(); }

@@ -322,6 +322,8 @@ struct mph_case {
     bool level0_done = false;           // this step's level-0 multigrid stencils were written by the assembly
     bool step_f64 = false;              // this step's FP64 solve may run on k_f64op.cu's operator in parts
     long long f64_slots = 0;            // slots the pair records have room for (their two arrays' split)
+    int cr_cap = -1;                    // blocks of the resident iteration its device holds at once (-1: not asked yet)
+    bool pen_attr = false, tail_attr = false;   // its kernels' shared-memory limits are set on its device
     bool shared_gpu = false;            // other cases step on this GPU meanwhile (a batch of several, a server)
     bool step_pen = false;              // this step's inner CR runs on k_penalty.cu's operator
     int pmax = 0;                       // longest P-list of the current lists
