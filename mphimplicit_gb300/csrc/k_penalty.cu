@@ -64,8 +64,11 @@ constexpr int kCrBlocks = 2 * 152;
 // but the blocks of a solve hold their SMs until it ends: an ensemble of 64
 // two-dimensional cases on their streams takes 52.9, 46.3, 37.9 and 37.5 ms
 // with 192, 256, 384 and 512.
-constexpr int kCrAhead = 3;        // staged neighbours a thread loads while alpha and beta are formed, in blocks alone on their SM
 constexpr int kCrMinRows3 = 192, kCrMinRows2 = 384;
+// Staged neighbours a thread loads while alpha and beta are formed: in blocks
+// alone on their SM, and in two blocks an SM (in 3-D none there: its twelve
+// registers would spill; a step of 89,000 particles 3.31 ms, 3.49 with one)
+constexpr int kCrAhead = 3, kCrShared3 = 0, kCrShared2 = 1;
 constexpr int kCrSmem = 100 * 1024;   // dynamic: two blocks an SM with their 7 KB of static shared memory
 // Staged neighbours a block of `rows` rows has room for.  Blocks of a
 // 3.5-spacing cell order have about 2.8 (256 rows) to 3.9 (64) times their
@@ -343,7 +346,10 @@ __device__ __forceinline__ bool grid_sums(const float* v, const PenArgs& A, int 
 // wait for the block's count or the row's length (both buffers have room for
 // every index read here); what lies beyond is not used.  A block's time is
 // this chain of loads, so nothing in it waits that need not.
-constexpr int kPreCols = 3, kPreWords = 4;
+// (Three columns and three words: a solve of three steps on 1.3 million particles
+// 66.7 ms, of one on 326,592 7.78; with four words, whose registers k_pen_t
+// spilled, 67.5 and 8.03, with two words 67.7, with two columns 70.2.)
+constexpr int kPreCols = 3, kPreWords = 3;
 struct PenPre {
     int col[kPreCols];
     uint2 word[kPreWords];
@@ -701,7 +707,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_pen_vec(PenArgs A, int n, in
 // cases whose rows fit the chip at once (up to 155,648 particles).  Such a
 // case's iteration is not bound by anything a kernel does but by three
 // launches, their load chains and their last-block reductions (19 us on 22,000
-// particles, 33 on 155,000; resident 8.2 and 20.5).  Here a block keeps its
+// particles, 33 on 155,000; resident 8.2 and 19.3).  Here a block keeps its
 // rows' neighbours' positions and ranks in shared memory and its vectors in
 // registers for the whole phase, and an iteration crosses the grid's barrier
 // twice:
@@ -858,7 +864,7 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
         ul[k] = j;
         sa[k] = A.ipos[j];
     }
-    int j0[PF];   // the thread's first staged neighbours
+    int j0[PF > 0 ? PF : 1];   // the thread's first staged neighbours
 #pragma unroll
     for (int u = 0; u < PF; ++u) j0[u] = tid + u * nth < U ? ul[tid + u * nth] : -1;
     int ng = 0;
@@ -915,7 +921,7 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
     bool ok = cr_cross(C.count, C.v3, val_s, 6, ++epoch, lb, nb, tid, A.flags);   // every row's s is out
     // a crossing's first loads: the thread's first neighbour's records, while
     // alpha and beta are formed
-    CrRec pre[PF];
+    CrRec pre[PF > 0 ? PF : 1];
 #pragma unroll
     for (int u = 0; u < PF; ++u) pre[u] = cr_load<D>(C.rec, j0[u], A.Nf);
     while (ok) {
@@ -1553,7 +1559,7 @@ static int cr_capacity(mph_case* c)
         int sms = 0, coop = 0, nb = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
-        const void* f[2] = {c->dim == 2 ? (const void*)k_pen_cr<2, 1> : (const void*)k_pen_cr<3, 1>,
+        const void* f[2] = {c->dim == 2 ? (const void*)k_pen_cr<2, kCrShared2> : (const void*)k_pen_cr<3, kCrShared3>,
                             c->dim == 2 ? (const void*)k_pen_cr<2, kCrAhead> : (const void*)k_pen_cr<3, kCrAhead>};
         for (const void* k : f) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCrSmem);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f[0], kCrThreads, kCrSmem);
@@ -1848,8 +1854,8 @@ int launch_pen_resident(mph_case* c, int cap, double scale)
     const size_t smem = cr_smem(c, c->pen_rows, c->pen_umax);
     // a block an SM and the device to itself: the form with more registers
     const bool alone = nb <= kCrBlocks / 2 && !c->shared_gpu;
-    const void* f = c->dim == 2 ? (alone ? (const void*)k_pen_cr<2, kCrAhead> : (const void*)k_pen_cr<2, 1>)
-                                : (alone ? (const void*)k_pen_cr<3, kCrAhead> : (const void*)k_pen_cr<3, 1>);
+    const void* f = c->dim == 2 ? (alone ? (const void*)k_pen_cr<2, kCrAhead> : (const void*)k_pen_cr<2, kCrShared2>)
+                                : (alone ? (const void*)k_pen_cr<3, kCrAhead> : (const void*)k_pen_cr<3, kCrShared3>);
     MPH_CUDA(cudaLaunchCooperativeKernel(f, dim3(nb), blk, args, smem, c->stream));
     MPH_COUNT_LAUNCH();
     return MPH_OK;
