@@ -1629,6 +1629,7 @@ static int launch_pen_lists(mph_case* c)
 {
     DeviceState& d = c->d;
     const DevParams& P = c->dp;
+    c->pen_staged = false;
     pen_shape(c);
     c->pen_pw4 = (c->pmax + 3) / 4;
     const int nsl = (P.N + 31) / 32, nb = (int)grid_for(P.N, c->pen_rows), ucap = pen_ucap(c->pen_rows);
@@ -1666,6 +1667,7 @@ static int launch_pen_lists(mph_case* c)
     c->loc_blocks[0] = h[2];
     c->loc_blocks[1] -= h[2];
     c->loc_cols = (long long)(unsigned)h[3];
+    c->pen_staged = true;
     return MPH_OK;
 }
 
@@ -1815,7 +1817,7 @@ static PenArgs pen_args(const mph_case* c, int cap)
     A.idx = d.pidx;
     A.groups = d.pgroups;
     A.uniq = d.puniq;
-    A.ucount = c->inner_local ? d.pucount : nullptr;
+    A.ucount = c->pen_staged ? d.pucount : nullptr;   // as the assembly built the lists: the option may have changed since
     A.ncp = d.ncp;
     A.nindP = d.nindP;
     A.nptrP = d.nptrP;

@@ -328,6 +328,7 @@ struct mph_case {
     bool step_pen = false;              // this step's inner CR runs on k_penalty.cu's operator
     int pmax = 0;                       // longest P-list of the current lists
     int pen_rows = 0, pen_w = 0;        // its rows a block and threads a row
+    bool pen_staged = false;            // the assembly built the row blocks' ranks and columns (option inner_local as it was then)
     bool pen_resident = false;          // a phase's CR iterations in one cooperative kernel (the case's rows fit the chip at once)
     int pen_pw4 = 0, pen_umax = 0;      // 8-byte words a row has room for; largest staged count (rounded up)
     double pen_tol = 0.0;               // what a refinement phase leaves at least (the viscous part outside the operator)
