@@ -1193,6 +1193,7 @@ __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __re
                 }
             }
         }
+        if (j == i && fluid) continue;   // the sum's slot: one store, by the lane that has it (nothing orders two lanes' stores)
 #pragma unroll
         for (int r = 0; r < D; ++r) cval[(b + a) * D + r] = cv[r];
     }

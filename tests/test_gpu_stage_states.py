@@ -6,6 +6,7 @@ import pytest
 
 from mphimplicit_gb300 import casegen, engine
 from mphimplicit_gb300.cabi import PRECISION_MIXED
+from parity_util import csr_blocks_oracle, rel
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +51,19 @@ def test_staging_is_the_assemblys(engine_lib, dim, at_assembly):
         assert np.array_equal(a.export("Velocity"), b.export("Velocity"))
         a.step(1)
         b.step(1)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_c_of_the_mixed_form(engine_lib, oracle_built, dim):
+    """C as the point-Jacobi mixed form's assembly writes it with four threads
+    a row, own slots (the sum of a row's others) included, against the
+    oracle's, to the bound of the FP64 form's parity tests."""
+    params, parts = _parts(dim)
+    o = oracle_built.Oracle(params, parts, dim, threads=1)
+    o.init()
+    g = _mixed(params, parts, dim)
+    for s in BEFORE_SOLVE[:5]:
+        getattr(o, s)()
+        g.stage(s)
+    want = csr_blocks_oracle(o.array("CsrPtrC"), o.array("CsrCofC"), g.fluid_count, g.export("NeighborCountP"), dim, per_block=False)
+    assert rel(g.export("CsrCofC"), want) <= 1e-12
