@@ -281,7 +281,10 @@ int mph_case_set_option(mph_case* c, const char* name, double value);
  *   solve as one CUDA graph whose refinement and CR loops are device-side
  *   conditional while nodes (no host poll; same bits); not with profiling.
  *   "mg_depth" -1 (default) / 0 / 1 .. 24: mixed form only.  The inner CR's
- *   preconditioner: -1 point Jacobi (D^-1 from the pair terms; no multigrid
+ *   preconditioner: -1 point Jacobi (D^-1 from the assembly, with the
+ *   lattice's viscous part; InvDiagA exports the row's own, formed when it is
+ *   read, and fails with MPH_ERR_STATE between the start of a step or
+ *   mph_case_set_state and the next assembly; no multigrid
  *   levels are built, so their export fails with MPH_ERR_STATE), 0 the
  *   reference's V-cycle over every level (preconditionWithMultiGrid,
  *   main.cpp:4122), k the V-cycle cut after its first k levels.

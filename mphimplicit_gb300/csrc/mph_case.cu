@@ -494,6 +494,7 @@ static int grow(void** p, long long* cap, long long need, size_t elem)
 // ---- stages --------------------------------------------------------------------
 int stage_step_begin(mph_case* c)
 {
+    c->system_current = false;
     launch_step_begin(c);
     c->densa_valid = false;
     // WallCenter += WallVelocity*Dt after the particles moved (main.cpp:2123-2127)
@@ -506,6 +507,7 @@ int stage_step_begin(mph_case* c)
 
 int stage_cellsort(mph_case* c)
 {
+    c->system_current = false;
     launch_cell_keys(c);
     if (c->cell_sort) MPH_TRY(launch_counting_sort(c));
     else launch_bitonic_sort(c);
@@ -529,6 +531,7 @@ int stage_cellsort(mph_case* c)
 
 int stage_neighbors(mph_case* c)
 {
+    c->system_current = false;
     const int N = c->dp.N;
     cudaEvent_t pe = nullptr;
     int pon = prof_begin(c, 3, &pe);
@@ -567,8 +570,10 @@ int stage_explicit(mph_case* c)
 int stage_assemble(mph_case* c)
 {
     if (c->stage < 4) return fail(MPH_ERR_STATE, "assemble before the explicit stage");
+    c->system_current = false;
     MPH_TRY(launch_assemble(c));
     MPH_CUDA(cudaGetLastError());
+    c->system_current = true;
     c->stage = 5;
     return MPH_OK;
 }

@@ -81,7 +81,10 @@ static int build_export(mph_case* c, const std::string& name, Out& o)
     if (name == "VectorP") return f64(d.pvec, N);
     if (name == "VectorB") return f64(d.bvec, (size_t)Nf * D);
     if (name == "InvDiagA") {
-        if (c->step_pen) MPH_TRY(pen_exact_diag(c));   // the step itself keeps the FP32 D^-1 with the lattice's viscous part
+        if (c->step_pen) {   // formed now, from the step's lists and C (the step itself keeps the FP32 D^-1 with the lattice's viscous part)
+            if (!c->system_current) return fail(MPH_ERR_STATE, "InvDiagA of the point-Jacobi mixed form is read between its step's assembly and the next step");
+            MPH_TRY(pen_exact_diag(c));
+        }
         return f64(d.invDiag, (size_t)Nf * D);
     }
     if (name == "CellFluidParticleBegin" || name == "CellFluidParticleEnd" || name == "CellWallParticleBegin" ||
@@ -397,6 +400,7 @@ int case_set_state(mph_case* c, const mph_particles* parts, const double* wall_c
     if (wall_center) std::memcpy(&c->wallC[0][0], wall_center, sizeof(c->wallC));
     c->time = parts->time;
     c->densa_valid = false;
+    c->system_current = false;
     // a state from outside has no velocity history, unless the caller
     // declares (option keep_history) that it continues this case's own
     // trajectory in the case's particle order

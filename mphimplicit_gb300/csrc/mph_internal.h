@@ -325,6 +325,7 @@ struct mph_case {
     int cr_cap = -1;                    // blocks of the resident iteration its device holds at once (-1: not asked yet)
     bool pen_attr = false, tail_attr = false;   // its kernels' shared-memory limits are set on its device
     bool shared_gpu = false;            // other cases step on this GPU meanwhile (a batch of several, a server)
+    bool system_current = false;        // positions, types and lists are those of the last assembly
     bool step_pen = false;              // this step's inner CR runs on k_penalty.cu's operator
     int pmax = 0;                       // longest P-list of the current lists
     int pen_rows = 0, pen_w = 0;        // its rows a block and threads a row

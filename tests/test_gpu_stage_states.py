@@ -67,3 +67,29 @@ def test_c_of_the_mixed_form(engine_lib, oracle_built, dim):
         g.stage(s)
     want = csr_blocks_oracle(o.array("CsrPtrC"), o.array("CsrCofC"), g.fluid_count, g.export("NeighborCountP"), dim, per_block=False)
     assert rel(g.export("CsrCofC"), want) <= 1e-12
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_diagonal_is_of_its_step_or_refused(engine_lib, dim):
+    """InvDiagA of the point-Jacobi form is formed when it is read, from the
+    step's lists and C: the same values from the assembly to the end of the
+    step, and refused where positions or lists are newer (a later step's first
+    stages, a new state)."""
+    params, parts = _parts(dim)
+    g = _mixed(params, parts, dim)
+    for s in BEFORE_SOLVE[:5]:
+        g.stage(s)
+    want = g.export("InvDiagA")
+    for s in ("mg_build", "solve", "step_end"):
+        g.stage(s)
+        assert np.array_equal(g.export("InvDiagA"), want), s
+    for s in BEFORE_SOLVE[:4]:
+        g.stage(s)
+        with pytest.raises(engine.MphError) as e:
+            g.export("InvDiagA")
+        assert e.value.status == 9, s
+    g.stage("assemble")
+    assert len(g.export("InvDiagA")) == len(want)
+    g.set_state(parts)
+    with pytest.raises(engine.MphError):
+        g.export("InvDiagA")
