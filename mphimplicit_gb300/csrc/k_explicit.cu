@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(128) k_density(DevParams P, const int* __restr
 #pragma unroll
     for (int d = 0; d < D; ++d) sg[d] *= cg;
     store_vec<D>(gcen, i, sg);
-    vsp[i] = __fma_rn(P.kfp, sp, -P.N0p);
+    if (vsp) vsp[i] = __fma_rn(P.kfp, sp, -P.N0p);
 }
 
 __global__ void k_pressure_a(DevParams P, const int* __restrict__ type, const double* __restrict__ densA, double* __restrict__ presA)
@@ -373,15 +373,19 @@ static void launch_density_p(mph_case* c)
     else L == 4 ? go(k_density_p<3, 4>) : go(k_density_p<3, 1>);
 }
 
-// The full density pass (DensityA, GravityCenter, DensityP) and PressureA.
+// The full density pass (DensityA, GravityCenter, and DensityP where CofA is
+// not all zero) and PressureA.  Without surface tension VolStrainP is
+// k_density_p's, always: its sums run in another order than this pass's, and a
+// reader's request must not change what the step goes on with.
 void launch_density_full(mph_case* c)
 {
     const DevParams& P = c->dp;
     const unsigned g = grid_for(P.N, 128);
+    double* vsp = P.surface ? c->d.vsp : nullptr;
     if (c->dim == 2)
-        { k_density<2><<<g, 128, 0, c->stream>>>(P, c->d.type, c->d.pos, c->d.nc, c->d.nptr, c->d.nind, c->d.densA, c->d.gcen, c->d.vsp); MPH_COUNT_LAUNCH(); }
+        { k_density<2><<<g, 128, 0, c->stream>>>(P, c->d.type, c->d.pos, c->d.nc, c->d.nptr, c->d.nind, c->d.densA, c->d.gcen, vsp); MPH_COUNT_LAUNCH(); }
     else
-        { k_density<3><<<g, 128, 0, c->stream>>>(P, c->d.type, c->d.pos, c->d.nc, c->d.nptr, c->d.nind, c->d.densA, c->d.gcen, c->d.vsp); MPH_COUNT_LAUNCH(); }
+        { k_density<3><<<g, 128, 0, c->stream>>>(P, c->d.type, c->d.pos, c->d.nc, c->d.nptr, c->d.nind, c->d.densA, c->d.gcen, vsp); MPH_COUNT_LAUNCH(); }
     { k_pressure_a<<<grid_for(P.N, 256), 256, 0, c->stream>>>(P, c->d.type, c->d.densA, c->d.presA); MPH_COUNT_LAUNCH(); }
     c->densa_valid = true;
 }
@@ -424,6 +428,7 @@ void launch_explicit(mph_case* c)
 void launch_explicit_density_only(mph_case* c)
 {
     launch_density_full(c);
+    if (!c->dp.surface) launch_density_p(c);
 }
 
 void launch_output_fields(mph_case* c)
@@ -433,7 +438,7 @@ void launch_output_fields(mph_case* c)
     // with every CofA zero the frame needs VolStrainP alone of the density
     // pass (DensityA and the rest follow when a reader asks for them)
     if (P.surface) ensure_density_a(c);
-    else if (!c->densa_valid) launch_density_p(c);
+    else launch_density_p(c);
     DeviceState& d = c->d;
     auto go = [&](auto dp, auto of) {
         dp<<<g, 128, 0, c->stream>>>(P, d.type, d.pos, d.vel, d.ncp, d.nptrP, d.nindP, d.vsp, d.divP, d.presP);

@@ -93,3 +93,27 @@ def test_diagonal_is_of_its_step_or_refused(engine_lib, dim):
     g.set_state(parts)
     with pytest.raises(engine.MphError):
         g.export("InvDiagA")
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_reading_the_density_changes_nothing(engine_lib, dim):
+    """Without surface tension DensityA, GravityCenter and PressureA are formed
+    when they are read; VolStrainP and the step's result keep their bits."""
+    params, parts = _parts(dim)
+    a, b = engine.Case(params, parts, dim), engine.Case(params, parts, dim)
+    first = a.export("VolStrainP")
+    a.export("DensityA")
+    a.stage("output_fields")
+    assert np.array_equal(a.export("VolStrainP"), first)
+    for s in BEFORE_SOLVE[:4]:
+        a.stage(s)
+        b.stage(s)
+    vsp = a.export("VolStrainP")
+    for n in ("DensityA", "GravityCenter", "PressureA"):
+        a.export(n)
+    assert np.array_equal(a.export("VolStrainP"), vsp)
+    for s in ("assemble", "mg_build", "solve", "step_end", "output_fields"):
+        a.stage(s)
+        b.stage(s)
+    for n in ("VectorB", "Velocity", "VolStrainP", "PressureP"):
+        assert np.array_equal(a.export(n), b.export(n)), n
