@@ -451,7 +451,7 @@ int launch_assemble(mph_case* c)
         const int pon = prof_begin(c, 2, &pe);
         MPH_TRY(launch_pen_assemble(c));
         if (pon) prof_end(c, 2, pe);
-        return MPH_OK;
+        if (c->step_pen) return MPH_OK;
     }
     // slice pointers
     // the fluid rows' slices padded to a multiple of 4 slots (zero padding

@@ -74,10 +74,10 @@ __global__ void k_cell_keys(DevParams P, const double* __restrict__ pos, const i
                             int* __restrict__ key, int* __restrict__ perm, int* __restrict__ bbox, int* __restrict__ wrap)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 3) {   // what k_fluid_bbox and k_fixed_positions accumulate into
+    if (i < 3) {   // what k_fluid_bbox and the assembly accumulate into
         bbox[i] = P.cc[i];
         bbox[3 + i] = 0;
-        if (i < 2) wrap[i] = 0;
+        wrap[i] = 0;
     }
     if (i >= P.nPow) return;
     if (i < P.N) {

@@ -39,6 +39,7 @@
 // give the same bits.
 #include <algorithm>
 #include <climits>
+#include <cstring>
 #include <mutex>
 #include <type_traits>
 
@@ -76,37 +77,36 @@ constexpr int kCrSmem = 100 * 1024;   // dynamic: two blocks an SM with their 7 
 // blocks of 599 on average: 9.12 ms staged, 9.34 gathered) gains little.
 static int pen_ucap(int rows) { return 4 * rows + 128; }
 
-// Fixed-point positions of the penalty operator (ipos, units of RadiusP /
-// 2^22 over the whole domain) and of the viscous pairs (vpos, RadiusP / 2^26
-// modulo 2^32: a pair's separation is exact while it is shorter than 32
-// RadiusP), both with the particle's type; and whether a pair can be a
-// periodic image: bits 0-2 of *wrap, a particle within MaxRadius of the
-// domain's lower face of an axis, bits 3-5 of the upper one.
+// Fixed-point positions with the particle's type, of the penalty operator and
+// of the viscous pairs.  An axis's unit is its domain width / (m 2^32), m the
+// integer that brings it next to MaxRadius / 2^30, and the 32 bits are kept: a
+// difference modulo 2^32 is the minimum image by itself, in domains of any
+// width, and the lists' separations (at most MaxRadius, or half the width) fit
+// it exactly.  A difference in units of RadiusP is its float times fix_c, with
+// FP32's relative rounding down to distances of 2^24 units: the phases' true
+// residual meets the directions' error enlarged by the depth of the fluid in
+// spacings (a pair's share of the pressure against the net force).  Units of
+// RadiusP / 2^22 over the whole domain took 480 iterations instead of 170 for
+// a pair of particles 0.01 spacings apart in 504, and did not converge at
+// 0.001.
 template <int D>
 __global__ void __launch_bounds__(256) k_fixed_positions(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
-                                                         int4* __restrict__ ipos, int4* __restrict__ vpos, int* __restrict__ wrap)
+                                                         int4* __restrict__ ipos)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned near = 0u;
-    if (i < P.N) {
-        double x[3];
-        load_vec<D>(pos, i, x);
-        int u[3] = {0, 0, 0}, v[3] = {0, 0, 0};
+    if (i >= P.N) return;
+    double x[3];
+    load_vec<D>(pos, i, x);
+    int u[3] = {0, 0, 0};
 #pragma unroll
-        for (int d = 0; d < D; ++d) {
-            const double r = x[d] - P.dmin[d];
-            u[d] = __double2int_rn(r * P.fix_scale);
-            v[d] = (int)(unsigned)(unsigned long long)__double2ll_rn(r * P.vfix_scale);
-            near |= (r < P.maxR ? 1u << d : 0u) | (P.dw[d] - r < P.maxR ? 8u << d : 0u);
-        }
-        const int t = type[i];
-        ipos[i] = make_int4(u[0], u[1], u[2], t);
-        vpos[i] = make_int4(v[0], v[1], v[2], t);
-    }
-    near = __reduce_or_sync(0xffffffffu, near);
-    if (near && (threadIdx.x & 31) == 0) atomicOr((unsigned*)wrap, near);
+    for (int d = 0; d < D; ++d) u[d] = (int)(unsigned)(unsigned long long)__double2ll_rn((x[d] - P.dmin[d]) * P.fix_scale[d]);
+    ipos[i] = make_int4(u[0], u[1], u[2], type[i]);
 }
-__device__ __forceinline__ bool may_wrap(int w) { return (w & (w >> 3) & 7) != 0; }
+// x_j - x_i of an axis, in units of RadiusP
+__device__ __forceinline__ float fixed_sep(const DevParams& P, int d, int uj, int ui)
+{
+    return __fmul_rn(__int2float_rn((int)((unsigned)uj - (unsigned)ui)), P.fix_c[d]);
+}
 
 // The P-lists of a block of rows as 2-byte ranks among the block's distinct
 // columns: uniq[block][0 .. U) the columns in ascending order, idx the rank of
@@ -120,7 +120,8 @@ __device__ __forceinline__ bool may_wrap(int w) { return (w & (w >> 3) & 7) != 0
 __global__ void __launch_bounds__(kCrThreads) k_plist_ranks(int N, int Nf, int pw4, int ucap, const int* __restrict__ ncp,
                                                              const long long* __restrict__ nptrP, const int* __restrict__ nindP,
                                                              uint2* __restrict__ idx, int* __restrict__ groups,
-                                                             int* __restrict__ uniq, int* __restrict__ ucount)
+                                                             int* __restrict__ uniq, int* __restrict__ ucount,
+                                                             const int* __restrict__ near)
 {
     extern __shared__ unsigned pl_smem[];
     unsigned* bm = pl_smem;
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(kCrThreads) k_plist_ranks(int N, int Nf, int p
     __shared__ unsigned wsum[32];
     const int tid = threadIdx.x, lane = tid & 31, wl = tid >> 5, nwl = blockDim.x >> 5;
     const int i = blockIdx.x * blockDim.x + tid;
+    if (blockIdx.x == 0 && tid == 0) ucount[gridDim.x + 4] = *near;   // rides in the host's read
     const int n = i < N ? ncp[i] : 0;
     const int* col = nindP + (i < N ? nptrP[i] : 0);
     int lf = INT_MAX, hf = -1, lw = INT_MAX, hw = -1;
@@ -236,35 +238,25 @@ __global__ void __launch_bounds__(kCrThreads) k_plist_ranks(int N, int Nf, int p
     }
 }
 
-// q = x_j - x_i in the positions' units and cf = 1 / |q| - 1 / RadiusP (0
-// beyond RadiusP), so that C_ij = kfp (2 / RadiusP) cf q.  um = u_i - kMagic.
-// |q| = 0 (the row itself, coincident particles) gives a finite cf, and zero
-// with its q.  WRAP: some pair of the step is a periodic image.
-constexpr int kMagic = 0x4b400000;   // 1.5 2^23: adding d, |d| <= 2^22, gives the float 1.5 2^23 + d
-template <int D, bool WRAP>
-__device__ __forceinline__ float pen_coef(const DevParams& P, const int* um, const int* uj, float* q)
+// q = x_j - x_i in units of RadiusP and cf = 1 / |q| - 1 (0 beyond RadiusP),
+// so that C_ij = kfp (2 / RadiusP) cf q.  |q| = 0 (the row itself, coincident
+// particles) gives a finite cf, and zero with its q.
+template <int D>
+__device__ __forceinline__ float pen_coef(const DevParams& P, const int* ui, const int* uj, float* q)
 {
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-        int v = uj[d] - um[d];
-        if (WRAP) {
-            const int w = v - kMagic;
-            v += w > P.fix_h[d] ? -P.fix_w[d] : (w < -P.fix_h[d] ? P.fix_w[d] : 0);
-        }
-        q[d] = __fadd_rn(__int_as_float(v), -12582912.f);
-    }
+    for (int d = 0; d < D; ++d) q[d] = fixed_sep(P, d, uj[d], ui[d]);
     float r2 = __fmul_rn(q[0], q[0]);
     r2 = __fmaf_rn(q[1], q[1], r2);
     if (D == 3) r2 = __fmaf_rn(q[2], q[2], r2);
     float inv;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(fmaxf(r2, 1.f)));
-    return fmaxf(__fadd_rn(inv, -P.fix_inv), 0.f);
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(fmaxf(r2, 1e-18f)));
+    return fmaxf(__fadd_rn(inv, -1.f), 0.f);
 }
 
 struct PenArgs {
     int N, Nf, pw4, ucap, umax, cap;
     const int4* ipos;
-    const int* wrap;
     const uint2* idx;
     const int *groups, *uniq, *ucount;      // ucount null: every block gathers by column
     const int *ncp, *nindP;
@@ -425,7 +417,6 @@ __device__ __forceinline__ void pen_t_body(const DevParams& P, const PenArgs& A,
     const int tid = threadIdx.y * rows + threadIdx.x, nth = rows * W;
     const int i = lb * rows + threadIdx.x;
     const int done = A.flags[kFlagDone];
-    const bool wrap = may_wrap(*A.wrap);
     PenPre R;
     pen_prefetch(A, lb, i, A.N, tid, nth, threadIdx.y, W, R);
     int4 pi = make_int4(0, 0, 0, 0);
@@ -456,11 +447,11 @@ __device__ __forceinline__ void pen_t_body(const DevParams& P, const PenArgs& A,
     });
     __syncthreads();
     float acc = 0.f;
-    const int um[3] = {pi.x - kMagic, pi.y - kMagic, pi.z - kMagic};
-    auto sum = [&](auto WR) {
+    const int ui[3] = {pi.x, pi.y, pi.z};
+    if (R.n > 0) {
         auto one = [&](const int* uj, const float* sj) {
             float q[3];
-            const float cf = pen_coef<D, decltype(WR)::value>(P, um, uj, q);
+            const float cf = pen_coef<D>(P, ui, uj, q);
             float dot = __fmul_rn(q[0], __fadd_rn(si[0], -sj[0]));
             dot = __fmaf_rn(q[1], __fadd_rn(si[1], -sj[1]), dot);
             if (D == 3) dot = __fmaf_rn(q[2], __fadd_rn(si[2], -sj[2]), dot);
@@ -490,10 +481,6 @@ __device__ __forceinline__ void pen_t_body(const DevParams& P, const PenArgs& A,
                 }
                 one(uj, sj);
             });
-    };
-    if (R.n > 0) {
-        if (wrap) sum(std::true_type());
-        else sum(std::false_type());
     }
     if (W > 1) {   // the row's partial sums in the order of w
         __shared__ float part[kMaxPenRows];
@@ -519,7 +506,6 @@ __device__ __forceinline__ void pen_y_body(const DevParams& P, const PenArgs& A,
     const int rows = blockDim.x, W = blockDim.y;
     const int tid = threadIdx.y * rows + threadIdx.x, nth = rows * W;
     const int done = A.flags[kFlagDone], it = A.flags[kFlagIter];
-    const bool wrap = may_wrap(*A.wrap);
     if (done) return;   // block-uniform: set before this launch
     int4* sa = pen_smem;
     float v[3] = {0.f, 0.f, 0.f};
@@ -551,11 +537,11 @@ __device__ __forceinline__ void pen_y_body(const DevParams& P, const PenArgs& A,
         });
         __syncthreads();
         float y[3] = {0.f, 0.f, 0.f};
-        const int um[3] = {pi.x - kMagic, pi.y - kMagic, pi.z - kMagic};
-        auto sum = [&](auto WR) {
+        const int ui[3] = {pi.x, pi.y, pi.z};
+        if (R.n > 0) {
             auto one = [&](const int* uj, float tj) {
                 float q[3];
-                const float c = __fmul_rn(pen_coef<D, decltype(WR)::value>(P, um, uj, q), __fadd_rn(tj, ti));
+                const float c = __fmul_rn(pen_coef<D>(P, ui, uj, q), __fadd_rn(tj, ti));
 #pragma unroll
                 for (int d = 0; d < D; ++d) y[d] = __fmaf_rn(c, q[d], y[d]);
             };
@@ -571,10 +557,6 @@ __device__ __forceinline__ void pen_y_body(const DevParams& P, const PenArgs& A,
                     const int uj[3] = {p.x, p.y, p.z};
                     one(uj, A.t[j]);
                 });
-        };
-        if (R.n > 0) {
-            if (wrap) sum(std::true_type());
-            else sum(std::false_type());
         }
         if (W > 1) {
             __shared__ float part[kMaxPenRows * D];
@@ -855,7 +837,6 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
     float* st = reinterpret_cast<float*>(sb + (D == 3 ? A.umax : 0));    // lambda t
     int* ul = reinterpret_cast<int*>(st + A.umax);                       // the staged columns
     uint2* words = reinterpret_cast<uint2*>(ul + A.umax);                // the rows' ranks, word by word
-    const bool wrap = may_wrap(*A.wrap);
     // what the phase keeps
     const int U = A.ucount ? A.ucount[lb] : -1;
     const int n = i < A.N ? A.ncp[i] : 0;
@@ -874,7 +855,7 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
         for (int g = w; g < ng; g += W) words[(size_t)g * rows + threadIdx.x] = ip[(long long)g * 32];
     }
     const int4 pi = i < A.N ? A.ipos[i] : make_int4(0, 0, 0, 0);
-    const int um[3] = {pi.x - kMagic, pi.y - kMagic, pi.z - kMagic};
+    const int ui[3] = {pi.x, pi.y, pi.z};
     const bool fluid = i < A.Nf, mine = w == 0 && fluid;
     int it = A.flags[kFlagIter];
     const int it_end = it + kCrMaxIter;
@@ -974,38 +955,34 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
         // lambda t
         float acc = 0.f;
         if (n > 0) {
-            auto sum = [&](auto WR) {
-                auto one = [&](const int* uj, const float* sj) {
-                    float dq[3];
-                    const float cf = pen_coef<D, decltype(WR)::value>(P, um, uj, dq);
-                    float dot = __fmul_rn(dq[0], __fadd_rn(si[0], -sj[0]));
-                    dot = __fmaf_rn(dq[1], __fadd_rn(si[1], -sj[1]), dot);
-                    if (D == 3) dot = __fmaf_rn(dq[2], __fadd_rn(si[2], -sj[2]), dot);
-                    acc = __fmaf_rn(cf, dot, acc);
-                };
-                slots([&](int k) {
-                    if (U >= 0) {
-                        const int4 pj = sa[k];
-                        const int uj[3] = {pj.x, pj.y, pj.z};
-                        if (D == 3) {
-                            const float2 v = sb[k];
-                            const float sj[3] = {__int_as_float(pj.w), v.x, v.y};
-                            one(uj, sj);
-                        } else {
-                            const float sj[3] = {__int_as_float(pj.z), __int_as_float(pj.w), 0.f};
-                            one(uj, sj);
-                        }
+            auto one = [&](const int* uj, const float* sj) {
+                float dq[3];
+                const float cf = pen_coef<D>(P, ui, uj, dq);
+                float dot = __fmul_rn(dq[0], __fadd_rn(si[0], -sj[0]));
+                dot = __fmaf_rn(dq[1], __fadd_rn(si[1], -sj[1]), dot);
+                if (D == 3) dot = __fmaf_rn(dq[2], __fadd_rn(si[2], -sj[2]), dot);
+                acc = __fmaf_rn(cf, dot, acc);
+            };
+            slots([&](int k) {
+                if (U >= 0) {
+                    const int4 pj = sa[k];
+                    const int uj[3] = {pj.x, pj.y, pj.z};
+                    if (D == 3) {
+                        const float2 v = sb[k];
+                        const float sj[3] = {__int_as_float(pj.w), v.x, v.y};
+                        one(uj, sj);
                     } else {
-                        const int4 pj = A.ipos[k];
-                        const int uj[3] = {pj.x, pj.y, pj.z};
-                        float sj[3];
-                        cr_combine<D>(cr_load<D>(C.rec, k, A.Nf), alpha, beta, sj);
+                        const float sj[3] = {__int_as_float(pj.z), __int_as_float(pj.w), 0.f};
                         one(uj, sj);
                     }
-                });
-            };
-            if (wrap) sum(std::true_type());
-            else sum(std::false_type());
+                } else {
+                    const int4 pj = A.ipos[k];
+                    const int uj[3] = {pj.x, pj.y, pj.z};
+                    float sj[3];
+                    cr_combine<D>(cr_load<D>(C.rec, k, A.Nf), alpha, beta, sj);
+                    one(uj, sj);
+                }
+            });
         }
         float ti = acc;
         if (W > 1) {   // the row's partial sums in the order of w
@@ -1035,21 +1012,17 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
         // y = M s
         float y[3] = {0.f, 0.f, 0.f};
         if (fluid && n > 0) {
-            auto sum = [&](auto WR) {
-                auto one = [&](const int* uj, float tj) {
-                    float dq[3];
-                    const float cf = __fmul_rn(pen_coef<D, decltype(WR)::value>(P, um, uj, dq), __fadd_rn(tj, ti));
+            auto one = [&](const int* uj, float tj) {
+                float dq[3];
+                const float cf = __fmul_rn(pen_coef<D>(P, ui, uj, dq), __fadd_rn(tj, ti));
 #pragma unroll
-                    for (int d = 0; d < D; ++d) y[d] = __fmaf_rn(cf, dq[d], y[d]);
-                };
-                slots([&](int k) {
-                    const int4 pj = U >= 0 ? sa[k] : A.ipos[k];
-                    const int uj[3] = {pj.x, pj.y, pj.z};
-                    one(uj, U >= 0 ? st[k] : __ldcg(A.t + k));
-                });
+                for (int d = 0; d < D; ++d) y[d] = __fmaf_rn(cf, dq[d], y[d]);
             };
-            if (wrap) sum(std::true_type());
-            else sum(std::false_type());
+            slots([&](int k) {
+                const int4 pj = U >= 0 ? sa[k] : A.ipos[k];
+                const int uj[3] = {pj.x, pj.y, pj.z};
+                one(uj, U >= 0 ? st[k] : __ldcg(A.t + k));
+            });
         }
         if (W > 1) {
 #pragma unroll
@@ -1151,12 +1124,16 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
 // pipe: 1.2 ms on 1.3 million particles.  C, the transposed lists (0.69 ms),
 // b with the pair terms (2.06) and their slicing (1.04) took 5.0 ms in passes
 // of their own.
+// *near: nonzero (FP32 bits) for a pair closer than MaxRadius / 256, where the
+// positions' units no longer hold its direction to FP32: the step then takes
+// the pair-term operator (mph_case::pen_near).
+constexpr float kNearMin = 2.5e-4f, kNearMax = 0.05f;
 template <int D, int L>
 __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
                                                     const double* __restrict__ vel, const int* __restrict__ ncp,
                                                     const long long* __restrict__ nptrP, const int* __restrict__ nindP,
                                                     const double* __restrict__ pvec, double* __restrict__ cval,
-                                                    double* __restrict__ bvec, float* __restrict__ invD)
+                                                    double* __restrict__ bvec, float* __restrict__ invD, int* __restrict__ near)
 {
     const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) / L, part = threadIdx.x % L;
     const int i = min(i0, P.N - 1);
@@ -1167,7 +1144,8 @@ __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __re
     const long long b = nptrP[i];
     const int n = i0 < P.N ? ncp[i] : 0;
     double self[3] = {0, 0, 0}, cp[3] = {0, 0, 0};
-    float dp[3] = {0.f, 0.f, 0.f};
+    float dp[3] = {0.f, 0.f, 0.f}, nearest = 0.f;
+    const int tf = fluid ? type[i] : 0;
     int selfk = 0;
     for (int a = part; a < n; a += L) {
         const int j = nindP[b + a];
@@ -1181,9 +1159,11 @@ __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __re
             const double r2 = norm2_fma<D>(q);
             if (r2_pos_below(r2, rP2)) {
                 // w' / r = kf (-2 / RadiusP) (1 - r / RadiusP) / r
-                const double f = K * (rsqrt(r2) - P.inv_rp);
+                const double inv = rsqrt(r2), f = K * (inv - P.inv_rp);
                 const double pj = fluid ? pvec[j] : 0.0;
-                const float lam = P.lambda32[type[j]];
+                const int tj = type[j];
+                const float lam = P.lambda32[tj], turn = (float)inv * P.near_r;   // MaxRadius / |q|
+                nearest = fmaxf(nearest, turn > 256.f ? __int_as_float(0x7f800000) : 0.f);
 #pragma unroll
                 for (int r = 0; r < D; ++r) {
                     cv[r] = q[r] * f;
@@ -1204,8 +1184,10 @@ __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __re
         dp[r] = row_sum<L>(dp[r]);
     }
     selfk = row_sum<L>(selfk);   // set by one lane
+    const int warp_near = __reduce_max_sync(0xffffffffu, fluid ? __float_as_int(nearest) : 0);
+    if ((threadIdx.x & 31) == 0 && warp_near > __float_as_int(kNearMin) && warp_near > *(volatile int*)near) atomicMax(near, warp_near);
     if (!fluid || i0 >= P.N || part != 0) return;
-    const int ti = type[i];
+    const int ti = tf;
     const double pi = pvec[i];
     double v[3];
     load_vec<D>(vel, i, v);
@@ -1381,11 +1363,9 @@ __device__ __forceinline__ void pen_ct64(const DevParams& P, int tid, const int*
 // ms for x_0, 0.82 for z.
 // The launch's first nbT blocks form lambda t of C^T x meanwhile (pen_ct64).
 template <int D, int L, bool FIRST, int LT>
-__global__ void __launch_bounds__(256) k_pen_visc(DevParams P, int nbT, const int4* __restrict__ vpos, const int* __restrict__ nfc,
+__global__ void __launch_bounds__(256) k_pen_visc(DevParams P, int nbT, const int4* __restrict__ ipos, const int* __restrict__ nfc,
                                                   const long long* __restrict__ nptr, const int* __restrict__ nind,
-                                                  const float4* __restrict__ rec, int* __restrict__ wrap,
-                                                  const int* __restrict__ type, const double* __restrict__ pos,
-                                                  const float* __restrict__ pos32, const float* __restrict__ poslo32, double scale,
+                                                  const float4* __restrict__ rec, const int* __restrict__ type, double scale,
                                                   const double* __restrict__ scale_src, double* __restrict__ vacc,
                                                   const int* __restrict__ ncp, const long long* __restrict__ nptrP,
                                                   const int* __restrict__ nindP, const double* __restrict__ cval,
@@ -1403,54 +1383,30 @@ __global__ void __launch_bounds__(256) k_pen_visc(DevParams P, int nbT, const in
         const float4 hi = rec[i];
         const float4 li = FIRST ? rec[P.Nf + i] : make_float4(0.f, 0.f, 0.f, 0.f);
         const float4* lo = rec + P.Nf;
-        if (!may_wrap(*wrap)) {
-            const int4 pi = vpos[i];
-            const float vm0 = pi.w ? P.pen_vm[1][0] : P.pen_vm[0][0], vm1 = pi.w ? P.pen_vm[1][1] : P.pen_vm[0][1];
+        const int4 pi = ipos[i];
+        const float vm0 = pi.w ? P.pen_vm[1][0] : P.pen_vm[0][0], vm1 = pi.w ? P.pen_vm[1][1] : P.pen_vm[0][1];
 #pragma unroll 4
-            for (int k = lane; k < n; k += L) {
-                const int j = col[k];
-                const int4 pj = vpos[j];
-                const float4 h = rec[j];
-                const float q[3] = {(float)(pj.x - pi.x), (float)(pj.y - pi.y), D == 3 ? (float)(pj.z - pi.z) : 0.f};
-                float dx[3] = {hi.x - h.x, hi.y - h.y, D == 3 ? hi.z - h.z : 0.f};
-                if (FIRST) {
-                    const float4 l = lo[j];
-                    dx[0] += li.x - l.x;
-                    dx[1] += li.y - l.y;
-                    if (D == 3) dx[2] += li.z - l.z;
-                }
-                float r2 = q[0] * q[0] + q[1] * q[1];
-                if (D == 3) r2 += q[2] * q[2];
-                const float inv = rsqrtf(fmaxf(r2, 1.f));
-                // visc mu_ij w' / |q|, w' = (1 - |q| / RadiusV) up to the constants in vm; q / |q| twice
-                const float c = (pj.w ? vm1 : vm0) * fmaxf(inv - P.pen_vk, 0.f) * (inv * inv);
-                float dot = q[0] * dx[0] + q[1] * dx[1];
-                if (D == 3) dot += q[2] * dx[2];
-                const float t = c * dot;
-#pragma unroll
-                for (int d = 0; d < D; ++d) y[d] += t * q[d];
+        for (int k = lane; k < n; k += L) {
+            const int j = col[k];
+            const int4 pj = ipos[j];
+            const float4 h = rec[j];
+            const float q[3] = {fixed_sep(P, 0, pj.x, pi.x), fixed_sep(P, 1, pj.y, pi.y), D == 3 ? fixed_sep(P, 2, pj.z, pi.z) : 0.f};
+            float dx[3] = {hi.x - h.x, hi.y - h.y, D == 3 ? hi.z - h.z : 0.f};
+            if (FIRST) {
+                const float4 l = lo[j];
+                dx[0] += li.x - l.x;
+                dx[1] += li.y - l.y;
+                if (D == 3) dx[2] += li.z - l.z;
             }
-        } else {   // periodic images: the general pair term
-            const int ti = type[i];
-            float ph[3], pl[3];
-            load_f32<D>(pos32, i, ph);
-            load_f32<D>(poslo32, i, pl);
-            for (int k = lane; k < n; k += L) {
-                const int j = col[k];
-                float e[3] = {0.f, 0.f, 0.f}, f = 0.f;
-                pair_ef<D>(P, i, j, ti, ph, pl, type, pos, pos32, poslo32, wrap + 1, e, f);
-                const float4 h = rec[j];
-                float dx[3] = {hi.x - h.x, hi.y - h.y, hi.z - h.z};
-                if (FIRST) {
-                    const float4 l = lo[j];
-                    dx[0] += li.x - l.x;
-                    dx[1] += li.y - l.y;
-                    dx[2] += li.z - l.z;
-                }
-                const float t = f * (e[0] * dx[0] + e[1] * dx[1] + e[2] * dx[2]);
+            float r2 = q[0] * q[0] + q[1] * q[1];
+            if (D == 3) r2 += q[2] * q[2];
+            const float inv = rsqrtf(fmaxf(r2, 1e-18f));
+            // visc mu_ij w' / |q|, w' = (1 - |q| / RadiusV) up to the constants in vm; q / |q| twice (the row itself: 0)
+            float dot = q[0] * dx[0] + q[1] * dx[1];
+            if (D == 3) dot += q[2] * dx[2];
+            const float t = (pj.w ? vm1 : vm0) * fmaxf(inv - P.pen_vk, 0.f) * (dot * inv) * inv;
 #pragma unroll
-                for (int d = 0; d < D; ++d) y[d] += t * e[d];
-            }
+            for (int d = 0; d < D; ++d) y[d] += t * q[d];
         }
     }
 #pragma unroll
@@ -1596,16 +1552,14 @@ static void pen_shape(mph_case* c)
     else { c->pen_rows = 64; c->pen_w = 4; }
 }
 
-// The positions' unit is RadiusP / 2^20 or finer (domains up to about 1900
-// RadiusP wide); in wider ones the stored operator's records are closer to C.
-// (The viscous pairs' separations hold MaxRadius below 16 RadiusP.)
+// (The positions' unit is MaxRadius / 2^30, which stays fine in RadiusP.)
 bool pen_applies(const mph_case* c)
 {
     const DevParams& P = c->dp;
-    if (!(c->step_pairs && mixed_jacobi(c) && P.fix_inv <= 1.0f / 1048576.0f && P.maxR <= 16.0 * P.rP)) return false;
+    if (!(c->step_pairs && mixed_jacobi(c) && P.maxR <= 16.0 * P.rP)) return false;
     for (int t = 0; t < 2; ++t)
         for (int u = 0; u < 2; ++u)
-            if (!(P.pen_vm[t][u] <= 1.0e30f)) return false;   // unit systems far outside FP32's range
+            if (!(P.pen_vm[t][u] <= 1.0e25f)) return false;   // unit systems far outside FP32's range
     return true;
 }
 
@@ -1636,7 +1590,7 @@ static int launch_pen_lists(mph_case* c)
     const int nsl = (P.N + 31) / 32, nb = (int)grid_for(P.N, c->pen_rows), ucap = pen_ucap(c->pen_rows);
     if (!d.pgroups) MPH_CUDA(cudaMalloc((void**)&d.pgroups, (size_t)nsl * sizeof(int)));
     MPH_TRY(grow_t(&d.puniq, &d.cap_puniq, (long long)nb * ucap));
-    MPH_TRY(grow_t(&d.pucount, &d.cap_pucount, nb + 4));
+    MPH_TRY(grow_t(&d.pucount, &d.cap_pucount, nb + 5));
     if (c->pen_resident && !d.cr_rec) {
         MPH_CUDA(cudaMalloc((void**)&d.cr_rec, (size_t)P.Nf * 3 * sizeof(float4)));
         MPH_CUDA(cudaMalloc((void**)&d.cr_vals, (size_t)(8 * kCrBlocks + 32) * sizeof(float)));
@@ -1647,7 +1601,18 @@ static int launch_pen_lists(mph_case* c)
     c->loc_blocks[1] = (int)grid_for(P.Nf, c->pen_rows);
     c->loc_cols = 0;
     c->loc_ct_blocks = 0;
-    if (!c->inner_local) return MPH_OK;
+    auto near_of = [](int bits) {
+        float f;
+        std::memcpy(&f, &bits, sizeof(f));
+        return f;
+    };
+    int h[5] = {};
+    if (!c->inner_local) {
+        MPH_CUDA(cudaMemcpyAsync(h, d.wrap32 + 2, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        MPH_CUDA(cudaStreamSynchronize(c->stream));
+        c->pen_near = near_of(h[0]);
+        return MPH_OK;
+    }
     const size_t smem = 2 * kPlWords * sizeof(unsigned);
     if (!c->pen_attr) {   // once a case; fixed maxima: host threads of a batch would race on per-launch values
         const int t = (pen_ucap(kMaxPenRows) + 256) * 24, y = (pen_ucap(kMaxPenRows) + 256) * 16;
@@ -1657,10 +1622,9 @@ static int launch_pen_lists(mph_case* c)
         MPH_CUDA(c->dim == 2 ? cudaFuncSetAttribute(k_pen_y<2>, a, y) : cudaFuncSetAttribute(k_pen_y<3>, a, y));
         c->pen_attr = true;
     }
-    MPH_CUDA(cudaMemsetAsync(d.pucount + nb, 0, 4 * sizeof(int), c->stream));
+    MPH_CUDA(cudaMemsetAsync(d.pucount + nb, 0, 5 * sizeof(int), c->stream));
     { k_plist_ranks<<<nb, c->pen_rows, smem, c->stream>>>(P.N, P.Nf, c->pen_pw4, ucap, d.ncp, d.nptrP, d.nindP, d.pidx, d.pgroups,
-                                                         d.puniq, d.pucount); MPH_COUNT_LAUNCH(); }
-    int h[4] = {};
+                                                         d.puniq, d.pucount, d.wrap32 + 2); MPH_COUNT_LAUNCH(); }
     MPH_CUDA(cudaMemcpyAsync(h, d.pucount + nb, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
     MPH_CUDA(cudaStreamSynchronize(c->stream));
     c->pen_umax = (h[0] + 127) / 128 * 128;   // rounded up: small changes keep the captured graphs
@@ -1668,12 +1632,14 @@ static int launch_pen_lists(mph_case* c)
     c->loc_blocks[0] = h[2];
     c->loc_blocks[1] -= h[2];
     c->loc_cols = (long long)(unsigned)h[3];
+    c->pen_near = near_of(h[4]);
     c->pen_staged = true;
     return MPH_OK;
 }
 
 // The assembly stage of the point-Jacobi mixed form: no blocks, no pair terms,
-// no slices and no transposed lists.
+// no slices and no transposed lists.  Leaves step_pen false where a pair is too
+// close for the operator (the caller then assembles the pair terms).
 int launch_pen_assemble(mph_case* c)
 {
     DeviceState& d = c->d;
@@ -1683,7 +1649,6 @@ int launch_pen_assemble(mph_case* c)
     c->nslots = 0;
     c->level0_done = c->ct_ready = false;
     if (!d.ipos) MPH_CUDA(cudaMalloc((void**)&d.ipos, (size_t)P.N * sizeof(int4)));
-    if (!d.vpos) MPH_CUDA(cudaMalloc((void**)&d.vpos, (size_t)P.N * sizeof(int4)));
     if (!d.z4) {   // components that a record does not use stay zero
         MPH_CUDA(cudaMalloc((void**)&d.z4, (size_t)P.Nf * 2 * sizeof(float4)));
         MPH_CUDA(cudaMemsetAsync(d.z4, 0, (size_t)P.Nf * 2 * sizeof(float4), st));
@@ -1699,14 +1664,14 @@ int launch_pen_assemble(mph_case* c)
     float* invD = d.v32 + 7 * vec32_stride(n);
     const int L = plist_lanes(P.N);
     auto system = [&](auto kern) {
-        kern<<<grid_for((long long)P.N * L, 128), 128, 0, st>>>(P, d.type, d.pos, d.vel, d.ncp, d.nptrP, d.nindP, d.pvec, d.cval, d.bvec, invD);
+        kern<<<grid_for((long long)P.N * L, 128), 128, 0, st>>>(P, d.type, d.pos, d.vel, d.ncp, d.nptrP, d.nindP, d.pvec, d.cval, d.bvec, invD, d.wrap32 + 2);
         MPH_COUNT_LAUNCH();
     };
     if (c->dim == 2) {
-        { k_fixed_positions<2><<<g, 256, 0, st>>>(P, d.type, d.pos, d.ipos, d.vpos, d.wrap32); MPH_COUNT_LAUNCH(); }
+        { k_fixed_positions<2><<<g, 256, 0, st>>>(P, d.type, d.pos, d.ipos); MPH_COUNT_LAUNCH(); }
         L == 4 ? system(k_pen_system<2, 4>) : system(k_pen_system<2, 1>);
     } else {
-        { k_fixed_positions<3><<<g, 256, 0, st>>>(P, d.type, d.pos, d.ipos, d.vpos, d.wrap32); MPH_COUNT_LAUNCH(); }
+        { k_fixed_positions<3><<<g, 256, 0, st>>>(P, d.type, d.pos, d.ipos); MPH_COUNT_LAUNCH(); }
         L == 4 ? system(k_pen_system<3, 4>) : system(k_pen_system<3, 1>);
     }
     auto walls = [&](auto kern, int lanes) {
@@ -1715,7 +1680,9 @@ int launch_pen_assemble(mph_case* c)
     };
     if (c->dim == 2) walls(k_pen_wall<2, 8>, 8);
     else walls(k_pen_wall<3, 16>, 16);
-    return launch_pen_lists(c);
+    MPH_TRY(launch_pen_lists(c));
+    c->step_pen = c->pen_near <= kNearMax;
+    return MPH_OK;
 }
 
 // D^-1 as a reader gets it (FP64 array), from the current step's lists and C
@@ -1739,7 +1706,7 @@ static void pen_residual_t(mph_case* c, double scale, const double* scale_src)
     cudaStream_t st = c->stream;
     const unsigned nbT = grid_for((long long)P.N * LT, 256);
     { k_pen_visc<D, L, FIRST, LT><<<nbT + grid_for((long long)P.Nf * L, 256), 256, 0, st>>>(
-          P, (int)nbT, d.vpos, d.nfc, d.nptr, d.nind, d.z4, d.wrap32, d.type, d.pos, d.pos32, d.poslo32, scale, scale_src, d.vacc,
+          P, (int)nbT, d.ipos, d.nfc, d.nptr, d.nind, d.z4, d.type, scale, scale_src, d.vacc,
           d.ncp, d.nptrP, d.nindP, d.cval, d.x, d.tct); MPH_COUNT_LAUNCH(); }
     { k_pen_resid<D, LT><<<grid_for((long long)P.Nf * LT, 128), 128, 0, st>>>(P, d.type, d.nc, d.nfc, d.ncp, d.nptrP, d.nindP, d.cval, d.tct, d.sdiag64, d.vacc,
                                                           d.x, d.bvec, d.r, d.partials, (unsigned*)(d.flags + kFlagCounter), d.scal + kSRR); MPH_COUNT_LAUNCH(); }
@@ -1814,7 +1781,6 @@ static PenArgs pen_args(const mph_case* c, int cap)
     A.umax = c->pen_umax;
     A.cap = cap;
     A.ipos = d.ipos;
-    A.wrap = d.wrap32;
     A.idx = d.pidx;
     A.groups = d.pgroups;
     A.uniq = d.puniq;

@@ -211,11 +211,10 @@ static int derive(mph_case* c, const mph_particles* parts)
         // the inner operator of the point-Jacobi form keeps 0.6 of a row's
         // viscous diagonal (fsum mu / dim) and leaves the rest, at most about
         // 0.7 of it, to the outer residual
-        P.vfix_scale = std::ldexp(1.0, 26) / P.rP;
-        P.pen_vk = (float)(1.0 / (P.rV * P.vfix_scale));
+        P.pen_vk = (float)(P.rP / P.rV);
         for (int t = 0; t < 2; ++t) {
             P.pen_vd[t] = (float)(fsum * std::fabs(P.mu[t]) / c->dim);
-            for (int u = 0; u < 2; ++u) P.pen_vm[t][u] = (float)(P.visc * P.muij[t][u] * (-P.kfv * P.m2h_rv) * P.vfix_scale);
+            for (int u = 0; u < 2; ++u) P.pen_vm[t][u] = (float)(P.visc * P.muij[t][u] * (-P.kfv * P.m2h_rv) / P.rP);
         }
         for (int t = 0; t < kTypeCount; ++t) P.pen_diag32[t] = (float)(P.inert64[t] + 0.6 * fsum * std::fabs(P.mu[t]) / c->dim);
         c->pen_tol = 0.7 * fsum * mu_max / c->dim / (rho_min / P.dt);
@@ -261,22 +260,14 @@ static int derive(mph_case* c, const mph_particles* parts)
         P.hw[d] = 0.5 * P.dw[d];
         P.wsafe[d] = 0.75 * P.dw[d];
     }
-    // fixed-point positions in units of RadiusP / 2^e, e = 22 (a separation
-    // within RadiusP is then an FP32 integer) or less where the domain is too
-    // wide for 31 bits (k_penalty.cu uses them down to e = 20)
-    {
-        double wide = 0.0;
-        for (int d = 0; d < c->dim; ++d) wide = std::max(wide, P.dw[d]);
-        int e = 22;
-        while (e > 1 && std::ldexp(wide / P.rP, e) > 2.0e9) --e;
-        P.fix_scale = std::ldexp(1.0, e) / P.rP;
-        P.fix_inv = (float)std::ldexp(1.0, -e);
-        for (int d = 0; d < c->dim; ++d) {
-            const double w = std::nearbyint(P.dw[d] * P.fix_scale);
-            P.fix_w[d] = w < 2.0e9 ? (int)w : 0;
-            P.fix_h[d] = P.fix_w[d] / 2;
-        }
+    // fixed-point positions modulo 2^32, a whole number of turns a domain width
+    // (k_penalty.cu)
+    for (int d = 0; d < c->dim; ++d) {
+        const double turns = std::max(1.0, std::floor(P.dw[d] / P.maxR * std::ldexp(1.0, -2)));
+        P.fix_scale[d] = std::ldexp(turns, 32) / P.dw[d];
+        P.fix_c[d] = (float)(1.0 / (P.fix_scale[d] * P.rP));
     }
+    P.near_r = (float)P.maxR;
     double cnt[3];
     cnt[0] = std::floor((dmax[0] - P.dmin[0]) / P.maxR);
     cnt[1] = std::floor((dmax[1] - P.dmin[1]) / P.maxR);
@@ -368,7 +359,7 @@ int case_alloc_particles(mph_case* c)
     MPH_TRY(dalloc(c, &d.poslo32, N * VSn));
     if (c->dim == 2) MPH_TRY(dalloc(c, &d.pt32, N));
     else d.pt32 = reinterpret_cast<float4*>(d.pos32);   // its w holds the type bits
-    MPH_TRY(dalloc(c, &d.wrap32, 2));
+    MPH_TRY(dalloc(c, &d.wrap32, 3));
     MPH_TRY(dalloc(c, &d.type, N));
     MPH_TRY(dalloc(c, &d.id, N));
     MPH_TRY(dalloc(c, &d.type_alt, N));
@@ -723,7 +714,7 @@ int case_destroy(mph_case* c)
                     (void*)d.tct32, (void*)d.pes32, (void*)d.sdiag32, (void*)d.sdiag64, (void*)d.cvl32, (void*)d.psptr, (void*)d.ctsptr,
                     (void*)d.pswidth, (void*)d.ctswidth, (void*)d.pscol, (void*)d.ctscol, (void*)d.psval, (void*)d.ctsval,
                     (void*)d.grec16, (void*)d.grec32, (void*)d.pscale, (void*)d.lcol16, (void*)d.uniq, (void*)d.ucount,
-                    (void*)d.ctuniq, (void*)d.ctucount, (void*)d.ipos, (void*)d.cr_rec, (void*)d.cr_vals, (void*)d.vpos, (void*)d.z4, (void*)d.vacc, (void*)d.pidx, (void*)d.pgroups, (void*)d.puniq, (void*)d.pucount, (void*)d.wkey, (void*)d.wval, (void*)d.ccell,
+                    (void*)d.ctuniq, (void*)d.ctucount, (void*)d.ipos, (void*)d.cr_rec, (void*)d.cr_vals, (void*)d.z4, (void*)d.vacc, (void*)d.pidx, (void*)d.pgroups, (void*)d.puniq, (void*)d.pucount, (void*)d.wkey, (void*)d.wval, (void*)d.ccell,
                     (void*)d.io3, (void*)d.vprev, (void*)d.vprev_alt, (void*)d.sort_cnt, (void*)d.sort_off, d.scan_tmp})
         if (p) cudaFree(p);
     for (auto& p : c->prof.pending) {

@@ -65,12 +65,11 @@ struct DevParams {
     float lambda32[kTypeCount];
     float vm32[kTypeCount][kTypeCount];        // FP32 visc * muij, -kfv * m2h_rv, 1/h, rV^2 (pair terms)
     float wdA32, inv_rv32, rV2_32;
-    double fix_scale;                          // fixed-point positions: units a length (2^e / RadiusP), 2^-e, and the
-    float fix_inv;                             // domain's width and half width in units
-    int fix_w[3], fix_h[3];
-    double vfix_scale;                         // the same for the viscous pairs: 2^26 / RadiusP, modulo 2^32
-    float pen_vm[2][2], pen_vk, pen_vd[2];     // visc mu_ij w' and 1/RadiusV of the fluid pairs in those units; the lattice's
+    double fix_scale[3];                       // fixed-point positions: an axis's units a length, and a unit in RadiusP
+    float fix_c[3];
+    float pen_vm[2][2], pen_vk, pen_vd[2];     // visc mu_ij w' and 1/RadiusV of the fluid pairs over 1/RadiusP; the lattice's
                                                // viscous diagonal of a fluid row
+    float near_r;                              // MaxRadius
     float pen_diag32[kTypeCount];              // inner operator of the point-Jacobi form: its diagonal, lambda kfp 2/RadiusP,
     float pen_lam32[kTypeCount], pen_w32;      // and kfp 2/RadiusP
     int exact_only;                            // 1: skip the FP32 pre-classification
@@ -175,7 +174,6 @@ struct DeviceState {
     // slice, the row blocks' distinct columns and their counts (statistics
     // after the blocks)
     int4* ipos = nullptr;
-    int4* vpos = nullptr;
     float4* z4 = nullptr;              // the solution or its last correction, a record a row (two where it is in two floats)
     double* vacc = nullptr;            // viscous fluid pairs of A x, added up over the refinement phases
     uint2* pidx = nullptr;
@@ -332,6 +330,7 @@ struct mph_case {
     bool pen_staged = false;            // the assembly built the row blocks' ranks and columns (option inner_local as it was then)
     bool pen_resident = false;          // a phase's CR iterations in one cooperative kernel (the case's rows fit the chip at once)
     int pen_pw4 = 0, pen_umax = 0;      // 8-byte words a row has room for; largest staged count (rounded up)
+    double pen_near = 0.0;              // infinite: a pair of this step's is too close for the operator
     double pen_tol = 0.0;               // what a refinement phase leaves at least (the viscous part outside the operator)
     int loc_smem = 0;                   // shared memory of k_visc_pen32's staged s (0: gathers by column)
     int loc_cap = 0;                    // staged neighbours a block of the pair-term operator has room for
