@@ -1124,9 +1124,14 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
 // pipe: 1.2 ms on 1.3 million particles.  C, the transposed lists (0.69 ms),
 // b with the pair terms (2.06) and their slicing (1.04) took 5.0 ms in passes
 // of their own.
-// *near: nonzero (FP32 bits) for a pair closer than MaxRadius / 256, where the
-// positions' units no longer hold its direction to FP32: the step then takes
-// the pair-term operator (mph_case::pen_near).
+// *near: the largest f / inertia of a P-list's viscous pair in FP32 bits where
+// it is above kNearMin, infinite for a pair closer than MaxRadius / 256.  A
+// lattice's pairs are some 1e-4; one pair close together has f ~ 1 / r, and a
+// refinement phase leaves 2 f / inertia of the pair's own motion, so a phase
+// asks for no more than that, and beyond kNearMax, or where the positions'
+// units no longer hold the pair's direction to FP32, the step takes the
+// pair-term operator (mph_case::pen_near; 0.01 spacings apart at mu = 0.1 in
+// 180 particles of 2-D: not converged with the lattice's target).
 constexpr float kNearMin = 2.5e-4f, kNearMax = 0.05f;
 template <int D, int L>
 __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __restrict__ type, const double* __restrict__ pos,
@@ -1144,7 +1149,7 @@ __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __re
     const long long b = nptrP[i];
     const int n = i0 < P.N ? ncp[i] : 0;
     double self[3] = {0, 0, 0}, cp[3] = {0, 0, 0};
-    float dp[3] = {0.f, 0.f, 0.f}, nearest = 0.f;
+    float dp[3] = {0.f, 0.f, 0.f}, nearest = 0.f;   // the row's f / inertia
     const int tf = fluid ? type[i] : 0;
     int selfk = 0;
     for (int a = part; a < n; a += L) {
@@ -1163,7 +1168,7 @@ __global__ void __launch_bounds__(128) k_pen_system(DevParams P, const int* __re
                 const double pj = fluid ? pvec[j] : 0.0;
                 const int tj = type[j];
                 const float lam = P.lambda32[tj], turn = (float)inv * P.near_r;   // MaxRadius / |q|
-                nearest = fmaxf(nearest, turn > 256.f ? __int_as_float(0x7f800000) : 0.f);
+                nearest = fmaxf(nearest, turn > 256.f ? __int_as_float(0x7f800000) : P.near_f[tf][tj] * (turn - P.near_k));
 #pragma unroll
                 for (int r = 0; r < D; ++r) {
                     cv[r] = q[r] * f;

@@ -267,7 +267,11 @@ static int derive(mph_case* c, const mph_particles* parts)
         P.fix_scale[d] = std::ldexp(turns, 32) / P.dw[d];
         P.fix_c[d] = (float)(1.0 / (P.fix_scale[d] * P.rP));
     }
+    // f / inertia of a viscous pair (f as above)
     P.near_r = (float)P.maxR;
+    P.near_k = (float)(P.maxR / P.rV);
+    for (int t = 0; t < 2; ++t)
+        for (int u = 0; u < kTypeCount; ++u) P.near_f[t][u] = (float)(P.visc * P.muij[t][u] * (-P.kfv * P.m2h_rv) / P.maxR / P.inert64[t]);
     double cnt[3];
     cnt[0] = std::floor((dmax[0] - P.dmin[0]) / P.maxR);
     cnt[1] = std::floor((dmax[1] - P.dmin[1]) / P.maxR);

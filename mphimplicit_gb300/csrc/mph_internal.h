@@ -69,7 +69,7 @@ struct DevParams {
     float fix_c[3];
     float pen_vm[2][2], pen_vk, pen_vd[2];     // visc mu_ij w' and 1/RadiusV of the fluid pairs over 1/RadiusP; the lattice's
                                                // viscous diagonal of a fluid row
-    float near_r;                              // MaxRadius
+    float near_f[2][kTypeCount], near_r, near_k;   // f / inertia of a pair = near_f (MaxRadius / r - near_k); MaxRadius
     float pen_diag32[kTypeCount];              // inner operator of the point-Jacobi form: its diagonal, lambda kfp 2/RadiusP,
     float pen_lam32[kTypeCount], pen_w32;      // and kfp 2/RadiusP
     int exact_only;                            // 1: skip the FP32 pre-classification
@@ -330,7 +330,7 @@ struct mph_case {
     bool pen_staged = false;            // the assembly built the row blocks' ranks and columns (option inner_local as it was then)
     bool pen_resident = false;          // a phase's CR iterations in one cooperative kernel (the case's rows fit the chip at once)
     int pen_pw4 = 0, pen_umax = 0;      // 8-byte words a row has room for; largest staged count (rounded up)
-    double pen_near = 0.0;              // infinite: a pair of this step's is too close for the operator
+    double pen_near = 0.0;              // the closest viscous pair's f / inertia this step (0: none beyond a lattice's; infinite: too close)
     double pen_tol = 0.0;               // what a refinement phase leaves at least (the viscous part outside the operator)
     int loc_smem = 0;                   // shared memory of k_visc_pen32's staged s (0: gathers by column)
     int loc_cap = 0;                    // staged neighbours a block of the pair-term operator has room for

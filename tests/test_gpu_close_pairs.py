@@ -52,3 +52,17 @@ def test_direction(engine_lib, dim, distance):
     assert s["status"] == 0 and f["status"] == 0
     assert np.linalg.norm(v - want) <= 1e-8 * np.linalg.norm(want)
     assert s["iter"] <= 1.5 * apart["iter"]
+
+
+@pytest.mark.parametrize("mu", [0.1, 1.0])
+@pytest.mark.parametrize("distance", [0.3, 0.1, 0.03, 0.015, 0.01])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_viscous_pair(engine_lib, dim, distance, mu):
+    """A pair that is stiff against the inertia (f / inertia up to 0.1)."""
+    v, s = _solve(dim, distance, mu, precision=PRECISION_MIXED)
+    _, apart = _solve(dim, 1.0, mu, precision=PRECISION_MIXED)
+    want, f = _solve(dim, distance, mu)
+    print(dim, distance, mu, s["iter"], s["outer"], apart["iter"])
+    assert s["status"] == 0 and f["status"] == 0
+    assert np.linalg.norm(v - want) <= 1e-8 * np.linalg.norm(want)
+    assert s["iter"] <= 1.5 * apart["iter"]
