@@ -206,8 +206,8 @@ int mph_server_poll(mph_server* s, mph_server_result* out, int max, int wait_ms,
 int mph_server_stats_get(mph_server* s, mph_server_stats* out);
 int mph_server_destroy(mph_server* s);
 /* Solver tolerances (as mph_case_set_solver) and engine options (as
- * mph_case_set_option; the mixed form's own options skip FP64 cases) for the
- * cases of requests submitted from now on; each case gets them when it is
+ * mph_case_set_option; the mixed form's own options skip FP64 cases, which
+ * "factored" reaches too) for the cases of requests submitted from now on; each case gets them when it is
  * created.  An invalid option fails that request with the option's error.
  * Option "extrapolate" adds its velocity history to the admission footprint. */
 int mph_server_set_solver(mph_server* s, double outer_rel_residual, double inner_rel_residual, int max_outer);

@@ -417,8 +417,8 @@ int server_submit(mph_server* s, const mph_params* prm, const mph_particles* par
             if (o.first == "extrapolate" && o.second > 0.0) fp += 4LL * parts->count * (dim == 2 ? 2 : 4) * 8;
     } else {
         for (auto& o : s->options)   // options of the mixed form do not apply to FP64 cases
-            if (o.first != "extrapolate" && o.first != "dense_coarse" && o.first != "factored" && o.first != "inner_blocks" &&
-                o.first != "inner_local" && o.first != "mixed_extra_sweeps")
+            if (o.first != "extrapolate" && o.first != "dense_coarse" && o.first != "inner_blocks" && o.first != "inner_local" &&
+                o.first != "mixed_extra_sweeps")   // "factored" chooses the FP64 operator in 3-D
                 r->options.push_back(o);
     }
     if (fp > s->budget) {
