@@ -32,7 +32,7 @@ NVCC_FLAGS += [f for f in os.environ.get("MPH_NVCC_DEFINES", "").split() if f.st
 LIB_SOURCES = ["k_particles.cu", "k_neighbor.cu", "k_explicit.cu", "k_assemble.cu", "k_multigrid.cu",
                "k_solver.cu", "k_mixed.cu", "k_assemble_cells.cu", "k_factored.cu", "k_penalty.cu", "k_f64op.cu", "k_resid_noalloc.cu", "mph_case.cu", "mph_export.cu",
                "mph_io.cpp", "mph_batch.cpp", "mph_capi.cpp"]
-HEADERS = ["mph_internal.h", "mph_device.cuh", "mph_solver.cuh", "mph_pairs.cuh", "mph_twofloat.cuh", os.path.join("..", "..", "include", "mph_gb300.h")]
+HEADERS = ["mph_internal.h", "mph_device.cuh", "mph_solver.cuh", "mph_pairs.cuh", "mph_twofloat.cuh", "mph_shapes.h", os.path.join("..", "..", "include", "mph_gb300.h")]
 
 
 def _nvcc() -> str:

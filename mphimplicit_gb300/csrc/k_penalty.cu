@@ -45,6 +45,7 @@
 
 #include "mph_device.cuh"
 #include "mph_pairs.cuh"
+#include "mph_shapes.h"
 #include "mph_solver.cuh"
 #include "mph_twofloat.cuh"
 
@@ -1514,7 +1515,8 @@ static size_t cr_smem(const mph_case* c, int rows, int umax)
     return (size_t)umax * (c->dim == 3 ? 32 : 24) + (size_t)rows * ((c->pmax + 3) / 4) * sizeof(uint2) + 16;
 }
 
-// Blocks of the resident iteration that the device holds at once (0: none)
+// Blocks of the resident iteration that the device holds at once (0: none), two
+// an SM and, in c->cr_alone, one an SM in the form with more registers
 static int cr_capacity(mph_case* c)
 {
     if (c->cr_cap < 0) {   // once a case: the attributes and the count belong to its device
@@ -1526,35 +1528,21 @@ static int cr_capacity(mph_case* c)
         for (const void* k : f) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCrSmem);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f[0], kCrThreads, kCrSmem);
         c->cr_cap = std::min(coop ? sms * nb : 0, kCrBlocks);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f[1], kCrThreads, kCrSmem);
+        c->cr_alone = coop && nb > 0 ? std::min(sms, kCrBlocks / 2) : 0;
     }
     return c->cr_cap;
 }
 
-// Rows a block and threads a row.  Up to 155,648 particles the iteration is
-// resident: up to 512 threads a block, the rows spread evenly over at most two
-// blocks an SM (the choice does not depend on what a step's blocks stage, so
-// that staged and gathering runs keep one order of sums).  Beyond, and for
-// lists too long for shared memory, 256 rows a block in the per-iteration
-// kernels (a row's share of the staged neighbours falls with the block), or
-// fewer and several threads a row where the blocks would not reach every SM.
 static void pen_shape(mph_case* c)
 {
-    const int N = c->dp.N;
     const int cap = cr_capacity(c);
-    int rows = std::max(c->dim == 2 ? kCrMinRows2 : kCrMinRows3, cap > 0 ? ((N + cap - 1) / cap + 31) / 32 * 32 : 0);
-    // as long as the rows fit, one block an SM: half the blocks at a crossing
-    // and twice the registers (kCrAhead).  A step of 33,600
-    // particles in 3-D 2.44 -> 2.03 ms, 57,000 2.61 -> 2.42, 71,000 3.03 ->
-    // 2.75; 2-D the same either way.  (One block of up to 1024 threads an SM
-    // beyond 77,824 particles, with the registers of two: no difference.)
-    const int one = ((N + kCrBlocks / 2 - 1) / (kCrBlocks / 2) + 31) / 32 * 32;
     auto fits = [c](int r) { return r <= kCrThreads && cr_smem(c, r, (pen_ucap(r) + 127) / 128 * 128) <= (size_t)kCrSmem; };
-    if (cap == kCrBlocks && one > rows && fits(one)) rows = one;
-    c->pen_resident = fits(rows) && (long long)rows * cap >= N;
-    if (c->pen_resident) { c->pen_rows = rows; c->pen_w = kCrThreads / rows; }
-    else if (N > 152 * 512) { c->pen_rows = 256; c->pen_w = 1; }
-    else if (N > 152 * 192) { c->pen_rows = 128; c->pen_w = 2; }
-    else { c->pen_rows = 64; c->pen_w = 4; }
+    const PenShape S = pen_shape_for(c->dp.N, c->dim == 2 ? kCrMinRows2 : kCrMinRows3, kCrThreads, cap, c->cr_alone, fits);
+    c->pen_rows = S.rows;
+    c->pen_w = S.w;
+    c->pen_resident = S.resident;
+    c->pen_alone = S.alone;
 }
 
 // (The positions' unit is MaxRadius / 2^30, which stays fine in RadiusP.)
@@ -1826,8 +1814,8 @@ int launch_pen_resident(mph_case* c, int cap, double scale)
     const dim3 blk(c->pen_rows, c->pen_w);
     void* args[] = {&c->dp, &A, &C};
     const size_t smem = cr_smem(c, c->pen_rows, c->pen_umax);
-    // a block an SM and the device to itself: the form with more registers
-    const bool alone = nb <= kCrBlocks / 2 && !c->shared_gpu;
+    // a block an SM and the device to itself (or too few SMs for the other form): the form with more registers
+    const bool alone = c->pen_alone && (!c->shared_gpu || nb > c->cr_cap);
     const void* f = c->dim == 2 ? (alone ? (const void*)k_pen_cr<2, kCrAhead> : (const void*)k_pen_cr<2, kCrShared2>)
                                 : (alone ? (const void*)k_pen_cr<3, kCrAhead> : (const void*)k_pen_cr<3, kCrShared3>);
     MPH_CUDA(cudaLaunchCooperativeKernel(f, dim3(nb), blk, args, smem, c->stream));

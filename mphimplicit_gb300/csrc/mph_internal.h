@@ -320,7 +320,7 @@ struct mph_case {
     bool level0_done = false;           // this step's level-0 multigrid stencils were written by the assembly
     bool step_f64 = false;              // this step's FP64 solve may run on k_f64op.cu's operator in parts
     long long f64_slots = 0;            // slots the pair records have room for (their two arrays' split)
-    int cr_cap = -1;                    // blocks of the resident iteration its device holds at once (-1: not asked yet)
+    int cr_cap = -1, cr_alone = 0;      // blocks of the resident iteration its device holds at once, two and one an SM (-1: not asked yet)
     bool pen_attr = false, tail_attr = false;   // its kernels' shared-memory limits are set on its device
     bool shared_gpu = false;            // other cases step on this GPU meanwhile (a batch of several, a server)
     bool system_current = false;        // positions, types and lists are those of the last assembly
@@ -328,6 +328,7 @@ struct mph_case {
     int pmax = 0;                       // longest P-list of the current lists
     int pen_rows = 0, pen_w = 0;        // its rows a block and threads a row
     bool pen_staged = false;            // the assembly built the row blocks' ranks and columns (option inner_local as it was then)
+    bool pen_alone = false;             // its blocks fit one an SM
     bool pen_resident = false;          // a phase's CR iterations in one cooperative kernel (the case's rows fit the chip at once)
     int pen_pw4 = 0, pen_umax = 0;      // 8-byte words a row has room for; largest staged count (rounded up)
     double pen_near = 0.0;              // the closest viscous pair's f / inertia this step (0: none beyond a lattice's; infinite: too close)
