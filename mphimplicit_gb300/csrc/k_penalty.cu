@@ -1584,9 +1584,9 @@ static int launch_pen_lists(mph_case* c)
     if (!d.pgroups) MPH_CUDA(cudaMalloc((void**)&d.pgroups, (size_t)nsl * sizeof(int)));
     MPH_TRY(grow_t(&d.puniq, &d.cap_puniq, (long long)nb * ucap));
     MPH_TRY(grow_t(&d.pucount, &d.cap_pucount, nb + 5));
-    if (c->pen_resident && !d.cr_rec) {
-        MPH_CUDA(cudaMalloc((void**)&d.cr_rec, (size_t)P.Nf * 3 * sizeof(float4)));
-        MPH_CUDA(cudaMalloc((void**)&d.cr_vals, (size_t)(8 * kCrBlocks + 32) * sizeof(float)));
+    if (c->pen_resident) {   // each asked for on its own: one may have failed before
+        if (!d.cr_rec) MPH_CUDA(cudaMalloc((void**)&d.cr_rec, (size_t)P.Nf * 3 * sizeof(float4)));
+        if (!d.cr_vals) MPH_CUDA(cudaMalloc((void**)&d.cr_vals, (size_t)(8 * kCrBlocks + 32) * sizeof(float)));
     }
     MPH_TRY(grow_t(&d.pidx, &d.cap_pidx, (long long)nsl * c->pen_pw4 * 32));
     c->pen_umax = 0;
