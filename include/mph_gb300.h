@@ -305,6 +305,12 @@ int mph_case_set_option(mph_case* c, const char* name, double value);
  *   "pair_fuse" 0 (default) / 1: point-Jacobi mixed form on the pair path;
  *   1 writes the sliced pair terms in one kernel without the per-slot
  *   pair-term list (16 bytes a neighbour slot less device memory; slower).
+ *   "launch_iterations" 1 .. 4096 (default), "wait_polls" 1 .. 2097152
+ *   (default): point-Jacobi mixed form of a case whose rows fit the chip at
+ *   once (up to 155,648 particles).  The CR iterations one cooperative launch
+ *   runs at most (the solve then goes on in the next), and the polls of its
+ *   grid barrier after which it gives up (MPH_ERR_CUDA; the case can be given
+ *   a state and stepped again).
  *   "split_apply" 0 (default) / 1: pair-term inner operator only; 1 runs the
  *   transposed apply on a side stream beside the viscous kernel and adds
  *   lambda C t in a third kernel.  The forms of these three options reach

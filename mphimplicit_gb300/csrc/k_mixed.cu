@@ -692,6 +692,7 @@ struct MixedRun {
     int host_flags[kFlagCount] = {};
     double hs[32] = {};
     bool bad = false;
+    bool scaled = false;              // scale is set
 
     void init(mph_case* c_)
     {
@@ -773,7 +774,8 @@ struct MixedRun {
         if (c->step_pen && c->pen_resident && outer > 0 && !host_flags[kFlagDone]) --outer;
         if (hs[kSRR] / hs[kSRR0] < tol_out2 || outer >= c->max_outer || hs[kSRR] == 0.0) return MPH_OK;
         if (outer > 0 && host_flags[kFlagIter] >= cap) return MPH_OK;
-        if (outer == 0) scale = std::sqrt(hs[kSRR]);
+        if (!scaled) scale = std::sqrt(hs[kSRR]);   // once a solve: the directions are in its units
+        scaled = true;
         if (c->step_pen) {
             ++outer;
             launch_pen_phase(c, 1.0 / scale, nullptr, tol_in2, tol_out2);

@@ -708,10 +708,9 @@ __global__ void __launch_bounds__(kReduceThreads) k_pen_vec(PenArgs A, int n, in
 // us an iteration; a warp's own terms are summed in FP32 as elsewhere.
 //
 // All blocks are resident (cooperative launch), so a wait ends; it is bounded
-// all the same, and a block whose wait runs out raises kFlagStall and leaves,
-// as the others then do.  A launch runs at most kCrMaxIter iterations.
-constexpr int kCrMaxIter = 4096;
-constexpr int kCrSpin = 1 << 21;
+// all the same (option wait_polls), and a block whose wait runs out raises
+// kFlagStall and leaves, as the others then do.  A launch runs at most
+// mph_case::cr_iters iterations (option launch_iterations).
 
 struct PenCr {
     float4* rec;                   // per row 3 records: s, a = D^-1 y, b = D^-1 q
@@ -720,6 +719,7 @@ struct PenCr {
     // the phase's end: x += scale z, z as records for the residual, the
     // velocity array
     double scale;
+    int iters, polls;              // iterations of a launch, polls of a wait at most
     double *x, *vel;
     float4* z4;
 };
@@ -731,7 +731,7 @@ struct PenCr {
 // word per block and value that every block polls instead was slower (nb^2
 // polls).
 __device__ __forceinline__ bool cr_cross(unsigned* count, float* vals, const float* mine, int nv, unsigned epoch, int lb, int nb, int tid,
-                                         int* flags)
+                                         int* flags, int polls)
 {
     __shared__ int ok_s;
     __syncthreads();
@@ -745,7 +745,7 @@ __device__ __forceinline__ bool cr_cross(unsigned* count, float* vals, const flo
             int n = 0;
             do {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-            } while ((int)(v - target) < 0 && ++n < kCrSpin);
+            } while ((int)(v - target) < 0 && ++n < polls);
             ok_s = (int)(v - target) >= 0;
             if (!ok_s) flags[kFlagStall] = 1;
         }
@@ -859,7 +859,7 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
     const int ui[3] = {pi.x, pi.y, pi.z};
     const bool fluid = i < A.Nf, mine = w == 0 && fluid;
     int it = A.flags[kFlagIter];
-    const int it_end = it + kCrMaxIter;
+    const int it_end = it + C.iters;
     const F2 stop_rr = f2_of(A.scal[kSTol2] * A.scal[kSIn0]);
     // thread 0's: (s, y) and (q, D^-1 q) of the last iteration
     F2 rho = f2_of(A.scal[rho_slot32(it - 1)]), qu = f2_of(A.scal[kSQUPrev]);
@@ -900,7 +900,7 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
     float alpha = 0.f, beta = 0.f;
     bool first = true;
     if (tid < 6) val_s[tid] = 0.f;
-    bool ok = cr_cross(C.count, C.v3, val_s, 6, ++epoch, lb, nb, tid, A.flags);   // every row's s is out
+    bool ok = cr_cross(C.count, C.v3, val_s, 6, ++epoch, lb, nb, tid, A.flags, C.polls);   // every row's s is out
     // a crossing's first loads: the thread's first neighbour's records, while
     // alpha and beta are formed
     CrRec pre[PF > 0 ? PF : 1];
@@ -995,7 +995,7 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
         ti = n > 0 ? lam * ti : 0.f;
         if (w == 0 && i < A.N) A.t[i] = ti;
         // every particle's lambda t (and every block's (r, r)) is out
-        if (!(ok = cr_cross(C.count, C.v1, val_s, 2, ++epoch, lb, nb, tid, A.flags))) break;
+        if (!(ok = cr_cross(C.count, C.v1, val_s, 2, ++epoch, lb, nb, tid, A.flags, C.polls))) break;
         if (!first && warp == (nth >> 5) - 1) {   // the stop test
             const F2 v = cr_sum(C.v1, 2, nb, lane);
             if (lane == 0) {
@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(kCrThreads, PF > 1 ? 1 : 2) k_pen_cr(DevParams
             }
         }
         // every row's s, a, b and every block's dot products are out
-        if (!(ok = cr_cross(C.count, C.v3, val_s, 6, ++epoch, lb, nb, tid, A.flags))) break;
+        if (!(ok = cr_cross(C.count, C.v3, val_s, 6, ++epoch, lb, nb, tid, A.flags, C.polls))) break;
 #pragma unroll
         for (int u = 0; u < PF; ++u) pre[u] = cr_load<D>(C.rec, j0[u], A.Nf);
         if (warp < 3) {
@@ -1808,6 +1808,8 @@ int launch_pen_resident(mph_case* c, int cap, double scale)
     C.v1 = d.cr_vals + 6 * kCrBlocks;
     C.count = cr_count(c);   // zeroed by k_pen_phase
     C.scale = scale;
+    C.iters = c->cr_iters;
+    C.polls = c->cr_polls;
     C.x = d.x;
     C.vel = d.vel;
     C.z4 = d.z4;

@@ -147,6 +147,14 @@ int mph_case_set_option(mph_case* c, const char* name, double value)
         (n == "pair_block" ? c->pair_block : n == "ct_block" ? c->ct_block : c->chunk) = v;
         return MPH_OK;
     }
+    if (std::string(name) == "launch_iterations" || std::string(name) == "wait_polls") {
+        const bool it = name[0] == 'l';
+        const int most = it ? 4096 : 1 << 21;
+        if (!(value >= 1.0 && value <= most) || (double)(int)value != value)
+            return mph::fail(MPH_ERR_ARG, "options launch_iterations 1 .. 4096, wait_polls 1 .. 2097152");
+        (it ? c->cr_iters : c->cr_polls) = (int)value;
+        return MPH_OK;
+    }
     if (std::string(name) == "keep_history") {
         c->keep_history = value != 0.0;
         return MPH_OK;

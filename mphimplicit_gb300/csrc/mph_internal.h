@@ -321,6 +321,7 @@ struct mph_case {
     bool step_f64 = false;              // this step's FP64 solve may run on k_f64op.cu's operator in parts
     long long f64_slots = 0;            // slots the pair records have room for (their two arrays' split)
     int cr_cap = -1, cr_alone = 0;      // blocks of the resident iteration its device holds at once, two and one an SM (-1: not asked yet)
+    int cr_iters = 4096, cr_polls = 1 << 21;   // options launch_iterations, wait_polls
     bool pen_attr = false, tail_attr = false;   // its kernels' shared-memory limits are set on its device
     bool shared_gpu = false;            // other cases step on this GPU meanwhile (a batch of several, a server)
     bool system_current = false;        // positions, types and lists are those of the last assembly
