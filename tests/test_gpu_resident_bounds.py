@@ -50,3 +50,33 @@ def test_launch_bound(engine_lib, dim, bound):
     va, vb = (vec_proj(c.export("Velocity"), dim)[:c.fluid_count] for c in (a, b))
     assert np.linalg.norm(vb - va) <= 1e-8 * np.linalg.norm(va)
     assert sb["iter"] <= 1.1 * sa["iter"] + 5
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_wait_runs_out(engine_lib, dim):
+    """One poll a wait: a block that arrives before the others gives up, every
+    block leaves, the step fails with a status that the host reads, and the
+    case given its state again steps to a new case's bits."""
+    g, parts = _new(dim, wait_polls=1)
+    with pytest.raises(engine.MphError) as e:
+        g.step(1)
+    assert "barrier" in str(e.value)
+    g.set_option("wait_polls", 1 << 21)
+    g.set_state(parts)
+    h, _ = _new(dim)
+    h.set_state(parts)
+    for _ in range(2):
+        g.step(1)
+        h.step(1)
+        assert g.solve_stats()["status"] == 0
+    assert np.array_equal(g.export("ParticleIndex"), h.export("ParticleIndex"))
+    assert np.array_equal(g.export("Velocity"), h.export("Velocity"))
+
+
+def test_bounds_are_checked(engine_lib):
+    g, _ = _new(2)
+    for name, value in (("launch_iterations", 0), ("launch_iterations", 4097), ("launch_iterations", 2.5), ("wait_polls", 0),
+                        ("wait_polls", float("nan")), ("wait_polls", 2097153)):
+        with pytest.raises(engine.MphError) as e:
+            g.set_option(name, value)
+        assert e.value.status == 1
