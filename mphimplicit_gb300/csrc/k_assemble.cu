@@ -431,6 +431,7 @@ int launch_assemble(mph_case* c)
     // the form of this step's system decides which block arrays exist: FP64
     // blocks unless the FP64 operator is factored, FP32 blocks for the mixed
     // form unless its inner operator runs without blocks
+    c->no_levels = false;
     c->step_factored = factored_applies(c);
     c->step_pairs = c->step_factored && !c->inner_blocks && c->visc_nonneg;
     c->step_pen = pen_applies(c);
@@ -451,7 +452,10 @@ int launch_assemble(mph_case* c)
         const int pon = prof_begin(c, 2, &pe);
         MPH_TRY(launch_pen_assemble(c));
         if (pon) prof_end(c, 2, pe);
-        if (c->step_pen) return MPH_OK;
+        if (c->step_pen) {
+            c->no_levels = true;
+            return MPH_OK;
+        }
     }
     // slice pointers
     // the fluid rows' slices padded to a multiple of 4 slots (zero padding
@@ -541,6 +545,7 @@ int launch_assemble(mph_case* c)
     }
     const int* only = cells ? c->d.cell_flags : nullptr;
     if (skip_rows) {
+        c->no_levels = true;
         if (c->step_pairs) MPH_TRY(launch_pairs_to_slices(c));
         if (pon) prof_end(c, 2, pe);
         return MPH_OK;

@@ -865,7 +865,7 @@ static void vcycle_t(mph_case* c, const TQ* q, TQ* u, const TQ* invDiag, const T
     // mixed form's options mg_pre / mg_post; the mixed form's option mg_depth
     // (>= 2) cuts the cycle after that many levels (the last one coarsest)
     const bool mixed = std::is_same<T, float>::value;
-    if (mixed && c->mg_depth < 0) {   // no grid levels: point Jacobi on the particles
+    if (mixed && mixed_jacobi(c)) {   // no grid levels: point Jacobi on the particles
         const long long n = (long long)c->dp.Nf * D;
         const int blocks = std::min<int>(grid_for(n, 256), kReduceBlocks);
         { k_jacobi_dot<TQ><<<blocks, 256, 0, c->stream>>>(n, invDiag, q, u, c->d.partials, (unsigned*)(c->d.flags + kFlagCounter),

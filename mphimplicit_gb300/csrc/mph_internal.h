@@ -324,6 +324,7 @@ struct mph_case {
     int cr_iters = 4096, cr_polls = 1 << 21;   // options launch_iterations, wait_polls
     bool pen_attr = false, tail_attr = false;   // its kernels' shared-memory limits are set on its device
     bool shared_gpu = false;            // other cases step on this GPU meanwhile (a batch of several, a server)
+    bool no_levels = false;             // the assembly left out what multigrid levels are built from (mg_depth as it was then)
     bool system_current = false;        // positions, types and lists are those of the last assembly
     bool step_pen = false;              // this step's inner CR runs on k_penalty.cu's operator
     int pmax = 0;                       // longest P-list of the current lists
@@ -470,7 +471,7 @@ bool batch_solve_eligible(const mph_case* c);
 
 // the mixed form preconditioned by point Jacobi (option mg_depth -1): no
 // multigrid levels are built or used
-inline bool mixed_jacobi(const mph_case* c) { return c->precision == MPH_PRECISION_MIXED && c->mg_depth < 0; }
+inline bool mixed_jacobi(const mph_case* c) { return c->precision == MPH_PRECISION_MIXED && (c->mg_depth < 0 || c->no_levels); }
 bool pair_path_expected(const mph_params* prm, const mph_particles* parts, int dim);
 int launch_pair_terms(mph_case* c);
 void launch_resid_factored(mph_case* c, const double* x, double* r, double* out);

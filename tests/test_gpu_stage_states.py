@@ -53,6 +53,33 @@ def test_staging_is_the_assemblys(engine_lib, dim, at_assembly):
         b.step(1)
 
 
+@pytest.mark.parametrize("pairs", [False, True])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_levels_are_the_assemblys(engine_lib, dim, pairs):
+    """Option mg_depth set to 0 between an assembly without multigrid levels
+    and the solve: the step keeps point Jacobi (levels would be built from
+    stencils that the assembly did not write), the next one has its levels.
+    pairs: the pair-term operator (two particles close together)."""
+    params, parts = _parts(dim)
+    if pairs:
+        parts.pos[1] = parts.pos[0] + 1e-3 * parts.spacing * np.array([0.6, 0.8, 0.0])
+        parts.vel[1] = parts.vel[0]
+    a, b = _mixed(params, parts, dim), _mixed(params, parts, dim)
+    for s in BEFORE_SOLVE[:5]:
+        a.stage(s)
+    a.set_option("mg_depth", 0)
+    for s in ("mg_build", "solve"):
+        a.stage(s)
+    with pytest.raises(engine.MphError):
+        a.export("MultiGridCsrCofA:0")
+    a.stage("step_end")
+    b.step(1)
+    assert a.solve_stats()["status"] == 0
+    assert np.array_equal(a.export("Velocity"), b.export("Velocity"))
+    a.step(1)
+    assert a.solve_stats()["status"] == 0 and len(a.export("MultiGridCsrCofA:0")) > 0
+
+
 @pytest.mark.parametrize("dim", [2, 3])
 def test_c_of_the_mixed_form(engine_lib, oracle_built, dim):
     """C as the point-Jacobi mixed form's assembly writes it with four threads
