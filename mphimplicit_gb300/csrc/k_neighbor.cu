@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(128) k_neighbors(DevParams P, int rx, int ry, 
 // as the per-thread walk's, written with coalesced stores.  A walk that does
 // not wrap around the periodic grid (and a grid of at least 2 range + 3 cells
 // on every axis) needs no minimum-image correction in FP32.  A bucket with
-// more than kNbMaxP particles, a pass with more than kNbCap candidates, a walk
+// more than kNbMaxP particles, a pass with more candidates than a block has room for, a walk
 // of more than 27 cells or the exact-only mode runs the per-thread walk.
 //
 // The walk is bound by the integer pipe, some 45 instructions a chunk of 32
@@ -163,11 +163,19 @@ __global__ void __launch_bounds__(128) k_neighbors(DevParams P, int rx, int ry, 
 // small and many: 64 threads and room for 512 candidates (30 KB of shared
 // memory a block of eight warps held an SM to seven blocks and left their
 // start and staging latencies uncovered).  Both passes on 412,000 particles 1.0 -> 0.63
-// ms (0.71 with 128 threads).  In 3-D, 30 and 810: 256 threads, 1536.
-template <int D> constexpr int kNbThreads = D == 2 ? 64 : 256;   // at least two warps: one a pass reads the walk's buckets
-template <int D> constexpr int kNbCap = D == 2 ? 512 : 1536;
+// ms (0.71 with 128 threads).  In 3-D, 30 and 810: 256 threads, 1536.  Those
+// also in 2-D where a cell has more than 32 particles (a MaxRadius beyond some
+// 5.5 spacings, a compressed fluid): such a grid has few cells, and two warps
+// each leave the chip empty (94,536 particles with a MaxRadius of 8.5, 12 and 14
+// spacings: 0.29, 0.61 and 1.21 ms, in small blocks and, beyond their room,
+// per-thread walks 0.86, 2.34 and 3.84); up to 32 a walk's 9 cells hold no more
+// than 288 candidates.
+struct NbSmall { static constexpr int threads = 64, cap = 512; };     // at least two warps: one a pass reads the walk's buckets
+struct NbLarge { static constexpr int threads = 256, cap = 1536; };
+constexpr int kNbSmallCell = 32;
 constexpr int kNbMaxP = 256;
-static_assert(kNbThreads<2> >= 64 && kNbThreads<3> >= 64, "a warp for each of the two passes");
+static_assert(NbSmall::threads >= 64 && NbLarge::threads >= 64, "a warp for each of the two passes");
+static_assert(9 * kNbSmallCell <= NbSmall::cap, "a 2-D walk's candidates");
 
 // The FP32 squared distance of a staged candidate (the minimum image only
 // for a walk that wraps), as classify computes it.
@@ -196,15 +204,15 @@ __device__ __forceinline__ int classify_exact(const DevParams& P, const double* 
     return 1 | (r2 <= P.rP2 ? 2 : 0);
 }
 
-template <int D, bool FILL>
-__global__ void __launch_bounds__(kNbThreads<D>) k_neighbors_cells(DevParams P, int rx, int ry, int rz, int wB, int wE,
+template <int D, bool FILL, typename B>
+__global__ void __launch_bounds__(B::threads) k_neighbors_cells(DevParams P, int rx, int ry, int rz, int wB, int wE,
                                                                 const int* __restrict__ key, const int* __restrict__ bucket,
                                                                 const double* __restrict__ pos, const float* __restrict__ pos32,
                                                                 int* __restrict__ nc, int* __restrict__ nfc, int* __restrict__ ncp,
                                                                 const long long* __restrict__ nptr, const long long* __restrict__ nptrP,
                                                                 int* __restrict__ nind, int* __restrict__ nindP)
 {
-    __shared__ float4 spos[kNbCap<D>];
+    __shared__ float4 spos[B::cap];
     __shared__ int coff[2][28];
     __shared__ int cbeg[2][27];
     __shared__ int sn0[kNbMaxP], snp0[kNbMaxP];
@@ -251,7 +259,7 @@ __global__ void __launch_bounds__(kNbThreads<D>) k_neighbors_cells(DevParams P, 
             if (lane == 0) coff[pass][0] = 0;
         }
         __syncthreads();
-        slow = coff[0][ncell] > kNbCap<D> || coff[1][ncell] > kNbCap<D>;
+        slow = coff[0][ncell] > B::cap || coff[1][ncell] > B::cap;
     }
     if (slow) {   // the same for every thread of the block
         for (int i = r0 + tid; i < r1; i += blockDim.x)
@@ -565,13 +573,14 @@ static void launch_neighbors_cells(mph_case* c, const int* r)
 {
     const unsigned g = (unsigned)(2 * c->dp.T);
     DeviceState& d = c->d;
-    if (c->dim == 2)
-        k_neighbors_cells<2, FILL><<<g, kNbThreads<2>, 0, c->stream>>>(c->dp, r[0], r[1], r[2], c->wB, c->wE, d.key, d.bucket, d.pos, d.pos32,
-                                                                    d.nc, d.nfc, d.ncp, d.nptr, d.nptrP, d.nind, d.nindP);
-    else
-        k_neighbors_cells<3, FILL><<<g, kNbThreads<3>, 0, c->stream>>>(c->dp, r[0], r[1], r[2], c->wB, c->wE, d.key, d.bucket, d.pos, d.pos32,
-                                                                    d.nc, d.nfc, d.ncp, d.nptr, d.nptrP, d.nind, d.nindP);
-    MPH_COUNT_LAUNCH();
+    auto go = [&](auto kern, int threads) {
+        kern<<<g, threads, 0, c->stream>>>(c->dp, r[0], r[1], r[2], c->wB, c->wE, d.key, d.bucket, d.pos, d.pos32, d.nc, d.nfc, d.ncp,
+                                           d.nptr, d.nptrP, d.nind, d.nindP);
+        MPH_COUNT_LAUNCH();
+    };
+    if (c->dim == 3) go(k_neighbors_cells<3, FILL, NbLarge>, NbLarge::threads);
+    else if (c->cell_max <= kNbSmallCell) go(k_neighbors_cells<2, FILL, NbSmall>, NbSmall::threads);
+    else go(k_neighbors_cells<2, FILL, NbLarge>, NbLarge::threads);
 }
 
 void launch_neighbor_count(mph_case* c)

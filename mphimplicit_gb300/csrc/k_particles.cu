@@ -78,6 +78,7 @@ __global__ void k_cell_keys(DevParams P, const double* __restrict__ pos, const i
         bbox[i] = P.cc[i];
         bbox[3 + i] = 0;
         wrap[i] = 0;
+        if (i == 0) bbox[8] = 0;
     }
     if (i >= P.nPow) return;
     if (i < P.N) {
@@ -328,6 +329,10 @@ __global__ void k_fluid_bbox(const int* __restrict__ bucket, DevParams P, int* _
         bbox[6] = bucket[P.T];
         bbox[7] = bucket[2 * P.T];
     }
+    // and the most particles of a cell, fluid or wall
+    const int most = c < P.T ? max(bucket[c + 1] - bucket[c], bucket[P.T + c + 1] - bucket[P.T + c]) : 0;
+    const int warp_most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0 && warp_most > *(volatile int*)(bbox + 8)) atomicMax(bbox + 8, warp_most);
     if (c >= P.T) return;
     if (bucket[c + 1] - bucket[c] > 0) {
         const int p[3] = {(c / (P.cc[1] * P.cc[2])) % P.cc[0], (c / P.cc[2]) % P.cc[1], c % P.cc[2]};

@@ -404,7 +404,7 @@ int case_alloc_particles(mph_case* c)
     MPH_TRY(dalloc(c, &d.partials, (size_t)std::max<size_t>(kReduceBlocks, Nf / 16 + 64)));   // three values a 64-row block
     MPH_TRY(dalloc(c, &d.scal, 32 + kFlagCount * sizeof(int) / sizeof(double)));
     d.flags = reinterpret_cast<int*>(d.scal + 32);   // one read brings both
-    MPH_TRY(dalloc(c, &d.bbox, 8));
+    MPH_TRY(dalloc(c, &d.bbox, 9));
     MPH_TRY(dalloc(c, &d.totals, 8));
     MPH_TRY(dalloc(c, &d.dmax, 4));
     MPH_CUDA(cudaMemsetAsync(d.flags, 0, kFlagCount * sizeof(int), c->stream));
@@ -508,7 +508,7 @@ int stage_cellsort(mph_case* c)
     else launch_bitonic_sort(c);
     launch_cell_ranges_and_permute(c);
     launch_fluid_bbox(c);
-    int hb[8];   // the fluid's cell box, the ends of the fluid and the wall particles
+    int hb[9];   // the fluid's cell box, the ends of the fluid and the wall particles, the most particles of a cell
     MPH_CUDA(cudaMemcpyAsync(hb, c->d.bbox, sizeof(hb), cudaMemcpyDeviceToHost, c->stream));
     MPH_CUDA(cudaStreamSynchronize(c->stream));
     MPH_CUDA(cudaGetLastError());
@@ -517,6 +517,7 @@ int stage_cellsort(mph_case* c)
     c->fE = ends[0];
     c->wB = ends[0];
     c->wE = ends[1];
+    c->cell_max = hb[8];
     if (c->fE != c->dp.Nf) return fail(MPH_ERR_STATE, "fluid count changed in the cell sort");
     for (int k = 0; k < 6; ++k) c->bbox[k] = hb[k];
     MPH_TRY(mg_geometry(c));

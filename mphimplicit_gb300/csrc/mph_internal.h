@@ -327,6 +327,7 @@ struct mph_case {
     bool no_levels = false;             // the assembly left out what multigrid levels are built from (mg_depth as it was then)
     bool system_current = false;        // positions, types and lists are those of the last assembly
     bool step_pen = false;              // this step's inner CR runs on k_penalty.cu's operator
+    int cell_max = 0;                   // most fluid or wall particles of a cell at the last sort
     int pmax = 0;                       // longest P-list of the current lists
     int pen_rows = 0, pen_w = 0;        // its rows a block and threads a row
     bool pen_staged = false;            // the assembly built the row blocks' ranks and columns (option inner_local as it was then)
