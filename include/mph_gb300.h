@@ -108,7 +108,11 @@ typedef struct mph_solve_stats {
     int inner_gather_blocks;
     long long inner_local_cols;  /* distinct neighbour columns summed over the staged row blocks */
     int inner_ct_local_blocks;   /* particle blocks of the transposed apply staging s */
-    int inner_reserved;          /* 0 */
+    int inner_kernel;            /* inner_form 2: 0 the pair-term kernels (options pair_block, ct_block, pair_pack,
+                                pair_recompute, pair_fuse, split_apply, chunk, graphs and device_loop act), 1 a kernel
+                                each for C^T s, the rest of the operator and the vectors (chunk, graphs, device_loop
+                                and batch_solve act), 2 all iterations of a refinement phase in one resident kernel
+                                (none of these acts) */
 } mph_solve_stats;
 
 typedef struct mph_case mph_case;
@@ -207,8 +211,8 @@ int mph_server_stats_get(mph_server* s, mph_server_stats* out);
 int mph_server_destroy(mph_server* s);
 /* Solver tolerances (as mph_case_set_solver) and engine options (as
  * mph_case_set_option; the mixed form's own options skip FP64 cases, which
- * "factored" reaches too) for the cases of requests submitted from now on; each case gets them when it is
- * created.  An invalid option fails that request with the option's error.
+ * "factored" reaches too) for the cases of requests submitted from now on;
+ * each case gets them when it is created.  An invalid option fails that request with the option's error.
  * Option "extrapolate" adds its velocity history to the admission footprint. */
 int mph_server_set_solver(mph_server* s, double outer_rel_residual, double inner_rel_residual, int max_outer);
 int mph_server_set_option(mph_server* s, const char* name, double value);
@@ -243,11 +247,13 @@ int mph_case_set_solver(mph_case* c, double outer_rel_residual, double inner_rel
  *   smoothing sweeps before and after the rest of its V-cycle.
  *   "inner_blocks" 0 (default) / 1: factored mixed form only.  0: the inner
  *   FP32 operator is inertia and C Lambda C^T evaluated from the P-lists (the
- *   viscous pairs are left to the FP64 outer residual) or, with mg_depth >= 0
- *   and in domains over about 1900 RadiusP wide, runs on the sliced FP32 pair
- *   terms and P-lists; no blocks are written (CsrCofA export then fails with MPH_ERR_STATE; the
- *   block columns CsrIndA still export).  1: FP32 blocks are assembled and
- *   the inner SpMV runs on them.
+ *   viscous pairs are left to the FP64 outer residual) or, with mg_depth >= 0,
+ *   with MaxRadius above 16 RadiusP and in steps with particles closer
+ *   together than MaxRadius / 256 or a viscous pair above 0.05 of the inertia,
+ *   runs on the sliced FP32 pair terms and P-lists; no blocks are written
+ *   (CsrCofA export then fails with MPH_ERR_STATE; the block columns CsrIndA
+ *   still export).  1: FP32 blocks are assembled and the inner SpMV runs on
+ *   them.
  *   "inner_local" 1 (default) / 0: inner operator without blocks only.  1: each
  *   block of rows (particles, for the transposed apply) whose distinct
  *   neighbours fit stages their values in shared memory; 0: every block gathers s
@@ -271,15 +277,18 @@ int mph_case_set_option(mph_case* c, const char* name, double value);
  *   "pair_block" 128 / 256 / 512 (default), "ct_block" 128 / 256 (default),
  *   "chunk" 4 / 8 (default) / 16 / 32: mixed form's launch shapes (block
  *   widths of the pair-term operator and of the transposed apply, CR
- *   iterations per captured graph chunk); mphimplicit_gb300/autotune.py
- *   chooses them by measurement.
+ *   iterations per captured graph chunk); they act where
+ *   mph_solve_stats::inner_kernel says so, and mphimplicit_gb300/autotune.py
+ *   chooses those by measurement.
  *   "keep_history" 0 (default) / 1: with 1, mph_case_set_state keeps the
  *   extrapolation history: the caller declares that the state continues this
  *   case's own steps in the case's particle order (e.g. the state it read back
  *   with mph_get_fields); the start value only changes the iteration count.
  *   "device_loop" 0 (default) / 1: mixed form with graphs.  1 runs the whole
  *   solve as one CUDA graph whose refinement and CR loops are device-side
- *   conditional while nodes (no host poll; same bits); not with profiling.
+ *   conditional while nodes (no host poll; same bits); not with profiling, nor
+ *   for a point-Jacobi case that fits the chip at once (inner_kernel 2: its
+ *   phases are one launch each without it).
  *   "mg_depth" -1 (default) / 0 / 1 .. 24: mixed form only.  The inner CR's
  *   preconditioner: -1 point Jacobi (D^-1 from the assembly, with the
  *   lattice's viscous part; InvDiagA exports the row's own, formed when it is
@@ -297,13 +306,17 @@ int mph_case_set_option(mph_case* c, const char* name, double value);
  *   "pair_recompute" 0 (default) / 1: pair-term inner operator only; 1
  *   evaluates g per slot from the staged FP32 positions (2 bytes a slot).
  *   "batch_solve" 0 (default) / 1: in mph_batch_step, the point-Jacobi
- *   mixed cases on the pair path solve together: each refinement phase's CR
+ *   mixed cases with a kernel each for the parts of an iteration
+ *   (inner_kernel 1: beyond 155,648 particles, or lists too long for the
+ *   resident kernel; the others solve one by one) solve together: each
+ *   refinement phase's CR
  *   iterations are one launch per kernel over all of them (a block runs its
  *   case's single-case kernel body with that case's block decomposition, so
  *   every case keeps the bits of its own solve); the stages before the solve
  *   then run for all cases before any solve starts.
- *   "pair_fuse" 0 (default) / 1: point-Jacobi mixed form on the pair path;
- *   1 writes the sliced pair terms in one kernel without the per-slot
+ *   "pair_fuse" 0 (default) / 1: point-Jacobi mixed form on the pair-term
+ *   operator (inner_kernel 0: a step with particles too close together for
+ *   the other operator, or MaxRadius above 16 RadiusP); 1 writes the sliced pair terms in one kernel without the per-slot
  *   pair-term list (16 bytes a neighbour slot less device memory; slower).
  *   "launch_iterations" 1 .. 4096 (default), "wait_polls" 1 .. 2097152
  *   (default): point-Jacobi mixed form of a case whose rows fit the chip at

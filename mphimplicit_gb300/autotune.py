@@ -10,9 +10,14 @@ Three launch shapes of the mixed form are runtime options of a case:
 * ``chunk``: CR iterations in one captured CUDA-graph chunk, i.e. how often
   the host reads the solver's flags (4, 8, 16, 32).
 
+Which of them act depends on the kernels a case's iteration runs on
+(``solve_stats()["inner_kernel"]``): none on the resident kernel (point-Jacobi
+cases that fit the chip at once), the chunk on the P-list kernels beyond, all
+three on the pair-term operator.
+
 ``tune`` times whole steps of fresh copies of a case for each candidate by
-coordinate descent (one option at a time, the others at their best so far)
-and returns the fastest settings with every timing.  ``tune_table`` does this
+coordinate descent (one option at a time, the others at their best so far; the
+options that act) and returns the fastest settings with every timing.  ``tune_table`` does this
 for one case of each size class (dimension and octave of the fluid count) of
 a workload and ``choose`` picks a case's settings from such a table, so that
 cases run measured settings deterministically: the block widths set the
@@ -35,14 +40,23 @@ def apply(case, settings: Dict[str, int]) -> None:
         case.set_option(k, v)
 
 
-def _ms_per_step(make_case: Callable, settings: Dict[str, int], steps: int, warmup: int) -> float:
+def _acting(case) -> Optional[tuple]:
+    """The options that change what the case's last solve ran (None: all)."""
+    s = case.solve_stats() if hasattr(case, "solve_stats") else {}
+    if s.get("inner_form") != 2:
+        return None
+    return {2: (), 1: ("chunk",)}.get(s.get("inner_kernel"))
+
+
+def _ms_per_step(make_case: Callable, settings: Dict[str, int], steps: int, warmup: int):
+    """Milliseconds per step with these settings, and the options that act."""
     c = make_case()
     try:
         apply(c, settings)
         c.step(warmup)
         t0 = time.perf_counter()
         c.step(steps)   # a step ends with the host reading its solve's results
-        return (time.perf_counter() - t0) * 1000.0 / steps
+        return (time.perf_counter() - t0) * 1000.0 / steps, _acting(c)
     finally:
         c.close()
 
@@ -57,14 +71,17 @@ def tune(make_case: Callable, steps: int = 3, warmup: int = 2, candidates=CANDID
     only for a candidate at least `margin` faster."""
     best = dict(DEFAULTS)
     timings: Dict[tuple, float] = {}
+    timings[tuple(sorted(best.items()))], acting = _ms_per_step(make_case, best, steps, warmup)
     for name, values in candidates:
+        if acting is not None and name not in acting:
+            continue
         res = {}
         for v in values:
             trial = dict(best)
             trial[name] = v
             key = tuple(sorted(trial.items()))
             if key not in timings:
-                timings[key] = _ms_per_step(make_case, trial, steps, warmup)
+                timings[key], _ = _ms_per_step(make_case, trial, steps, warmup)
             res[v] = timings[key]
         fastest = min(res, key=res.get)
         if res[fastest] < (1.0 - margin) * res[best[name]]:
