@@ -451,7 +451,7 @@ static void pq_precond(mph_case* c, cudaStream_t st, int n, unsigned rb, const f
 // what the inner operator leaves of the true one (k_penalty.cu).
 static double inner_target2(const mph_case* c)
 {
-    const double t = c->step_pen ? std::max(c->tol_inner, std::min(std::max(c->pen_tol, 2.0 * c->pen_near), 0.1)) : c->tol_inner;
+    const double t = c->step_pen ? std::max(c->tol_inner, pen_floor(c)) : c->tol_inner;
     return t * t;
 }
 

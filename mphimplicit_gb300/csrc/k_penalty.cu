@@ -39,6 +39,7 @@
 // give the same bits.
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <type_traits>
@@ -1476,12 +1477,17 @@ __global__ void __launch_bounds__(128) k_pen_resid(DevParams P, const int* __res
 }
 
 // Start of a refinement phase: r32 = r / scale, s = D^-1 r32, z = 0, the inner
-// reference norm (r32, r32), the phase's target (reduce it by tol_in, but no
-// further than half of what the outer test still asks for) and the done flag.
+// reference norm (r32, r32), the phase's target and the done flag.  The target
+// is a reduction by tol_in or, in the phase that may meet the outer test with
+// it (an iteration takes some 0.86, so a phase lands up to that much below its
+// target), the fraction aim of what that test still asks for, less or more than
+// tol_in, but no less than the inner operator leaves of the true residual
+// (floor): where a solve lands under its tolerance then does not depend on
+// where the phases before happened to end.
 __global__ void __launch_bounds__(kReduceThreads) k_pen_phase(int n, const double* __restrict__ r, const float* __restrict__ invD,
                                                               float* __restrict__ s, float* __restrict__ z, double inv_scale,
                                                               const double* __restrict__ scale_src, double tol_in2, double tol_out2,
-                                                              double* __restrict__ scal, int* __restrict__ flags,
+                                                              double aim2, double floor2, double* __restrict__ scal, int* __restrict__ flags,
                                                               double* __restrict__ partials, unsigned* __restrict__ counter,
                                                               unsigned* __restrict__ crossings)
 {
@@ -1495,9 +1501,8 @@ __global__ void __launch_bounds__(kReduceThreads) k_pen_phase(int n, const doubl
         acc += v * v;
     }
     if (reduce_finalize_last(acc, partials, counter, scal + kSIn0)) {
-
-        const double need = 0.25 * tol_out2 * scal[kSRR0] / scal[kSRR];
-        const double tol2 = need > tol_in2 ? need : tol_in2;
+        const double left = tol_out2 * scal[kSRR0] / scal[kSRR];
+        const double tol2 = 0.5 * tol_in2 < left ? fmax(aim2 * left, floor2) : tol_in2;
         scal[kSTol2] = tol2;
         const F2 stop = f2_of(tol2 * scal[kSIn0]);
         reinterpret_cast<float2*>(scal)[kSStop] = make_float2(stop.h, stop.l);
@@ -1746,19 +1751,29 @@ void launch_pen_refine(mph_case* c, double scale, const double* scale_src, const
 
 static unsigned* cr_count(const mph_case* c) { return (unsigned*)(c->d.cr_vals + 8 * kCrBlocks); }
 
-// The last phase aims at half of the outer tolerance, and at an eighth of one
-// below 5e-11: such a tolerance is asked for where forces and pressures are
-// read off the velocities' divergence, which shows the solve's error enlarged
-// (2-D frames at 1e-11: 4 to 11e-10 of the forces at a half, 1.4 to 3.5e-10 at
-// an eighth, for 8 to 11 more of some 130 iterations).
+// What the inner operator leaves of the true residual, at least: the viscous
+// pairs outside it (the lattice's, or a close pair's).
+double pen_floor(const mph_case* c) { return std::min(std::max(c->pen_tol, 2.0 * c->pen_near), 0.1); }
+
+// The last phase aims at a quarter of the outer tolerance, and from 1e-10 down
+// to 1e-11 at ever less, at a tenth beyond: such tolerances are asked for
+// where forces and pressures are read off the velocities' divergence, which
+// shows the solve's error enlarged (2-D frames at 1e-11: 4 to 11e-10 of the
+// forces at a half, 1.4 to 3.5e-10 at an eighth).  At a half, solves refined to
+// 1e-10 were up to 60% further from the 64-bit solution than with the pair-term
+// operator (412,000 particles in 2-D 5.0e-11 and 3.2e-11; at a quarter 2.6e-11);
+// a quarter takes some five of 150 iterations more (22,000 particles and three
+// steps 6.0 -> 6.2 ms).
 void launch_pen_phase(mph_case* c, double inv_scale, const double* scale_src, double tol_in2, double tol_out2)
 {
     DeviceState& d = c->d;
-    if (c->tol_outer < 5.0e-11) tol_out2 *= 1.0 / 16.0;
+    const double aim = std::max(0.1, 0.25 * std::min(1.0, std::pow(c->tol_outer * 1.0e10, 0.39794)));
+    const double floor = pen_floor(c);
     const int n = c->dp.Nf * c->dim;
     float* v = d.v32;
     { k_pen_phase<<<std::min<int>(grid_for(n, kReduceThreads), kReduceBlocks), kReduceThreads, 0, c->stream>>>(
-          n, d.r, v + 7 * vec32_stride(n), v + 2 * vec32_stride(n), v + vec32_stride(n), inv_scale, scale_src, tol_in2, tol_out2, d.scal, d.flags, d.partials,
+          n, d.r, v + 7 * vec32_stride(n), v + 2 * vec32_stride(n), v + vec32_stride(n), inv_scale, scale_src, tol_in2, tol_out2,
+          aim * aim, floor * floor, d.scal, d.flags, d.partials,
           (unsigned*)(d.flags + kFlagCounter), c->pen_resident ? cr_count(c) : nullptr); MPH_COUNT_LAUNCH(); }
 }
 

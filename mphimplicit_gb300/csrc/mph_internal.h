@@ -456,6 +456,7 @@ int launch_pen_assemble(mph_case* c);
 int pen_exact_diag(mph_case* c);
 void launch_pen_start_residual(mph_case* c);
 void launch_pen_refine(mph_case* c, double scale, const double* scale_src, const int* flags);
+double pen_floor(const mph_case* c);
 void launch_pen_phase(mph_case* c, double inv_scale, const double* scale_src, double tol_in2, double tol_out2);
 int launch_pen_resident(mph_case* c, int cap, double scale);
 void launch_pen_residual(mph_case* c, double scale);
