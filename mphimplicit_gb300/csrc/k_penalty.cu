@@ -110,6 +110,17 @@ __device__ __forceinline__ float fixed_sep(const DevParams& P, int d, int uj, in
     return __fmul_rn(__int2float_rn((int)((unsigned)uj - (unsigned)ui)), P.fix_c[d]);
 }
 
+// The same in units of RadiusV with the unit in two floats, for the viscous
+// pairs that the outer residual carries: their roundings are then at random,
+// and no constant's own (the unit's, 1 / RadiusV, mu_00: exact or applied in
+// FP64) goes through every pair.  A frame of 326,592 particles is 5.3e-11 from
+// the 64-bit one, 6.6e-11 with the constants rounded.
+__device__ __forceinline__ float fixed_sep_v(const DevParams& P, int d, int uj, int ui)
+{
+    const float v = __int2float_rn((int)((unsigned)uj - (unsigned)ui));
+    return __fmaf_rn(v, P.fix_v[d], __fmul_rn(v, P.fix_vl[d]));
+}
+
 // The P-lists of a block of rows as 2-byte ranks among the block's distinct
 // columns: uniq[block][0 .. U) the columns in ascending order, idx the rank of
 // every slot, four slots of a row in one 8-byte word, a row's words 32 words
@@ -1397,7 +1408,7 @@ __global__ void __launch_bounds__(256) k_pen_visc(DevParams P, int nbT, const in
             const int j = col[k];
             const int4 pj = ipos[j];
             const float4 h = rec[j];
-            const float q[3] = {fixed_sep(P, 0, pj.x, pi.x), fixed_sep(P, 1, pj.y, pi.y), D == 3 ? fixed_sep(P, 2, pj.z, pi.z) : 0.f};
+            const float q[3] = {fixed_sep_v(P, 0, pj.x, pi.x), fixed_sep_v(P, 1, pj.y, pi.y), D == 3 ? fixed_sep_v(P, 2, pj.z, pi.z) : 0.f};
             float dx[3] = {hi.x - h.x, hi.y - h.y, D == 3 ? hi.z - h.z : 0.f};
             if (FIRST) {
                 const float4 l = lo[j];
@@ -1408,10 +1419,10 @@ __global__ void __launch_bounds__(256) k_pen_visc(DevParams P, int nbT, const in
             float r2 = q[0] * q[0] + q[1] * q[1];
             if (D == 3) r2 += q[2] * q[2];
             const float inv = rsqrtf(fmaxf(r2, 1e-18f));
-            // visc mu_ij w' / |q|, w' = (1 - |q| / RadiusV) up to the constants in vm; q / |q| twice (the row itself: 0)
+            // mu_ij w' / |q|, w' = 1 - |q|, up to the constants in pen_v0; q / |q| twice (the row itself: 0)
             float dot = q[0] * dx[0] + q[1] * dx[1];
             if (D == 3) dot += q[2] * dx[2];
-            const float t = (pj.w ? vm1 : vm0) * fmaxf(inv - P.pen_vk, 0.f) * (dot * inv) * inv;
+            const float t = (pj.w ? vm1 : vm0) * fmaxf(inv - 1.f, 0.f) * (dot * inv) * inv;
 #pragma unroll
             for (int d = 0; d < D; ++d) y[d] += t * q[d];
         }
@@ -1423,7 +1434,8 @@ __global__ void __launch_bounds__(256) k_pen_visc(DevParams P, int nbT, const in
     if (i < P.Nf && lane < D) {
         const float yl = lane == 0 ? y[0] : (lane == 1 ? y[1] : y[2]);
         const size_t k = (size_t)i * D + lane;
-        vacc[k] = FIRST ? (double)yl : vacc[k] + (scale_src ? *scale_src : scale) * (double)yl;
+        const double v = P.pen_v0 * (double)yl;
+        vacc[k] = FIRST ? v : vacc[k] + (scale_src ? *scale_src : scale) * v;
     }
 }
 
@@ -1557,7 +1569,7 @@ bool pen_applies(const mph_case* c)
     if (!(c->step_pairs && mixed_jacobi(c) && P.maxR <= 16.0 * P.rP)) return false;
     for (int t = 0; t < 2; ++t)
         for (int u = 0; u < 2; ++u)
-            if (!(P.pen_vm[t][u] <= 1.0e25f)) return false;   // unit systems far outside FP32's range
+            if (!(P.pen_v0 * P.pen_vm[t][u] <= 1.0e25)) return false;   // unit systems far outside FP32's range
     return true;
 }
 

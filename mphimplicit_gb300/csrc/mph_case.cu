@@ -211,10 +211,11 @@ static int derive(mph_case* c, const mph_particles* parts)
         // the inner operator of the point-Jacobi form keeps 0.6 of a row's
         // viscous diagonal (fsum mu / dim) and leaves the rest, at most about
         // 0.7 of it, to the outer residual
-        P.pen_vk = (float)(P.rP / P.rV);
+        P.pen_v0 = P.visc * P.muij[0][0] * (-P.kfv * P.m2h_rv) / P.rV;
+        if (!(P.pen_v0 > 0.0)) P.pen_v0 = 1.0;
         for (int t = 0; t < 2; ++t) {
             P.pen_vd[t] = (float)(fsum * std::fabs(P.mu[t]) / c->dim);
-            for (int u = 0; u < 2; ++u) P.pen_vm[t][u] = (float)(P.visc * P.muij[t][u] * (-P.kfv * P.m2h_rv) / P.rP);
+            for (int u = 0; u < 2; ++u) P.pen_vm[t][u] = (float)(P.visc * P.muij[t][u] * (-P.kfv * P.m2h_rv) / P.rV / P.pen_v0);
         }
         for (int t = 0; t < kTypeCount; ++t) P.pen_diag32[t] = (float)(P.inert64[t] + 0.6 * fsum * std::fabs(P.mu[t]) / c->dim);
         c->pen_tol = 0.7 * fsum * mu_max / c->dim / (rho_min / P.dt);
@@ -266,6 +267,9 @@ static int derive(mph_case* c, const mph_particles* parts)
         const double turns = std::max(1.0, std::floor(P.dw[d] / P.maxR * std::ldexp(1.0, -2)));
         P.fix_scale[d] = std::ldexp(turns, 32) / P.dw[d];
         P.fix_c[d] = (float)(1.0 / (P.fix_scale[d] * P.rP));
+        const double v = 1.0 / (P.fix_scale[d] * P.rV);
+        P.fix_v[d] = (float)v;
+        P.fix_vl[d] = (float)(v - (double)P.fix_v[d]);
     }
     // f / inertia of a viscous pair (f as above)
     P.near_r = (float)P.maxR;

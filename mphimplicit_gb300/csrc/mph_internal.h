@@ -66,9 +66,9 @@ struct DevParams {
     float vm32[kTypeCount][kTypeCount];        // FP32 visc * muij, -kfv * m2h_rv, 1/h, rV^2 (pair terms)
     float wdA32, inv_rv32, rV2_32;
     double fix_scale[3];                       // fixed-point positions: an axis's units a length, and a unit in RadiusP
-    float fix_c[3];
-    float pen_vm[2][2], pen_vk, pen_vd[2];     // visc mu_ij w' and 1/RadiusV of the fluid pairs over 1/RadiusP; the lattice's
-                                               // viscous diagonal of a fluid row
+    float fix_c[3], fix_v[3], fix_vl[3];       // (in RadiusV: two floats)
+    double pen_v0;                             // visc mu_00 w' of the fluid pairs over 1/RadiusV
+    float pen_vm[2][2], pen_vd[2];             // mu_ij over mu_00; the lattice's viscous diagonal of a fluid row
     float near_f[2][kTypeCount], near_r, near_k;   // f / inertia of a pair = near_f (MaxRadius / r - near_k); MaxRadius
     float pen_diag32[kTypeCount];              // inner operator of the point-Jacobi form: its diagonal, lambda kfp 2/RadiusP,
     float pen_lam32[kTypeCount], pen_w32;      // and kfp 2/RadiusP
