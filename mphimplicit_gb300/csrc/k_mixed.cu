@@ -531,7 +531,8 @@ static int device_solve(mph_case* c, double* hs, int* hflags)
     const long long extra[] = {have, c->max_outer, (long long)(vprev != nullptr), (long long)(uintptr_t)d.vel,
                                (long long)(uintptr_t)d.force, (long long)(uintptr_t)d.type, (long long)(uintptr_t)d.vprev};
     sig = fnv1a(sig, extra, sizeof(extra));
-    sig = fnv1a(sig, &tol_out2, sizeof(tol_out2));
+    const double tols[] = {tol_out2, c->step_pen ? pen_floor(c) : 0.0};
+    sig = fnv1a(sig, tols, sizeof(tols));
     int slot = -1;
     for (int k = 0; k < 2; ++k)
         if (c->sx_exec[k] && c->sx_sig[k] == sig) slot = k;

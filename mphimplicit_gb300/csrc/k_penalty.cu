@@ -1611,10 +1611,10 @@ static int launch_pen_lists(mph_case* c)
     c->loc_blocks[1] = (int)grid_for(P.Nf, c->pen_rows);
     c->loc_cols = 0;
     c->loc_ct_blocks = 0;
-    auto near_of = [](int bits) {
+    auto near_of = [](int bits) {   // rounded up to a quarter of an octave: small changes keep the captured solve
         float f;
         std::memcpy(&f, &bits, sizeof(f));
-        return f;
+        return f > 0.f ? std::exp2(std::ceil(4.0 * std::log2((double)f)) / 4.0) : 0.0;
     };
     int h[5] = {};
     if (!c->inner_local) {

@@ -66,3 +66,27 @@ def test_viscous_pair(engine_lib, dim, distance, mu):
     assert s["status"] == 0 and f["status"] == 0
     assert np.linalg.norm(v - want) <= 1e-8 * np.linalg.norm(want)
     assert s["iter"] <= 1.5 * apart["iter"]
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_footprint_with_a_close_pair(engine_lib, dim):
+    """A step that meets a pair too close for the penalty operator assembles the
+    pair terms beside what that operator had: the admission bound holds both."""
+    torch = pytest.importorskip("torch")
+    from mphimplicit_gb300 import serving
+    torch.cuda.init()
+    l0, dt = (0.01, 1e-4) if dim == 2 else (0.005, 5e-5)
+    parts = casegen.dam_case(dim, (100, 100) if dim == 2 else (30, 30, 30), (120, 110) if dim == 2 else (33, 33, 33), l0, seed=3)
+    params = casegen.baseline_params(dim, l0, dt)
+    parts.pos[1] = parts.pos[0] + 1e-3 * l0 * np.array([0.6, 0.8, 0.0])
+    fp = serving.footprint(params, parts, dim, PRECISION_MIXED)
+    free0, _ = torch.cuda.mem_get_info()
+    g = engine.Case(params, parts, dim, precision=PRECISION_MIXED)
+    g.set_solver(1e-10, 1e-3, 50)
+    g.step(2)
+    free1, _ = torch.cuda.mem_get_info()
+    s = g.solve_stats()
+    g.close()
+    print(dim, free0 - free1, fp)
+    assert s["inner_kernel"] == 0
+    assert free0 - free1 <= fp

@@ -50,7 +50,17 @@ def _beyond():
     return _start(casegen.baseline_params(2, 0.01, 1.0e-4), casegen.dam_case(2, (417, 373), (600, 420), 0.01, seed=10), 2)
 
 
-ITERATED = {"long2d": lambda: _long2((61, 53), 1), "long3d": lambda: _long3((12, 13, 12), 11), "beyond2d": _beyond}
+def _long2_close():
+    """With two particles whose viscous pair sets the phases' target, a new one every step."""
+    dim, params, parts = _long2((61, 53), 1)
+    params.shear_viscosity = (20.0, 20.0, 20.0, 20.0)
+    a, b = 30 * 53 + 20, 30 * 53 + 21
+    parts.pos[b] = parts.pos[a] + 0.06 * parts.spacing * np.array([0.6, 0.8, 0.0])
+    parts.vel[b] = parts.vel[a] + np.array([3.0, 4.0, 0.0])
+    return dim, params, parts
+
+
+ITERATED = {"long2d": lambda: _long2((61, 53), 1), "close2d": _long2_close, "long3d": lambda: _long3((12, 13, 12), 11), "beyond2d": _beyond}
 
 
 def _run(case, options, steps=2):
