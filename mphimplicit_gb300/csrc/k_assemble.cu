@@ -497,13 +497,19 @@ int launch_assemble(mph_case* c)
     long long h_cn = 0;
     MPH_CUDA(cudaMemcpyAsync(&h_cn, c->d.nptrP + Nf, sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
     MPH_CUDA(cudaStreamSynchronize(c->stream));
-    const int crows = c->step_f64 ? P.N : Nf;   // the operator in parts reads C^T from every particle's own row
-    if (c->step_f64) h_cn = c->nnbP;
     {
         void* p = c->d.cval;
-        MPH_TRY(ensure(&p, &c->d.cap_cval, h_cn * D, sizeof(double)));
+        // the operator in parts reads C^T from every particle's own row; without
+        // the memory for it the stored blocks are applied
+        if (c->step_f64 && ensure(&p, &c->d.cap_cval, c->nnbP * D, sizeof(double)) != MPH_OK) {
+            cudaGetLastError();
+            c->step_f64 = false;
+        }
+        const int st = c->step_f64 ? MPH_OK : ensure(&p, &c->d.cap_cval, h_cn * D, sizeof(double));
         c->d.cval = (double*)p;
+        MPH_TRY(st);
     }
+    const int crows = c->step_f64 ? P.N : Nf;
     const unsigned gf = grid_for(Nf, 128);
     Level0Map M{};
     const mph::LevelGeom& g0 = c->lv[0];

@@ -390,11 +390,17 @@ int f64_parts_build(mph_case* c, bool* ok)
         d.cap_f64g = (long long)want;
     }
     c->f64_slots = d.cap_f64g / 3;
-    if (!d.f64rec) MPH_CUDA(cudaMalloc((void**)&d.f64rec, (size_t)P.Nf * (sizeof(float4) + sizeof(float2))));
-    if (!d.f64type) MPH_CUDA(cudaMalloc((void**)&d.f64type, (size_t)P.N * sizeof(int)));
-    if (!d.vacc) MPH_CUDA(cudaMalloc((void**)&d.vacc, (size_t)P.Nf * 3 * sizeof(double)));
-    if (!d.tct) MPH_CUDA(cudaMalloc((void**)&d.tct, (size_t)(P.N + 1) * sizeof(double)));
-    if (!d.sdiag64) MPH_CUDA(cudaMalloc((void**)&d.sdiag64, (size_t)P.Nf * 8 * sizeof(double)));
+    auto have = [](auto** p, size_t bytes) {
+        if (!*p && cudaMalloc((void**)p, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            *p = nullptr;
+        }
+        return *p != nullptr;
+    };
+    if (!have(&d.f64rec, (size_t)P.Nf * (sizeof(float4) + sizeof(float2))) || !have(&d.f64type, (size_t)P.N * sizeof(int)) ||
+        !have(&d.vacc, (size_t)P.Nf * 3 * sizeof(double)) || !have(&d.tct, (size_t)(P.N + 1) * sizeof(double)) ||
+        !have(&d.sdiag64, (size_t)P.Nf * 8 * sizeof(double)))
+        return MPH_OK;
     { k_f64_pairs<<<grid_for(P.N, 128), 128, 0, c->stream>>>(P, f64_inert(c), d.type, d.pos, d.nc, d.nfc, d.nptr, d.nind, d.sptr, d.acol,
                                                               d.f64g, c->f64_slots, d.sdiag64, d.f64type); MPH_COUNT_LAUNCH(); }
     MPH_CUDA(cudaGetLastError());
