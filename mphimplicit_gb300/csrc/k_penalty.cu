@@ -41,8 +41,6 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
-#include <mutex>
-#include <type_traits>
 
 #include "mph_device.cuh"
 #include "mph_pairs.cuh"
@@ -77,7 +75,7 @@ constexpr int kCrSmem = 100 * 1024;   // dynamic: two blocks an SM with their 7 
 // 3.5-spacing cell order have about 2.8 (256 rows) to 3.9 (64) times their
 // rows of them, against some 20 slots a row; one with more (a solve of 211
 // blocks of 599 on average: 9.12 ms staged, 9.34 gathered) gains little.
-static int pen_ucap(int rows) { return 4 * rows + 128; }
+static constexpr int pen_ucap(int rows) { return 4 * rows + 128; }
 
 // Fixed-point positions with the particle's type, of the penalty operator and
 // of the viscous pairs.  An axis's unit is its domain width / (m 2^32), m the
@@ -1624,12 +1622,10 @@ static int launch_pen_lists(mph_case* c)
         return MPH_OK;
     }
     const size_t smem = 2 * kPlWords * sizeof(unsigned);
-    if (!c->pen_attr) {   // once a case; fixed maxima: host threads of a batch would race on per-launch values
-        const int t = (pen_ucap(kMaxPenRows) + 256) * 24, y = (pen_ucap(kMaxPenRows) + 256) * 16;
-        const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        MPH_CUDA(cudaFuncSetAttribute(k_plist_ranks, a, (int)smem));
-        MPH_CUDA(c->dim == 2 ? cudaFuncSetAttribute(k_pen_t<2>, a, t) : cudaFuncSetAttribute(k_pen_t<3>, a, t));
-        MPH_CUDA(c->dim == 2 ? cudaFuncSetAttribute(k_pen_y<2>, a, y) : cudaFuncSetAttribute(k_pen_y<3>, a, y));
+    // (what the iteration's kernels stage is within a block's default limit)
+    static_assert(pen_ucap(kMaxPenRows) % 128 == 0 && pen_ucap(kMaxPenRows) * 24 + 4096 <= 48 * 1024, "k_pen_t's shared memory");
+    if (!c->pen_attr) {   // once a case: the attribute belongs to its device
+        MPH_CUDA(cudaFuncSetAttribute(k_plist_ranks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         c->pen_attr = true;
     }
     MPH_CUDA(cudaMemsetAsync(d.pucount + nb, 0, 5 * sizeof(int), c->stream));
@@ -1928,14 +1924,6 @@ void batch_pen_fill(const mph_case* c, int cap, void* table, int k, int* nb)
 // staged count of the batch).
 void launch_batch_pen(const void* table, const int* b0, int nc, int dim, int rows, int W, int umax, const int* nb, cudaStream_t st)
 {
-    static std::once_flag once;
-    std::call_once(once, [] {
-        const int t = (pen_ucap(kMaxPenRows) + 256) * 24, y = (pen_ucap(kMaxPenRows) + 256) * 16;
-        cudaFuncSetAttribute(k_batch_pen_t<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, t);
-        cudaFuncSetAttribute(k_batch_pen_t<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, t);
-        cudaFuncSetAttribute(k_batch_pen_y<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, y);
-        cudaFuncSetAttribute(k_batch_pen_y<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, y);
-    });
     const BatchPen* cs = (const BatchPen*)table;
     const dim3 blk(rows, W);
     if (nb[0] > 0) {
