@@ -12,7 +12,8 @@
 // eigenvalues lie between 0 and about 1.3 of that diagonal, so a refinement
 // phase leaves at most about 0.7 of diagonal / inertia of the residual (4e-4
 // in the benchmark's tank, below the phase's own target of 1e-3, which is
-// raised to that bound where the fluid is more viscous).
+// raised to that bound where the fluid is more viscous, and to what a close
+// pair leaves, k_pen_system).
 //
 // C is not stored: C_ik = w(|q|) q / |q| with q = x_k - x_i and
 // C_ii = sum_k C_ik, so with P-lists that are symmetric (k in P(i) <=> i in
@@ -24,12 +25,11 @@
 // and both sums run over one list with a 2-byte index a slot (40 MB on
 // 1.3 million particles, which stays in L2 from one iteration to the next)
 // instead of two lists of 16-byte records (640 MB, read from HBM every time).
-// Positions are fixed point in units of RadiusP / 2^22: their differences are
-// exact (C_ik = -C_ki to the bit), good to 2^-22 of RadiusP, and become floats
-// by an addition to the bits of 1.5 2^23 (integer-to-float conversions run on
-// the quarter-rate pipe of the reciprocal square root).
+// Positions are fixed point, about MaxRadius / 2^30 a unit and modulo 2^32, so
+// that their differences are exact minimum images (C_ik = -C_ki to the bit)
+// and good to FP32's own rounding down to MaxRadius / 256 (k_fixed_positions).
 //
-// On 1,297,696 particles an application takes 95 us (k_pen_t 51, k_pen_y 44;
+// On 1,297,696 particles an application takes 93 us (k_pen_t 49, k_pen_y 44;
 // the viscous pairs and stored records: 398) and the vectors 20 us in one
 // kernel (43 in two), with 142 CR iterations where there were 140.
 //
@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_pen_vec(PenArgs A, int n, in
 // cases whose rows fit the chip at once (up to 155,648 particles).  Such a
 // case's iteration is not bound by anything a kernel does but by three
 // launches, their load chains and their last-block reductions (19 us on 22,000
-// particles, 33 on 155,000; resident 8.2 and 19.3).  Here a block keeps its
+// particles, 33 on 155,000; resident 8.1 and 18.4).  Here a block keeps its
 // rows' neighbours' positions and ranks in shared memory and its vectors in
 // registers for the whole phase, and an iteration crosses the grid's barrier
 // twice:
@@ -1375,8 +1375,8 @@ __device__ __forceinline__ void pen_ct64(const DevParams& P, int tid, const int*
 // for x_0) and some 35 instructions; bound by the L1's gather rate.  Against
 // the stored FP32 g and columns (16 bytes a slot streamed, x in six 4-byte
 // gathers: 1.33 ms on 1.3 million particles with the P-part) it needs no pair
-// terms, which took three passes to build: with C^T x in the same launch 0.93
-// ms for x_0, 0.82 for z.
+// terms, which took three passes to build: with C^T x in the same launch 0.92
+// ms for x_0, 0.74 for z.
 // The launch's first nbT blocks form lambda t of C^T x meanwhile (pen_ct64).
 template <int D, int L, bool FIRST, int LT>
 __global__ void __launch_bounds__(256) k_pen_visc(DevParams P, int nbT, const int4* __restrict__ ipos, const int* __restrict__ nfc,

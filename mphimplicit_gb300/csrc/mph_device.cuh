@@ -1,10 +1,11 @@
 // mph_device.cuh - device helpers shared by the kernels.
 //
-// Exact arithmetic: the cell keys, neighbour decisions, particle motion and
-// the particle-number densities are computed with explicitly rounded
-// operations (__dadd_rn, __dmul_rn, ...), which the compiler never contracts
-// into FMAs.  They reproduce the reference's FP64 expressions operation by
-// operation, so sort permutations and neighbour lists match it bit for bit.
+// Exact arithmetic: the cell keys, neighbour decisions and particle motion are
+// computed with explicitly rounded operations (__dadd_rn, __dmul_rn, ...),
+// which the compiler never contracts into FMAs.  They reproduce the reference's
+// FP64 expressions operation by operation, so sort permutations and neighbour
+// lists match it bit for bit.  (The densities, forces and matrices are FP64
+// sums with FMAs and constants taken out, to rounding.)
 #pragma once
 
 #include <cuda_runtime.h>
