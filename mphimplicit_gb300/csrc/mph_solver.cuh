@@ -89,6 +89,8 @@ __device__ __forceinline__ int cr_stop(const double* __restrict__ scal, const in
 // the last block of a launch of 1688 took 13 round trips to L2 in line)
 __device__ __forceinline__ double partials_sum(const double* partials, int nb)
 {
+    if (nb <= (int)blockDim.x)   // (the sum of eight below is four FP64 additions in line, some hundred clocks each)
+        return (int)threadIdx.x < nb ? __ldcg(partials + threadIdx.x) : 0.0;
     double s = 0.0;
     for (int b = threadIdx.x; b < nb; b += 8 * blockDim.x) {
         double v[8];
