@@ -102,8 +102,8 @@ typedef struct mph_solve_stats {
     int outer_iterations;    /* mixed form: FP64 refinement steps (0 for the FP64 form) */
     int inner_form;          /* operator of the CR iterations: 0 FP64 blocks, 1 FP32 blocks,
                                 2 FP32 without blocks (mixed form, factored, option inner_blocks 0) */
-    int inner_local_blocks;  /* inner_form 2: blocks of fluid rows (64, 128 or 256 by the particle count; 512 with
-                                mg_depth >= 0) whose neighbours' values are staged in shared memory, and the
+    int inner_local_blocks;  /* inner_form 2: blocks of fluid rows (64 to 512 by the particle count; option pair_block
+                                where inner_kernel is 0) whose neighbours' values are staged in shared memory, and the
                                 rest, which gather by column */
     int inner_gather_blocks;
     long long inner_local_cols;  /* distinct neighbour columns summed over the staged row blocks */
